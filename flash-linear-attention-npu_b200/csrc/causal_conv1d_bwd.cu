@@ -406,9 +406,9 @@ __global__ void __launch_bounds__(kBwdThreads, 2) conv_bwd_kernel(ConvBwdParams 
 
 
 struct ConvBwdReduceParams {
-  const float* part; float* dw; float* db;
+  const float* part; void* dw; void* db;
   int64_t dw_sd, dw_sw;
-  int tiles, W, D;
+  int tiles, W, D, dw_f32, db_f32;
 };
 
 __global__ void conv_bwd_reduce_kernel(ConvBwdReduceParams p) {
@@ -417,8 +417,11 @@ __global__ void conv_bwd_reduce_kernel(ConvBwdReduceParams p) {
   if (d >= p.D) return;
   float acc = 0.f;
   for (int t = 0; t < p.tiles; ++t) acc += p.part[(int64_t(t) * (p.W + 1) + j) * p.D + d];
-  if (j < p.W) p.dw[d * p.dw_sd + j * p.dw_sw] = acc;
-  else if (p.db) p.db[d] = acc;
+  void* out = j < p.W ? p.dw : p.db;
+  const int64_t off = j < p.W ? d * p.dw_sd + j * p.dw_sw : d;
+  if (!out) return;
+  if (j < p.W ? p.dw_f32 : p.db_f32) static_cast<float*>(out)[off] = acc;
+  else static_cast<bf16*>(out)[off] = __float2bfloat16_rn(acc);
 }
 
 inline bool vec_ok3(const fla_tensor_t& t) {
@@ -448,7 +451,7 @@ extern "C" FLA_API int fla_b200_causal_conv1d_bwd(const fla_causal_conv1d_bwd_ar
   const fla_tensor_t &x = a->x, &dy = a->dy, &dx = a->dx, &w = a->weight, &dw = a->dw;
   if (!x.data || !dy.data || !dx.data || !w.data || !dw.data) return FLA_ERR_NULL;
   if (x.ndim != 3 || dy.ndim != 3 || dx.ndim != 3 || w.ndim != 2 || dw.ndim != 2) return FLA_ERR_SHAPE;
-  if (x.dtype != FLA_BF16 || dy.dtype != FLA_BF16 || dx.dtype != FLA_BF16 || w.dtype != FLA_BF16 || dw.dtype != FLA_F32)
+  if (x.dtype != FLA_BF16 || dy.dtype != FLA_BF16 || dx.dtype != FLA_BF16 || w.dtype != FLA_BF16 || (dw.dtype != FLA_F32 && dw.dtype != FLA_BF16))
     return FLA_ERR_DTYPE;
   const int64_t B = x.shape[0], T = x.shape[1], D = x.shape[2], W = w.shape[1];
   if (w.shape[0] != D || dw.shape[0] != D || dw.shape[1] != W || W < 2 || W > 4 || D % 8 || B <= 0 || T <= 0) return FLA_ERR_SHAPE;
@@ -476,10 +479,10 @@ extern "C" FLA_API int fla_b200_causal_conv1d_bwd(const fla_causal_conv1d_bwd_ar
     if (a->bias.ndim != 1 || a->bias.shape[0] != D || a->bias.dtype != FLA_BF16 || a->bias.stride[0] != 1 || !aligned16(a->bias.data)) return FLA_ERR_SHAPE;
     p.bias = static_cast<const bf16*>(a->bias.data);
   }
-  float* db = nullptr;
+  void* db = nullptr;
   if (a->db.data) {
-    if (a->db.ndim != 1 || a->db.shape[0] != D || a->db.dtype != FLA_F32 || a->db.stride[0] != 1) return FLA_ERR_SHAPE;
-    db = static_cast<float*>(a->db.data);
+    if (a->db.ndim != 1 || a->db.shape[0] != D || (a->db.dtype != FLA_F32 && a->db.dtype != FLA_BF16) || a->db.stride[0] != 1) return FLA_ERR_SHAPE;
+    db = a->db.data;
   }
   for (int which = 0; which < 3; ++which) {
     const fla_tensor_t& s = which == 0 ? a->initial_state : which == 1 ? a->dht : a->dh0;
@@ -510,7 +513,7 @@ extern "C" FLA_API int fla_b200_causal_conv1d_bwd(const fla_causal_conv1d_bwd_ar
 #undef FLA_LAUNCH_BWD
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
-  ConvBwdReduceParams r{p.part, static_cast<float*>(dw.data), db, dw.stride[0], dw.stride[1], int(B) * tiles, int(W), int(D)};
+  ConvBwdReduceParams r{p.part, dw.data, db, dw.stride[0], dw.stride[1], int(B) * tiles, int(W), int(D), dw.dtype == FLA_F32, a->db.dtype == FLA_F32};
   conv_bwd_reduce_kernel<<<dim3(unsigned((D + 255) / 256), unsigned(W + 1)), 256, 0, st>>>(r);
   return cuda_status(cudaGetLastError());
 }

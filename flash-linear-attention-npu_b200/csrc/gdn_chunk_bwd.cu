@@ -45,7 +45,8 @@ struct GdnBwdParams {
   int64_t q_st, q_sh, k_st, k_sh, v_st, v_sh, do_st, do_sh, beta_st;
   int64_t dq_st, dq_sh, dk_st, dk_sh, dv_st, dv_sh;
   int64_t total_tokens;
-  int N, T, HK, HV, beta_is_f32, grads_f32;
+  int N, T, HK, HV, beta_is_f32;
+  int dq_f32, dk_f32, dv_f32, dg_f32, dbeta_f32;   // gradients leave in the dtypes of their inputs: f32, else bf16
   int V, nvb;          // value head dim (128 or 256) and its number of 64-column blocks
   int n0;              // first sequence of this launch (the backward may be launched as two halves of the batch)
   float scale;
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, con
     const int64_t gidx = (tok0 + i) * p.HV + hvf;
     if (live) {
       const float db = bz - egi * g_ + ma;
-      if (p.grads_f32) static_cast<float*>(p.dbeta)[gidx] = db;
+      if (p.dbeta_f32) static_cast<float*>(p.dbeta)[gidx] = db;
       else static_cast<bf16*>(p.dbeta)[gidx] = __float2bfloat16_rn(db);
     }
 #pragma unroll
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, con
     for (int w = 0; w < 8; ++w) tot += sds_s2[fb][w];
     const float dgv = suf + __expf(gl) * tot + fin_s[1][0] + fin_s[1][1];
     if (live) {
-      if (p.grads_f32) static_cast<float*>(p.dg)[gidx] = dgv;
+      if (p.dg_f32) static_cast<float*>(p.dg)[gidx] = dgv;
       else static_cast<bf16*>(p.dg)[gidx] = __float2bfloat16_rn(dgv);
     }
     asm volatile("bar.sync 2, 64;" ::: "memory");   // fin_s is free again
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, con
     else if (tok < rows) {   // the last head: the rows are complete
       void* base = kside ? p.dk : p.dq;
       const int64_t off = kside ? (tok0 + tok) * p.dk_st + hk * p.dk_sh + half * 64 : (tok0 + tok) * p.dq_st + hk * p.dq_sh + half * 64;
-      if (p.grads_f32) {
+      if (kside ? p.dk_f32 : p.dq_f32) {
         float* dst = static_cast<float*>(base) + off;
 #pragma unroll
         for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(part[i], part[i + 1], part[i + 2], part[i + 3]);
@@ -515,8 +516,6 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   if ((st = check_tok3(a->beta, B, T, HV, false))) return st;
   if ((st = check_tok3(a->dg, B, T, HV, true))) return st;
   if ((st = check_tok3(a->dbeta, B, T, HV, true))) return st;
-  const int gdt = a->dq.dtype;
-  if (a->dk.dtype != gdt || a->dv.dtype != gdt || a->dg.dtype != gdt || a->dbeta.dtype != gdt) return FLA_ERR_DTYPE;
   const fla_tensor_t &gam = a->gam, &X = a->x_inv;
   if (!gam.data || !X.data || !a->s_img.data || !a->vn_img.data || !a->p_img.data) return FLA_ERR_NULL;
   if (gam.dtype != FLA_F32 || gam.ndim != 3 || gam.shape[0] != B || gam.shape[1] != T || gam.shape[2] != HV ||
@@ -564,7 +563,9 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   p.dv_st = a->dv.stride[1]; p.dv_sh = a->dv.stride[2];
   p.total_tokens = B * T;
   p.N = N; p.T = int(T); p.HK = int(HK); p.HV = int(HV); p.V = int(V); p.nvb = int(nvb);
-  p.beta_is_f32 = a->beta.dtype == FLA_F32; p.grads_f32 = gdt == FLA_F32;
+  p.beta_is_f32 = a->beta.dtype == FLA_F32;
+  p.dq_f32 = a->dq.dtype == FLA_F32; p.dk_f32 = a->dk.dtype == FLA_F32; p.dv_f32 = a->dv.dtype == FLA_F32;
+  p.dg_f32 = a->dg.dtype == FLA_F32; p.dbeta_f32 = a->dbeta.dtype == FLA_F32;
   p.scale = a->scale;
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);

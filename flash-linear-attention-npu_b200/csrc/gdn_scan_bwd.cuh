@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
   auto store_dv = [&](int c) {
     const int rows = min(kC, sq.len - c * kC);
     const int64_t off = (int64_t(sq.bos) + c * kC) * p.dv_st + hv * p.dv_sh + vb * 128;
-    void* g = p.grads_f32 ? static_cast<void*>(static_cast<float*>(p.dv) + off) : static_cast<void*>(static_cast<bf16*>(p.dv) + off);
-    store_rows_transposed(smem + bO, ov, g, p.dv_st, p.grads_f32 != 0, rows, half, vrow, tid);
+    void* g = p.dv_f32 ? static_cast<void*>(static_cast<float*>(p.dv) + off) : static_cast<void*>(static_cast<bf16*>(p.dv) + off);
+    store_rows_transposed(smem + bO, ov, g, p.dv_st, p.dv_f32 != 0, rows, half, vrow, tid);
   };
 
   for (int s = 0; s < nt; ++s) {

@@ -43,7 +43,8 @@ struct KdaBwdParams {
   int64_t v_st, v_sh, do_st, do_sh, beta_st;
   int64_t dq_st, dq_sh, dk_st, dk_sh, dv_st, dv_sh, dg_st, dg_sh;
   int64_t total_tokens;
-  int N, T, HK, HV, beta_is_f32, grads_f32;
+  int N, T, HK, HV, beta_is_f32;
+  int dq_f32, dk_f32, dv_f32, dg_f32, dbeta_f32;   // gradients leave in the dtypes of their inputs: f32, else bf16
   int n0;              // first sequence of this launch (the backward may be launched as two halves of the batch)
   int V, nvb;          // value head dim (128 or 256) and its number of 64-column blocks
   float scale;
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_dhu_kernel(KdaBwdParams p) {
       if (tok < rows) {
         p.bz[(int64_t(vb * 2 + half) * p.total_tokens + tok0 + tok) * p.HV + hv] = bzsum;
         const int64_t off = (tok0 + tok) * p.dv_st + hv * p.dv_sh + vb * kBV + c0;
-        if (p.grads_f32) {
+        if (p.dv_f32) {
           float* dst = static_cast<float*>(p.dv) + off;
 #pragma unroll
           for (int i = 0; i < 32; i += 4)
@@ -625,7 +626,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
       float bz = 0.f;
       for (int s = 0; s < NVB; ++s) bz += p.bz[(2 * s) * bzs + gidx] + p.bz[(2 * s + 1) * bzs + gidx];
       const float db = bz - (red[0][0][i] + red[0][1][i]) + (red[1][0][i] + red[1][1][i]);
-      if (p.grads_f32) static_cast<float*>(p.dbeta)[gidx] = db;
+      if (p.dbeta_f32) static_cast<float*>(p.dbeta)[gidx] = db;
       else static_cast<bf16*>(p.dbeta)[gidx] = __float2bfloat16_rn(db);
     }
     ok = mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT);
@@ -732,7 +733,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
         for (int j = 0; j < 8; ++j) {
           const int t = r0 + blk * 8 + j;
           if (t < rows) {
-            if (p.grads_f32) static_cast<float*>(p.dg)[base + t * p.dg_st] = vals[j];
+            if (p.dg_f32) static_cast<float*>(p.dg)[base + t * p.dg_st] = vals[j];
             else static_cast<bf16*>(p.dg)[base + t * p.dg_st] = __float2bfloat16_rn(vals[j]);
           }
         }
@@ -744,7 +745,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
   if (ok && tok < rows) {
     void* base = kside ? p.dk : p.dq;
     const int64_t off = kside ? (tok0 + tok) * p.dk_st + hk * p.dk_sh + half * 64 : (tok0 + tok) * p.dq_st + hk * p.dq_sh + half * 64;
-    if (p.grads_f32) {
+    if (kside ? p.dk_f32 : p.dq_f32) {
       float* dst = static_cast<float*>(base) + off;
 #pragma unroll
       for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(acc_out[i], acc_out[i + 1], acc_out[i + 2], acc_out[i + 3]);
@@ -845,8 +846,6 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   if ((st = kda_bwd_check_tok(a->dg, B, T, HV, kK, true))) return st;
   if ((st = kda_bwd_check_tok3(a->beta, B, T, HV, false))) return st;
   if ((st = kda_bwd_check_tok3(a->dbeta, B, T, HV, true))) return st;
-  const int gdt = a->dq.dtype;
-  if (a->dk.dtype != gdt || a->dv.dtype != gdt || a->dg.dtype != gdt || a->dbeta.dtype != gdt) return FLA_ERR_DTYPE;
   for (const fla_tensor_t* s : {&a->initial_state, &a->dht, &a->dh0}) {
     if (!s->data) continue;
     if (s->dtype != FLA_F32) return FLA_ERR_DTYPE;
@@ -901,7 +900,9 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   p.dv_st = a->dv.stride[1]; p.dv_sh = a->dv.stride[2]; p.dg_st = a->dg.stride[1]; p.dg_sh = a->dg.stride[2];
   p.total_tokens = B * T;
   p.N = N; p.T = int(T); p.HK = int(HK); p.HV = int(HV); p.V = int(V); p.nvb = int(nvb);
-  p.beta_is_f32 = f.beta_is_f32; p.grads_f32 = gdt == FLA_F32;
+  p.beta_is_f32 = f.beta_is_f32;
+  p.dq_f32 = a->dq.dtype == FLA_F32; p.dk_f32 = a->dk.dtype == FLA_F32; p.dv_f32 = a->dv.dtype == FLA_F32;
+  p.dg_f32 = a->dg.dtype == FLA_F32; p.dbeta_f32 = a->dbeta.dtype == FLA_F32;
   p.scale = a->scale;
   p.status = f.status;
 

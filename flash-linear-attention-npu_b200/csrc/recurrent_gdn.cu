@@ -29,7 +29,7 @@ struct RecurrentParams {
   const void* state_in;    // [blocks, HV, K, V] (or [.., V, K] when v-first)
   void* state_out;         // may alias state_in
   void* out;               // [T, HV, V]
-  const int32_t* cu_seqlens;           // [N+1] or null (then every sequence has tokens_per_seq tokens)
+  const int32_t* cu_seqlens;           // [N+1] or null (then every sequence has tokens_per_seq tokens); offsets, or lengths behind a prefix
   const int32_t* state_indices;        // [T] or null (then sequence n uses block n, written once at the end)
   const int32_t* num_accepted_tokens;  // [N] or null
   int64_t q_stride_t, q_stride_h, k_stride_t, k_stride_h, v_stride_t, v_stride_h;
@@ -39,6 +39,7 @@ struct RecurrentParams {
   int64_t gk_stride_t, gk_stride_h;
   int g_is_f32, beta_is_f32, out_is_f32, l2norm, gk_is_f32, gate_mode, beta_mode;
   int act_f16, out_is_f16;   // q, k, v are fp16 (read exactly: the arithmetic is fp32) / out is fp16
+  int cu_is_lengths;
   float scale, lower_bound;
 };
 
@@ -122,7 +123,12 @@ __global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(Recurrent
   const int rg = tid / TPR, c0 = (tid % TPR) * 4;
 
   int t0, t1;
-  if (p.cu_seqlens) {
+  if (p.cu_seqlens && p.cu_is_lengths) {   // offsets from the lengths: every warp adds up the entries before its sequence
+    int sum = 0;
+    for (int i = tid % 32; i <= seq; i += 32) sum += p.cu_seqlens[i];
+    t0 = __reduce_add_sync(0xffffffffu, sum);
+    t1 = t0 + p.cu_seqlens[seq + 1];
+  } else if (p.cu_seqlens) {
     t0 = p.cu_seqlens[seq];
     t1 = p.cu_seqlens[seq + 1];
   } else {
@@ -383,6 +389,7 @@ extern "C" FLA_API int fla_b200_recurrent_gdn(const fla_recurrent_gdn_args* a, v
   p.HK = int(HK); p.HV = int(HV); p.tokens_per_seq = a->tokens_per_seq;
   p.nblocks_in = int(si.shape[0]); p.nblocks_out = int(so.shape[0]);
   p.g_is_f32 = a->g.dtype == FLA_F32; p.beta_is_f32 = a->beta.dtype == FLA_F32; p.out_is_f32 = o.dtype == FLA_F32;
+  p.cu_is_lengths = a->cu_is_lengths;
   p.l2norm = a->use_qk_l2norm; p.scale = a->scale;
   p.gk = a->gk.data; p.a_log = static_cast<const float*>(a->a_log.data); p.dt_bias = static_cast<const float*>(a->dt_bias.data);
   p.gk_stride_t = a->gk.data ? a->gk.stride[0] : 0; p.gk_stride_h = a->gk.data ? a->gk.stride[1] : 0;

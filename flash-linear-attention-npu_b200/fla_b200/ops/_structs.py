@@ -10,7 +10,7 @@ class RecurrentGdnArgs(ctypes.Structure):
                                            "dt_bias")] + [
         ("scale", ctypes.c_float), ("lower_bound", ctypes.c_float), ("tokens_per_seq", ctypes.c_int32),
         ("state_v_first", ctypes.c_int32), ("use_qk_l2norm", ctypes.c_int32), ("gate_mode", ctypes.c_int32),
-        ("beta_mode", ctypes.c_int32)]
+        ("beta_mode", ctypes.c_int32), ("cu_is_lengths", ctypes.c_int32)]
 
 
 class CausalConv1dFwdArgs(ctypes.Structure):

@@ -135,6 +135,7 @@ typedef struct fla_recurrent_gdn_args {
   int32_t use_qk_l2norm; /* normalise q and k rows as x * rsqrt(sum x^2 + 1e-6) first */
   int32_t gate_mode;
   int32_t beta_mode;
+  int32_t cu_is_lengths; /* cu_seqlens holds [skipped prefix length, length of sequence 0, 1, ...] instead of offsets */
 } fla_recurrent_gdn_args;
 FLA_API int fla_b200_recurrent_gdn_workspace_size(const fla_recurrent_gdn_args* args, uint64_t* bytes);
 FLA_API int fla_b200_recurrent_gdn(const fla_recurrent_gdn_args* args, void* workspace, uint64_t workspace_bytes,
@@ -168,8 +169,8 @@ FLA_API int fla_b200_causal_conv1d_fwd(const fla_causal_conv1d_fwd_args* args, v
  * torch_custom/fla_npu/test/test_npu_causal_conv1d_bwd.py:33-127).
  *   x, dy, dx [B, T, D] bf16;  weight [D, W] bf16 (any strides);  bias [D] bf16 optional (enters the recomputed
  *   pre-activation);  y_pre [B, T, D] bf16 optional: the forward's pre-activation, read instead of recomputed;
- *   initial_state, dht [N, D, W-1] bf16 optional (gradient of the final state);  dw [D, W] f32 (any strides);
- *   db [D] f32 optional;  dh0 [N, D, W-1] bf16|f32 optional;  cu_seqlens as in the forward.
+ *   initial_state, dht [N, D, W-1] bf16 optional (gradient of the final state);  dw [D, W] f32|bf16 (any strides);
+ *   db [D] f32|bf16 optional;  dh0 [N, D, W-1] bf16|f32 optional;  cu_seqlens as in the forward.
  * Workspace: per-tile partial sums of dw / db (reduced in a fixed order: results are deterministic). */
 typedef struct fla_causal_conv1d_bwd_args {
   fla_tensor_t x, weight, bias, dy, y_pre, initial_state, dht;
@@ -249,7 +250,7 @@ FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* args, void* wor
  * Unlike the reference's composition it also consumes the final-state cotangent dht and produces dh0.
  *   q, k, v, beta, gam, x_inv, s_img, vn_img, p_img: the forward's inputs and saved outputs (same shapes as there)
  *   d_o [B, T, HV, V] bf16;   dht [N, HV, 128, V] f32, optional
- *   dq, dk [B, T, HK, 128], dv [B, T, HV, V], dg, dbeta [B, T, HV]: all bf16 or all f32;  dh0 [N, HV, 128, V] f32, optional
+ *   dq, dk [B, T, HK, 128], dv [B, T, HV, V], dg, dbeta [B, T, HV]: each bf16 or f32;  dh0 [N, HV, 128, V] f32, optional
  *   dq / dk are summed over the value heads of each GVA group inside the kernel (deterministic).
  * Workspace (size from the _workspace_size call): status block + state-gradient images + [dO; dZ] images + row sums. */
 typedef struct fla_gdn_chunk_bwd_args {
@@ -408,7 +409,7 @@ FLA_API int fla_b200_kda_gate_bwd(const fla_kda_gate_args* args, void* workspace
  *   q, k, v, g, beta, initial_state, cu_seqlens ...: the forward's inputs;  d_o [B, T, HV, 128] bf16;
  *   dht [N, HV, 128, 128] f32 optional (gradient of the final state);
  *   dq, dk [B, T, HK, 128] (summed over the value heads of a group), dv [B, T, HV, 128], dg [B, T, HV, 128],
- *   dbeta [B, T, HV]: all bf16 or all f32;  dh0 [N, HV, 128, 128] f32 optional.
+ *   dbeta [B, T, HV]: each bf16 or f32;  dh0 [N, HV, 128, 128] f32 optional.
  * Workspace: the forward's workspace plus about 250 KB per (chunk, value head). */
 typedef struct fla_kda_chunk_bwd_args {
   fla_tensor_t q, k, v, g, beta, initial_state;
@@ -461,6 +462,10 @@ FLA_API int fla_b200_fast_gelu_bwd(const fla_fast_gelu_args* args, void* stream)
  *   made token-major in the same pass).  Rows of a multiple of 8 elements at 16-byte aligned addresses take the
  *   vector path.  Single-phase (no workspace). */
 FLA_API int fla_b200_convert(const fla_tensor_t* src, const fla_tensor_t* dst, void* stream);
+
+/* Chunk bookkeeping of a packed batch on the device: chunk_offsets[n] = sum over i < n of ceil(length_i / 64), from the
+ * sequence boundaries cu_seqlens (both int32 [N+1], dense).  Single-phase (no workspace). */
+FLA_API int fla_b200_chunk_offsets(const fla_tensor_t* cu_seqlens, const fla_tensor_t* chunk_offsets, void* stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Stand-alone stages of the chunked gated-delta-rule forward: one entry point per low-level reference operator,
