@@ -39,3 +39,29 @@ def load_library() -> ctypes.CDLL:
         mode = ctypes.RTLD_GLOBAL | getattr(os, "RTLD_NOW", 2)
         _LIB = ctypes.CDLL(str(path), mode=mode)
     return _LIB
+
+
+_HOST = None
+
+
+def host():
+    """The C++ binding of the hot operators (``lib/_host.so``, built beside the kernel library), bound to it on first use."""
+    global _HOST
+    if _HOST is None:
+        lib = load_library()
+        path = Path(__file__).resolve().parent / "lib" / "_host.so"
+        if not path.exists():
+            raise RuntimeError(f"fla_b200: operator binding not found at {path}. Build it with "
+                               f"`python {Path(__file__).resolve().parent.parent / 'build.py'}`. There is no fallback path.")
+        import importlib.util
+        from importlib.machinery import ExtensionFileLoader
+
+        import torch  # noqa: F401  (its libraries have to be in the process before the binding is)
+        loader = ExtensionFileLoader("_host", str(path))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
+        loader.exec_module(mod)
+        mod.bind(lib._handle)
+        from ._runtime import device_status_check
+        mod.check_status(device_status_check())
+        _HOST = mod
+    return _HOST

@@ -1,4 +1,5 @@
-"""ctypes call layer between the Python operators and libfla_b200.so.
+"""ctypes call layer between the stage operators and libfla_b200.so (the hot operators go through the C++ binding,
+csrc/host, which does the same things natively).
 
 Mirrors the reference's FFI runtime (torch_custom/fla_npu/fla_npu/ops/ascendc/_runtime.py):
 tensor descriptors built from shape / strides / dtype / data pointer (:210-256), a device guard
@@ -14,7 +15,7 @@ from typing import Iterable, Optional, Sequence
 
 import torch
 
-from . import load_library
+from . import host, load_library
 
 FLA_MAX_DIMS = 6
 
@@ -103,10 +104,9 @@ def _check_arch(dev: torch.device, op: str) -> None:
 # Operators whose kernels wait on barriers: byte 0 of their workspace is an int32 status word that a wait which ran
 # out sets to FLA_ERR_TIMEOUT (include/fla_b200.h, "Device-side failure reporting").
 _STATUS_WORD_OPS = frozenset({
-    "gdn_chunk_fwd", "gdn_chunk_bwd", "kda_chunk_fwd", "kda_chunk_bwd", "chunk_local_cumsum", "chunk_scaled_dot_kkt",
-    "solve_tri", "recompute_w_u_fwd", "chunk_gated_delta_rule_fwd_h", "chunk_fwd_o", "chunk_bwd_dv_local",
-    "chunk_gated_delta_rule_bwd_dhu", "chunk_bwd_dqkwg", "prepare_wy_repr_bwd", "prepare_wy_repr_bwd_da",
-    "prepare_wy_repr_bwd_full",
+    "chunk_local_cumsum", "chunk_scaled_dot_kkt", "solve_tri", "recompute_w_u_fwd", "chunk_gated_delta_rule_fwd_h",
+    "chunk_fwd_o", "chunk_bwd_dv_local", "chunk_gated_delta_rule_bwd_dhu", "chunk_bwd_dqkwg", "prepare_wy_repr_bwd",
+    "prepare_wy_repr_bwd_da", "prepare_wy_repr_bwd_full",
 })
 
 _check_device_status = os.environ.get("FLA_B200_CHECK", "0") not in ("", "0")
@@ -120,7 +120,12 @@ def set_device_status_check(enabled: bool) -> bool:
     stay asynchronous and a caller can check a workspace itself with :func:`read_device_status`."""
     global _check_device_status
     prev, _check_device_status = _check_device_status, bool(enabled)
+    host().check_status(_check_device_status)
     return prev
+
+
+def device_status_check() -> bool:
+    return _check_device_status
 
 
 def read_device_status(workspace: torch.Tensor, op: str = "operator") -> None:

@@ -8,12 +8,9 @@ activation, cu_seqlens, output_final_state).  States are `[N,D,W-1]` (the last W
 """
 from __future__ import annotations
 
-from typing import Optional
-
 import torch
 
-from .. import _runtime as rt
-from ._structs import CausalConv1dBwdArgs, CausalConv1dFwdArgs, CausalConv1dUpdateArgs
+from .. import host
 
 
 def _act(activation) -> int:
@@ -28,116 +25,28 @@ def causal_conv1d_bwd(x, weight, dy, bias=None, initial_state=None, dht=None, ac
                       y_pre=None, need_dh0=None):
     """Gradients of :func:`causal_conv1d` (layouts as there).  Returns ``(dx, dw [D,W] f32, db [D] f32, dh0 | None)``.
     The pre-activation is recomputed from x (and bias) unless ``y_pre`` holds it."""
-    B, T, D = x.shape
-    W = weight.shape[1]
-    if x.stride(-1) != 1:
-        x = x.contiguous()
-    dy = dy.contiguous() if dy.stride(-1) != 1 or dy.dtype != x.dtype else dy
-    if dy.dtype != x.dtype:
-        dy = dy.to(x.dtype)
-    cu = None
-    N = B
-    if cu_seqlens is not None:
-        cu = cu_seqlens.to(device=x.device, dtype=torch.int32)
-        N = cu.numel() - 1
-    dx = torch.empty_like(x)
-    dw = torch.empty((D, W), dtype=torch.float32, device=x.device)
-    db = torch.empty((D,), dtype=torch.float32, device=x.device)
     want_dh0 = (initial_state is not None) if need_dh0 is None else need_dh0
-    dh0 = torch.zeros((N, D, W - 1), dtype=torch.float32, device=x.device) if want_dh0 else None
-    a = CausalConv1dBwdArgs()
-    a.x, a.weight, a.bias, a.dy, a.y_pre = rt.desc(x), rt.desc(weight), rt.desc(bias), rt.desc(dy), rt.desc(y_pre)
-    a.initial_state, a.dht = rt.desc(initial_state), rt.desc(dht)
-    a.dx, a.dw, a.db, a.dh0, a.cu_seqlens = rt.desc(dx), rt.desc(dw), rt.desc(db), rt.desc(dh0), rt.desc(cu)
-    a.activation_silu = _act(activation)
-    rt.call("causal_conv1d_bwd", a, [x, weight, bias, dy, y_pre, initial_state, dht, dx, dw, db, dh0, cu])
-    return dx, dw, db, dh0
-
-
-class CausalConv1dFunction(torch.autograd.Function):
-    """Autograd glue of :func:`causal_conv1d` (the reference wires its operator the same way,
-    examples/flash_gated_delta_rule.py:323-419): saves the inputs, the backward recomputes the pre-activation."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, residual, initial_state, output_final_state, activation, cu_seqlens):
-        y, final = _causal_conv1d_fwd(x, weight, bias, residual, initial_state, output_final_state, activation, cu_seqlens)
-        ctx.save_for_backward(x, weight, bias, initial_state, cu_seqlens)
-        ctx.activation, ctx.has_residual = activation, residual is not None
-        return y, final
-
-    @staticmethod
-    def backward(ctx, dy, dfinal):
-        x, weight, bias, initial_state, cu = ctx.saved_tensors
-        dht = None if dfinal is None else dfinal.to(x.dtype)
-        dx, dw, db, dh0 = causal_conv1d_bwd(x, weight, dy, bias, initial_state, dht, ctx.activation, cu)
-        return (dx, dw.to(weight.dtype), None if bias is None else db.to(bias.dtype), dy if ctx.has_residual else None,
-                None if dh0 is None else dh0.to(initial_state.dtype), None, None, None)
+    return host().conv_bwd(x, weight, dy, bias, initial_state, dht, _act(activation), cu_seqlens, y_pre, want_dh0)
 
 
 def causal_conv1d(x, weight=None, bias=None, residual=None, initial_state=None, output_final_state=False,
                   activation=None, cu_seqlens=None):
     """x `[B,T,D]` bf16; weight `[D,W]`; initial_state / final_state `[N,D,W-1]`.
-    Returns ``(y [B,T,D], final_state | None)``; differentiable in x, weight, bias, residual and initial_state."""
+    Returns ``(y [B,T,D], final_state | None)``; differentiable in x, weight, bias, residual and initial_state (the reference
+    wires its operator the same way, examples/flash_gated_delta_rule.py:323-419): the inputs are saved, the backward
+    recomputes the pre-activation."""
     if weight is None:
         raise RuntimeError("causal_conv1d: weight is required")
-    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, weight, bias, residual, initial_state)):
-        return CausalConv1dFunction.apply(x, weight, bias, residual, initial_state, output_final_state, activation, cu_seqlens)
-    return _causal_conv1d_fwd(x, weight, bias, residual, initial_state, output_final_state, activation, cu_seqlens)
-
-
-def _causal_conv1d_fwd(x, weight=None, bias=None, residual=None, initial_state=None, output_final_state=False,
-                       activation=None, cu_seqlens=None, head_num=0):
-    """`head_num` > 0: y comes out head-first, `[B, head_num, T, D // head_num]`, written in that layout by the kernel."""
-    op = "causal_conv1d"
-    if x.dim() != 3:
-        raise RuntimeError(f"{op}: x must be [B,T,D], got {tuple(x.shape)}")
-    if weight is None:
-        raise RuntimeError(f"{op}: weight is required")
-    B, T, D = x.shape
-    W = weight.shape[1]
-    if x.stride(-1) != 1:
-        x = x.contiguous()
-    cu = None
-    N = B
-    if cu_seqlens is not None:
-        cu = cu_seqlens.to(device=x.device, dtype=torch.int32)
-        N = cu.numel() - 1
-    head_num = int(head_num)
-    if head_num > 0:
-        if D % head_num or (D // head_num) % 8:
-            raise RuntimeError(f"{op}: head_num={head_num} must divide D={D} into heads of a multiple of 8 channels")
-        y = torch.empty((B, head_num, T, D // head_num), dtype=x.dtype, device=x.device)
-    else:
-        y = torch.empty_like(x)
-    final = torch.empty((N, D, W - 1), dtype=x.dtype, device=x.device) if output_final_state else None
-    a = CausalConv1dFwdArgs()
-    a.x, a.weight, a.bias, a.residual = rt.desc(x), rt.desc(weight), rt.desc(bias), rt.desc(residual)
-    a.initial_state, a.y, a.final_state, a.cu_seqlens = rt.desc(initial_state), rt.desc(y), rt.desc(final), rt.desc(cu)
-    a.activation_silu = _act(activation)
-    rt.call("causal_conv1d_fwd", a, [x, weight, bias, residual, initial_state, y, final, cu])
-    return y, final
+    return host().conv(x, weight, bias, residual, initial_state, output_final_state, _act(activation), cu_seqlens)
 
 
 def causal_conv1d_update(x, cache, residual=None, weight=None, bias=None, activation=None, cache_indices=None,
                          num_accepted_tokens=None, pad_slot_id=-1):
     """Decode step.  x `[N,D]` or `[N,T,D]`; cache `[slots,D,S]` (S >= W-1), updated in place.
     Returns y with the shape of x."""
-    op = "causal_conv1d_update"
     if weight is None:
-        raise RuntimeError(f"{op}: weight is required")
-    rt.reject_requires_grad(op, cache=cache)
-    squeeze = x.dim() == 2
-    x3 = x.unsqueeze(1) if squeeze else x
-    r3 = None if residual is None else (residual.unsqueeze(1) if squeeze else residual)
-    y3 = torch.empty_like(x3)
-    a = CausalConv1dUpdateArgs()
-    a.x, a.weight, a.bias, a.residual = rt.desc(x3), rt.desc(weight), rt.desc(bias), rt.desc(r3)
-    a.conv_state, a.y = rt.desc(cache), rt.desc(y3)
-    a.cache_indices, a.num_accepted_tokens = rt.desc(cache_indices), rt.desc(num_accepted_tokens)
-    a.activation_silu, a.pad_slot_id = _act(activation), int(pad_slot_id)
-    rt.call("causal_conv1d_update", a, [x3, weight, bias, r3, cache, y3, cache_indices, num_accepted_tokens])
-    rt.mark_mutated(cache)
-    return y3.squeeze(1) if squeeze else y3
+        raise RuntimeError("causal_conv1d_update: weight is required")
+    return host().conv_update(x, cache, residual, weight, bias, _act(activation), cache_indices, num_accepted_tokens, pad_slot_id)
 
 
 def npu_causal_conv1d(x, weight, bias=None, conv_states=None, *, query_start_loc=None, cache_indices=None,
@@ -172,7 +81,8 @@ def npu_causal_conv1d(x, weight, bias=None, conv_states=None, *, query_start_loc
     init = None
     idx = as_i32(cache_indices)
     if st is not None:
-        rt.reject_requires_grad(op, conv_states=conv_states)
+        if conv_states.requires_grad:
+            raise RuntimeError(f"{op}: conv_states is updated in place and must not require grad")
         if st.shape[2] != W - 1:
             raise RuntimeError(f"{op}: prefill expects conv_states with state_len == W-1")
         if initial_state_mode is not None:
@@ -180,7 +90,7 @@ def npu_causal_conv1d(x, weight, bias=None, conv_states=None, *, query_start_loc
             mode = as_i32(initial_state_mode).bool()
             init = torch.where(mode[:, None, None], sel, torch.zeros_like(sel))
     if head_num:   # prefill output as [B, head_num, T, D / head_num] ([head_num, T, D / head_num] for packed input)
-        y, final = _causal_conv1d_fwd(x3, w_dw, bias, None, init, st is not None, int(activation_mode), cu, head_num=head_num)
+        y, final = host().conv_fwd(x3, w_dw, bias, None, init, st is not None, _act(int(activation_mode)), cu, head_num)
     else:
         y, final = causal_conv1d(x3, w_dw, bias, None, init, st is not None, int(activation_mode), cu)
     if st is not None:
@@ -189,7 +99,7 @@ def npu_causal_conv1d(x, weight, bias=None, conv_states=None, *, query_start_loc
         else:
             keep = idx != pad_slot_id
             st[idx[keep].long()] = final[keep]
-        rt.mark_mutated(conv_states)
+        torch.autograd.graph.increment_version(conv_states)
     return y.squeeze(0) if varlen else y   # packed input with head_num: [head_num, T, D / head_num]
 
 

@@ -17,107 +17,14 @@ import ctypes
 import torch
 
 from .. import _runtime as rt
-from .. import load_library
-from ._structs import KdaChunkBwdArgs, KdaChunkFwdArgs
+from .. import host, load_library
 from .gdn import CHUNK, _as_rows, _varlen_meta
-
-
-def _kda_forward(q, k, v, g, beta, scale, initial_state, output_final_state, gate_mode, A_log, dt_bias, lower_bound,
-                 meta, return_gate_cumsum, output_dtype, keep_for_backward=False, scores=None):
-    B, T, HK, K = q.shape
-    HV, V = v.shape[2], v.shape[3]
-    cu, co, N, max_len, total_chunks = meta
-    dev = q.device
-    o = torch.empty((B, T, HV, V), dtype=output_dtype or q.dtype, device=dev)
-    ht = torch.empty((N, HV, K, V), dtype=torch.float32, device=dev) if output_final_state else None
-    gk = torch.empty((B, T, HV, K), dtype=torch.float32, device=dev) if return_gate_cumsum else None
-    a = KdaChunkFwdArgs()
-    a.q, a.k, a.v, a.g, a.beta = rt.desc(q), rt.desc(k), rt.desc(v), rt.desc(g), rt.desc(beta)
-    a.a_log, a.dt_bias = rt.desc(A_log if gate_mode else None), rt.desc(dt_bias if gate_mode else None)
-    a.initial_state, a.o, a.final_state, a.gk = rt.desc(initial_state), rt.desc(o), rt.desc(ht), rt.desc(gk)
-    a.cu_seqlens, a.chunk_offsets = rt.desc(cu), rt.desc(co)
-    a.scale, a.lower_bound, a.gate_mode = scale, float(lower_bound or 0.0), gate_mode
-    a.chunk_size, a.max_seqlen, a.total_chunks = CHUNK, int(max_len), int(total_chunks)
-    if scores is not None:   # (aqk, akk) as [B,T,HV,64] views, filled from the forward's score images
-        a.aqk, a.akk = rt.desc(scores[0]), rt.desc(scores[1])
-    saved = None
-    if keep_for_backward:   # the reference's disable_recompute=True: keep the intermediates instead of recomputing them
-        nbytes = ctypes.c_uint64(0)
-        status = load_library().fla_b200_kda_chunk_saved_size(ctypes.byref(a), ctypes.byref(nbytes))
-        if status:
-            raise RuntimeError(f"kda_chunk_saved_size failed with status={status}")
-        saved = torch.empty((nbytes.value + 1) // 2, dtype=torch.bfloat16, device=dev)
-        a.saved = rt.desc(saved)
-    rt.call("kda_chunk_fwd", a, [q, k, v, g, beta, initial_state, o, ht, gk, cu, co, saved] + list(scores or ()))
-    if keep_for_backward:
-        return o, ht, saved
-    return o, ht, gk
 
 
 def kda_chunk_bwd(q, k, v, g, beta, scale, initial_state, do, dht, meta, grad_dtype=None, saved=None):
     """Complete KDA chunk backward (g = per-channel log decay).  Returns dq, dk, dv, dg, dbeta, dh0.
-    `saved` is the buffer a forward with ``keep_for_backward`` returned; without it the forward is recomputed."""
-    B, T, HK, K = q.shape
-    HV, V = v.shape[2], v.shape[3]
-    cu, co, N, max_len, total_chunks = meta
-    dev = q.device
-    gdt = grad_dtype or torch.float32
-    dq = torch.empty((B, T, HK, K), dtype=gdt, device=dev)
-    dk = torch.empty_like(dq)
-    dv = torch.empty((B, T, HV, V), dtype=gdt, device=dev)
-    dg = torch.empty((B, T, HV, K), dtype=gdt, device=dev)
-    dbeta = torch.empty((B, T, HV), dtype=gdt, device=dev)
-    dh0 = torch.empty((N, HV, K, V), dtype=torch.float32, device=dev) if initial_state is not None else None
-    if do.dtype != torch.bfloat16:
-        from ._convert import convert
-        do = convert(do, torch.bfloat16, "chunk_kda_bwd")
-    do = _as_rows(do)
-    if dht is not None:
-        dht = dht.float().contiguous()
-    a = KdaChunkBwdArgs()
-    a.q, a.k, a.v, a.g, a.beta = rt.desc(q), rt.desc(k), rt.desc(v), rt.desc(g), rt.desc(beta)
-    a.initial_state, a.d_o, a.dht = rt.desc(initial_state), rt.desc(do), rt.desc(dht)
-    a.dq, a.dk, a.dv, a.dg, a.dbeta, a.dh0 = (rt.desc(x) for x in (dq, dk, dv, dg, dbeta, dh0))
-    a.cu_seqlens, a.chunk_offsets, a.saved = rt.desc(cu), rt.desc(co), rt.desc(saved)
-    a.scale = scale
-    a.chunk_size, a.max_seqlen, a.total_chunks = CHUNK, int(max_len), int(total_chunks)
-    rt.call("kda_chunk_bwd", a, [q, k, v, g, beta, initial_state, do, dht, dq, dk, dv, dg, dbeta, dh0, cu, co, saved])
-    return dq, dk, dv, dg, dbeta, dh0
-
-
-class ChunkKdaFunction(torch.autograd.Function):
-    """Autograd glue of `chunk_kda` (gate already activated): saves only the inputs, the backward recomputes."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, beta, initial_state, scale, output_final_state, meta, output_dtype, disable_recompute,
-                qk_l2norm=False):
-        ctx.qk_l2norm = qk_l2norm
-        rstd = ()
-        if qk_l2norm:   # q, k <- x * rsqrt(sum x^2 + 1e-6) stored in the input dtype; rstd kept for the backward
-            from .l2norm import l2norm_fwd
-            q, q_rstd = l2norm_fwd(q)
-            k, k_rstd = l2norm_fwd(k)
-            rstd = (q_rstd, k_rstd)
-        o, ht, saved = _kda_forward(q, k, v, g, beta, scale, initial_state, output_final_state, 0, None, None, None, meta,
-                                    False, output_dtype, keep_for_backward=disable_recompute)
-        ctx.save_for_backward(q, k, v, g, beta, initial_state, saved if disable_recompute else None, *rstd)
-        ctx.scale, ctx.meta = scale, meta
-        ctx.in_dtypes = (q.dtype, k.dtype, v.dtype, g.dtype, beta.dtype)
-        return o, ht
-
-    @staticmethod
-    def backward(ctx, do, dht):
-        q, k, v, g, beta, h0, saved = ctx.saved_tensors[:7]
-        dq, dk, dv, dg, dbeta, dh0 = kda_chunk_bwd(q, k, v, g, beta, ctx.scale, h0, do.contiguous(), dht, ctx.meta,
-                                                   saved=saved, grad_dtype=torch.float32 if ctx.qk_l2norm else None)
-        if ctx.qk_l2norm:
-            from .l2norm import l2norm_bwd
-            q_rstd, k_rstd = ctx.saved_tensors[7:9]
-            dq = l2norm_bwd(q, q_rstd, dq)
-            dk = l2norm_bwd(k, k_rstd, dk)
-        dts = ctx.in_dtypes
-        return (dq.to(dts[0]), dk.to(dts[1]), dv.to(dts[2]), dg.to(dts[3]), dbeta.to(dts[4]), dh0,
-                None, None, None, None, None, None)
+    `saved` is the buffer a forward that kept its intermediates returned; without it the forward is recomputed."""
+    return host().kda_bwd(q, k, v, g, beta, scale, initial_state, do, dht, *meta, *(grad_dtype,) * 5, saved)
 
 
 def chunk_kda_fwd_bwd(q, k, v, g, beta, do, scale=None, initial_state=None, dht=None, output_dtype=None, grad_dtype=None,
@@ -129,10 +36,9 @@ def chunk_kda_fwd_bwd(q, k, v, g, beta, do, scale=None, initial_state=None, dht=
     scale = q.shape[-1] ** -0.5 if scale is None else float(scale)
     q, k, v, g, beta = (_as_rows(x) for x in (q, k, v, g, beta))
     meta = (None, None, B, T, B * ((T + CHUNK - 1) // CHUNK))
-    o, ht, saved = _kda_forward(q, k, v, g, beta, scale, initial_state, True, 0, None, None, None, meta, False, output_dtype,
-                                keep_for_backward=disable_recompute)
-    grads = kda_chunk_bwd(q, k, v, g, beta, scale, initial_state, do, dht, meta, grad_dtype=grad_dtype,
-                          saved=saved if disable_recompute else None)
+    o, ht, _, saved = host().kda_fwd(q, k, v, g, beta, initial_state, None, None, *meta, scale, 0.0, 0, True, disable_recompute,
+                                     False, output_dtype, None, None)
+    grads = kda_chunk_bwd(q, k, v, g, beta, scale, initial_state, do, dht, meta, grad_dtype=grad_dtype, saved=saved)
     return o, ht, grads
 
 
@@ -205,84 +111,25 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
         # beta arrives as logits.  It is a [B,T,HV] tensor, 1/128 of the gate's bytes: the activation (and, through autograd,
         # its gradient) is one elementwise pass in front of the kernels rather than a mode of them.
         beta = torch.sigmoid(beta.float())
-    if torch.float16 in (q.dtype, k.dtype, v.dtype):
-        # fp16 tensors (the reference's published 4-stage case is fp16, fla/ops/ascendc/kda/KDA_FORWARD_VALIDATION_REPORT.md:133-146):
-        # q, k, v are rounded to the bf16 operands of the tensor-core products by the library's conversion kernel, fp16
-        # gates become fp32, o is computed in fp32 and converted to fp16 once; gradients return through the same conversions
-        if not (q.dtype == k.dtype == v.dtype):
-            raise TypeError(f"{op}: q, k, v must share one dtype, got {q.dtype}, {k.dtype}, {v.dtype}")
-        from ._convert import to_dtype
-        q, k, v = (to_dtype(x, torch.bfloat16, op) for x in (q, k, v))
-        g, beta = (to_dtype(x, torch.float32, op) if x.dtype == torch.float16 else x for x in (g, beta))
-        if export_scores is not None and any(x.dtype == torch.float16 for x in export_scores):
-            raise NotImplementedError(f"{op}: export_scores takes bf16 or fp32 views")
-        res = chunk_kda(q, k, v, g, beta, scale=scale, initial_state=initial_state, output_final_state=output_final_state,
-                        use_qk_l2norm_in_kernel=use_qk_l2norm_in_kernel, use_gate_in_kernel=use_gate_in_kernel,
-                        use_beta_sigmoid_in_kernel=False, cu_seqlens=cu_seqlens, safe_gate=safe_gate, lower_bound=lower_bound,
-                        A_log=A_log, dt_bias=dt_bias, return_gate_cumsum=return_gate_cumsum, output_dtype=torch.float32,
-                        disable_recompute=disable_recompute, export_scores=export_scores, _return_saved=_return_saved)
-        return (to_dtype(res[0], output_dtype or torch.float16, op),) + tuple(res[1:])
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        if t.dtype != torch.bfloat16:
-            raise TypeError(f"{op}: {name} must be bfloat16 or float16, got {t.dtype}")
-    if q.dim() != 4 or q.shape != k.shape or v.dim() != 4 or v.shape[:2] != q.shape[:2]:
-        raise RuntimeError(f"{op}: expected q,k [B,T,HK,K] and v [B,T,HV,V]")
-    B, T, HK, K = q.shape
-    HV, V = v.shape[2], v.shape[3]
-    if K != 128 or V not in (128, 256):
-        raise RuntimeError(f"{op}: this build supports K = 128 and V = 128 or 256, got K={K}, V={V}")
-    if HV % HK:
-        raise RuntimeError(f"{op}: HV={HV} must be a multiple of HK={HK}")
-    if tuple(g.shape) != (B, T, HV, K) or tuple(beta.shape) != (B, T, HV):
-        raise RuntimeError(f"{op}: g must be {(B, T, HV, K)} and beta {(B, T, HV)}")
-    scale = K ** -0.5 if scale is None else float(scale)
-    needs_grad = torch.is_grad_enabled() and any(
-        t is not None and t.requires_grad for t in (q, k, v, g, beta, initial_state, A_log, dt_bias))
+    scale = q.shape[-1] ** -0.5 if scale is None else float(scale)
     gate_mode = 0
     if use_gate_in_kernel:
         if A_log is None:
             raise RuntimeError(f"{op}: use_gate_in_kernel needs A_log")
         if safe_gate and lower_bound is None:
             raise RuntimeError(f"{op}: safe_gate needs lower_bound")
+        needs_grad = torch.is_grad_enabled() and any(
+            t is not None and t.requires_grad for t in (q, k, v, g, beta, initial_state, A_log, dt_bias))
         if needs_grad or _return_saved:   # the kernels keep their intermediates only for gates given as they are
             g = _gate_activation(g, A_log, dt_bias, safe_gate, lower_bound)
         else:
             gate_mode = 2 if safe_gate else 1
-            A_log = A_log.float().contiguous()
-            dt_bias = None if dt_bias is None else dt_bias.float().reshape(HV, K).contiguous()
-    q, k, v, g, beta = (_as_rows(x) for x in (q, k, v, g, beta))
-    dev = q.device
-    cu = co = None
-    N, max_len, total_chunks = B, T, B * ((T + CHUNK - 1) // CHUNK)
-    if cu_seqlens is not None:
-        if B != 1:
-            raise RuntimeError(f"{op}: cu_seqlens requires batch size 1 (packed sequences)")
-        cu, co, max_len, total_chunks, N, total = _varlen_meta(cu_seqlens, dev)
-        if total != T:
-            raise RuntimeError(f"{op}: cu_seqlens[-1]={total} must equal T={T}")
-    if initial_state is not None:
-        if tuple(initial_state.shape) != (N, HV, K, V):
-            raise RuntimeError(f"{op}: initial_state must be {(N, HV, K, V)}, got {tuple(initial_state.shape)}")
-        initial_state = initial_state.float().contiguous()
-    meta = (cu, co, N, max_len, total_chunks)
-    if needs_grad:
-        if return_gate_cumsum or export_scores is not None:
-            raise NotImplementedError(f"{op}: return_gate_cumsum / export_scores are not available on the differentiable path")
-        o, ht = ChunkKdaFunction.apply(q, k, v, g, beta, initial_state, scale, output_final_state, meta, output_dtype,
-                                       bool(disable_recompute), bool(use_qk_l2norm_in_kernel))
-        return o, ht
-    if use_qk_l2norm_in_kernel:   # x * rsqrt(sum x^2 + 1e-6), stored in the input dtype (the l2norm kernels)
-        from .l2norm import l2norm_fwd
-        q, k = l2norm_fwd(q)[0], l2norm_fwd(k)[0]
+    aqk, akk = export_scores if export_scores is not None else (None, None)
     if _return_saved:
-        o, ht, saved = _kda_forward(q, k, v, g, beta, scale, initial_state, output_final_state, 0, None, None, None, meta,
-                                    False, output_dtype, keep_for_backward=True, scores=export_scores)
-        return o, ht, saved, meta, (q, k, v, beta)
-    o, ht, gk = _kda_forward(q, k, v, g, beta, scale, initial_state, output_final_state, gate_mode, A_log, dt_bias,
-                             lower_bound, meta, return_gate_cumsum, output_dtype, scores=export_scores)
-    if return_gate_cumsum:
-        return o, ht, gk
-    return o, ht
+        return host().kda_saved(q, k, v, g, beta, initial_state, cu_seqlens, scale, output_final_state, use_qk_l2norm_in_kernel,
+                                output_dtype, aqk, akk)
+    return host().kda(q, k, v, g, beta, initial_state, A_log, dt_bias, cu_seqlens, scale, lower_bound or 0.0, gate_mode,
+                      output_final_state, use_qk_l2norm_in_kernel, disable_recompute, return_gate_cumsum, output_dtype, aqk, akk)
 
 
 def kda_chunk_intermediates(q, k, v, beta, saved, meta, *, full, state_v_first=False, dtype=None):
