@@ -34,6 +34,7 @@ namespace fla {
 struct GdnBwdParams {
   const bf16* q; const bf16* k; const bf16* v; const bf16* dO;
   const void* beta;
+  const float* q_rstd; const float* k_rstd;   // [tokens, HK] or null: q, k are normalised rows, dq / dk go through the normalisation
   const float* gam; const bf16* X;
   const bf16* s_img; const bf16* vn_img; const bf16* p_img;
   bf16* ds_img;        // [chunks, HV, V/64, 2, 128x64]  state gradient entering each chunk (hi, lo)
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, con
   __shared__ float gam_s2[2][kC], beta_s2[2][kC];
   __shared__ float red2[2][5][2][kC];  // qdq, kdk, rkG, rkB, ma : [half][row]
   __shared__ float sds_s2[2][8];
+  __shared__ float ndot_s[2][2 * kC];  // q.dq / k.dk of the complete rows, per half of the columns (normalised q, k only)
   __shared__ float fin_s[2][2];
   __shared__ uint32_t tmem_base_s;
   __shared__ __align__(8) uint64_t mma_bar, load_bar, qk_bar;
@@ -401,8 +403,25 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, con
 #pragma unroll
       for (int i = 0; i < 64; ++i) part[i] += t[i];
     }
-    if (h + 1 < G) tmem_st_row64(trow + rColAcc + half * 64, part);
-    else if (tok < rows) {   // the last head: the rows are complete
+    if (h + 1 < G) {
+      tmem_st_row64(trow + rColAcc + half * 64, part);
+    } else if (p.q_rstd) {   // the rows are complete: through the normalisation, rstd (dx - x (x . dx)), while they are in registers
+      float t = 0.f;
+      row_dot64(smem + rOffQK, rQKPanel, row, half * 64, part, t);
+      ndot_s[half][row] = t;
+      __syncthreads();
+      t = ndot_s[0][row] + ndot_s[1][row];
+      const float rs = (kside ? p.k_rstd : p.q_rstd)[(tok0 + min(tok, rows - 1)) * p.HK + hk];
+      const uint8_t* pan = smem + rOffQK + half * rQKPanel;
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        float f[8];
+        unpack_bf16x8(*reinterpret_cast<const uint4*>(pan + panel_chunk_off(row, ch)), f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) part[ch * 8 + j] = (part[ch * 8 + j] - t * f[j]) * rs;
+      }
+    }
+    if (h + 1 == G && tok < rows) {   // the last head
       void* base = kside ? p.dk : p.dq;
       const int64_t off = kside ? (tok0 + tok) * p.dk_st + hk * p.dk_sh + half * 64 : (tok0 + tok) * p.dq_st + hk * p.dq_sh + half * 64;
       if (kside ? p.dk_f32 : p.dq_f32) {
@@ -536,6 +555,13 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
     if (s->stride[3] != 1 || s->stride[2] != V || s->stride[1] != kK * V || s->stride[0] != HV * kK * V || !aligned16(s->data))
       return FLA_ERR_LAYOUT;
   }
+  if (a->q_rstd.data || a->k_rstd.data) {
+    for (const fla_tensor_t* t : {&a->q_rstd, &a->k_rstd}) {
+      if (!t->data) return FLA_ERR_NULL;
+      if (t->dtype != FLA_F32) return FLA_ERR_DTYPE;
+      if ((st = check_tok3(*t, B, T, HK, true))) return st;
+    }
+  }
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
   uint64_t off_ds, off_dz, off_bz;
   const uint64_t need = bwd_ws_layout(total_chunks, HV, nvb, B * T, &off_ds, &off_dz, &off_bz);
@@ -544,6 +570,7 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   GdnBwdParams p{};
   p.q = static_cast<const bf16*>(a->q.data); p.k = static_cast<const bf16*>(a->k.data);
   p.v = static_cast<const bf16*>(a->v.data); p.dO = static_cast<const bf16*>(a->d_o.data);
+  p.q_rstd = static_cast<const float*>(a->q_rstd.data); p.k_rstd = static_cast<const float*>(a->k_rstd.data);
   p.beta = a->beta.data; p.gam = static_cast<const float*>(gam.data); p.X = static_cast<const bf16*>(X.data);
   p.s_img = static_cast<const bf16*>(a->s_img.data); p.vn_img = static_cast<const bf16*>(a->vn_img.data);
   p.p_img = static_cast<const bf16*>(a->p_img.data);

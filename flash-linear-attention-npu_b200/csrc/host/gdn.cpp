@@ -10,7 +10,8 @@ using torch::autograd::variable_list;
 static Tensor state_f32(const Tensor& t) { return t.defined() ? t.to(at::kFloat).contiguous() : t; }
 
 std::tuple<Tensor, Tensor, GdnSaved> gdn_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, double scale,
-                                             const Tensor& h0_, bool want_final, const Tensor& cu, bool save, std::optional<at::ScalarType> out) {
+                                             const Tensor& h0_, bool want_final, const Tensor& cu, bool save, std::optional<at::ScalarType> out,
+                                             bool l2norm) {
   const char* op = "chunk_gated_delta_rule";
   for (auto& [name, t] : {std::pair<const char*, const Tensor&>{"q", q_}, {"k", k_}, {"v", v_}})
     TORCH_CHECK_TYPE(t.scalar_type() == at::kBFloat16, op, ": ", name, " must be bfloat16 (fp32 inputs are rejected like in the reference), got ", t.scalar_type());
@@ -40,7 +41,12 @@ std::tuple<Tensor, Tensor, GdnSaved> gdn_fwd(const Tensor& q_, const Tensor& k_,
     s.vn_img = empty({tiles * (V / 64) * 8192}, at::kBFloat16, d);
     s.p_img = empty({tiles * 8768}, at::kBFloat16, d);    // P tile (16 KB) + the chunk's factor record
   }
+  if (l2norm) {
+    s.qn = empty({B, T, HK, K}, at::kBFloat16, d), s.kn = empty({B, T, HK, K}, at::kBFloat16, d);
+    s.q_rstd = empty({B, T, HK}, at::kFloat, d), s.k_rstd = empty({B, T, HK}, at::kFloat, d);
+  }
   fla_gdn_chunk_fwd_args a{};
+  a.q_norm = desc(s.qn), a.k_norm = desc(s.kn), a.q_rstd = desc(s.q_rstd), a.k_rstd = desc(s.k_rstd);
   a.q = desc(q), a.k = desc(k), a.v = desc(v), a.g = desc(g), a.beta = desc(beta);
   a.initial_state = desc(h0), a.o = desc(o), a.final_state = desc(ht);
   a.gam = desc(s.gam), a.x_inv = desc(s.x_inv), a.s_img = desc(s.s_img), a.vn_img = desc(s.vn_img), a.p_img = desc(s.p_img);
@@ -65,6 +71,7 @@ std::vector<Tensor> gdn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, c
          dbeta = empty({B, T, HV}, ty.beta, d), dh0;
   if (want_dh0) dh0 = empty(hs, at::kFloat, d);
   fla_gdn_chunk_bwd_args a{};
+  a.q_rstd = desc(s.q_rstd), a.k_rstd = desc(s.k_rstd);
   a.q = desc(q), a.k = desc(k), a.v = desc(v), a.beta = desc(beta);
   a.gam = desc(s.gam), a.x_inv = desc(s.x_inv), a.s_img = desc(s.s_img), a.vn_img = desc(s.vn_img), a.p_img = desc(s.p_img);
   a.d_o = desc(d_o), a.dht = desc(dht);
@@ -90,12 +97,11 @@ std::array<Tensor, 3> fold_plan(const Tensor& q, const Tensor& k, const Tensor& 
   return f;
 }
 
-struct GdnInputs {      // what the kernels are given: row-major or folded views, q and k normalised when asked for
-  Tensor q, k, v, g, beta, h0, q_rstd, k_rstd;
+struct GdnInputs {      // what the kernels are given: row-major or folded views
+  Tensor q, k, v, g, beta, h0;
   bool folded = false;
 };
-static GdnInputs gdn_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& h0, const Tensor& cu,
-                            bool l2norm) {
+static GdnInputs gdn_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& h0, const Tensor& cu) {
   GdnInputs in;
   const auto f = fold_plan(q, k, v, cu);
   in.folded = f[0].defined();
@@ -107,10 +113,6 @@ static GdnInputs gdn_inputs(const Tensor& q, const Tensor& k, const Tensor& v, c
     if (h0.defined()) in.h0 = h0.reshape({1, B * HV, h0.size(2), h0.size(3)});
   } else {
     in.q = as_rows(q), in.k = as_rows(k), in.v = as_rows(v), in.g = as_rows(g), in.beta = as_rows(beta), in.h0 = h0;
-  }
-  if (l2norm) {
-    std::tie(in.q, in.q_rstd) = l2norm_fwd(in.q, 1e-6, std::nullopt);
-    std::tie(in.k, in.k_rstd) = l2norm_fwd(in.k, 1e-6, std::nullopt);
   }
   return in;
 }
@@ -124,18 +126,19 @@ struct GdnFn : torch::autograd::Function<GdnFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta,
                                const OptTensor& h0_, double scale, bool want_final, const OptTensor& cu_, int64_t out, bool l2norm) {
     const Tensor h0 = value(h0_), cu = value(cu_);
-    const GdnInputs in = gdn_inputs(q, k, v, g, beta, h0, cu, l2norm);
+    const GdnInputs in = gdn_inputs(q, k, v, g, beta, h0, cu);
     auto [o, ht, s] = gdn_fwd(in.q, in.k, in.v, in.g, in.beta, scale, in.h0, want_final, cu, true,
-                              out < 0 ? std::nullopt : std::optional<at::ScalarType>(at::ScalarType(out)));
+                              out < 0 ? std::nullopt : std::optional<at::ScalarType>(at::ScalarType(out)), l2norm);
     if (in.folded) std::tie(o, ht) = unfold_outputs(o, ht, q.size(0));
-    ctx->save_for_backward({in.q, in.k, in.v, in.beta, s.gam, s.x_inv, s.s_img, s.vn_img, s.p_img, in.q_rstd, in.k_rstd, s.geo.cu, s.geo.co});
+    ctx->save_for_backward({l2norm ? s.qn : in.q, l2norm ? s.kn : in.k, in.v, in.beta, s.gam, s.x_inv, s.s_img, s.vn_img, s.p_img, s.q_rstd,
+                            s.k_rstd, s.geo.cu, s.geo.co});
     auto& m = ctx->saved_data;
     m["geo"] = std::vector<int64_t>{s.geo.N, s.geo.max_len, s.geo.chunks};
     m["types"] = std::vector<int64_t>{int64_t(q.scalar_type()), int64_t(k.scalar_type()), int64_t(v.scalar_type()), int64_t(g.scalar_type()),
                                       int64_t(beta.scalar_type())};
     m["fold"] = in.folded ? q.size(0) : int64_t(0);
     m["o"] = o.sizes();
-    m["scale"] = scale, m["h0"] = h0.defined(), m["l2norm"] = l2norm;
+    m["scale"] = scale, m["h0"] = h0.defined();
     ctx->set_materialize_grads(false);
     if (want_final) return {o, ht};
     return {o};
@@ -144,9 +147,8 @@ struct GdnFn : torch::autograd::Function<GdnFn> {
     const variable_list sv = ctx->get_saved_variables();
     auto& m = ctx->saved_data;
     const std::vector<int64_t> geo = m["geo"].toIntVector(), ty = m["types"].toIntVector();
-    GdnSaved s{sv[4], sv[5], sv[6], sv[7], sv[8], Geometry{sv[11], sv[12], geo[0], geo[1], geo[2]}};
+    GdnSaved s{sv[4], sv[5], sv[6], sv[7], sv[8], Tensor(), Tensor(), sv[9], sv[10], Geometry{sv[11], sv[12], geo[0], geo[1], geo[2]}};
     const int64_t B = m["fold"].toInt();
-    const bool l2norm = m["l2norm"].toBool();
     Tensor d_o = grads[0].defined() ? grads[0] : at::zeros(m["o"].toIntVector(), sv[2].options());
     Tensor dht = grads.size() > 1 ? grads[1] : Tensor();
     if (B) {
@@ -154,15 +156,10 @@ struct GdnFn : torch::autograd::Function<GdnFn> {
       d_o = d_o.permute({1, 0, 2, 3}).reshape({1, T, -1, d_o.size(3)});      // a view when d_o has the strides of o
       if (dht.defined()) dht = dht.reshape({1, -1, dht.size(2), dht.size(3)});
     }
-    // gradients leave the kernels in the dtypes of their inputs; those of q and k stay fp32 when the normalisation follows
+    // gradients leave the kernels in the dtypes of their inputs
     auto kernel_type = [](int64_t t) { return at::ScalarType(t) == at::kBFloat16 ? at::kBFloat16 : at::kFloat; };
-    const GradTypes want{l2norm ? at::kFloat : kernel_type(ty[0]), l2norm ? at::kFloat : kernel_type(ty[1]), kernel_type(ty[2]), kernel_type(ty[3]),
-                         kernel_type(ty[4])};
+    const GradTypes want{kernel_type(ty[0]), kernel_type(ty[1]), kernel_type(ty[2]), kernel_type(ty[3]), kernel_type(ty[4])};
     auto r = gdn_bwd(sv[0], sv[1], sv[2], sv[3], s, d_o, dht, m["scale"].toDouble(), m["h0"].toBool(), want);
-    if (l2norm) {
-      r[0] = l2norm_bwd(sv[0], sv[9], r[0], 1e-6, std::nullopt);
-      r[1] = l2norm_bwd(sv[1], sv[10], r[1], 1e-6, std::nullopt);
-    }
     if (B) {
       for (int i = 0; i < 3; ++i) r[i] = r[i].view({r[i].size(1), B, -1, r[i].size(3)}).permute({1, 0, 2, 3});
       for (int i = 3; i < 5; ++i) r[i] = r[i].view({r[i].size(1), B, -1}).permute({1, 0, 2});
@@ -196,8 +193,8 @@ Pair gdn(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_,
     r = {l[0], l.size() > 1 ? l[1] : Tensor()};
   } else {
     Device(op)(q)(k)(v).get();
-    const GdnInputs in = gdn_inputs(q, k, v, g, beta, h0, cu, l2norm);
-    auto [o, ht, s] = gdn_fwd(in.q, in.k, in.v, in.g, in.beta, scale, in.h0, want_final, cu, false, inner);
+    const GdnInputs in = gdn_inputs(q, k, v, g, beta, h0, cu);
+    auto [o, ht, s] = gdn_fwd(in.q, in.k, in.v, in.g, in.beta, scale, in.h0, want_final, cu, false, inner, l2norm);
     r = in.folded ? unfold_outputs(o, ht, q.size(0)) : Pair{o, ht};
   }
   if (half) r.first = to_dtype(r.first, out.value_or(at::kHalf), op);

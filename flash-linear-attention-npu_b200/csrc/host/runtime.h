@@ -152,10 +152,11 @@ Pair recurrent_kda(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
 
 struct GdnSaved {
   Tensor gam, x_inv, s_img, vn_img, p_img;
+  Tensor qn, kn, q_rstd, k_rstd;      // normalised rows and their factors, when the operator normalises q and k
   Geometry geo;
 };
 std::tuple<Tensor, Tensor, GdnSaved> gdn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, double scale,
-                                             const Tensor& h0, bool want_final, const Tensor& cu, bool save, std::optional<at::ScalarType> out);
+                                             const Tensor& h0, bool want_final, const Tensor& cu, bool save, std::optional<at::ScalarType> out, bool l2norm = false);
 struct GradTypes {
   at::ScalarType q, k, v, g, beta;
 };
