@@ -86,6 +86,38 @@ __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 x
   *reinterpret_cast<uint2*>(p) = raw;
 }
 
+// one 16-byte piece of a state row <-> fp32
+template <typename T>
+__device__ __forceinline__ void load16(const T* p, float* f) {
+#pragma unroll
+  for (int i = 0; i < int(16 / sizeof(T)); i += 4) {
+    const float4 x = load4<T>(p + i);
+    f[i] = x.x; f[i + 1] = x.y; f[i + 2] = x.z; f[i + 3] = x.w;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void store16(T* p, const float* f) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+  } else {
+    uint4 raw;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    *reinterpret_cast<uint4*>(p) = raw;
+  }
+}
+template <>
+__device__ __forceinline__ void load16<__nv_bfloat16>(const __nv_bfloat16* p, float* f) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __low2float(h[i]);
+    f[2 * i + 1] = __high2float(h[i]);
+  }
+}
+
 // one activation element (q, k, v): bf16, or fp16 when f16
 __device__ __forceinline__ float load_act(const void* p, int64_t idx, int f16) {
   return f16 ? __half2float(static_cast<const __half*>(p)[idx]) : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[idx]);
@@ -94,35 +126,9 @@ __device__ __forceinline__ float load_scalar(const void* p, int64_t idx, int is_
   return is_f32 ? static_cast<const float*>(p)[idx] : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[idx]);
 }
 
-constexpr int kRecThreads = 256;
-
-// ROWS x COLS state tile held by one CTA (COLS contiguous in memory, LD elements between rows).  The columns of V
-// are independent recurrences, so a CTA owns VT of the V value channels: K-first ROWS = K, COLS = VT, LD = V;
-// V-first ROWS = VT, COLS = K, LD = K.
-template <int K, int V, int VT, typename ST, bool VFIRST>
-__global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(RecurrentParams p) {
-  constexpr int ROWS = VFIRST ? VT : K;
-  constexpr int COLS = VFIRST ? K : VT;
-  constexpr int LD = VFIRST ? K : V;
-  constexpr int NVB = V / VT;
-  constexpr int TPR = COLS / 4;              // threads per row
-  constexpr int RG = kRecThreads / TPR;      // row groups handled per pass
-  constexpr int R = ROWS / RG;               // rows per thread
-  static_assert(ROWS % RG == 0 && TPR <= 32, "unsupported head dims");
-
-  __shared__ float k_s[K], q_s[K], dk_s[K];
-  __shared__ __align__(16) float red[VFIRST ? 1 : RG][VFIRST ? 4 : COLS];
-  __shared__ float norm_s[2];
-
-  const int vb = blockIdx.x % NVB;
-  const int seq = (blockIdx.x / NVB) / p.HV, hv = (blockIdx.x / NVB) % p.HV;
-  const int v0 = vb * VT;                                   // first value channel of this CTA
-  const int64_t tile_off = VFIRST ? int64_t(v0) * LD : v0;  // offset of the tile inside the stored K x V (V x K) matrix
-  const int hk = hv / (p.HV / p.HK);
-  const int tid = threadIdx.x;
-  const int rg = tid / TPR, c0 = (tid % TPR) * 4;
-
-  int t0, t1;
+// Tokens [t0, t1) of sequence `seq` and the block its state starts from; false when there is nothing to do (no tokens, a padded
+// slot or a bad index: everything is left untouched).
+__device__ __forceinline__ bool sequence_of(const RecurrentParams& p, int seq, int tid, int& t0, int& t1, int& blk) {
   if (p.cu_seqlens && p.cu_is_lengths) {   // offsets from the lengths: every warp adds up the entries before its sequence
     int sum = 0;
     for (int i = tid % 32; i <= seq; i += 32) sum += p.cu_seqlens[i];
@@ -135,14 +141,59 @@ __global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(Recurrent
     t0 = seq * p.tokens_per_seq;
     t1 = t0 + p.tokens_per_seq;
   }
-  if (t1 <= t0) return;
-  int blk = seq;
+  if (t1 <= t0) return false;
+  blk = seq;
   if (p.state_indices) {
     int tok = t0;
     if (p.num_accepted_tokens) tok = t0 + p.num_accepted_tokens[seq] - 1;
     blk = p.state_indices[tok];
   }
-  if (blk < 0 || blk >= p.nblocks_in) return;  // padded slot or bad index: leave everything untouched
+  return blk >= 0 && blk < p.nblocks_in;
+}
+// Log decay of one key channel after the gate activation.
+template <int K>
+__device__ __forceinline__ float channel_gate(const RecurrentParams& p, float gate, int hv, int kc) {
+  if (p.gate_mode) {
+    const float eig = p.a_log ? __expf(p.a_log[hv]) : 1.f;
+    const float raw = gate + (p.dt_bias ? p.dt_bias[hv * K + kc] : 0.f);
+    if (p.gate_mode == 1) gate = -eig * (raw > 20.f ? raw : log1pf(__expf(raw)));
+    else gate = p.lower_bound / (1.f + __expf(-eig * raw));
+  }
+  return gate;
+}
+__device__ __forceinline__ void store_out(const RecurrentParams& p, int64_t off, float o) {
+  if (p.out_is_f32) static_cast<float*>(p.out)[off] = o;
+  else if (p.out_is_f16) static_cast<__half*>(p.out)[off] = __float2half_rn(o);
+  else static_cast<__nv_bfloat16*>(p.out)[off] = __float2bfloat16_rn(o);
+}
+
+constexpr int kRecThreads = 256;
+
+// K-first states ([K][V] in memory).  The columns of V are independent recurrences, so a CTA owns VT of the V value channels:
+// a thread keeps 4 channels of every RG-th key row.
+template <int K, int V, int VT, typename ST>
+__global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(RecurrentParams p) {
+  constexpr int ROWS = K, COLS = VT, LD = V;
+  constexpr int NVB = V / VT;
+  constexpr int TPR = COLS / 4;              // threads per row
+  constexpr int RG = kRecThreads / TPR;      // row groups handled per pass
+  constexpr int R = ROWS / RG;               // rows per thread
+  static_assert(ROWS % RG == 0 && TPR <= 32, "unsupported head dims");
+
+  __shared__ float k_s[K], q_s[K], dk_s[K];
+  __shared__ __align__(16) float red[RG][COLS];
+  __shared__ float norm_s[2];
+
+  const int vb = blockIdx.x % NVB;
+  const int seq = (blockIdx.x / NVB) / p.HV, hv = (blockIdx.x / NVB) % p.HV;
+  const int v0 = vb * VT;                                   // first value channel of this CTA
+  const int64_t tile_off = v0;                              // offset of the tile inside the stored K x V matrix
+  const int hk = hv / (p.HV / p.HK);
+  const int tid = threadIdx.x;
+  const int rg = tid / TPR, c0 = (tid % TPR) * 4;
+
+  int t0, t1, blk;
+  if (!sequence_of(p, seq, tid, t0, t1, blk)) return;
 
   float4 s[R];
   {
@@ -159,14 +210,7 @@ __global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(Recurrent
       q_s[tid - K] = load_act(p.q, t * p.q_stride_t + hk * p.q_stride_h + (tid - K), p.act_f16);
     }
     if (p.gk && tid < K) {   // per-channel decay of this token: exp(gate(gk))
-      float gate = load_scalar(p.gk, t * p.gk_stride_t + hv * p.gk_stride_h + tid, p.gk_is_f32);
-      if (p.gate_mode) {
-        const float eig = p.a_log ? __expf(p.a_log[hv]) : 1.f;
-        const float raw = gate + (p.dt_bias ? p.dt_bias[hv * K + tid] : 0.f);
-        if (p.gate_mode == 1) gate = -eig * (raw > 20.f ? raw : log1pf(__expf(raw)));
-        else gate = p.lower_bound / (1.f + __expf(-eig * raw));
-      }
-      dk_s[tid] = __expf(gate);
+      dk_s[tid] = __expf(channel_gate<K>(p, load_scalar(p.gk, t * p.gk_stride_t + hv * p.gk_stride_h + tid, p.gk_is_f32), hv, tid));
     }
     const float decay = p.g ? expf(load_scalar(p.g, t * p.g_stride_t + hv, p.g_is_f32)) : 1.f;
     float beta = p.beta ? load_scalar(p.beta, t * p.beta_stride_t + hv, p.beta_is_f32) : 1.f;
@@ -188,87 +232,55 @@ __global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(Recurrent
     }
 
     if (p.gk) {   // S <- diag(exp(gate)) S
-      if constexpr (!VFIRST) {
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-          const float d = dk_s[rg + i * RG];
-          s[i].x *= d; s[i].y *= d; s[i].z *= d; s[i].w *= d;
-        }
-      } else {
-        const float4 d = make_float4(dk_s[c0], dk_s[c0 + 1], dk_s[c0 + 2], dk_s[c0 + 3]);
-#pragma unroll
-        for (int i = 0; i < R; ++i) { s[i].x *= d.x; s[i].y *= d.y; s[i].z *= d.z; s[i].w *= d.w; }
-      }
-    }
-    if constexpr (!VFIRST) {
-      // rows are k, my 4 columns are v.  dot[v] = sum_k S[k][v] k[k]
-      float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < R; ++i) {
-        const float kk = k_s[rg + i * RG] * kscale;
-        part.x += s[i].x * kk; part.y += s[i].y * kk; part.z += s[i].z * kk; part.w += s[i].w * kk;
+        const float d = dk_s[rg + i * RG];
+        s[i].x *= d; s[i].y *= d; s[i].z *= d; s[i].w *= d;
       }
-      *reinterpret_cast<float4*>(&red[rg][c0]) = part;
-      __syncthreads();
-      float4 dot = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // rows are k, my 4 columns are v.  dot[v] = sum_k S[k][v] k[k]
+    float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const float kk = k_s[rg + i * RG] * kscale;
+      part.x += s[i].x * kk; part.y += s[i].y * kk; part.z += s[i].z * kk; part.w += s[i].w * kk;
+    }
+    *reinterpret_cast<float4*>(&red[rg][c0]) = part;
+    __syncthreads();
+    float4 dot = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < RG; ++r) {
+      const float4 x = *reinterpret_cast<const float4*>(&red[r][c0]);
+      dot.x += x.x; dot.y += x.y; dot.z += x.z; dot.w += x.w;
+    }
+    const int64_t voff = t * p.v_stride_t + hv * p.v_stride_h + v0 + c0;
+    const float4 vv = p.act_f16 ? load4<__half>(static_cast<const __half*>(p.v) + voff)
+                                : load4<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.v) + voff);
+    float4 d;
+    d.x = beta * (vv.x - decay * dot.x); d.y = beta * (vv.y - decay * dot.y);
+    d.z = beta * (vv.z - decay * dot.z); d.w = beta * (vv.w - decay * dot.w);
+    float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const float kk = k_s[rg + i * RG] * kscale, qq = q_s[rg + i * RG] * qscale;
+      s[i].x = decay * s[i].x + kk * d.x; s[i].y = decay * s[i].y + kk * d.y;
+      s[i].z = decay * s[i].z + kk * d.z; s[i].w = decay * s[i].w + kk * d.w;
+      po.x += s[i].x * qq; po.y += s[i].y * qq; po.z += s[i].z * qq; po.w += s[i].w * qq;
+    }
+    __syncthreads();  // everyone has consumed red[] for the dot
+    *reinterpret_cast<float4*>(&red[rg][c0]) = po;
+    __syncthreads();
+    if (rg == 0) {
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int r = 0; r < RG; ++r) {
         const float4 x = *reinterpret_cast<const float4*>(&red[r][c0]);
-        dot.x += x.x; dot.y += x.y; dot.z += x.z; dot.w += x.w;
+        o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
       }
-      const int64_t voff = t * p.v_stride_t + hv * p.v_stride_h + v0 + c0;
-      const float4 vv = p.act_f16 ? load4<__half>(static_cast<const __half*>(p.v) + voff)
-                                  : load4<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.v) + voff);
-      float4 d;
-      d.x = beta * (vv.x - decay * dot.x); d.y = beta * (vv.y - decay * dot.y);
-      d.z = beta * (vv.z - decay * dot.z); d.w = beta * (vv.w - decay * dot.w);
-      float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const float kk = k_s[rg + i * RG] * kscale, qq = q_s[rg + i * RG] * qscale;
-        s[i].x = decay * s[i].x + kk * d.x; s[i].y = decay * s[i].y + kk * d.y;
-        s[i].z = decay * s[i].z + kk * d.z; s[i].w = decay * s[i].w + kk * d.w;
-        po.x += s[i].x * qq; po.y += s[i].y * qq; po.z += s[i].z * qq; po.w += s[i].w * qq;
-      }
-      __syncthreads();  // everyone has consumed red[] for the dot
-      *reinterpret_cast<float4*>(&red[rg][c0]) = po;
-      __syncthreads();
-      if (rg == 0) {
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int r = 0; r < RG; ++r) {
-          const float4 x = *reinterpret_cast<const float4*>(&red[r][c0]);
-          o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
-        }
-        const int64_t off = t * p.out_stride_t + hv * p.out_stride_h + v0 + c0;
-        if (p.out_is_f32) store4<float>(static_cast<float*>(p.out) + off, o);
-        else if (p.out_is_f16) store4<__half>(static_cast<__half*>(p.out) + off, o);
-        else store4<__nv_bfloat16>(static_cast<__nv_bfloat16*>(p.out) + off, o);
-      }
-    } else {
-      // rows are v, my 4 columns are k.  Each row is reduced across the TPR lanes that share it.
-      const float4 kk = make_float4(k_s[c0] * kscale, k_s[c0 + 1] * kscale, k_s[c0 + 2] * kscale, k_s[c0 + 3] * kscale);
-      const float4 qq = make_float4(q_s[c0] * qscale, q_s[c0 + 1] * qscale, q_s[c0 + 2] * qscale, q_s[c0 + 3] * qscale);
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const int row = v0 + rg + i * RG;
-        float dot = s[i].x * kk.x + s[i].y * kk.y + s[i].z * kk.z + s[i].w * kk.w;
-#pragma unroll
-        for (int o = TPR / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        const float vv = load_act(p.v, t * p.v_stride_t + hv * p.v_stride_h + row, p.act_f16);
-        const float d = beta * (vv - decay * dot);
-        s[i].x = decay * s[i].x + d * kk.x; s[i].y = decay * s[i].y + d * kk.y;
-        s[i].z = decay * s[i].z + d * kk.z; s[i].w = decay * s[i].w + d * kk.w;
-        float o = s[i].x * qq.x + s[i].y * qq.y + s[i].z * qq.z + s[i].w * qq.w;
-#pragma unroll
-        for (int sft = TPR / 2; sft > 0; sft >>= 1) o += __shfl_xor_sync(0xffffffffu, o, sft);
-        if (tid % TPR == 0) {
-          const int64_t off = t * p.out_stride_t + hv * p.out_stride_h + row;
-          if (p.out_is_f32) static_cast<float*>(p.out)[off] = o;
-          else if (p.out_is_f16) static_cast<__half*>(p.out)[off] = __float2half_rn(o);
-          else static_cast<__nv_bfloat16*>(p.out)[off] = __float2bfloat16_rn(o);
-        }
-      }
+      const int64_t off = t * p.out_stride_t + hv * p.out_stride_h + v0 + c0;
+      if (p.out_is_f32) store4<float>(static_cast<float*>(p.out) + off, o);
+      else if (p.out_is_f16) store4<__half>(static_cast<__half*>(p.out) + off, o);
+      else store4<__nv_bfloat16>(static_cast<__nv_bfloat16*>(p.out) + off, o);
     }
 
     const bool last = (t == t1 - 1);
@@ -283,17 +295,143 @@ __global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(Recurrent
   }
 }
 
+// V-first states ([V][K] in memory; the state-pool operators).  Four lanes share a value row (K / 4 key channels each, in 16-byte
+// pieces dealt out in turn so that the four lanes read 64 contiguous bytes), so the two dot products of a token take two
+// shuffles each, for VT / 64 rows per thread.  A whole warp per row, which the 4-channel layout of the K-first kernel would
+// give, spent ten shuffles and a dependent global load of v on each of sixteen rows: 36.7 us for 24 sequences x 16 heads with one
+// to four draft tokens (bf16 pool) against the 7 us its bytes take.  The next token's q, k, v are requested before the current one is worked on
+// (q, k, v are double-buffered: one barrier per token, two with the normalisation).
+template <int K, int V, int VT, typename ST>
+__global__ void __launch_bounds__(kRecThreads, 2) recurrent_gdn_vfirst_kernel(RecurrentParams p) {
+  constexpr int NVB = V / VT;
+  constexpr int E = 16 / sizeof(ST);               // channels per 16-byte piece
+  constexpr int P = K / (4 * E);                   // pieces per lane
+  constexpr int R = VT / 64;                       // rows per thread
+  static_assert(VT % 64 == 0 && K % (4 * E) == 0 && 2 * K <= kRecThreads && VT <= kRecThreads, "unsupported head dims");
+  __shared__ __align__(16) float k_s[2][K], q_s[2][K], dk_s[2][K];
+  __shared__ float v_s[2][VT], norm_s[2][2];
+
+  const int tid = threadIdx.x, lane4 = tid & 3, row = tid >> 2;
+  const int vb = blockIdx.x % NVB, seq = (blockIdx.x / NVB) / p.HV, hv = (blockIdx.x / NVB) % p.HV;
+  const int v0 = vb * VT, hk = hv / (p.HV / p.HK);
+  int t0, t1, blk;
+  if (!sequence_of(p, seq, tid, t0, t1, blk)) return;
+
+  float s[R][P * E];
+  {
+    const ST* src = static_cast<const ST*>(p.state_in) + blk * p.state_in_stride_b + hv * p.state_in_stride_h + int64_t(v0) * K;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int j = 0; j < P; ++j) load16<ST>(src + (row + r * 64) * K + (j * 4 + lane4) * E, &s[r][j * E]);
+  }
+  float pqk = 0.f, pv = 0.f, pg = 0.f, pdecay = 0.f, pbeta = 1.f;     // the next token's elements
+  auto request = [&](int t) {
+    if (tid < K) pqk = load_act(p.k, t * p.k_stride_t + hk * p.k_stride_h + tid, p.act_f16);
+    else if (tid < 2 * K) pqk = load_act(p.q, t * p.q_stride_t + hk * p.q_stride_h + (tid - K), p.act_f16);
+    if (tid < VT) pv = load_act(p.v, t * p.v_stride_t + hv * p.v_stride_h + v0 + tid, p.act_f16);
+    if (p.gk && tid < K) pg = load_scalar(p.gk, t * p.gk_stride_t + hv * p.gk_stride_h + tid, p.gk_is_f32);
+    if (p.g) pdecay = load_scalar(p.g, t * p.g_stride_t + hv, p.g_is_f32);
+    if (p.beta) pbeta = load_scalar(p.beta, t * p.beta_stride_t + hv, p.beta_is_f32);
+  };
+  request(t0);
+  for (int t = t0; t < t1; ++t) {
+    const int b = (t - t0) & 1;
+    if (tid < K) k_s[b][tid] = pqk;
+    else if (tid < 2 * K) q_s[b][tid - K] = pqk;
+    if (tid < VT) v_s[b][tid] = pv;
+    if (p.gk && tid < K) dk_s[b][tid] = __expf(channel_gate<K>(p, pg, hv, tid));
+    const float decay = p.g ? expf(pdecay) : 1.f;
+    const float beta = p.beta_mode ? float(p.beta_mode) / (1.f + __expf(-pbeta)) : pbeta;
+    if (t + 1 < t1) request(t + 1);
+    __syncthreads();
+    float kscale = 1.f, qscale = p.scale;
+    if (p.l2norm) {
+      if (tid < 64) {  // warp 0: |k|^2, warp 1: |q|^2
+        const float* src = tid < 32 ? k_s[b] : q_s[b];
+        float acc = 0.f;
+        for (int i = tid % 32; i < K; i += 32) acc += src[i] * src[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (tid % 32 == 0) norm_s[b][tid / 32] = rsqrtf(acc + 1e-6f);
+      }
+      __syncthreads();
+      kscale = norm_s[b][0];
+      qscale = p.scale * norm_s[b][1];
+    }
+    float dot[R], o[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) dot[r] = o[r] = 0.f;
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+#pragma unroll
+      for (int e4 = 0; e4 < E; e4 += 4) {
+        const int c = (j * 4 + lane4) * E + e4;
+        const float4 kk = *reinterpret_cast<const float4*>(&k_s[b][c]);
+        if (p.gk) {      // S <- diag(exp(gate)) S
+          const float4 d = *reinterpret_cast<const float4*>(&dk_s[b][c]);
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            float* x = &s[r][j * E + e4];
+            x[0] *= d.x; x[1] *= d.y; x[2] *= d.z; x[3] *= d.w;
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float* x = &s[r][j * E + e4];
+          dot[r] += x[0] * kk.x + x[1] * kk.y + x[2] * kk.z + x[3] * kk.w;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 1);
+      dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 2);
+      dot[r] = beta * (v_s[b][row + r * 64] - decay * dot[r] * kscale) * kscale;     // d, times the factor of k
+    }
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+#pragma unroll
+      for (int e4 = 0; e4 < E; e4 += 4) {
+        const int c = (j * 4 + lane4) * E + e4;
+        const float4 kk = *reinterpret_cast<const float4*>(&k_s[b][c]), qq = *reinterpret_cast<const float4*>(&q_s[b][c]);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float* x = &s[r][j * E + e4];
+          x[0] = decay * x[0] + dot[r] * kk.x; x[1] = decay * x[1] + dot[r] * kk.y;
+          x[2] = decay * x[2] + dot[r] * kk.z; x[3] = decay * x[3] + dot[r] * kk.w;
+          o[r] += x[0] * qq.x + x[1] * qq.y + x[2] * qq.z + x[3] * qq.w;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      o[r] += __shfl_xor_sync(0xffffffffu, o[r], 1);
+      o[r] += __shfl_xor_sync(0xffffffffu, o[r], 2);
+      if (lane4 == 0) store_out(p, t * p.out_stride_t + hv * p.out_stride_h + v0 + row + r * 64, o[r] * qscale);
+    }
+    const int wblk = p.state_indices ? p.state_indices[t] : (t == t1 - 1 ? seq : -1);
+    if (wblk >= 0 && wblk < p.nblocks_out) {
+      ST* dst = static_cast<ST*>(p.state_out) + wblk * p.state_out_stride_b + hv * p.state_out_stride_h + int64_t(v0) * K;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < P; ++j) store16<ST>(dst + (row + r * 64) * K + (j * 4 + lane4) * E, &s[r][j * E]);
+    }
+  }
+}
+
 template <int K, int V>
 int launch_recurrent(const RecurrentParams& p, int nseq, bool state_f32, bool vfirst, cudaStream_t st) {
   constexpr int VT = V > 128 ? 128 : V;
   const dim3 grid(nseq * p.HV * (V / VT)), block(kRecThreads);
   KernelTimer kt("recurrent_gdn", st);
   if (state_f32) {
-    if (vfirst) recurrent_gdn_kernel<K, V, VT, float, true><<<grid, block, 0, st>>>(p);
-    else recurrent_gdn_kernel<K, V, VT, float, false><<<grid, block, 0, st>>>(p);
+    if (vfirst) recurrent_gdn_vfirst_kernel<K, V, VT, float><<<grid, block, 0, st>>>(p);
+    else recurrent_gdn_kernel<K, V, VT, float><<<grid, block, 0, st>>>(p);
   } else {
-    if (vfirst) recurrent_gdn_kernel<K, V, VT, __nv_bfloat16, true><<<grid, block, 0, st>>>(p);
-    else recurrent_gdn_kernel<K, V, VT, __nv_bfloat16, false><<<grid, block, 0, st>>>(p);
+    if (vfirst) recurrent_gdn_vfirst_kernel<K, V, VT, __nv_bfloat16><<<grid, block, 0, st>>>(p);
+    else recurrent_gdn_kernel<K, V, VT, __nv_bfloat16><<<grid, block, 0, st>>>(p);
   }
   return cuda_status(cudaGetLastError());
 }

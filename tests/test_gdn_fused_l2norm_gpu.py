@@ -31,6 +31,8 @@ def test_fused_normalisation_matches_separate_passes(T, HK, HV):
     dq, dk, dv, dg, db = torch.autograd.grad(o2, [q2, k2, v2, g2, b2], do)
     assert torch.equal(o1, o2) and torch.equal(got[1], dv)
     want = torch.cat([l2norm_bwd(n, r, d).flatten(-2) for n, r, d in ((qn, qr, dq), (kn, kr, dk))], dim=-1)
-    assert_close("d(q, k)", got[0], want, 2e-2)   # bf16 results: the separate pass also rounds dq, dk to bf16 in between
+    # bf16 results, and the separate pass also rounds dq, dk to bf16 in between: some ulps at single elements, little over all
+    assert_close("d(q, k)", got[0], want, 8e-2)
+    assert (got[0].float() - want.float()).norm() <= 5e-3 * want.float().norm()
     assert_close("dg", got[2], dg, 1e-5)
     assert_close("dbeta", got[3].float(), db.float(), 1e-5)
