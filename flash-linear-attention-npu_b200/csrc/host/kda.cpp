@@ -23,6 +23,10 @@ KdaResult kda_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   a.aqk = desc(aqk), a.akk = desc(akk);
   a.scale = float(o.scale), a.lower_bound = float(o.lower_bound), a.gate_mode = int32_t(o.gate_mode);
   a.chunk_size = kChunk, a.max_seqlen = int32_t(geo.max_len), a.total_chunks = int32_t(geo.chunks);
+  if (o.l2norm) {
+    r.q_rstd = empty({B, T, q.size(2)}, at::kFloat, d), r.k_rstd = empty({B, T, q.size(2)}, at::kFloat, d);
+    a.q_rstd = desc(r.q_rstd), a.k_rstd = desc(r.k_rstd);
+  }
   if (o.keep) {      // the reference's disable_recompute=True: keep the intermediates for the backward instead of recomputing them
     uint64_t bytes = 0;
     ok_or_throw("kda_chunk_saved_size", lib.kda_chunk_saved_size(&a, &bytes));
@@ -34,7 +38,8 @@ KdaResult kda_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
 }
 
 std::vector<Tensor> kda_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, double scale, const Tensor& h0,
-                            const Tensor& do_in, const Tensor& dht_in, const Geometry& geo, GradTypes ty, const Tensor& saved) {
+                            const Tensor& do_in, const Tensor& dht_in, const Geometry& geo, GradTypes ty, const Tensor& saved,
+                            const Tensor& q_rstd, const Tensor& k_rstd) {
   const int64_t B = q.size(0), T = q.size(1), HK = q.size(2), K = q.size(3), HV = v.size(2), V = v.size(3);
   const at::Device d = Device("kda_chunk_bwd")(q)(k)(v)(g)(beta)(h0)(do_in)(dht_in)(saved).get();
   const Tensor d_o = as_rows(do_in.scalar_type() == at::kBFloat16 ? do_in : convert(do_in, at::kBFloat16, "chunk_kda_bwd"));
@@ -47,6 +52,7 @@ std::vector<Tensor> kda_bwd(const Tensor& q, const Tensor& k, const Tensor& v, c
   a.initial_state = desc(h0), a.d_o = desc(d_o), a.dht = desc(dht);
   a.dq = desc(dq), a.dk = desc(dk), a.dv = desc(dv), a.dg = desc(dg), a.dbeta = desc(dbeta), a.dh0 = desc(dh0);
   a.cu_seqlens = desc(geo.cu), a.chunk_offsets = desc(geo.co), a.saved = desc(saved);
+  a.q_rstd = desc(q_rstd), a.k_rstd = desc(k_rstd);
   a.scale = float(scale), a.chunk_size = kChunk, a.max_seqlen = int32_t(geo.max_len), a.total_chunks = int32_t(geo.chunks);
   two_phase("kda_chunk_bwd", lib.kda_chunk_bwd_workspace_size, lib.kda_chunk_bwd, a, d, true);
   return {dq, dk, dv, dg, dbeta, dh0};
@@ -54,23 +60,18 @@ std::vector<Tensor> kda_bwd(const Tensor& q, const Tensor& k, const Tensor& v, c
 
 // Saves the inputs, and the forward's operand images when they are kept; otherwise the backward recomputes them.
 struct KdaFn : torch::autograd::Function<KdaFn> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& q_, const Tensor& k_, const Tensor& v, const Tensor& g, const Tensor& beta,
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta,
                                const OptTensor& h0_, const OptTensor& cu_, const OptTensor& co_, std::vector<int64_t> geo, double scale, bool want_final,
                                int64_t out, bool keep, bool l2norm) {
     const Tensor h0 = value(h0_), cu = value(cu_), co = value(co_);
-    Tensor q = q_, k = k_, q_rstd, k_rstd;
-    if (l2norm) {
-      std::tie(q, q_rstd) = l2norm_fwd(q_, 1e-6, std::nullopt);
-      std::tie(k, k_rstd) = l2norm_fwd(k_, 1e-6, std::nullopt);
-    }
     KdaOptions o;
-    o.scale = scale, o.want_final = want_final, o.keep = keep;
+    o.scale = scale, o.want_final = want_final, o.keep = keep, o.l2norm = l2norm;
     if (out >= 0) o.out = at::ScalarType(out);
     KdaResult r = kda_fwd(q, k, v, g, beta, h0, Tensor(), Tensor(), Geometry{cu, co, geo[0], geo[1], geo[2]}, o, Tensor(), Tensor());
-    ctx->save_for_backward({q, k, v, g, beta, h0, r.saved, q_rstd, k_rstd, cu, co});
+    ctx->save_for_backward({q, k, v, g, beta, h0, r.saved, r.q_rstd, r.k_rstd, cu, co});
     auto& m = ctx->saved_data;
     m["geo"] = geo;
-    m["scale"] = scale, m["l2norm"] = l2norm;
+    m["scale"] = scale;
     ctx->set_materialize_grads(false);
     if (want_final) return {r.o, r.ht};
     return {r.o};
@@ -79,17 +80,11 @@ struct KdaFn : torch::autograd::Function<KdaFn> {
     const variable_list s = ctx->get_saved_variables();
     auto& m = ctx->saved_data;
     const std::vector<int64_t> geo = m["geo"].toIntVector();
-    const bool l2norm = m["l2norm"].toBool();
     const Tensor d_o = grads[0].defined() ? grads[0].contiguous() : at::zeros(s[2].sizes(), s[2].options());
     auto kernel_type = [](const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kFloat; };
-    const GradTypes want{l2norm ? at::kFloat : kernel_type(s[0]), l2norm ? at::kFloat : kernel_type(s[1]), kernel_type(s[2]), kernel_type(s[3]),
-                         kernel_type(s[4])};
+    const GradTypes want{kernel_type(s[0]), kernel_type(s[1]), kernel_type(s[2]), kernel_type(s[3]), kernel_type(s[4])};
     auto r = kda_bwd(s[0], s[1], s[2], s[3], s[4], m["scale"].toDouble(), s[5], d_o, grads.size() > 1 ? grads[1] : Tensor(),
-                     Geometry{s[9], s[10], geo[0], geo[1], geo[2]}, want, s[6]);
-    if (l2norm) {
-      r[0] = l2norm_bwd(s[0], s[7], r[0], 1e-6, std::nullopt);
-      r[1] = l2norm_bwd(s[1], s[8], r[1], 1e-6, std::nullopt);
-    }
+                     Geometry{s[9], s[10], geo[0], geo[1], geo[2]}, want, s[6], s[7], s[8]);
     for (int i = 0; i < 5; ++i) r[i] = r[i].to(s[i].scalar_type());
     variable_list out(14);
     for (int i = 0; i < 6; ++i) out[i] = r[i];
@@ -143,7 +138,10 @@ KdaCall kda(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& 
     c.r.o = l[0];
     if (l.size() > 1) c.r.ht = l[1];
   } else {
-    if (o.l2norm) q = l2norm_fwd(q, 1e-6, std::nullopt).first, k = l2norm_fwd(k, 1e-6, std::nullopt).first;
+    if (o.l2norm && return_saved) {      // the export pass behind it reads the normalised rows
+      q = l2norm_fwd(q, 1e-6, std::nullopt).first, k = l2norm_fwd(k, 1e-6, std::nullopt).first;
+      o.l2norm = false;
+    }
     Tensor a_log, dt_bias;
     if (o.gate_mode) {
       a_log = a_log_.to(at::kFloat).contiguous();

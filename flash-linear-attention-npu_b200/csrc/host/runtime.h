@@ -172,12 +172,13 @@ struct KdaOptions {
   std::optional<at::ScalarType> out;
 };
 struct KdaResult {
-  Tensor o, ht, gk, saved;
+  Tensor o, ht, gk, saved, q_rstd, k_rstd;
 };
 KdaResult kda_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& h0, const Tensor& a_log,
                   const Tensor& dt_bias, const Geometry& geo, const KdaOptions& o, const Tensor& aqk, const Tensor& akk);
 std::vector<Tensor> kda_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, double scale, const Tensor& h0,
-                            const Tensor& d_o, const Tensor& dht, const Geometry& geo, GradTypes types, const Tensor& saved);
+                            const Tensor& d_o, const Tensor& dht, const Geometry& geo, GradTypes types, const Tensor& saved,
+                            const Tensor& q_rstd = Tensor(), const Tensor& k_rstd = Tensor());
 struct KdaCall {
   KdaResult r;
   Geometry geo;

@@ -31,6 +31,9 @@ namespace fla {
 
 struct KdaBwdParams {
   const bf16* v; const bf16* dO; const void* beta;
+  const bf16* q; const bf16* k;               // raw rows, read only when dq / dk go through the normalisation:
+  const float* q_rstd; const float* k_rstd;   // [tokens, HK] or null
+  int64_t q_st, q_sh, k_st, k_sh;
   const bf16* qk_img; const bf16* kn_img; const bf16* p_img; const bf16* x_img;
   const float* vec; const float* gk;
   const bf16* s_img; const bf16* vn_img;
@@ -399,7 +402,9 @@ __device__ __forceinline__ float warp_column_sums32(const float* v, int lane) {
 
 // The chunk's gk rows arrive as TMA tiles once the phase-1 buffers are free; the last epilogue reads them from
 // shared memory (their global loads used to sit, one round trip each, on the critical path).
-template <int NVB>   // 64-column blocks of V per head (2 or 4): a compile-time trip count keeps the block loop unrolled
+// NVB: 64-column blocks of V per head (2 or 4), a compile-time trip count that keeps the block loop unrolled.  NORM: dq, dk go through
+// the q/k normalisation at the end (a kernel of its own: the epilogue's registers would spill in the other: 2.24 -> 2.5 ms).
+template <int NVB, bool NORM>
 __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, const __grid_constant__ CUtensorMap tm_gk) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -407,6 +412,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
   __shared__ float red[2][2][kC];      // rkG, ma : [half][row]
   __shared__ float sds_s[2][kK];       // sum_v dS'a * Sa per key channel, by column half
   __shared__ float colsum_s[2][kK];    // per 32-row part: column sums of the dgk tiles
+  __shared__ float ndot_s[NORM ? 2 : 1][2 * kC];  // q.dq / k.dk of the complete rows, per half of the columns (normalised q, k only)
   __shared__ float t1col_s[2][kK];     // per 32-row quadrant: sum_i Kn_i (Vn dS'a^T)_i of the last-row term
   __shared__ uint32_t tmem_base_s;
   __shared__ __align__(8) uint64_t mma_bar, load_bar, img_bar, gk_bar;
@@ -742,6 +748,36 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
     __syncthreads();
   }
 
+  if constexpr (NORM) {   // the rows are complete: rstd (dx - x (x . dx)) with x the normalised row, made again from the raw one
+    const int64_t r = tok0 + min(tok, rows - 1);
+    const float rs = (kside ? p.k_rstd : p.q_rstd)[r * p.HK + hk];
+    const bf16* src = kside ? p.k + r * p.k_st + hk * p.k_sh : p.q + r * p.q_st + hk * p.q_sh;
+    uint4 raw[8];
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch) raw[ch] = *reinterpret_cast<const uint4*>(src + half * 64 + ch * 8);
+    float t = 0.f;
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch) {
+      float f[8];
+      unpack_bf16x8(raw[ch], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rs;
+      raw[ch] = pack8(f);
+      unpack_bf16x8(raw[ch], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) t += f[j] * acc_out[ch * 8 + j];
+    }
+    ndot_s[half][row] = t;
+    __syncthreads();
+    t = ndot_s[0][row] + ndot_s[1][row];
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch) {
+      float f[8];
+      unpack_bf16x8(raw[ch], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc_out[ch * 8 + j] = (acc_out[ch * 8 + j] - t * f[j]) * rs;
+    }
+  }
   if (ok && tok < rows) {
     void* base = kside ? p.dk : p.dq;
     const int64_t off = kside ? (tok0 + tok) * p.dk_st + hk * p.dk_sh + half * 64 : (tok0 + tok) * p.dq_st + hk * p.dq_sh + half * 64;
@@ -853,6 +889,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
     if (s->stride[3] != 1 || s->stride[2] != V || s->stride[1] != kK * V || s->stride[0] != HV * kK * V || !aligned16(s->data))
       return FLA_ERR_LAYOUT;
   }
+  if ((st = kda_check_rstd(a->q_rstd, a->k_rstd, B, T, HK))) return st;
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
   uint64_t off[3], off_saved, so[4], fo[6];
   const bool have_saved = a->saved.data != nullptr;
@@ -885,8 +922,11 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   f.N = N; f.T = int(T); f.HK = int(HK); f.HV = int(HV); f.total_tokens = B * T; f.V = int(V); f.nvb = int(nvb);
   f.g_is_f32 = a->g.dtype == FLA_F32; f.beta_is_f32 = a->beta.dtype == FLA_F32;
   f.gate_mode = 0; f.scale = a->scale;
+  f.q_rstd = static_cast<float*>(a->q_rstd.data); f.k_rstd = static_cast<float*>(a->k_rstd.data);   // (written again by the recomputed forward)
 
   KdaBwdParams p{};
+  p.q = f.q; p.k = f.k; p.q_rstd = f.q_rstd; p.k_rstd = f.k_rstd;
+  p.q_st = f.q_st; p.q_sh = f.q_sh; p.k_st = f.k_st; p.k_sh = f.k_sh;
   p.v = f.v; p.dO = static_cast<const bf16*>(a->d_o.data); p.beta = a->beta.data;
   p.qk_img = f.qk_img; p.kn_img = f.kn_img; p.p_img = f.p_img; p.x_img = f.x_img; p.vec = f.vec; p.gk = f.gk_out;
   p.s_img = f.s_img; p.vn_img = f.vn_img;
@@ -915,8 +955,8 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
   if (!attr_done_dev[dev]) {
     if (cudaFuncSetAttribute(kda_bwd_dhu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaDhuSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
-    if (cudaFuncSetAttribute(kda_bwd_par_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaParSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
-    if (cudaFuncSetAttribute(kda_bwd_par_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaParSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
+    for (auto* par : {kda_bwd_par_kernel<2, false>, kda_bwd_par_kernel<4, false>, kda_bwd_par_kernel<2, true>, kda_bwd_par_kernel<4, true>})
+      if (cudaFuncSetAttribute(par, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaParSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     attr_done_dev[dev] = true;
   }
   CUtensorMap tm_gk;
@@ -925,8 +965,9 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
     kda_bwd_dhu_kernel<<<dim3(unsigned(nvb), unsigned(HV), nseq), 256, kKdaDhuSmem + 1024, st_>>>(pp);
   };
   auto launch_par = [&](const KdaBwdParams& pp, int nseq, cudaStream_t st_) {
-    if (nvb == 2) kda_bwd_par_kernel<2><<<dim3(nt_max, unsigned(HK), nseq), 256, kKdaParSmem + 1024, st_>>>(pp, tm_gk);
-    else kda_bwd_par_kernel<4><<<dim3(nt_max, unsigned(HK), nseq), 256, kKdaParSmem + 1024, st_>>>(pp, tm_gk);
+    auto* par = nvb == 2 ? (pp.q_rstd ? kda_bwd_par_kernel<2, true> : kda_bwd_par_kernel<2, false>)
+                         : (pp.q_rstd ? kda_bwd_par_kernel<4, true> : kda_bwd_par_kernel<4, false>);
+    par<<<dim3(nt_max, unsigned(HK), nseq), 256, kKdaParSmem + 1024, st_>>>(pp, tm_gk);
   };
   // more scan chains (one CTA per SM each) than SMs: two halves of the batch on two streams, so that the chunk-parallel
   // kernel of the first half fills the SMs the second half's scan leaves idle (aux_stream.h)

@@ -1,12 +1,14 @@
 // Parameter block and image sizes shared by the KDA chunk forward and backward translation units.
 #pragma once
 #include "gdn_common.cuh"
+#include "fla_b200_internal.h"
 
 namespace fla {
 
 struct KdaParams {
   const bf16* q; const bf16* k; const bf16* v;
   const void* g; const void* beta;
+  float* q_rstd; float* k_rstd;   // [tokens, HK] optional out: when given, the prep kernel normalises the rows of q and k first
   const float* a_log; const float* dt_bias;   // optional gate parameters: [HV], [HV, K]
   float* gk_out;        // [tokens, HV, K] cumulative gate (optional)
   bf16* qk_img;         // [chunks, HV, {hi, lo}, 2 panels x 128 rows]  rows 0-63 Qp, rows 64-127 Kp
@@ -37,6 +39,8 @@ uint64_t kda_ws_layout(int64_t total_chunks, int64_t HV, uint64_t off[6]);
 // Layout of the buffer a training forward leaves for the backward: the forward workspace (operand images), gk, the
 // Sa images and the v_new images; returns the total size.
 uint64_t kda_saved_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, uint64_t off[4]);
+// q_rstd, k_rstd of an argument block: both absent, or both dense [B, T, HK] f32; an FLA_ERR_* status otherwise.
+int kda_check_rstd(const fla_tensor_t& q, const fla_tensor_t& k, int64_t B, int64_t T, int64_t HK);
 // prep -> inverse -> forward scan on `stream`; 0 or an FLA_ERR_* status.
 int kda_launch_forward(const KdaParams& p, int nt_max, cudaStream_t stream);
 

@@ -314,6 +314,8 @@ typedef struct fla_kda_chunk_fwd_args {
   fla_tensor_t q, k, v, g, beta, a_log, dt_bias, initial_state;
   fla_tensor_t o, final_state, gk;
   fla_tensor_t cu_seqlens, chunk_offsets;
+  fla_tensor_t q_rstd, k_rstd;   /* optional out (both or none) [B, T, HK] f32 dense: when given, the rows of q and k are normalised first,
+                                    x * rsqrt(sum x^2 + 1e-6) rounded to bf16 (use_qk_l2norm_in_kernel), and their factors left here */
   fla_tensor_t saved;   /* optional out, 1-D bf16 of fla_b200_kda_chunk_saved_size bytes: what the backward otherwise recomputes */
   fla_tensor_t aqk, akk; /* optional out [B, T, HV, 64] bf16|f32 (any strides, e.g. head-first views): the per-chunk blocks
                             scale tril(q k^T 2^{gk_i-gk_j}) and (I + beta strict(k k^T 2^{gk_i-gk_j}))^-1 that npu_chunk_kda_fwd returns */
@@ -423,6 +425,8 @@ typedef struct fla_kda_chunk_bwd_args {
   fla_tensor_t d_o, dht;
   fla_tensor_t dq, dk, dv, dg, dbeta, dh0;
   fla_tensor_t cu_seqlens, chunk_offsets;
+  fla_tensor_t q_rstd, k_rstd;   /* optional (both or none): the factors the forward left; q, k are the rows before the normalisation
+                                    and dq, dk their gradients */
   fla_tensor_t saved;   /* optional in: the buffer the forward filled; skips the internal recomputation */
   float scale;
   int32_t chunk_size;
