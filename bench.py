@@ -64,7 +64,6 @@ KERNEL_FLOPS = {
     "kda_bwd_dhu": 131072.0,   # Kn dS'a, P^T dO, X^T dVn, [Qp^T|Kp^T][dO~; dR]
     "kda_bwd_par": 229376.0,   # [Qp;Kp]Kn^T, [dO;dZ]Vn^T, [dO;dZ]Sa^T, Vn dS'a^T, [dP;dM]Kn, [dP^T|dM^T][Qp;Kp]
     "gdn_prep": 16384.0,
-    "tri_inverse": 8192.0,     # 2 * 64^2 FLOP per token-head of the triangular solve (CUDA cores; shown against the tensor peak)
 }
 # Algorithmic HBM bytes of the stand-alone stages: every input read once, every output written once
 # (bf16 token tensors, fp32 A and gates, bf16 per-chunk states).
@@ -91,7 +90,7 @@ STAGE_BYTES = {
     "prepare_wy_repr_bwd_group_sum": lambda c: _th(c, "HV", 128, 4) + _th(c, "HK", 128, 2),
 }
 KERNEL_SYMBOL = {"gdn_fwd": "gdn_scan_fwd_kernel", "gdn_bwd_dhu": "gdn_scan_bwd_kernel", "gdn_bwd_par": "gdn_bwd_par_kernel",
-                 "kda_fwd": "kda_fwd_kernel", "kda_prep": "kda_prep_kernel", "kda_bwd_dhu": "kda_bwd_dhu_kernel", "kda_bwd_par": "kda_bwd_par_kernel", "gdn_prep": "gdn_prep_kernel", "tri_inverse": "tri_inverse_kernel",
+                 "kda_fwd": "kda_fwd_kernel", "kda_prep": "kda_prep_kernel", "kda_bwd_dhu": "kda_bwd_dhu_kernel", "kda_bwd_par": "kda_bwd_par_kernel", "gdn_prep": "gdn_prep_kernel",
                  "recurrent_gdn": "recurrent_gdn_kernel", "causal_conv1d_fwd": "conv_fwd_kernel",
                  "causal_conv1d_update": "conv_update1_kernel", "causal_conv1d_bwd": "conv_bwd_kernel",
                  "chunk_local_cumsum": "stage_cumsum_kernel", "chunk_scaled_dot_kkt": "stage_kkt_kernel",
@@ -294,7 +293,7 @@ class Workload:
         return self.graph_out
 
     def launches_per_step(self):
-        n = {"gdn_fwd_bwd": 5, "gdn_fwd_conv": 4, "kda_fwd": 3, "kda_fwd_bwd": 5, "decode": 2, "conv_prefill": 1, "conv_bwd": 2,
+        n = {"gdn_fwd_bwd": 4, "gdn_fwd_conv": 3, "kda_fwd": 2, "kda_fwd_bwd": 4, "decode": 2, "conv_prefill": 1, "conv_bwd": 2,
              "gdn_stage_fwd": 6, "gdn_stage_fwd_bwd": 13}[self.name]
         c = self.cfg
         if self.name in ("gdn_fwd_bwd", "kda_fwd_bwd") and c["B"] >= 2:
@@ -305,10 +304,10 @@ class Workload:
         return n
 
     def kernel_names(self):
-        return {"gdn_fwd_bwd": ["gdn_prep", "tri_inverse", "gdn_fwd", "gdn_bwd_dhu", "gdn_bwd_par"],
-                "gdn_fwd_conv": ["causal_conv1d_fwd", "gdn_prep", "tri_inverse", "gdn_fwd"],
-                "kda_fwd": ["kda_prep", "tri_inverse", "kda_fwd"],
-                "kda_fwd_bwd": ["kda_prep", "tri_inverse", "kda_fwd", "kda_bwd_dhu", "kda_bwd_par"], "decode": ["causal_conv1d_update", "recurrent_gdn"],
+        return {"gdn_fwd_bwd": ["gdn_prep", "gdn_fwd", "gdn_bwd_dhu", "gdn_bwd_par"],
+                "gdn_fwd_conv": ["causal_conv1d_fwd", "gdn_prep", "gdn_fwd"],
+                "kda_fwd": ["kda_prep", "kda_fwd"],
+                "kda_fwd_bwd": ["kda_prep", "kda_fwd", "kda_bwd_dhu", "kda_bwd_par"], "decode": ["causal_conv1d_update", "recurrent_gdn"],
                 "conv_prefill": ["causal_conv1d_fwd"], "conv_bwd": ["causal_conv1d_bwd"],
                 "gdn_stage_fwd": ["chunk_local_cumsum", "chunk_scaled_dot_kkt", "solve_tri", "recompute_w_u_fwd", "chunk_fwd_h",
                                   "chunk_fwd_o"],

@@ -2,8 +2,8 @@
 //
 //  gdn_prep_kernel   (parallel over chunks): gam = chunk-local cumsum(g);
 //                    A[i,j] = beta_i exp(gam_i - gam_j) k_i.k_j (j < i);  X = (I + A)^-1
-//                    KK^T on tcgen05 (shared by the value heads of a GVA group); the unit-lower
-//                    triangular inverse runs in tri_inverse_kernel (fp32 forward substitution on CUDA cores).
+//                    KK^T on tcgen05 (shared by the value heads of a GVA group); the unit lower-triangular inverse by
+//                    blocks in fp32 on CUDA cores (tri_inverse.cuh).
 //                    Replaces chunk_local_cumsum + chunk_scaled_dot_kkt + solve_tri of the reference
 //                    (examples/flash_gated_delta_rule.py:811-838).
 //  gdn_scan_fwd_kernel (gdn_scan_fwd.cuh; sequential over chunks, one CTA per (sequence, value head, 128-column block of V)):
@@ -22,7 +22,7 @@
 #include "gdn_common.cuh"
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
-#include "tri_inverse.h"
+#include "tri_inverse.cuh"
 #include "tensor_map.h"
 
 namespace fla {
@@ -34,7 +34,6 @@ struct GdnFwdParams {
   const void* g; const void* beta;
   float* gam;          // [tokens, HV]      chunk-local cumulative log decay (saved for backward)
   bf16* X;             // [chunks, HV, 2, 8 x 64 x 8]  the chunk's (I + A)^-1 as value + residual strips (saved for backward)
-  float* at;           // [chunks, HV, 64, 64] scratch: A^T handed to the triangular-inverse kernel
   bf16* p_img;         // [chunks, HV, kPImg]: tril(Q K^T * decay) as value / residual strips, then the chunk's factor record (reused by backward)
   const float* h0;     // [N, HV, K, V] or null
   float* ht;           // [N, HV, K, V] or null
@@ -57,16 +56,25 @@ namespace fla {
 // One CTA per (chunk, q/k head).  One M = 128 product [q; k] k^T leaves Q K^T in TMEM lanes 0..63 and K K^T in
 // lanes 64..127.  Eight warps: warp w reads lane quadrant w % 4 and the half w / 4 of the 64 columns, so a thread keeps
 // half a row (32 values) in registers; per value head of the GVA group the q-side threads emit their half of
-// P = tril(Q K^T * e^{gam_i - gam_j}) as split operand panels and the k-side threads their half of A^T.  (With four warps
+// P = tril(Q K^T * e^{gam_i - gam_j}) as split operand panels and the k-side threads their half of A^T, which stays in shared
+// memory (where q and k were) and is inverted on the spot, two heads at a time with four warps each: A^T through memory to a kernel
+// of its own and back cost 16 KB each way per tile.  (With four warps
 // and whole rows per thread the kernel took 0.245 ms at the benchmark shape: it is a chain of latencies, and half the
 // work per thread at twice the warps per SM shortens it.)
+// eight consecutive floats of shared memory, 16-byte aligned
+__device__ __forceinline__ void gather8(const float* p, float* f) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
 constexpr int kPrepThreads = 256;
+constexpr int kPrepSmem = 2 * kTriTile * 4;      // [q; k] panels (32 KB), then the A^T tiles of two heads
+static_assert(kPrepSmem >= 32768, "the panels must fit");
 __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* qk_pan = smem;                        // 2 panels x 128 rows: rows 0..63 q, rows 64..127 k
-  __shared__ float gam_s[kC];
-  __shared__ float wsum_s[2];
+  __shared__ __align__(16) float gam_s[2][kC];   // gam log2(e): the decays are powers of two of its differences
+  __shared__ float wsum_s[4];
   __shared__ uint32_t tmem_base_s;
   __shared__ __align__(8) uint64_t bar;
 
@@ -144,33 +152,28 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
   const bool kside = row >= 64;
   const int tok = row & 63;
   const int j0 = half * 32;                         // my 32 columns
-  // the gate / beta values of a head are requested one head ahead (and those of the first head before the product is waited for)
-  auto fetch_g = [&](int hv) { return (warp < 2 && tok < rows) ? ld_scalar(p.g, (tok0 + tok) * p.g_st + hv, p.g_is_f32) : 0.f; };
-  auto fetch_b = [&](int hv) { return (kside && tok < rows) ? ld_scalar(p.beta, (tok0 + tok) * p.beta_st + hv, p.beta_is_f32) : 0.f; };
-  float g_next = fetch_g(hk * G), b_next = fetch_b(hk * G);
-  const bool ok = mbar_wait(&bar, 0, p.status, FLA_ERR_TIMEOUT);
+  // Two value heads at a time.  Their gates are requested a pair ahead (those of the first pair before the product is waited for):
+  // warps 0..3 hold g of (head warp / 2, token (warp % 2) * 32 + lane), the k-side threads beta of both heads.
+  const int sh = warp >> 1, st = (warp & 1) * 32 + lane;
+  auto fetch_g = [&](int h) { return (warp < 4 && h + sh < G && st < rows) ? ld_scalar(p.g, (tok0 + st) * p.g_st + hk * G + h + sh, p.g_is_f32) : 0.f; };
+  auto fetch_b = [&](int h) { return (kside && h < G && tok < rows) ? ld_scalar(p.beta, (tok0 + tok) * p.beta_st + hk * G + h, p.beta_is_f32) : 0.f; };
+  float g_next = fetch_g(0), b_next[2] = {fetch_b(0), fetch_b(1)};
+  const bool ok = __syncthreads_and(mbar_wait(&bar, 0, p.status, FLA_ERR_TIMEOUT));
   tc_fence_after();
-  float sc[32];   // my half of row `tok` of Q K^T (q side) or K K^T (k side)
-  if (ok) {
-    tmem_ld32(tmem_addr(tbase, quad * 32, j0), sc);
-    tmem_ld_wait();
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tbase, 64);
-  if (!ok) return;
 
-  for (int h = 0; h < G; ++h) {
-    const int hv = hk * G + h;
-    const int64_t cidx = (int64_t(sq.cbase) + blockIdx.x) * p.HV + hv;
-    // chunk-local cumulative sum of g (warps 0 and 1: the q-side rows of the first column half)
+  for (int h0 = 0; ok && h0 < G; h0 += 2) {      // (a wait that ran out did so for the whole CTA)
+    const int pair = min(2, G - h0);
+    float sc[32];   // my half of row `tok` of Q K^T (q side) or K K^T (k side): read again for each pair, the inverse needs the registers
+    tmem_ld32(tmem_addr(tbase, quad * 32, j0), sc);
+    // chunk-local cumulative sums of g
     float gv = g_next;
-    const float bi = b_next;
-    if (h + 1 < G) {
-      g_next = fetch_g(hv + 1);
-      b_next = fetch_b(hv + 1);
+    const float bi[2] = {b_next[0], b_next[1]};
+    if (h0 + 2 < G) {
+      g_next = fetch_g(h0 + 2);
+      b_next[0] = fetch_b(h0 + 2);
+      b_next[1] = fetch_b(h0 + 3);
     }
-    if (warp < 2) {
+    if (warp < 4) {
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const float up = __shfl_up_sync(0xffffffffu, gv, o);
@@ -179,53 +182,81 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
       if (lane == 31) wsum_s[warp] = gv;
     }
     __syncthreads();
-    if (warp < 2) {
-      if (warp == 1) gv += wsum_s[0];
-      gam_s[tok] = gv;
-      if (tok < rows) p.gam[(tok0 + tok) * p.HV + hv] = gv;
+    if (warp < 4) {
+      if (warp & 1) gv += wsum_s[warp - 1];
+      gam_s[sh][st] = gv * kLog2e;
+      if (sh < pair && st < rows) p.gam[(tok0 + st) * p.HV + hk * G + h0 + sh] = gv;
     }
     __syncthreads();
-    const float gam_i = gam_s[tok];
-    if (!kside) {
-      // my half of the P row as split bf16, in strips of 8 columns ([j / 8][row i][16 bytes], value then residual): the 16
-      // bytes a thread stores for a strip lie next to its neighbours' (512 contiguous bytes per warp store), and the scans
-      // read the image as an operand with the reduction along j (forward) or along i (reverse) by the descriptor alone
-      uint8_t* img = reinterpret_cast<uint8_t*>(p.p_img + cidx * kPImg);
+    tmem_ld_wait();
+    const bool below = j0 <= (quad & 1) * 32 + 31;      // my warp's quarter of the tile reaches below the diagonal
+    for (int hh = 0; hh < pair; ++hh) {
+      const int64_t cidx = (int64_t(sq.cbase) + blockIdx.x) * p.HV + hk * G + h0 + hh;
+      const float* gam = gam_s[hh];
+      const float gam_i = gam[tok];
+      if (!kside) {
+        // my half of the P row as split bf16, in strips of 8 columns ([j / 8][row i][16 bytes], value then residual): the 16
+        // bytes a thread stores for a strip lie next to its neighbours' (512 contiguous bytes per warp store), and the scans
+        // read the image as an operand with the reduction along j (forward) or along i (reverse) by the descriptor alone
+        uint8_t* img = reinterpret_cast<uint8_t*>(p.p_img + cidx * kPImg);
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        float t[8];
+        for (int ch = 0; ch < 4; ++ch) {
+          uint4 hi = make_uint4(0, 0, 0, 0), lo = hi;
+          if (below) {
+            float t[8];
+            gather8(gam + j0 + ch * 8, t);
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          const int j = j0 + ch * 8 + jj;
-          const float e = __expf(fminf(gam_i - gam_s[j], 0.f));
-          t[jj] = sc[ch * 8 + jj] * ((j <= tok) ? e : 0.f);
+            for (int jj = 0; jj < 8; ++jj) {
+              const int j = j0 + ch * 8 + jj;
+              t[jj] = (j <= tok) ? sc[ch * 8 + jj] * exp2_fast(gam_i - t[jj]) : 0.f;
+            }
+            split8(t, hi, lo);
+          }
+          const uint32_t off = uint32_t(half * 4 + ch) * 1024u + uint32_t(tok) * 16u;
+          *reinterpret_cast<uint4*>(img + off) = hi;
+          *reinterpret_cast<uint4*>(img + 8192 + off) = lo;
         }
-        uint4 hi, lo;
-        split8(t, hi, lo);
-        const uint32_t off = uint32_t(half * 4 + ch) * 1024u + uint32_t(tok) * 16u;
-        *reinterpret_cast<uint4*>(img + off) = hi;
-        *reinterpret_cast<uint4*>(img + 8192 + off) = lo;
-      }
-    } else {
-      if (half == 0) {   // the chunk's per-token factors for the scans, behind the P tile (rows past the end: beta = 0, gam = gam_L)
-        ScanFactors* f = reinterpret_cast<ScanFactors*>(reinterpret_cast<uint8_t*>(p.p_img + cidx * kPImg) + kPTileBytes);
-        const float eg = __expf(gam_i), gl = gam_s[rows - 1];
-        f->b[tok] = bi;
-        f->bg[tok] = bi * eg;
-        f->se[tok] = p.scale * eg;
-        f->dk[tok] = __expf(gl - gam_i);
-        if (tok == 0) f->dl = __expf(gl);
-      }
-      // A^T[j][i] = beta_i exp(gam_i - gam_j) (k_i . k_j) for j < i, written coalesced along i
-      float* at = p.at + cidx * (kC * kC);
+      } else {
+        const float b = bi[hh];
+        if (half == 0) {   // the chunk's per-token factors for the scans, behind the P tile (rows past the end: beta = 0, gam = gam_L)
+          ScanFactors* f = reinterpret_cast<ScanFactors*>(reinterpret_cast<uint8_t*>(p.p_img + cidx * kPImg) + kPTileBytes);
+          const float eg = exp2_fast(gam_i), gl = gam[rows - 1];
+          f->b[tok] = b;
+          f->bg[tok] = b * eg;
+          f->se[tok] = p.scale * eg;
+          f->dk[tok] = exp2_fast(gl - gam_i);
+          if (tok == 0) f->dl = exp2_fast(gl);
+        }
+        // A^T[j][i] = beta_i exp(gam_i - gam_j) (k_i . k_j) for j < i, else 0
+        float* at = reinterpret_cast<float*>(smem) + hh * kTriTile;
+        if (below) {
 #pragma unroll
-      for (int jl = 0; jl < 32; ++jl) {
-        const int j = j0 + jl;
-        if (j < tok) at[j * kC + tok] = bi * __expf(gam_i - gam_s[j]) * sc[jl];
+          for (int ch = 0; ch < 4; ++ch) {
+            float t[8];
+            gather8(gam + j0 + ch * 8, t);
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) {
+              const int j = j0 + ch * 8 + jj;
+              at[j * kTriStride + tok] = j < tok ? b * exp2_fast(gam_i - t[jj]) * sc[ch * 8 + jj] : 0.f;
+            }
+          }
+        }
       }
     }
     __syncthreads();
+    {      // the tiles are complete: four warps each
+      const int grp = tid >> 7, t = tid & 127;
+      if (grp < pair) {
+        float* tile = reinterpret_cast<float*>(smem) + grp * kTriTile;
+        tri_invert(tile, t, 1 + grp);
+        tri_store_strips(tile, reinterpret_cast<uint8_t*>(p.X + ((int64_t(sq.cbase) + blockIdx.x) * p.HV + hk * G + h0 + grp) * 8192), rows, t);
+      }
+    }
+    if (h0 + 2 < G) __syncthreads();
   }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tbase, 64);
 }
 
 }  // namespace fla
@@ -256,8 +287,8 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd_workspace_size(const fla_gdn_chunk
   int64_t chunks = a->q.shape[0] * ((a->q.shape[1] + kC - 1) / kC);
   if (a->cu_seqlens.data) chunks = a->total_chunks;
   if (chunks <= 0) return FLA_ERR_VALUE;
-  // status block + A^T scratch for the inverse + P panels (unless the caller keeps them for the backward)
-  *bytes = 256 + uint64_t(chunks) * a->v.shape[2] * (kC * kC * 4 + (a->p_img.data ? 0 : kPImgBytes));
+  // status block + P panels (unless the caller keeps them for the backward)
+  *bytes = 256 + uint64_t(chunks) * a->v.shape[2] * (a->p_img.data ? 0 : kPImgBytes);
   return FLA_OK;
 }
 
@@ -333,14 +364,13 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   p.status = static_cast<int*>(workspace);
   {
     const uint64_t per = uint64_t(total_chunks) * HV;
-    if (workspace_bytes < 256 + per * (kC * kC * 4 + (a->p_img.data ? 0 : kPImgBytes))) return FLA_ERR_WORKSPACE;
-    p.at = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + 256);
+    if (workspace_bytes < 256 + per * (a->p_img.data ? 0 : kPImgBytes)) return FLA_ERR_WORKSPACE;
     if (a->p_img.data) {
       const fla_tensor_t& pi = a->p_img;
       if (pi.dtype != FLA_BF16 || pi.ndim != 1 || pi.shape[0] != int64_t(per) * kPImg || !aligned16(pi.data)) return FLA_ERR_SHAPE;
       p.p_img = static_cast<bf16*>(pi.data);
     } else {
-      p.p_img = reinterpret_cast<bf16*>(static_cast<uint8_t*>(workspace) + 256 + per * kC * kC * 4);
+      p.p_img = reinterpret_cast<bf16*>(static_cast<uint8_t*>(workspace) + 256);
     }
   }
 
@@ -360,7 +390,7 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(workspace, 0, 256, cs) != cudaSuccess) return FLA_ERR_CUDA;
-  const int prep_smem = 32768 + 1024;
+  const int prep_smem = kPrepSmem + 1024;
   static std::atomic<bool> attr_done_dev[64] = {};   // per device ordinal; setting the attributes twice is harmless
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
@@ -377,11 +407,6 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
     gdn_prep_kernel<<<dim3(nt_max, unsigned(HK), N), kPrepThreads, prep_smem, cs>>>(p);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
-  {
-    KernelTimer kt("tri_inverse", cs);
-    TriInverseParams tp{p.at, nullptr, p.X, nullptr, nullptr, p.cu_seqlens, p.chunk_offsets, p.T, p.HV, 0};
-    if (launch_tri_inverse(tp, nt_max, N, cs)) return FLA_ERR_CUDA;
-  }
   CUtensorMap tm_q, tm_k;
   const uint64_t nst = uint64_t(HK) * kK;   // the normalised rows are dense
   if (p.qn ? (make_row_tile_map(&tm_q, p.qn, kK, uint64_t(HK), uint64_t(B * T), kK, nst) ||

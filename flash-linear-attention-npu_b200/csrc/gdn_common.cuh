@@ -40,6 +40,14 @@ __device__ __forceinline__ float ld_scalar(const void* p, int64_t idx, int is_f3
   return is_f32 ? static_cast<const float*>(p)[idx] : __bfloat162float(static_cast<const bf16*>(p)[idx]);
 }
 
+constexpr float kLog2e = 1.4426950408889634f;
+// 2^x in one instruction (results below the normal range are zero): decays of arguments already scaled by log2(e)
+__device__ __forceinline__ float exp2_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Load 64 consecutive fp32 accumulator columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld_row64(uint32_t taddr, float* v) {
   tmem_ld32(taddr, v);

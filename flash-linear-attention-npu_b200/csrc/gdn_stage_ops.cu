@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(128) stage_kkt_kernel(StageParams p) {
 
 // ----------------------------------------------------------------------------- solve_tri
 // X = (I + A)^-1 per chunk, A strictly lower triangular (entries on and above the diagonal are ignored), fp32
-// forward substitution, one thread per column (the scheme of tri_inverse.cu), two matrices per CTA.
+// forward substitution, one thread per column, two matrices per CTA.
 constexpr int kSolveStride = 68;
 constexpr int kSolveTiles = 2;   // matrices per CTA; small CTAs under a register bound keep ten solves in flight per SM
 __global__ void __launch_bounds__(64 * kSolveTiles, 5) stage_solve_tri_kernel(StageParams p) {

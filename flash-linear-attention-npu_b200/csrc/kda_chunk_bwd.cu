@@ -891,7 +891,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   }
   if ((st = kda_check_rstd(a->q_rstd, a->k_rstd, B, T, HK))) return st;
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
-  uint64_t off[3], off_saved, so[4], fo[6];
+  uint64_t off[3], off_saved, so[4], fo[5];
   const bool have_saved = a->saved.data != nullptr;
   const uint64_t need = kda_bwd_ws_layout(total_chunks, HV, nvb, B * T, have_saved, &off_saved, off);
   if (!workspace || workspace_bytes < need || !aligned16(workspace)) return FLA_ERR_WORKSPACE;
@@ -911,7 +911,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   f.status = reinterpret_cast<int*>(ws);
   f.qk_img = reinterpret_cast<bf16*>(fws + fo[0]); f.kn_img = reinterpret_cast<bf16*>(fws + fo[1]);
   f.p_img = reinterpret_cast<bf16*>(fws + fo[2]); f.x_img = reinterpret_cast<bf16*>(fws + fo[3]);
-  f.vec = reinterpret_cast<float*>(fws + fo[4]); f.at = reinterpret_cast<float*>(fws + fo[5]);
+  f.vec = reinterpret_cast<float*>(fws + fo[4]);
   f.s_img = reinterpret_cast<bf16*>(sv + so[2]); f.vn_img = reinterpret_cast<bf16*>(sv + so[3]);
   f.h0 = static_cast<const float*>(a->initial_state.data);
   f.cu_seqlens = static_cast<const int32_t*>(a->cu_seqlens.data);

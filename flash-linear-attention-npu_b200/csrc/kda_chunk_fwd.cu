@@ -15,7 +15,7 @@
 #include "gdn_common.cuh"
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
-#include "tri_inverse.h"
+#include "tri_inverse.cuh"
 #include "kda_common.cuh"
 #include "tensor_map.h"
 
@@ -225,12 +225,15 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
     mma_commit(&bar);
   }
   // 5. q-side rows: P = tril(Aqk) written straight into its split panel image;
-  //    k-side rows: Akk^T = (beta_i Kp Kn^T)^T for the inverse kernel (coalesced along i)
+  //    k-side rows: Akk^T = (beta_i Kp Kn^T)^T into shared memory, where the operand panels were, and inverted there
   const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane, tok = row & 63;
   // requested before the product is waited for
   const float bi = (quad >= 2 && tok < rows) ? ld_scalar(p.beta, (tok0 + tok) * p.beta_st + hv, p.beta_is_f32) : 0.f;
   const bool ok = mbar_wait(&bar, 0, p.status, FLA_ERR_TIMEOUT);
+  if (tid == 0) bulk_wait_read();     // the images have left the panels
   tc_fence_after();
+  __syncthreads();
+  float* at = reinterpret_cast<float*>(smem);
   if (ok) {
     float sc[32];
     tmem_ld32(tmem_addr(tbase, quad * 32, half * 32), sc);
@@ -248,17 +251,20 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
         *reinterpret_cast<uint4*>(img + 8192 + off) = lo;
       }
     } else {
-      float* at = p.at + cidx * (kC * kC);
 #pragma unroll
       for (int jj = 0; jj < 32; ++jj) {
         const int j = half * 32 + jj;
-        if (j < tok) at[j * kC + tok] = bi * sc[jj];
+        at[j * kTriStride + tok] = j < tok ? bi * sc[jj] : 0.f;      // select: entries above the diagonal may be inf
       }
     }
   }
-  if (tid == 0) bulk_wait_all();
   tc_fence_before();
   __syncthreads();
+  if (tid < 128) {
+    tri_invert(at, tid, 1);
+    tri_store_panels(at, reinterpret_cast<uint8_t*>(p.x_img + cidx * kKdaXImg), rows, tid);
+  }
+  if (tid == 0) bulk_wait_all();
   if (warp == 0) tmem_dealloc(tbase, 64);
 }
 
@@ -576,7 +582,7 @@ __global__ void __launch_bounds__(128) kda_export_scores_kernel(KdaExportParams 
 
 using namespace fla;
 
-uint64_t fla::kda_ws_layout(int64_t total_chunks, int64_t HV, uint64_t off[6]) {
+uint64_t fla::kda_ws_layout(int64_t total_chunks, int64_t HV, uint64_t off[5]) {
   uint64_t o = 256;
   const uint64_t per = uint64_t(total_chunks) * HV;
   off[0] = o; o += align_up(per * kKdaQkImg * 2, 256);
@@ -584,12 +590,11 @@ uint64_t fla::kda_ws_layout(int64_t total_chunks, int64_t HV, uint64_t off[6]) {
   off[2] = o; o += align_up(per * kKdaPImg * 2, 256);
   off[3] = o; o += align_up(per * kKdaXImg * 2, 256);
   off[4] = o; o += align_up(per * kKdaVecs * kK * 4, 256);
-  off[5] = o; o += align_up(per * kC * kC * 4, 256);
   return o;
 }
 
 uint64_t fla::kda_saved_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, uint64_t off[4]) {
-  uint64_t fo[6];
+  uint64_t fo[5];
   const uint64_t per = uint64_t(total_chunks) * HV;
   uint64_t o = 0;
   off[0] = o; o += align_up(kda_ws_layout(total_chunks, HV, fo), 256);
@@ -622,7 +627,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd_workspace_size(const fla_kda_chunk
   int64_t total_chunks; int N, max_len;
   const int st = kda_geometry(a, &total_chunks, &N, &max_len);
   if (st) return st;
-  uint64_t off[6];
+  uint64_t off[5];
   *bytes = a->saved.data ? 256 : kda_ws_layout(total_chunks, a->v.shape[2], off);
   return FLA_OK;
 }
@@ -704,7 +709,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
   }
   if ((st = kda_check_rstd(a->q_rstd, a->k_rstd, B, T, HK))) return st;
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
-  uint64_t off[6];
+  uint64_t off[5];
   uint64_t need = kda_ws_layout(total_chunks, HV, off);
   uint8_t* images = static_cast<uint8_t*>(workspace);   // where the operand images go
   uint64_t soff[4] = {0, 0, 0, 0};
@@ -735,7 +740,6 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
   p.qk_img = reinterpret_cast<bf16*>(ws + off[0]); p.kn_img = reinterpret_cast<bf16*>(ws + off[1]);
   p.p_img = reinterpret_cast<bf16*>(ws + off[2]); p.x_img = reinterpret_cast<bf16*>(ws + off[3]);
   p.vec = reinterpret_cast<float*>(ws + off[4]);
-  p.at = reinterpret_cast<float*>(ws + off[5]);
   p.h0 = static_cast<const float*>(a->initial_state.data); p.ht = static_cast<float*>(a->final_state.data);
   p.o = a->o.data;
   p.cu_seqlens = static_cast<const int32_t*>(a->cu_seqlens.data);
@@ -788,11 +792,6 @@ int fla::kda_launch_forward(const KdaParams& p, int nt_max, cudaStream_t cs) {
     kda_prep_kernel<<<dim3(nt_max, unsigned(p.HV), p.N), 256, kKdaPrepSmem + 1024, cs>>>(p, tm_q, tm_k);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
-  {
-    KernelTimer kt("tri_inverse", cs);
-    TriInverseParams tp{p.at, nullptr, nullptr, p.x_img, p.x_img + kC * kC, p.cu_seqlens, p.chunk_offsets, p.T, p.HV, int(kKdaXImg)};
-    if (launch_tri_inverse(tp, nt_max, p.N, cs)) return FLA_ERR_CUDA;
-  }
   {
     KernelTimer kt("kda_fwd", cs);
     kda_fwd_kernel<<<dim3(unsigned(p.nvb), unsigned(p.HV), p.N), 256, kKdaFwdSmem + 1024, cs>>>(p);

@@ -14,8 +14,7 @@ struct KdaParams {
   bf16* qk_img;         // [chunks, HV, {hi, lo}, 2 panels x 128 rows]  rows 0-63 Qp, rows 64-127 Kp
   bf16* kn_img;         // [chunks, HV, {hi, lo}, 2 panels x 64 rows]
   bf16* p_img;          // [chunks, HV, {hi, lo}, 64 x 64]   tril(Qp Kn^T)
-  bf16* x_img;          // [chunks, HV, {hi, lo}, 64 x 64]   (I + Akk)^-1 (written by the inverse kernel)
-  float* at;            // [chunks, HV, 64, 64] scratch: Akk^T for the inverse kernel
+  bf16* x_img;          // [chunks, HV, {hi, lo}, 64 x 64]   (I + Akk)^-1 
   float* vec;           // [chunks, HV, 3, K]  e^a, e^{gk_L - a}, a
   bf16* s_img;          // optional out for the backward: [chunks, HV, V/64, {hi, lo}, 128 x 64]  Sa = diag(e^a) S at chunk start
   bf16* vn_img;         // optional out for the backward: [chunks, HV, V/64, {hi, lo}, 64 x 64]   v_new
@@ -34,14 +33,14 @@ constexpr int64_t kKdaQkImg = 32768, kKdaKnImg = 16384, kKdaPImg = 8192, kKdaXIm
 constexpr int64_t kKdaSImg = 16384, kKdaVnImg = 8192;   // per 64-column block of V
 constexpr int kKdaVecs = 3;
 
-// Workspace layout of the forward (offsets of qk_img, kn_img, p_img, x_img, vec, at); returns the total size.
-uint64_t kda_ws_layout(int64_t total_chunks, int64_t HV, uint64_t off[6]);
+// Workspace layout of the forward (offsets of qk_img, kn_img, p_img, x_img, vec); returns the total size.
+uint64_t kda_ws_layout(int64_t total_chunks, int64_t HV, uint64_t off[5]);
 // Layout of the buffer a training forward leaves for the backward: the forward workspace (operand images), gk, the
 // Sa images and the v_new images; returns the total size.
 uint64_t kda_saved_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, uint64_t off[4]);
 // q_rstd, k_rstd of an argument block: both absent, or both dense [B, T, HK] f32; an FLA_ERR_* status otherwise.
 int kda_check_rstd(const fla_tensor_t& q, const fla_tensor_t& k, int64_t B, int64_t T, int64_t HK);
-// prep -> inverse -> forward scan on `stream`; 0 or an FLA_ERR_* status.
+// prep -> forward scan on `stream`; 0 or an FLA_ERR_* status.
 int kda_launch_forward(const KdaParams& p, int nt_max, cudaStream_t stream);
 
 }  // namespace fla
