@@ -49,7 +49,7 @@ struct GdnBwdParams {
   int N, T, HK, HV, beta_is_f32;
   int dq_f32, dk_f32, dv_f32, dg_f32, dbeta_f32;   // gradients leave in the dtypes of their inputs: f32, else bf16
   int V, nvb;          // value head dim (128 or 256) and its number of 64-column blocks
-  int n0;              // first sequence of this launch (the backward may be launched as two halves of the batch)
+  int n0, n1;          // sequences of this launch (the backward may be launched as two halves of the batch)
   float scale;
   int* status;
 };
@@ -106,10 +106,11 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, con
   __shared__ __align__(8) uint64_t mma_bar, load_bar, qk_bar;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int hk = blockIdx.y, n = blockIdx.z + p.n0;
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
-  const int c = blockIdx.x;
-  if (c >= sq.nt) return;
+  const int hk = blockIdx.y;
+  const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.n0, blockIdx.x);
+  if (pos.n < p.n0 || pos.n >= p.n1) return;      // half of a packed batch: the other half's chunks
+  const SeqInfo& sq = pos.sq;
+  const int c = pos.c;
   const int t0 = c * kC;
   const int rows = min(kC, sq.len - t0);
   const int64_t tok0 = int64_t(sq.bos) + t0;
@@ -466,19 +467,17 @@ static uint64_t bwd_ws_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int
   return o;
 }
 
-static int bwd_geometry(const fla_gdn_chunk_bwd_args* a, int64_t* total_chunks, int* N, int* max_len) {
+static int bwd_geometry(const fla_gdn_chunk_bwd_args* a, int64_t* total_chunks, int* N) {
   const fla_tensor_t& q = a->q;
   if (!q.data || q.ndim != 4 || !a->v.data || a->v.ndim != 4) return FLA_ERR_SHAPE;
   const int64_t B = q.shape[0], T = q.shape[1];
   *N = int(B);
   *total_chunks = B * ((T + kC - 1) / kC);
-  *max_len = int(T);
   if (a->cu_seqlens.data) {
     if (B != 1 || a->cu_seqlens.dtype != FLA_I32 || a->cu_seqlens.ndim != 1 || a->cu_seqlens.shape[0] < 2) return FLA_ERR_SHAPE;
     *N = int(a->cu_seqlens.shape[0] - 1);
     if (!a->chunk_offsets.data || a->chunk_offsets.dtype != FLA_I32 || a->chunk_offsets.shape[0] != *N + 1) return FLA_ERR_SHAPE;
     if (a->max_seqlen <= 0 || a->max_seqlen > T || a->total_chunks <= 0) return FLA_ERR_VALUE;
-    *max_len = a->max_seqlen;
     *total_chunks = a->total_chunks;
   }
   return FLA_OK;
@@ -486,8 +485,8 @@ static int bwd_geometry(const fla_gdn_chunk_bwd_args* a, int64_t* total_chunks, 
 
 extern "C" FLA_API int fla_b200_gdn_chunk_bwd_workspace_size(const fla_gdn_chunk_bwd_args* a, uint64_t* bytes) {
   if (!a || !bytes) return FLA_ERR_NULL;
-  int64_t total_chunks; int N, max_len;
-  int st = bwd_geometry(a, &total_chunks, &N, &max_len);
+  int64_t total_chunks; int N;
+  int st = bwd_geometry(a, &total_chunks, &N);
   if (st) return st;
   uint64_t o1, o2, o3;
   const int64_t V = a->v.shape[3];
@@ -518,8 +517,8 @@ static int check_tok3(const fla_tensor_t& t, int64_t B, int64_t T, int64_t heads
 static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, uint64_t workspace_bytes, void* stream,
                               bool allow_split) {
   if (!a) return FLA_ERR_NULL;
-  int64_t total_chunks; int N, max_len;
-  int st = bwd_geometry(a, &total_chunks, &N, &max_len);
+  int64_t total_chunks; int N;
+  int st = bwd_geometry(a, &total_chunks, &N);
   if (st) return st;
   const int64_t B = a->q.shape[0], T = a->q.shape[1], HK = a->q.shape[2], HV = a->v.shape[2];
   if (HK <= 0 || HV <= 0 || HV % HK) return FLA_ERR_SHAPE;
@@ -588,7 +587,7 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   p.beta_st = a->beta.stride[1];
   p.dq_st = a->dq.stride[1]; p.dq_sh = a->dq.stride[2]; p.dk_st = a->dk.stride[1]; p.dk_sh = a->dk.stride[2];
   p.dv_st = a->dv.stride[1]; p.dv_sh = a->dv.stride[2];
-  p.total_tokens = B * T;
+  p.total_tokens = B * T; p.n1 = N;
   p.N = N; p.T = int(T); p.HK = int(HK); p.HV = int(HV); p.V = int(V); p.nvb = int(nvb);
   p.beta_is_f32 = a->beta.dtype == FLA_F32;
   p.dq_f32 = a->dq.dtype == FLA_F32; p.dk_f32 = a->dk.dtype == FLA_F32; p.dv_f32 = a->dv.dtype == FLA_F32;
@@ -596,7 +595,6 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   p.scale = a->scale;
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(workspace, 0, 256, cs) != cudaSuccess) return FLA_ERR_CUDA;
   static std::atomic<bool> attr_done_dev[64] = {};   // per device ordinal; setting the attributes twice is harmless
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
@@ -612,13 +610,12 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
       make_row_tile_map(&tm_v, p.v, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.v_sh), uint64_t(p.v_st)) ||
       make_row_tile_map(&tm_d, p.dO, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.do_sh), uint64_t(p.do_st)))
     return FLA_ERR_CUDA;
-  const int nt_max = (max_len + kC - 1) / kC;
   auto launch_scan = [&](const GdnBwdParams& pp, int nseq, cudaStream_t st) {
     gdn_scan_bwd_kernel<<<dim3(unsigned(V / 128), unsigned(HV), nseq), kScanThreads, kScanBwdSmem + 1024, st>>>(pp, tm_q, tm_k, tm_v, tm_d);
   };
-  auto launch_par = [&](const GdnBwdParams& pp, int nseq, cudaStream_t st) {
-    if (nvb == 2) gdn_bwd_par_kernel<2><<<dim3(nt_max, unsigned(HK), nseq), 256, kParSmem + 1024, st>>>(pp, tm_q, tm_k);
-    else gdn_bwd_par_kernel<4><<<dim3(nt_max, unsigned(HK), nseq), 256, kParSmem + 1024, st>>>(pp, tm_q, tm_k);
+  auto launch_par = [&](const GdnBwdParams& pp, int64_t chunks, cudaStream_t st) {
+    if (nvb == 2) gdn_bwd_par_kernel<2><<<dim3(unsigned(chunks), unsigned(HK)), 256, kParSmem + 1024, st>>>(pp, tm_q, tm_k);
+    else gdn_bwd_par_kernel<4><<<dim3(unsigned(chunks), unsigned(HK)), 256, kParSmem + 1024, st>>>(pp, tm_q, tm_k);
   };
   // The reverse scan launches one CTA per (sequence, value head, 128 channels) and each needs a whole SM: when there are
   // more chains than SMs the last round leaves SMs idle for the length of a chain.  The batch is then launched as two
@@ -631,13 +628,15 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
     std::lock_guard<std::mutex> lk(aux->mu);   // the fork / join events are shared by the callers of this stream
     const int n1 = N / 2;
     GdnBwdParams p2 = p;
-    p2.n0 = n1;
+    p.n1 = p2.n0 = n1;
     bool okc = cudaEventRecord(aux->fork, cs) == cudaSuccess && cudaStreamWaitEvent(aux->s, aux->fork, 0) == cudaSuccess;
     if (!okc) return FLA_ERR_CUDA;
     launch_scan(p, n1, cs);
     launch_scan(p2, N - n1, aux->s);
-    launch_par(p, n1, cs);
-    launch_par(p2, N - n1, aux->s);
+    // a packed batch's halves hold chunk counts the host does not have: both launches cover all chunks and skip the other half's
+    const int64_t nt = (T + kC - 1) / kC;
+    launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs);
+    launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s);
     okc = cudaEventRecord(aux->join, aux->s) == cudaSuccess && cudaStreamWaitEvent(cs, aux->join, 0) == cudaSuccess;
     if (!okc) return FLA_ERR_CUDA;
     return cuda_status(cudaGetLastError());
@@ -649,7 +648,7 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
     KernelTimer kt("gdn_bwd_par", cs);
-    launch_par(p, N, cs);
+    launch_par(p, total_chunks, cs);
   }
   return cuda_status(cudaGetLastError());
 }
@@ -702,7 +701,7 @@ extern "C" FLA_API int fla_b200_gdn_chunk_bwd_noalloc(const fla_gdn_chunk_bwd_ar
     }
     scratch = g_static_ptr[dev];
   }
-  // The regular entry point clears the status block at the head of the scratch on `stream` and overwrites
+  // The regular entry point's first kernel clears the status word at the head of the scratch on `stream` and overwrites
   // every other byte it later reads, so nothing else of the previous call's contents matters.
   return gdn_chunk_bwd_impl(a, scratch, kStaticScratchBytes, stream, false);   // one stream: creating a second one may allocate
 }

@@ -79,10 +79,10 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
   __shared__ __align__(8) uint64_t bar;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int hk = blockIdx.y, n = blockIdx.z;
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
-  const int t0 = blockIdx.x * kC;
-  if (t0 >= sq.len) return;
+  const int hk = blockIdx.y;
+  const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, 0, blockIdx.x);
+  const SeqInfo& sq = pos.sq;
+  const int t0 = pos.c * kC;
   const int rows = min(kC, sq.len - t0);
   const int64_t tok0 = int64_t(sq.bos) + t0;
   {
@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
     tmem_relinquish();
   }
   if (tid == 0) {
+    clear_status(p.status, blockIdx.x + hk == 0);
     mbar_init(&bar, 1);
     mbar_init_fence();
   }
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
     tmem_ld_wait();
     const bool below = j0 <= (quad & 1) * 32 + 31;      // my warp's quarter of the tile reaches below the diagonal
     for (int hh = 0; hh < pair; ++hh) {
-      const int64_t cidx = (int64_t(sq.cbase) + blockIdx.x) * p.HV + hk * G + h0 + hh;
+      const int64_t cidx = (int64_t(sq.cbase) + pos.c) * p.HV + hk * G + h0 + hh;
       const float* gam = gam_s[hh];
       const float gam_i = gam[tok];
       if (!kside) {
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
       if (grp < pair) {
         float* tile = reinterpret_cast<float*>(smem) + grp * kTriTile;
         tri_invert(tile, t, 1 + grp);
-        tri_store_strips(tile, reinterpret_cast<uint8_t*>(p.X + ((int64_t(sq.cbase) + blockIdx.x) * p.HV + hk * G + h0 + grp) * 8192), rows, t);
+        tri_store_strips(tile, reinterpret_cast<uint8_t*>(p.X + ((int64_t(sq.cbase) + pos.c) * p.HV + hk * G + h0 + grp) * 8192), rows, t);
       }
     }
     if (h0 + 2 < G) __syncthreads();
@@ -316,13 +317,11 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
 
   int N = int(B);
   int64_t total_chunks = B * ((T + kC - 1) / kC);
-  int max_len = int(T);
   if (a->cu_seqlens.data) {
     if (B != 1 || a->cu_seqlens.dtype != FLA_I32 || a->cu_seqlens.ndim != 1 || a->cu_seqlens.shape[0] < 2) return FLA_ERR_SHAPE;
     N = int(a->cu_seqlens.shape[0] - 1);
     if (!a->chunk_offsets.data || a->chunk_offsets.dtype != FLA_I32 || a->chunk_offsets.shape[0] != N + 1) return FLA_ERR_SHAPE;
     if (a->max_seqlen <= 0 || a->max_seqlen > T || a->total_chunks <= 0) return FLA_ERR_VALUE;
-    max_len = a->max_seqlen;
     total_chunks = a->total_chunks;
   }
   const fla_tensor_t &gam = a->gam, &X = a->x_inv;
@@ -389,7 +388,6 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   }
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(workspace, 0, 256, cs) != cudaSuccess) return FLA_ERR_CUDA;
   const int prep_smem = kPrepSmem + 1024;
   static std::atomic<bool> attr_done_dev[64] = {};   // per device ordinal; setting the attributes twice is harmless
   int dev = 0;
@@ -401,10 +399,9 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
     if (cudaFuncSetAttribute(gdn_scan_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kScanFwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     attr_done = true;
   }
-  const int nt_max = (max_len + kC - 1) / kC;
   {
     KernelTimer kt("gdn_prep", cs);
-    gdn_prep_kernel<<<dim3(nt_max, unsigned(HK), N), kPrepThreads, prep_smem, cs>>>(p);
+    gdn_prep_kernel<<<dim3(unsigned(total_chunks), unsigned(HK)), kPrepThreads, prep_smem, cs>>>(p);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   CUtensorMap tm_q, tm_k;

@@ -36,6 +36,39 @@ __device__ __forceinline__ SeqInfo seq_info(const int32_t* cu_seqlens, const int
   return s;
 }
 
+// The chunk-parallel kernels launch one CTA (per head) for each chunk there is, numbered through all sequences: a grid of
+// (longest sequence) x (sequences) leaves most of a packed batch's CTAs with nothing to do (22 prompts of 11,003 tokens: 172 chunks, 1,034
+// CTAs per head, 178 us for the GDN prep kernel where the chunks alone take 120).
+struct ChunkPos {
+  SeqInfo sq;
+  int n, c;  // sequence, chunk inside it
+};
+// Called by whole warps.  `chunk` counts from the first chunk of sequence n0 (fixed lengths; packed: of the batch).
+__device__ __forceinline__ ChunkPos chunk_pos(const int32_t* cu_seqlens, const int32_t* chunk_offsets, int N, int T, int n0, int chunk) {
+  ChunkPos r;
+  if (!cu_seqlens) {
+    const int nt = (T + kC - 1) / kC, k = chunk / nt;
+    r.n = n0 + k;
+    r.sq = seq_info(nullptr, nullptr, r.n, T);
+    r.c = chunk - k * nt;
+    return r;
+  }
+  // the last sequence that starts at or before the chunk: 32 candidates at a time
+  int lo = 0, n = N;
+  const int lane = threadIdx.x & 31;
+  while (n > 1) {
+    const int step = (n + 31) / 32, i = lane * step;
+    const unsigned le = __ballot_sync(0xffffffffu, i < n && chunk_offsets[lo + i] <= chunk);
+    const int k = __popc(le) - 1;
+    lo += k * step;
+    n = min(step, n - k * step);
+  }
+  r.n = lo;
+  r.sq = seq_info(cu_seqlens, chunk_offsets, lo, T);
+  r.c = chunk - r.sq.cbase;
+  return r;
+}
+
 __device__ __forceinline__ float ld_scalar(const void* p, int64_t idx, int is_f32) {
   return is_f32 ? static_cast<const float*>(p)[idx] : __bfloat162float(static_cast<const bf16*>(p)[idx]);
 }
@@ -129,6 +162,12 @@ __device__ __forceinline__ void unpack_f16x8(const uint4& raw, float* f) {
     f[2 * i] = t.x;
     f[2 * i + 1] = t.y;
   }
+}
+
+// The first CTA of an operator's first kernel clears the status word (a memset of its own was a launch more per call).  A wait
+// that runs out does so after millions of polls: long after that CTA, which is the first to be scheduled, has passed here.
+__device__ __forceinline__ void clear_status(int* status, bool first) {
+  if (first && status) *status = 0;
 }
 
 // A wait that gives up records the timeout once; afterwards the thread stops waiting so that the kernel

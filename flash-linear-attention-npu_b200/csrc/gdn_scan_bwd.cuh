@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
     tmem_relinquish();
   }
   if (tid == 0) {
+    clear_status(p.status, vb + hv + n == 0);
     mbar_init(&mma_bar, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&qk_bar[i], 1);

@@ -48,7 +48,7 @@ struct KdaBwdParams {
   int64_t total_tokens;
   int N, T, HK, HV, beta_is_f32;
   int dq_f32, dk_f32, dv_f32, dg_f32, dbeta_f32;   // gradients leave in the dtypes of their inputs: f32, else bf16
-  int n0;              // first sequence of this launch (the backward may be launched as two halves of the batch)
+  int n0, n1;          // sequences of this launch (the backward may be launched as two halves of the batch)
   int V, nvb;          // value head dim (128 or 256) and its number of 64-column blocks
   float scale;
   int* status;
@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_dhu_kernel(KdaBwdParams p) {
     tmem_relinquish();
   }
   if (tid == 0) {
+    clear_status(p.status, vb + hv + n == 0);
     mbar_init(&bar, 1);
     mbar_init(&pbar, 1);
     mbar_init(&qk_bar, 1);
@@ -418,10 +419,11 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
   __shared__ __align__(8) uint64_t mma_bar, load_bar, img_bar, gk_bar;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int hk = blockIdx.y, n = blockIdx.z + p.n0;
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
-  const int c = blockIdx.x;
-  if (c >= sq.nt) return;
+  const int hk = blockIdx.y;
+  const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.n0, blockIdx.x);
+  if (pos.n < p.n0 || pos.n >= p.n1) return;      // half of a packed batch: the other half's chunks
+  const SeqInfo& sq = pos.sq;
+  const int c = pos.c;
   const int t0 = c * kC;
   const int rows = min(kC, sq.len - t0);
   const int64_t tok0 = int64_t(sq.bos) + t0;
@@ -813,19 +815,17 @@ static uint64_t kda_bwd_ws_layout(int64_t total_chunks, int64_t HV, int64_t nvb,
   return o;
 }
 
-static int kda_bwd_geometry(const fla_kda_chunk_bwd_args* a, int64_t* total_chunks, int* N, int* max_len) {
+static int kda_bwd_geometry(const fla_kda_chunk_bwd_args* a, int64_t* total_chunks, int* N) {
   const fla_tensor_t& q = a->q;
   if (!q.data || q.ndim != 4 || !a->v.data || a->v.ndim != 4) return FLA_ERR_SHAPE;
   const int64_t B = q.shape[0], T = q.shape[1];
   *N = int(B);
   *total_chunks = B * ((T + kC - 1) / kC);
-  *max_len = int(T);
   if (a->cu_seqlens.data) {
     if (B != 1 || a->cu_seqlens.dtype != FLA_I32 || a->cu_seqlens.ndim != 1 || a->cu_seqlens.shape[0] < 2) return FLA_ERR_SHAPE;
     *N = int(a->cu_seqlens.shape[0] - 1);
     if (!a->chunk_offsets.data || a->chunk_offsets.dtype != FLA_I32 || a->chunk_offsets.shape[0] != *N + 1) return FLA_ERR_SHAPE;
     if (a->max_seqlen <= 0 || a->max_seqlen > T || a->total_chunks <= 0) return FLA_ERR_VALUE;
-    *max_len = a->max_seqlen;
     *total_chunks = a->total_chunks;
   }
   return FLA_OK;
@@ -833,8 +833,8 @@ static int kda_bwd_geometry(const fla_kda_chunk_bwd_args* a, int64_t* total_chun
 
 extern "C" FLA_API int fla_b200_kda_chunk_bwd_workspace_size(const fla_kda_chunk_bwd_args* a, uint64_t* bytes) {
   if (!a || !bytes) return FLA_ERR_NULL;
-  int64_t total_chunks; int N, max_len;
-  const int st = kda_bwd_geometry(a, &total_chunks, &N, &max_len);
+  int64_t total_chunks; int N;
+  const int st = kda_bwd_geometry(a, &total_chunks, &N);
   if (st) return st;
   uint64_t off[3], off_saved;
   const int64_t V = a->v.shape[3];
@@ -864,8 +864,8 @@ static int kda_bwd_check_tok3(const fla_tensor_t& t, int64_t B, int64_t T, int64
 extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, void* workspace, uint64_t workspace_bytes,
                                               void* stream) {
   if (!a) return FLA_ERR_NULL;
-  int64_t total_chunks; int N, max_len;
-  int st = kda_bwd_geometry(a, &total_chunks, &N, &max_len);
+  int64_t total_chunks; int N;
+  int st = kda_bwd_geometry(a, &total_chunks, &N);
   if (st) return st;
   const int64_t B = a->q.shape[0], T = a->q.shape[1], HK = a->q.shape[2], HV = a->v.shape[2];
   if (HK <= 0 || HV <= 0 || HV % HK) return FLA_ERR_SHAPE;
@@ -938,7 +938,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   p.v_st = f.v_st; p.v_sh = f.v_sh; p.do_st = a->d_o.stride[1]; p.do_sh = a->d_o.stride[2]; p.beta_st = f.beta_st;
   p.dq_st = a->dq.stride[1]; p.dq_sh = a->dq.stride[2]; p.dk_st = a->dk.stride[1]; p.dk_sh = a->dk.stride[2];
   p.dv_st = a->dv.stride[1]; p.dv_sh = a->dv.stride[2]; p.dg_st = a->dg.stride[1]; p.dg_sh = a->dg.stride[2];
-  p.total_tokens = B * T;
+  p.total_tokens = B * T; p.n1 = N;
   p.N = N; p.T = int(T); p.HK = int(HK); p.HV = int(HV); p.V = int(V); p.nvb = int(nvb);
   p.beta_is_f32 = f.beta_is_f32;
   p.dq_f32 = a->dq.dtype == FLA_F32; p.dk_f32 = a->dk.dtype == FLA_F32; p.dv_f32 = a->dv.dtype == FLA_F32;
@@ -947,9 +947,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   p.status = f.status;
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(workspace, 0, 256, cs) != cudaSuccess) return FLA_ERR_CUDA;
-  const int nt_max = (max_len + kC - 1) / kC;
-  if (!have_saved && (st = kda_launch_forward(f, nt_max, cs))) return st;
+  if (!have_saved && (st = kda_launch_forward(f, total_chunks, cs))) return st;
   static std::atomic<bool> attr_done_dev[64] = {};   // per device ordinal; setting the attributes twice is harmless
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
@@ -964,10 +962,10 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   auto launch_scan = [&](const KdaBwdParams& pp, int nseq, cudaStream_t st_) {
     kda_bwd_dhu_kernel<<<dim3(unsigned(nvb), unsigned(HV), nseq), 256, kKdaDhuSmem + 1024, st_>>>(pp);
   };
-  auto launch_par = [&](const KdaBwdParams& pp, int nseq, cudaStream_t st_) {
+  auto launch_par = [&](const KdaBwdParams& pp, int64_t chunks, cudaStream_t st_) {
     auto* par = nvb == 2 ? (pp.q_rstd ? kda_bwd_par_kernel<2, true> : kda_bwd_par_kernel<2, false>)
                          : (pp.q_rstd ? kda_bwd_par_kernel<4, true> : kda_bwd_par_kernel<4, false>);
-    par<<<dim3(nt_max, unsigned(HK), nseq), 256, kKdaParSmem + 1024, st_>>>(pp, tm_gk);
+    par<<<dim3(unsigned(chunks), unsigned(HK)), 256, kKdaParSmem + 1024, st_>>>(pp, tm_gk);
   };
   // more scan chains (one CTA per SM each) than SMs: two halves of the batch on two streams, so that the chunk-parallel
   // kernel of the first half fills the SMs the second half's scan leaves idle (aux_stream.h)
@@ -977,12 +975,14 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
     std::lock_guard<std::mutex> lk(aux->mu);
     const int n1 = N / 2;
     KdaBwdParams p2 = p;
-    p2.n0 = n1;
+    p.n1 = p2.n0 = n1;
     if (cudaEventRecord(aux->fork, cs) != cudaSuccess || cudaStreamWaitEvent(aux->s, aux->fork, 0) != cudaSuccess) return FLA_ERR_CUDA;
     launch_scan(p, n1, cs);
     launch_scan(p2, N - n1, aux->s);
-    launch_par(p, n1, cs);
-    launch_par(p2, N - n1, aux->s);
+    // a packed batch's halves hold chunk counts the host does not have: both launches cover all chunks and skip the other half's
+    const int64_t nt = (T + kC - 1) / kC;
+    launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs);
+    launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s);
     if (cudaEventRecord(aux->join, aux->s) != cudaSuccess || cudaStreamWaitEvent(cs, aux->join, 0) != cudaSuccess) return FLA_ERR_CUDA;
     return cuda_status(cudaGetLastError());
   }
@@ -993,7 +993,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
     KernelTimer kt("kda_bwd_par", cs);
-    launch_par(p, N, cs);
+    launch_par(p, total_chunks, cs);
   }
   return cuda_status(cudaGetLastError());
 }

@@ -48,11 +48,11 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
   __shared__ __align__(8) uint64_t bar, qk_bar;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int hv = blockIdx.y, n = blockIdx.z;
+  const int hv = blockIdx.y;
   const int hk = hv / (p.HV / p.HK);
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
-  const int c = blockIdx.x;
-  if (c >= sq.nt) return;
+  const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, 0, blockIdx.x);
+  const SeqInfo& sq = pos.sq;
+  const int c = pos.c;
   const int t0 = c * kC;
   const int rows = min(kC, sq.len - t0);
   const int64_t tok0 = int64_t(sq.bos) + t0;
@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
     tmem_relinquish();
   }
   if (tid == 0) {
+    clear_status(p.status, blockIdx.x + hv == 0);
     mbar_init(&bar, 1);
     mbar_init(&qk_bar, 1);
     mbar_init_fence();
@@ -763,9 +764,8 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
   }
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(workspace, 0, 256, cs) != cudaSuccess) return FLA_ERR_CUDA;
   const int nt_max = (max_len + kC - 1) / kC;
-  st = kda_launch_forward(p, nt_max, cs);
+  st = kda_launch_forward(p, total_chunks, cs);
   if (st || (!ep.out[0] && !ep.out[1])) return st;
   ep.img[0] = p.p_img; ep.img[1] = p.x_img;
   ep.cu_seqlens = p.cu_seqlens; ep.chunk_offsets = p.chunk_offsets; ep.T = p.T; ep.HV = p.HV; ep.scale = p.scale;
@@ -774,7 +774,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
   return cuda_status(cudaGetLastError());
 }
 
-int fla::kda_launch_forward(const KdaParams& p, int nt_max, cudaStream_t cs) {
+int fla::kda_launch_forward(const KdaParams& p, int64_t total_chunks, cudaStream_t cs) {
   static std::atomic<bool> attr_done_dev[64] = {};   // per device ordinal; setting the attributes twice is harmless
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
@@ -789,7 +789,7 @@ int fla::kda_launch_forward(const KdaParams& p, int nt_max, cudaStream_t cs) {
     return FLA_ERR_CUDA;
   {
     KernelTimer kt("kda_prep", cs);
-    kda_prep_kernel<<<dim3(nt_max, unsigned(p.HV), p.N), 256, kKdaPrepSmem + 1024, cs>>>(p, tm_q, tm_k);
+    kda_prep_kernel<<<dim3(unsigned(total_chunks), unsigned(p.HV)), 256, kKdaPrepSmem + 1024, cs>>>(p, tm_q, tm_k);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {

@@ -41,6 +41,6 @@ uint64_t kda_saved_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t
 // q_rstd, k_rstd of an argument block: both absent, or both dense [B, T, HK] f32; an FLA_ERR_* status otherwise.
 int kda_check_rstd(const fla_tensor_t& q, const fla_tensor_t& k, int64_t B, int64_t T, int64_t HK);
 // prep -> forward scan on `stream`; 0 or an FLA_ERR_* status.
-int kda_launch_forward(const KdaParams& p, int nt_max, cudaStream_t stream);
+int kda_launch_forward(const KdaParams& p, int64_t total_chunks, cudaStream_t stream);
 
 }  // namespace fla
