@@ -11,7 +11,7 @@ int g_sm_count[64] = {};
 
 int sm_count(int dev) {
   std::lock_guard<std::mutex> lk(g_aux_mu);
-  if (!g_sm_count[dev] && cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) g_sm_count[dev] = 1 << 30;
+  if (!g_sm_count[dev] && cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) g_sm_count[dev] = 148;
   return g_sm_count[dev];
 }
 

@@ -41,6 +41,9 @@ struct GdnBwdParams {
   bf16* dz_img;        // [chunks, HV, V/64, 192x64: rows 0-63 dO, rows 64-127 dZ rounded to bf16, rows 128-191 the residual of dZ]
   float* bz;           // [V/32, tokens, HV] partial sums of dZ * V over the 32-column slices of V
   const float* dht; float* dh0;
+  const bf16* seg_m;   // [segments, HV, 128x128 (value, residual)]  the forward's transition matrices (split chains only)
+  float* seg_dh;       // [segments, HV, V/128, 128, 128]
+  int seg_len;         // chunks per segment
   void* dq; void* dk; void* dv; void* dg; void* dbeta;
   const int32_t* cu_seqlens; const int32_t* chunk_offsets;
   int64_t q_st, q_sh, k_st, k_sh, v_st, v_sh, do_st, do_sh, beta_st;
@@ -458,12 +461,14 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, con
 
 using namespace fla;
 
-static uint64_t bwd_ws_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, uint64_t* off_ds, uint64_t* off_dz,
-                              uint64_t* off_bz) {
+static uint64_t bwd_ws_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, const SegPlan& plan, uint64_t* off_ds,
+                              uint64_t* off_dz, uint64_t* off_bz, uint64_t* off_seg) {
   uint64_t o = 256;  // status block
   *off_ds = o; o += align_up(uint64_t(total_chunks) * HV * nvb * kSImg * 2, 256);
   *off_dz = o; o += align_up(uint64_t(total_chunks) * HV * nvb * kDzImg * 2, 256);
   *off_bz = o; o += align_up(uint64_t(2 * nvb) * tokens * HV * 4, 256);
+  *off_seg = o;
+  if (plan.split) o += uint64_t(plan.count) * HV * (nvb / 2) * kSegHBytes;
   return o;
 }
 
@@ -483,15 +488,23 @@ static int bwd_geometry(const fla_gdn_chunk_bwd_args* a, int64_t* total_chunks, 
   return FLA_OK;
 }
 
+static SegPlan bwd_plan(const fla_gdn_chunk_bwd_args* a, int64_t total_chunks, int N) {
+  SegPlan whole;
+  whole.count = N;
+  if (!a->seg_m.data) return whole;
+  const bool packed = a->cu_seqlens.data != nullptr;
+  return gdn_segments(N, total_chunks, packed ? a->max_seqlen : a->q.shape[1], packed, a->v.shape[2], a->v.shape[3]);
+}
+
 extern "C" FLA_API int fla_b200_gdn_chunk_bwd_workspace_size(const fla_gdn_chunk_bwd_args* a, uint64_t* bytes) {
   if (!a || !bytes) return FLA_ERR_NULL;
   int64_t total_chunks; int N;
   int st = bwd_geometry(a, &total_chunks, &N);
   if (st) return st;
-  uint64_t o1, o2, o3;
+  uint64_t o1, o2, o3, o4;
   const int64_t V = a->v.shape[3];
   if (V != kV && V != 2 * kV) return FLA_ERR_SHAPE;
-  *bytes = bwd_ws_layout(total_chunks, a->v.shape[2], V / kBV, a->q.shape[0] * a->q.shape[1], &o1, &o2, &o3);
+  *bytes = bwd_ws_layout(total_chunks, a->v.shape[2], V / kBV, a->q.shape[0] * a->q.shape[1], bwd_plan(a, total_chunks, N), &o1, &o2, &o3, &o4);
   return FLA_OK;
 }
 
@@ -562,8 +575,12 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
     }
   }
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
-  uint64_t off_ds, off_dz, off_bz;
-  const uint64_t need = bwd_ws_layout(total_chunks, HV, nvb, B * T, &off_ds, &off_dz, &off_bz);
+  uint64_t off_ds, off_dz, off_bz, off_seg;
+  const SegPlan plan = bwd_plan(a, total_chunks, N);
+  if (plan.split && (a->seg_m.dtype != FLA_BF16 || a->seg_m.ndim != 1 || uint64_t(a->seg_m.shape[0]) * 2 < uint64_t(plan.count) * HV * kSegMBytes ||
+                     !aligned16(a->seg_m.data)))
+    return FLA_ERR_SHAPE;
+  const uint64_t need = bwd_ws_layout(total_chunks, HV, nvb, B * T, plan, &off_ds, &off_dz, &off_bz, &off_seg);
   if (!workspace || workspace_bytes < need || !aligned16(workspace)) return FLA_ERR_WORKSPACE;
 
   GdnBwdParams p{};
@@ -578,6 +595,9 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   p.ds_img = reinterpret_cast<bf16*>(ws + off_ds);
   p.dz_img = reinterpret_cast<bf16*>(ws + off_dz);
   p.bz = reinterpret_cast<float*>(ws + off_bz);
+  p.seg_m = static_cast<const bf16*>(a->seg_m.data);
+  p.seg_dh = reinterpret_cast<float*>(ws + off_seg);
+  p.seg_len = plan.len;
   p.dht = static_cast<const float*>(a->dht.data); p.dh0 = static_cast<float*>(a->dh0.data);
   p.dq = a->dq.data; p.dk = a->dk.data; p.dv = a->dv.data; p.dg = a->dg.data; p.dbeta = a->dbeta.data;
   p.cu_seqlens = static_cast<const int32_t*>(a->cu_seqlens.data);
@@ -599,7 +619,8 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
   if (!attr_done_dev[dev]) {
-    if (cudaFuncSetAttribute(gdn_scan_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kScanBwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
+    for (auto* scan : {gdn_scan_bwd_kernel<false, false>, gdn_scan_bwd_kernel<false, true>, gdn_scan_bwd_kernel<true, true>})
+      if (cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kScanBwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     if (cudaFuncSetAttribute(gdn_bwd_par_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kParSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     if (cudaFuncSetAttribute(gdn_bwd_par_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kParSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     attr_done_dev[dev] = true;
@@ -610,8 +631,11 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
       make_row_tile_map(&tm_v, p.v, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.v_sh), uint64_t(p.v_st)) ||
       make_row_tile_map(&tm_d, p.dO, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.do_sh), uint64_t(p.do_st)))
     return FLA_ERR_CUDA;
-  auto launch_scan = [&](const GdnBwdParams& pp, int nseq, cudaStream_t st) {
-    gdn_scan_bwd_kernel<<<dim3(unsigned(V / 128), unsigned(HV), nseq), kScanThreads, kScanBwdSmem + 1024, st>>>(pp, tm_q, tm_k, tm_v, tm_d);
+  auto launch_scan = [&](const GdnBwdParams& pp, int64_t segments, cudaStream_t st) {
+    const dim3 grid(unsigned(HV * (V / 128)), unsigned(segments));
+    if (plan.split) gdn_scan_bwd_kernel<true, true><<<grid, kScanThreads, kScanBwdSmem + 1024, st>>>(pp, tm_q, tm_k, tm_v, tm_d);
+    auto* scan = plan.split ? gdn_scan_bwd_kernel<false, true> : gdn_scan_bwd_kernel<false, false>;
+    scan<<<grid, kScanThreads, kScanBwdSmem + 1024, st>>>(pp, tm_q, tm_k, tm_v, tm_d);
   };
   auto launch_par = [&](const GdnBwdParams& pp, int64_t chunks, cudaStream_t st) {
     if (nvb == 2) gdn_bwd_par_kernel<2><<<dim3(unsigned(chunks), unsigned(HK)), 256, kParSmem + 1024, st>>>(pp, tm_q, tm_k);
@@ -623,7 +647,7 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   // leaves free.  Not while per-kernel timing is on (its events bracket single launches), not during stream capture, not
   // for the allocation-free entry (creating the second stream may allocate).
   AuxStream* aux = nullptr;
-  if (allow_split && N >= 2 && int64_t(V / 128) * HV * N > sm_count(dev) && !kernel_timing_enabled()) aux = aux_stream_for(dev, cs);
+  if (allow_split && N >= 2 && !plan.split && int64_t(V / 128) * HV * N > sm_count(dev) && !kernel_timing_enabled()) aux = aux_stream_for(dev, cs);
   if (aux) {
     std::lock_guard<std::mutex> lk(aux->mu);   // the fork / join events are shared by the callers of this stream
     const int n1 = N / 2;
@@ -643,7 +667,7 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   }
   {
     KernelTimer kt("gdn_bwd_dhu", cs);
-    launch_scan(p, N, cs);
+    launch_scan(p, plan.count, cs);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {

@@ -24,6 +24,7 @@
 #include "kernel_timer.h"
 #include "tri_inverse.cuh"
 #include "tensor_map.h"
+#include "aux_stream.h"
 
 namespace fla {
 
@@ -39,6 +40,9 @@ struct GdnFwdParams {
   float* ht;           // [N, HV, K, V] or null
   void* o;             // [tokens, HV, V]
   bf16* s_img;         // [chunks, HV, V/64, 2, 128x64] panel images of the state at chunk start (hi, lo), optional
+  bf16* seg_m;         // [segments, HV, 128x128 (value, residual)]  transition matrix of a segment (split chains only)
+  float* seg_h;        // [segments, HV, V/128, 128, 128]  its end state from the zero state (segment 0: from the initial one)
+  int seg_len;         // chunks per segment
   bf16* vn_img;        // [chunks, HV, V/64, 2, 64x64]  panel images of v_new (hi, lo), optional
   const int32_t* cu_seqlens; const int32_t* chunk_offsets;
   int64_t q_st, q_sh, k_st, k_sh, v_st, v_sh, o_st, o_sh, g_st, beta_st;
@@ -264,6 +268,46 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
 
 using namespace fla;
 
+// A forward step is 1; a state-only step takes as long (its outputs and score products are off the chain).
+fla::SegPlan fla::gdn_segments(int64_t N, int64_t total_chunks, int64_t max_len, bool packed, int64_t HV, int64_t V) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+  return plan_segments(N, total_chunks, (max_len + kC - 1) / kC, packed, HV * (V / 128), HV, 1.0, sm_count(dev));
+}
+
+static int geometry(const fla_gdn_chunk_fwd_args* a, int64_t* total_chunks, int* N, int* max_len) {
+  const int64_t B = a->q.shape[0], T = a->q.shape[1];
+  *N = int(B);
+  *total_chunks = B * ((T + kC - 1) / kC);
+  *max_len = int(T);
+  if (a->cu_seqlens.data) {
+    if (B != 1 || a->cu_seqlens.dtype != FLA_I32 || a->cu_seqlens.ndim != 1 || a->cu_seqlens.shape[0] < 2) return FLA_ERR_SHAPE;
+    *N = int(a->cu_seqlens.shape[0] - 1);
+    if (!a->chunk_offsets.data || a->chunk_offsets.dtype != FLA_I32 || a->chunk_offsets.shape[0] != *N + 1) return FLA_ERR_SHAPE;
+    if (a->max_seqlen <= 0 || a->max_seqlen > T || a->total_chunks <= 0) return FLA_ERR_VALUE;
+    *max_len = a->max_seqlen;
+    *total_chunks = a->total_chunks;
+  }
+  return FLA_OK;
+}
+static SegPlan plan_of(const fla_gdn_chunk_fwd_args* a, int64_t total_chunks, int N, int max_len) {
+  SegPlan whole;
+  whole.count = N;
+  if (a->s_img.data && !a->seg_m.data) return whole;      // the backward has to find the same segments' M
+  return gdn_segments(N, total_chunks, max_len, a->cu_seqlens.data != nullptr, a->v.shape[2], a->v.shape[3]);
+}
+
+// Size of the seg_m buffer a training forward keeps for its backward (0: the chains of this shape are not split).
+extern "C" FLA_API int fla_b200_gdn_chunk_segments_size(const fla_gdn_chunk_fwd_args* a, uint64_t* bytes) {
+  if (!a || !bytes) return FLA_ERR_NULL;
+  if (!a->q.data || a->q.ndim != 4 || !a->v.data || a->v.ndim != 4) return FLA_ERR_SHAPE;
+  int64_t total_chunks; int N, max_len;
+  if (int st = geometry(a, &total_chunks, &N, &max_len)) return st;
+  const SegPlan plan = gdn_segments(N, total_chunks, max_len, a->cu_seqlens.data != nullptr, a->v.shape[2], a->v.shape[3]);
+  *bytes = plan.split ? uint64_t(plan.count) * a->v.shape[2] * kSegMBytes : 0;
+  return FLA_OK;
+}
+
 static int check_token_tensor(const fla_tensor_t& t, int64_t heads, int64_t dim, int dtype_a, int dtype_b) {
   // [B, T, H, D] with D contiguous, rows 16-byte aligned, and batch rows laid out back to back
   if (!t.data) return FLA_ERR_NULL;
@@ -282,14 +326,20 @@ static int check_gate_tensor(const fla_tensor_t& t, int64_t B, int64_t T, int64_
   return FLA_OK;
 }
 
+static uint64_t workspace_bytes_of(const fla_gdn_chunk_fwd_args* a, int64_t chunks, const SegPlan& plan) {
+  const uint64_t HV = a->v.shape[2];
+  uint64_t b = 256 + uint64_t(chunks) * HV * (a->p_img.data ? 0 : kPImgBytes);
+  if (plan.split) b += uint64_t(plan.count) * HV * ((a->seg_m.data ? 0 : kSegMBytes) + kSegHBytes * (a->v.shape[3] / 128));
+  return b;
+}
 extern "C" FLA_API int fla_b200_gdn_chunk_fwd_workspace_size(const fla_gdn_chunk_fwd_args* a, uint64_t* bytes) {
   if (!a || !bytes) return FLA_ERR_NULL;
   if (!a->q.data || a->q.ndim != 4 || !a->v.data || a->v.ndim != 4) return FLA_ERR_SHAPE;
-  int64_t chunks = a->q.shape[0] * ((a->q.shape[1] + kC - 1) / kC);
-  if (a->cu_seqlens.data) chunks = a->total_chunks;
+  int64_t chunks; int N, max_len;
+  if (int st = geometry(a, &chunks, &N, &max_len)) return st;
   if (chunks <= 0) return FLA_ERR_VALUE;
-  // status block + P panels (unless the caller keeps them for the backward)
-  *bytes = 256 + uint64_t(chunks) * a->v.shape[2] * (a->p_img.data ? 0 : kPImgBytes);
+  // status block + P panels (unless the caller keeps them for the backward) + M and H of the segments of split chains
+  *bytes = workspace_bytes_of(a, chunks, plan_of(a, chunks, N, max_len));
   return FLA_OK;
 }
 
@@ -315,15 +365,10 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
   if (!(a->scale == a->scale)) return FLA_ERR_VALUE;
 
-  int N = int(B);
-  int64_t total_chunks = B * ((T + kC - 1) / kC);
-  if (a->cu_seqlens.data) {
-    if (B != 1 || a->cu_seqlens.dtype != FLA_I32 || a->cu_seqlens.ndim != 1 || a->cu_seqlens.shape[0] < 2) return FLA_ERR_SHAPE;
-    N = int(a->cu_seqlens.shape[0] - 1);
-    if (!a->chunk_offsets.data || a->chunk_offsets.dtype != FLA_I32 || a->chunk_offsets.shape[0] != N + 1) return FLA_ERR_SHAPE;
-    if (a->max_seqlen <= 0 || a->max_seqlen > T || a->total_chunks <= 0) return FLA_ERR_VALUE;
-    total_chunks = a->total_chunks;
-  }
+  int N, max_len;
+  int64_t total_chunks;
+  if ((st = geometry(a, &total_chunks, &N, &max_len))) return st;
+  const SegPlan plan = plan_of(a, total_chunks, N, max_len);
   const fla_tensor_t &gam = a->gam, &X = a->x_inv;
   if (!gam.data || !X.data) return FLA_ERR_NULL;
   if (gam.dtype != FLA_F32 || gam.ndim != 3 || gam.shape[0] != B || gam.shape[1] != T || gam.shape[2] != HV ||
@@ -363,13 +408,26 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   p.status = static_cast<int*>(workspace);
   {
     const uint64_t per = uint64_t(total_chunks) * HV;
-    if (workspace_bytes < 256 + per * (a->p_img.data ? 0 : kPImgBytes)) return FLA_ERR_WORKSPACE;
+    if (workspace_bytes < workspace_bytes_of(a, total_chunks, plan)) return FLA_ERR_WORKSPACE;
     if (a->p_img.data) {
       const fla_tensor_t& pi = a->p_img;
       if (pi.dtype != FLA_BF16 || pi.ndim != 1 || pi.shape[0] != int64_t(per) * kPImg || !aligned16(pi.data)) return FLA_ERR_SHAPE;
       p.p_img = static_cast<bf16*>(pi.data);
     } else {
       p.p_img = reinterpret_cast<bf16*>(static_cast<uint8_t*>(workspace) + 256);
+    }
+    p.seg_len = plan.len;
+    if (plan.split) {
+      uint8_t* ws = static_cast<uint8_t*>(workspace) + 256 + (a->p_img.data ? 0 : per * kPImgBytes);
+      if (a->seg_m.data) {
+        if (a->seg_m.dtype != FLA_BF16 || a->seg_m.ndim != 1 || uint64_t(a->seg_m.shape[0]) * 2 < uint64_t(plan.count) * HV * kSegMBytes || !aligned16(a->seg_m.data))
+          return FLA_ERR_SHAPE;
+        p.seg_m = static_cast<bf16*>(a->seg_m.data);
+      } else {
+        p.seg_m = reinterpret_cast<bf16*>(ws);
+        ws += uint64_t(plan.count) * HV * kSegMBytes;
+      }
+      p.seg_h = reinterpret_cast<float*>(ws);
     }
   }
 
@@ -395,8 +453,9 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   std::atomic<bool>& attr_done = attr_done_dev[dev];
   if (!attr_done) {
     if (cudaFuncSetAttribute(gdn_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem) != cudaSuccess) return FLA_ERR_CUDA;
-    if (cudaFuncSetAttribute(gdn_scan_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kScanFwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
-    if (cudaFuncSetAttribute(gdn_scan_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kScanFwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
+    for (auto* scan : {gdn_scan_fwd_kernel<kScanInfer, false>, gdn_scan_fwd_kernel<kScanSave, false>, gdn_scan_fwd_kernel<kScanInfer, true>,
+                       gdn_scan_fwd_kernel<kScanSave, true>, gdn_scan_fwd_kernel<kScanState, true>})
+      if (cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kScanFwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     attr_done = true;
   }
   {
@@ -415,9 +474,12 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   if (make_row_tile_map(&tm_v, p.v, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.v_sh), uint64_t(p.v_st))) return FLA_ERR_CUDA;
   {
     KernelTimer kt("gdn_fwd", cs);
-    const dim3 grid(unsigned(V / 128), unsigned(HV), N);
-    if (p.s_img) gdn_scan_fwd_kernel<true><<<grid, kFwdThreads, kScanFwdSmem + 1024, cs>>>(p, tm_q, tm_k, tm_v);
-    else gdn_scan_fwd_kernel<false><<<grid, kFwdThreads, kScanFwdSmem + 1024, cs>>>(p, tm_q, tm_k, tm_v);
+    const unsigned heads = unsigned(HV * (V / 128));
+    if (plan.split)
+      gdn_scan_fwd_kernel<kScanState, true><<<dim3(heads, unsigned(plan.count), 2), kFwdThreads, kScanFwdSmem + 1024, cs>>>(p, tm_q, tm_k, tm_v);
+    auto* scan = plan.split ? (p.s_img ? gdn_scan_fwd_kernel<kScanSave, true> : gdn_scan_fwd_kernel<kScanInfer, true>)
+                            : (p.s_img ? gdn_scan_fwd_kernel<kScanSave, false> : gdn_scan_fwd_kernel<kScanInfer, false>);
+    scan<<<dim3(heads, unsigned(plan.count)), kFwdThreads, kScanFwdSmem + 1024, cs>>>(p, tm_q, tm_k, tm_v);
   }
   return cuda_status(cudaGetLastError());
 }

@@ -15,8 +15,12 @@
 // the thread that owns the channel (coalesced):
 //     ds_img  dS' as [64-channel half][value | residual][16 strips of 8 key dims][64 rows x 16 bytes]   = 64 KB
 //     dz_img  [64-channel half][dO^T | dZ^T | residual of dZ^T][8 strips of 8 tokens][64 rows x 16 bytes] = 48 KB
+//
+// Split chains (scan_segments.cuh): a state-only pass gives each segment's dH (the gradient that leaves it on the left when none enters on
+// the right; the last segment starts from dht), the walk to a segment's own start goes through the transposes of the forward's M.
 #pragma once
 #include "scan_common.cuh"
+#include "scan_segments.cuh"
 
 namespace fla {
 
@@ -39,6 +43,8 @@ constexpr uint32_t bD = 163840;              // 2 x 16 KB: dO rows, same layout
 constexpr uint32_t bO = 196608;              // 16 KB: dV rows on their way out
 constexpr uint32_t bI = 212992;              // 8 KB: identity panel
 constexpr uint32_t kScanBwdSmem = 221184;
+// the image of M during the walk: four pieces of 16 KB in the buffers of odd steps
+__host__ __device__ constexpr uint32_t bwd_walk_piece(int i) { return i < 2 ? bQK + 32768 + i * 16384 : i == 2 ? bX + 16384 : bP + 16384; }
 
 struct ScanBwdBars {
   uint64_t *mma_bar, *qk_bar, *x_bar, *p_bar, *v_bar, *d_bar;
@@ -60,6 +66,7 @@ __device__ __forceinline__ bool scan_bwd_mma1(uint32_t tbase, uint32_t sb, int s
   mma_commit(bars.mma_bar, lead);
   return dead;
 }
+template <bool kState>
 __device__ __forceinline__ bool scan_bwd_mma2(uint32_t tbase, uint32_t sb, int s, ScanBwdBars bars, int* status, bool dead, uint32_t lead) {
   const int b = s & 1;
   const uint32_t ph = (s >> 1) & 1;
@@ -70,11 +77,13 @@ __device__ __forceinline__ bool scan_bwd_mma2(uint32_t tbase, uint32_t sb, int s
   mma_tile_ts(tbase + uW, tbase + uDVh, opXh, 64, 4, false, lead);
   mma_tile_ts(tbase + uW, tbase + uDVl, opXh, 64, 4, true, lead);
   mma_tile_ts(tbase + uW, tbase + uDVh, opXl, 64, 4, true, lead);
-  if (!dead && !mbar_wait(&bars.v_bar[b], ph, status, FLA_ERR_TIMEOUT)) dead = true;
   const Operand opI{sb + bI, 8192, 0};
   const Operand opDt{sb + bD + b * 16384, 8192, 1}, opVt{sb + bV + b * 16384, 8192, 1};
   mma_tile(tbase + uU, opDt, opI, 128, 64, 4, false, lead);                // dO^T, exact
-  mma_tile(tbase + uVT, opVt, opI, 128, 64, 4, false, lead);               // V^T, exact
+  if (!kState) {
+    if (!dead && !mbar_wait(&bars.v_bar[b], ph, status, FLA_ERR_TIMEOUT)) dead = true;
+    mma_tile(tbase + uVT, opVt, opI, 128, 64, 4, false, lead);             // V^T, exact
+  }
   mma_commit(bars.mma_bar, lead);
   return dead;
 }
@@ -85,6 +94,22 @@ __device__ __forceinline__ bool scan_bwd_mma3(uint32_t tbase, uint32_t sb, int s
   mma_tile_ts(tbase + uDS, tbase + uAh, opQK, 128, 8, true, lead);
   mma_tile_ts(tbase + uDS, tbase + uAl, opQK, 128, 8, true, lead);
   mma_commit(bars.mma_bar, lead);
+  return dead;
+}
+
+// One product of the walk over later segments: D^T = dS^T M, into the accumulators of W1 and U1 (64 start dims each)
+__device__ __forceinline__ bool scan_bwd_walk(uint32_t tbase, uint32_t sb, uint64_t* m_bar, uint32_t ph, uint64_t* mma_bar, int* status, bool dead, uint32_t lead) {
+  tc_fence_after();
+  if (!dead && !mbar_wait(m_bar, ph, status, FLA_ERR_TIMEOUT)) dead = true;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const Operand mh{sb + bwd_walk_piece(half * 2), 1024, 3}, ml{sb + bwd_walk_piece(half * 2 + 1), 1024, 3};
+    const uint32_t d = tbase + uW + half * 64;
+    mma_tile_ts(d, tbase + uAh, mh, 64, 8, false, lead);
+    mma_tile_ts(d, tbase + uAl, mh, 64, 8, true, lead);
+    mma_tile_ts(d, tbase + uAh, ml, 64, 8, true, lead);
+  }
+  mma_commit(mma_bar, lead);
   return dead;
 }
 
@@ -103,6 +128,7 @@ __device__ __forceinline__ float warp_transpose_reduce32(float* x, int lane) {
   return x[0];
 }
 
+template <bool kState, bool kSplit>     // kState: dH of a segment only.  kSplit: chains are split (whole chains have an instance without the walk)
 __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdParams p, const __grid_constant__ CUtensorMap tm_q,
                                                                         const __grid_constant__ CUtensorMap tm_k,
                                                                         const __grid_constant__ CUtensorMap tm_v,
@@ -111,22 +137,27 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ ScanFactors fac[3];
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(8) uint64_t mma_bar, qk_bar[2], x_bar[2], p_bar[2], v_bar[2], d_bar[2], f_bar[3];
+  __shared__ __align__(8) uint64_t mma_bar, m_bar, qk_bar[2], x_bar[2], p_bar[2], v_bar[2], d_bar[2], f_bar[3];
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int vb = blockIdx.x, hv = blockIdx.y, n = blockIdx.z + p.n0;
+  const int seg = blockIdx.y + p.n0, hv = blockIdx.x / (p.V / 128), vb = blockIdx.x % (p.V / 128);   // neighbours share q, k: heads first
   const int hk = hv / (p.HV / p.HK);
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
+  if (tid == 0) clear_status(p.status, seg + blockIdx.x == 0 && (kState || !kSplit));   // the backward's first kernel
+  SegPos pos;
+  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos)) return;
+  if (kState && pos.s == 0) return;
+  const SeqInfo& sq = pos.sq;
+  const int n = pos.n;
   const uint32_t sb = smem_u32(smem);
-  const int nt = sq.nt;
+  const int nt = pos.nt;
 
   if (warp == 0) {
     tmem_alloc(&tmem_base_s, 512);
     tmem_relinquish();
   }
   if (tid == 0) {
-    clear_status(p.status, vb + hv + n == 0);
     mbar_init(&mma_bar, 1);
+    mbar_init(&m_bar, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&qk_bar[i], 1);
       mbar_init(&x_bar[i], 1);
@@ -163,9 +194,11 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
       bulk_load(sb + bP + b * 16384, p.p_img + ((int64_t(sq.cbase) + c) * p.HV + hv) * kPImg, 16384, &p_bar[b]);
       mbar_arrive_expect_tx(&x_bar[b], 16384);
       bulk_load(sb + bX + b * 16384, p.X + ((int64_t(sq.cbase) + c) * p.HV + hv) * 8192, 16384, &x_bar[b]);
-      mbar_arrive_expect_tx(&v_bar[b], 16384);
-      tma_load_tile(sb + bV + b * 16384, &tm_v, vb * 128, hv, row0, &v_bar[b]);
-      tma_load_tile(sb + bV + b * 16384 + 8192, &tm_v, vb * 128 + 64, hv, row0, &v_bar[b]);
+      if (!kState) {
+        mbar_arrive_expect_tx(&v_bar[b], 16384);
+        tma_load_tile(sb + bV + b * 16384, &tm_v, vb * 128, hv, row0, &v_bar[b]);
+        tma_load_tile(sb + bV + b * 16384 + 8192, &tm_v, vb * 128 + 64, hv, row0, &v_bar[b]);
+      }
     };
     // the per-token factors of step s (chunk nt - 1 - s; made by the prep kernel, behind the chunk's P tile) into buffer s % 3
     auto load_factors = [&](int s) {
@@ -186,6 +219,19 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
       load_factors(1);
     }
     __syncwarp();
+    if (kSplit && !kState) {      // the images of the later segments' M, one at a time (scan_bwd_walk)
+      for (int i = pos.ns - 2; i > pos.s; --i) {
+        if (lane == 0) {
+          const bf16* img = p.seg_m + (int64_t(seg - pos.s + i) * p.HV + hv) * 32768;
+          mbar_arrive_expect_tx(&m_bar, 65536);
+#pragma unroll
+          for (int piece = 0; piece < 4; ++piece) bulk_load(sb + bwd_walk_piece(piece), img + piece * 8192, 16384, &m_bar);
+        }
+        __syncwarp();
+        scan_sync();                                        // the gradient's operand copy is in place
+        scan_sync();                                        // the product has been read
+      }
+    }
     scan_sync();   // (pairs with the epilogue warps' barrier after they have loaded the final-state gradient)
     for (int s = 0; s < nt; ++s) {
       scan_sync();                                          // sync 1: step s - 1 no longer reads the other buffers
@@ -213,16 +259,63 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
   const int k_lo = half * 64;
   uint32_t mphase = 0;
 
+  auto seg_dh = [&](int i) -> float* {      // dH of segment i of my sequence, at my channel's first key dim
+    return p.seg_dh + ((int64_t(seg - pos.s + i) * p.HV + hv) * (p.V / 128) + vb) * (kK * 128) + k_lo * 128 + vrow;
+  };
   {   // dht (or zero) into the accumulator columns
-    const float* src = p.dht ? p.dht + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow : nullptr;
+    const float* src = nullptr;
+    int64_t ld = p.V;
+    if (!kSplit || pos.s + 1 == pos.ns) {
+      if (p.dht) src = p.dht + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow;
+    } else if (!kState) {         // what left the last segment
+      src = seg_dh(pos.ns - 1);
+      ld = 128;
+    }
 #pragma unroll
     for (int part = 0; part < 4; ++part) {
       float s16[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) s16[i] = src ? src[int64_t(part * 16 + i) * p.V] : 0.f;
+      for (int i = 0; i < 16; ++i) s16[i] = src ? src[int64_t(part * 16 + i) * ld] : 0.f;
       tmem_st16(tlane + uDS + k_lo + part * 16, s16);
     }
     tmem_st_wait();
+  }
+  if (kSplit && !kState) {
+    for (int i = pos.ns - 2; i > pos.s; --i) {              // dS <- M_i^T dS + dH_i
+#pragma unroll 1
+      for (int part = 0; part < 4; ++part) {
+        float s16[16];
+        uint32_t hi[8], lo[8];
+        tmem_ld16(tlane + uDS + k_lo + part * 16, s16);
+        tmem_ld_wait();
+        split16(s16, hi, lo);
+        tmem_st8u(tlane + uAh + half * 32 + part * 8, hi);
+        tmem_st8u(tlane + uAl + half * 32 + part * 8, lo);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      scan_sync();
+      tc_fence_after();
+      if (warp_u == 0) dead = scan_bwd_walk(tbase_u, sb_u, &m_bar, (pos.ns - 2 - i) & 1, &mma_bar, p.status, dead, elect_one());
+      const float* src = seg_dh(i);
+      float h[64];
+#pragma unroll
+      for (int k = 0; k < 64; ++k) h[k] = src[k * 128];
+      wait_or_mark(&mma_bar, mphase, dead, p.status);
+      tc_fence_after();
+#pragma unroll
+      for (int part = 0; part < 4; ++part) {
+        float s16[16];
+        tmem_ld16(tlane + uW + k_lo + part * 16, s16);
+        tmem_ld_wait();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s16[k] += h[part * 16 + k];
+        tmem_st16(tlane + uDS + k_lo + part * 16, s16);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      scan_sync();
+    }
   }
   // The dO rows of a ragged last chunk that lie past the end of the sequence belong to whatever follows in memory: they
   // are zeroed in shared memory (every other operand meets a zero row of beta or of dVn there).
@@ -266,7 +359,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
         split16(s16, hi, lo);
         tmem_st8u(tlane + uAh + half * 32 + g4 * 8, hi);
         tmem_st8u(tlane + uAl + half * 32 + g4 * 8, lo);
-        {   // the dS' image for the chunk-parallel kernel: strips half * 8 + g4 * 2 and the next one of my channel's row
+        if (!kState) {   // the dS' image for the chunk-parallel kernel: strips half * 8 + g4 * 2 and the next one of my channel's row
           uint8_t* dst = s_row + (half * 8 + g4 * 2) * 1024;
           *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
           *reinterpret_cast<uint4*>(dst + 1024) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
@@ -316,7 +409,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
     tc_fence_before();
     scan_sync();                                   // sync 2
     tc_fence_after();
-    if (warp_u == 0) dead = scan_bwd_mma2(tbase_u, sb_u, s, bars, p.status, dead, elect_one());
+    if (warp_u == 0) dead = scan_bwd_mma2<kState>(tbase_u, sb_u, s, bars, p.status, dead, elect_one());
     wait_or_mark(&mma_bar, mphase, dead, p.status);
     tc_fence_after();
 
@@ -329,12 +422,12 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
       for (int g = 0; g < 2; ++g) {
         float dz[16], t16[16];
         tmem_ld16(tlane + uW + t_lo + g * 16, dz);
-        tmem_ld16(tlane + uVT + t_lo + g * 16, t16);     // V^T
+        if (!kState) tmem_ld16(tlane + uVT + t_lo + g * 16, t16);     // V^T
         tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) pr[g * 16 + i] = dz[i] * t16[i];
         uint32_t w8[8];
-        {
+        if (!kState) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) pr[g * 16 + i] = dz[i] * t16[i];
           uint32_t zl[8];
           split16(dz, w8, zl);     // dZ as value + residual: dA = -tril(dZ Vn^T) feeds dk, dg, dbeta through cancelling sums
           *reinterpret_cast<uint4*>(img + 8192 + (half * 4 + g * 2) * 1024) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
@@ -357,9 +450,11 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
         tmem_st8u(tlane + uAl + 32 + half * 16 + g * 8, lo);
         tmem_ld16(tlane + uU + t_lo + g * 16, t16);       // dO^T
         tmem_ld_wait();
-        pack16(t16, w8);                                  // exact: these are the bf16 inputs
-        *reinterpret_cast<uint4*>(img + (half * 4 + g * 2) * 1024) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
-        *reinterpret_cast<uint4*>(img + (half * 4 + g * 2 + 1) * 1024) = make_uint4(w8[4], w8[5], w8[6], w8[7]);
+        if (!kState) {
+          pack16(t16, w8);                                // exact: these are the bf16 inputs
+          *reinterpret_cast<uint4*>(img + (half * 4 + g * 2) * 1024) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
+          *reinterpret_cast<uint4*>(img + (half * 4 + g * 2 + 1) * 1024) = make_uint4(w8[4], w8[5], w8[6], w8[7]);
+        }
 #pragma unroll
         for (int i4 = 0; i4 < 16; i4 += 4) {
           const float4 s4 = *reinterpret_cast<const float4*>(&f.se[t_lo + g * 16 + i4]);
@@ -372,28 +467,32 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
       }
       tmem_st_wait();
       // sum over my warp's 32 channels of dZ V for each of my 32 tokens; lane l ends up with token t_lo + l
-      const float bzsum = warp_transpose_reduce32(pr, lane);
-      if (t_lo + lane < rows)
-        p.bz[(int64_t(vb * 4 + quad) * p.total_tokens + int64_t(sq.bos) + c * kC + t_lo + lane) * p.HV + hv] = bzsum;
+      if (!kState) {
+        const float bzsum = warp_transpose_reduce32(pr, lane);
+        if (t_lo + lane < rows)
+          p.bz[(int64_t(vb * 4 + quad) * p.total_tokens + int64_t(sq.bos) + c * kC + t_lo + lane) * p.HV + hv] = bzsum;
+      }
     }
     tc_fence_before();
     scan_sync();                                   // sync 3
     tc_fence_after();
     if (warp_u == 0) dead = scan_bwd_mma3(tbase_u, sb_u, s, bars, dead, elect_one());
-    store_dv(c);                                   // while the state-gradient update runs
+    if (!kState) store_dv(c);                      // while the state-gradient update runs
     wait_or_mark(&mma_bar, mphase, dead, p.status);
     tc_fence_after();
   }
 
-  if (!dead && p.dh0) {
-    float* dst = p.dh0 + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow;
+  float* dst = kState ? seg_dh(pos.s)
+                      : p.dh0 && (!kSplit || pos.s == 0) ? p.dh0 + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow : nullptr;
+  const int64_t ld = kState ? 128 : p.V;
+  if (!dead && dst) {
 #pragma unroll
     for (int part = 0; part < 4; ++part) {
       float s16[16];
       tmem_ld16(tlane + uDS + k_lo + part * 16, s16);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) dst[int64_t(part * 16 + i) * p.V] = s16[i];
+      for (int i = 0; i < 16; ++i) dst[int64_t(part * 16 + i) * ld] = s16[i];
     }
   }
   tc_fence_before();

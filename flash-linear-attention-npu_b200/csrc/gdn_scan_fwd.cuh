@@ -17,8 +17,12 @@
 // apart, had to be staged in shared memory and written by bulk copies: 0.83 ms per launch against 0.7x ms.
 //     s_img   [64-channel half][value | residual][16 strips of 8 key dims][64 rows x 16 bytes]   = 64 KB
 //     vn_img  [64-channel half][value | residual][8 strips of 8 tokens][64 rows x 16 bytes]      = 32 KB
+//
+// Long chains may be split into segments (scan_segments.cuh): the kernel then also runs as the state-only pass that gives each
+// segment's M and H.
 #pragma once
 #include "scan_common.cuh"
+#include "scan_segments.cuh"
 
 namespace fla {
 
@@ -41,6 +45,9 @@ constexpr uint32_t sV = 131072;              // 2 x 16 KB: v rows of the chunk, 
 constexpr uint32_t sO = 163840;              // 16 KB: the chunk's output rows on their way out
 constexpr uint32_t sI = 180224;              // 8 KB: identity panel
 constexpr uint32_t kScanFwdSmem = 188416;
+// four pieces of 16 KB in the buffers of odd chunks, free until chunk 0 is under way
+__host__ __device__ constexpr uint32_t walk_piece(int i) { return i < 2 ? sQK + 32768 + i * 16384 : i == 2 ? sX + 16384 : sP + 16384; }
+enum { kScanInfer = 0, kScanSave = 1, kScanState = 2 };
 
 // Epilogue warps of the forward scan: TMEM lane quadrant = warp % 4, warp / 4 selects which of the kFwdSplit column
 // ranges of a tile the warp owns (64 / kFwdSplit tokens, 128 / kFwdSplit key dims); the helper warp comes after them.
@@ -88,18 +95,27 @@ struct ScanBars {
 // The three batches of products of one chunk.  All of warp 0 runs them and the lane `lead` marks issues: built from
 // warp-uniform values in converged code a product costs a handful of instructions; out of line, or in a branch that one
 // thread takes, it cost some thirty and the tensor pipe waited for its issuer (0.65 -> 0.53 ms for the inference forward).
-__device__ __forceinline__ bool scan_fwd_mma1(uint32_t tbase, uint32_t sb, int c, ScanBars bars, int* status, bool dead, uint32_t lead) {
+template <int kMode>
+__device__ __forceinline__ bool scan_fwd_mma1(uint32_t tbase, uint32_t sb, int c, ScanBars bars, bool values, int* status, bool dead, uint32_t lead) {
   const int b = c & 1;
   const uint32_t ph = (c >> 1) & 1;
   tc_fence_after();
   if (!dead && !mbar_wait(&bars.qk_bar[b], ph, status, FLA_ERR_TIMEOUT)) dead = true;
-  const Operand opKQ{sb + sQK + b * 32768, 16384, 0};
-  mma_tile_ts(tbase + tKQ, tbase + tSAh, opKQ, 128, 8, false, lead);
-  mma_tile_ts(tbase + tKQ, tbase + tSAl, opKQ, 128, 8, true, lead);
+  if (kMode == kScanState) {
+    const Operand opK{sb + sQK + b * 32768 + 8192, 16384, 0};
+    mma_tile_ts(tbase + tKQ + 64, tbase + tSAh, opK, 64, 8, false, lead);
+    mma_tile_ts(tbase + tKQ + 64, tbase + tSAl, opK, 64, 8, true, lead);
+  } else {
+    const Operand opKQ{sb + sQK + b * 32768, 16384, 0};
+    mma_tile_ts(tbase + tKQ, tbase + tSAh, opKQ, 128, 8, false, lead);
+    mma_tile_ts(tbase + tKQ, tbase + tSAl, opKQ, 128, 8, true, lead);
+  }
   // V^T into the columns the decayed v_new of this chunk will occupy later
-  if (!dead && !mbar_wait(&bars.v_bar[b], ph, status, FLA_ERR_TIMEOUT)) dead = true;
-  const Operand opVt{sb + sV + b * 16384, 8192, 1}, opI{sb + sI, 8192, 0};
-  mma_tile(tbase + tVAh, opVt, opI, 128, 64, 4, false, lead);
+  if (kMode != kScanState || values) {
+    if (!dead && !mbar_wait(&bars.v_bar[b], ph, status, FLA_ERR_TIMEOUT)) dead = true;
+    const Operand opVt{sb + sV + b * 16384, 8192, 1}, opI{sb + sI, 8192, 0};
+    mma_tile(tbase + tVAh, opVt, opI, 128, 64, 4, false, lead);
+  }
   mma_commit(bars.mma_bar, lead);
   return dead;
 }
@@ -115,6 +131,7 @@ __device__ __forceinline__ bool scan_fwd_mma2(uint32_t tbase, uint32_t sb, int c
   mma_commit(bars.mma_bar, lead);
   return dead;
 }
+template <int kMode>
 __device__ __forceinline__ bool scan_fwd_mma3(uint32_t tbase, uint32_t sb, int c, ScanBars bars, int* status, bool dead, uint32_t lead) {
   const int b = c & 1;
   tc_fence_after();
@@ -122,6 +139,7 @@ __device__ __forceinline__ bool scan_fwd_mma3(uint32_t tbase, uint32_t sb, int c
   mma_tile_ts(tbase + tST, tbase + tVAh, opK, 128, 4, true, lead);
   mma_tile_ts(tbase + tST, tbase + tVAl, opK, 128, 4, true, lead);
   mma_commit(bars.mma_bar, lead);                                   // the state update: what the next chunk waits for
+  if (kMode == kScanState) return dead;
   if (!dead && !mbar_wait(&bars.p_bar[b], (c >> 1) & 1, status, FLA_ERR_TIMEOUT)) dead = true;
   const uint32_t pp = sb + sP + b * 16384;
   const Operand opPh{pp, 1024, 3}, opPl{pp + 8192, 1024, 3};   // P in strips of 8 columns: N = rows i, reduction along j
@@ -132,7 +150,25 @@ __device__ __forceinline__ bool scan_fwd_mma3(uint32_t tbase, uint32_t sb, int c
   return dead;
 }
 
-template <bool kSave>
+// One product of the walk over earlier segments: D^T = S^T M^T with S^T (value, residual) in tensor memory and the image of M in
+// the buffers of odd chunks (a 64-row half of the start dims: value and residual in two pieces of 16 KB).
+__device__ __forceinline__ bool scan_fwd_walk(uint32_t tbase, uint32_t sb, uint64_t* m_bar, uint32_t ph, uint64_t* mma_bar, int* status, bool dead, uint32_t lead) {
+  tc_fence_after();
+  if (!dead && !mbar_wait(m_bar, ph, status, FLA_ERR_TIMEOUT)) dead = true;
+  const Operand m0h{sb + walk_piece(0), 1024, 2}, m0l{sb + walk_piece(1), 1024, 2}, m1h{sb + walk_piece(2), 1024, 2}, m1l{sb + walk_piece(3), 1024, 2};
+  mma_tile_ts(tbase + tKQ, tbase + tSAh, m0h, 128, 4, false, lead);
+  mma_tile_ts(tbase + tKQ, tbase + tSAl, m0h, 128, 4, true, lead);
+  mma_tile_ts(tbase + tKQ, tbase + tSAh, m0l, 128, 4, true, lead);
+  mma_tile_ts(tbase + tKQ, tbase + tSAh + 32, m1h, 128, 4, true, lead);
+  mma_tile_ts(tbase + tKQ, tbase + tSAl + 32, m1h, 128, 4, true, lead);
+  mma_tile_ts(tbase + tKQ, tbase + tSAh + 32, m1l, 128, 4, true, lead);
+  mma_commit(mma_bar, lead);
+  return dead;
+}
+
+// kScanInfer: outputs only.  kScanSave: outputs and the images the backward reads.  kScanState: a segment's M (blockIdx.z = 1) or H (0) only.
+// kSplit: chains are split; whole chains have an instance without the walk, whose registers cost them 5 % (503 against 479 us, B=8 T=4096 HV=32).
+template <int kMode, bool kSplit>
 __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdParams p, const __grid_constant__ CUtensorMap tm_q,
                                                                         const __grid_constant__ CUtensorMap tm_k,
                                                                         const __grid_constant__ CUtensorMap tm_v) {
@@ -140,14 +176,22 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ ScanFactors fac[3];
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(8) uint64_t mma_bar, o_bar, qk_bar[2], x_bar[2], p_bar[2], v_bar[2], f_bar[3];
+  __shared__ __align__(8) uint64_t mma_bar, o_bar, m_bar, qk_bar[2], x_bar[2], p_bar[2], v_bar[2], f_bar[3];
+  constexpr bool kSave = kMode == kScanSave;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int vb = blockIdx.x, hv = blockIdx.y, n = blockIdx.z;
+  const int seg = blockIdx.y, hv = blockIdx.x / (p.V / 128), vb = blockIdx.x % (p.V / 128);   // neighbours share q, k: heads first
   const int hk = hv / (p.HV / p.HK);
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
+  SegPos pos;
+  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos)) return;
+  const bool values = blockIdx.z == 0;                     // (state-only) H, from the values; else M, from the identity
+  if (kMode == kScanState) {                               // H of every segment but the last, M of those between the first and the last
+    if (pos.s + 1 == pos.ns || (!values && (pos.s == 0 || vb > 0))) return;
+  }
+  const SeqInfo& sq = pos.sq;
+  const int n = pos.n;
   const uint32_t sb = smem_u32(smem);
-  const int nt = sq.nt;
+  const int nt = pos.nt;
 
   if (warp == 0) {
     tmem_alloc(&tmem_base_s, 512);
@@ -156,6 +200,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
   if (tid == 0) {
     mbar_init(&mma_bar, 1);
     mbar_init(&o_bar, 1);
+    mbar_init(&m_bar, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&qk_bar[i], 1);
       mbar_init(&x_bar[i], 1);
@@ -178,21 +223,27 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
     auto load_qk = [&](int c) {
       const int b = c & 1, row0 = sq.bos + c * kC;
       const uint32_t qk = sb + sQK + b * 32768;
-      mbar_arrive_expect_tx(&qk_bar[b], 32768);
-      tma_load_tile(qk, &tm_q, 0, hk, row0, &qk_bar[b]);
-      tma_load_tile(qk + 16384, &tm_q, 64, hk, row0, &qk_bar[b]);
+      mbar_arrive_expect_tx(&qk_bar[b], kMode == kScanState ? 16384 : 32768);
+      if (kMode != kScanState) {
+        tma_load_tile(qk, &tm_q, 0, hk, row0, &qk_bar[b]);
+        tma_load_tile(qk + 16384, &tm_q, 64, hk, row0, &qk_bar[b]);
+      }
       tma_load_tile(qk + 8192, &tm_k, 0, hk, row0, &qk_bar[b]);
       tma_load_tile(qk + 16384 + 8192, &tm_k, 64, hk, row0, &qk_bar[b]);
     };
     auto load_rest = [&](int c) {
       const int b = c & 1, row0 = sq.bos + c * kC;
-      mbar_arrive_expect_tx(&v_bar[b], 16384);
-      tma_load_tile(sb + sV + b * 16384, &tm_v, vb * 128, hv, row0, &v_bar[b]);
-      tma_load_tile(sb + sV + b * 16384 + 8192, &tm_v, vb * 128 + 64, hv, row0, &v_bar[b]);
+      if (kMode != kScanState || values) {
+        mbar_arrive_expect_tx(&v_bar[b], 16384);
+        tma_load_tile(sb + sV + b * 16384, &tm_v, vb * 128, hv, row0, &v_bar[b]);
+        tma_load_tile(sb + sV + b * 16384 + 8192, &tm_v, vb * 128 + 64, hv, row0, &v_bar[b]);
+      }
       mbar_arrive_expect_tx(&x_bar[b], 16384);
       bulk_load(sb + sX + b * 16384, p.X + ((int64_t(sq.cbase) + c) * p.HV + hv) * 8192, 16384, &x_bar[b]);
-      mbar_arrive_expect_tx(&p_bar[b], 16384);
-      bulk_load(sb + sP + b * 16384, p.p_img + ((int64_t(sq.cbase) + c) * p.HV + hv) * kPImg, 16384, &p_bar[b]);
+      if (kMode != kScanState) {
+        mbar_arrive_expect_tx(&p_bar[b], 16384);
+        bulk_load(sb + sP + b * 16384, p.p_img + ((int64_t(sq.cbase) + c) * p.HV + hv) * kPImg, 16384, &p_bar[b]);
+      }
     };
     // the per-token factors of chunk c (made by the prep kernel, behind the chunk's P tile) into buffer c % 3
     auto load_factors = [&](int c) {
@@ -214,6 +265,19 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
       load_factors(1);
     }
     __syncwarp();
+    if (kSplit && kMode != kScanState) {      // the images of the earlier segments' M, one at a time (scan_fwd_walk)
+      for (int i = 1; i < pos.s; ++i) {
+        if (lane == 0) {
+          const bf16* img = p.seg_m + (int64_t(seg - pos.s + i) * p.HV + hv) * 32768;
+          mbar_arrive_expect_tx(&m_bar, 65536);
+#pragma unroll
+          for (int piece = 0; piece < 4; ++piece) bulk_load(sb + walk_piece(piece), img + piece * 8192, 16384, &m_bar);
+        }
+        __syncwarp();
+        scan_sync();                                        // the state's operand copy is in place
+        scan_sync();                                        // the product has been read
+      }
+    }
     scan_sync();   // (pairs with the epilogue warps' barrier after they have loaded the initial state)
     for (int c = 0; c < nt; ++c) {
       scan_sync();                                          // sync 1: chunk c - 1 no longer reads the other buffers
@@ -248,15 +312,63 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
 
   // the initial state goes straight into the accumulator columns: every chunk starts by reading its state from there
   {
-    const float* src = p.h0 ? p.h0 + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow : nullptr;
+    const float* src = nullptr;
+    int64_t ld = p.V;
+    if (!kSplit || pos.s == 0) {
+      if (p.h0) src = p.h0 + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow;
+    } else if (kMode != kScanState) {                       // what segment 0 ended with
+      src = p.seg_h + ((int64_t(seg - pos.s) * p.HV + hv) * (p.V / 128) + vb) * (kK * 128) + k_lo * 128 + vrow;
+      ld = 128;
+    }
 #pragma unroll
     for (int part = 0; part < kFwdKT / 16; ++part) {
       float s16[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) s16[i] = src ? src[int64_t(part * 16 + i) * p.V] : 0.f;
+      for (int i = 0; i < 16; ++i) s16[i] = src ? src[int64_t(part * 16 + i) * ld] : 0.f;
+      if (kMode == kScanState && !values) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s16[i] = k_lo + part * 16 + i == vrow ? 1.f : 0.f;
+      }
       tmem_st16(tlane + tST + k_lo + part * 16, s16);
     }
     tmem_st_wait();
+  }
+  if (kSplit && kMode != kScanState) {
+    for (int i = 1; i < pos.s; ++i) {                       // S <- M_i S + H_i
+#pragma unroll
+      for (int part = 0; part < kFwdKT / 16; ++part) {
+        float s16[16];
+        uint32_t hi[8], lo[8];
+        tmem_ld16(tlane + tST + k_lo + part * 16, s16);
+        tmem_ld_wait();
+        split16(s16, hi, lo);
+        tmem_st8u(tlane + tSAh + cs * (kFwdKT / 2) + part * 8, hi);
+        tmem_st8u(tlane + tSAl + cs * (kFwdKT / 2) + part * 8, lo);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      scan_sync();
+      tc_fence_after();
+      if (warp_u == 0) dead = scan_fwd_walk(tbase_u, sb_u, &m_bar, (i - 1) & 1, &mma_bar, p.status, dead, elect_one());
+      const float* src = p.seg_h + ((int64_t(seg - pos.s + i) * p.HV + hv) * (p.V / 128) + vb) * (kK * 128) + k_lo * 128 + vrow;
+      float h[kFwdKT];
+#pragma unroll
+      for (int k = 0; k < kFwdKT; ++k) h[k] = src[k * 128];
+      wait_or_mark(&mma_bar, mphase, dead, p.status);
+      tc_fence_after();
+#pragma unroll
+      for (int part = 0; part < kFwdKT / 16; ++part) {
+        float s16[16];
+        tmem_ld16(tlane + tKQ + k_lo + part * 16, s16);
+        tmem_ld_wait();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s16[k] += h[part * 16 + k];
+        tmem_st16(tlane + tST + k_lo + part * 16, s16);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      scan_sync();
+    }
   }
   scan_sync();   // factors of chunk 0 are visible
 
@@ -323,7 +435,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
       }
       tmem_st_wait();
     }
-    if (c > 0) {   // the output accumulators of chunk c - 1: into registers before the next product overwrites them
+    if (kMode != kScanState && c > 0) {   // the output accumulators of chunk c - 1: into registers before the next product overwrites them
       wait_or_mark(&o_bar, ophase, dead, p.status);
       tc_fence_after();
       form_o(c - 1);
@@ -331,9 +443,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
     tc_fence_before();
     scan_sync();                                   // sync 1
     tc_fence_after();
-    if (warp_u == 0) dead = scan_fwd_mma1(tbase_u, sb_u, c, bars, p.status, dead, elect_one());
+    if (warp_u == 0) dead = scan_fwd_mma1<kMode>(tbase_u, sb_u, c, bars, values, p.status, dead, elect_one());
     // ---- while [QS^T | KS^T] runs: output rows of chunk c - 1
-    if (c > 0) store_o(c - 1);
+    if (kMode != kScanState && c > 0) store_o(c - 1);
     wait_or_mark(&mma_bar, mphase, dead, p.status);
     tc_fence_after();
 
@@ -343,7 +455,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
       for (int g = 0; g < kFwdTT / 16; ++g) {
         float ks[16], vt[16];
         tmem_ld16(tlane + tKQ + 64 + t_lo + g * 16, ks);
-        tmem_ld16(tlane + tVAh + t_lo + g * 16, vt);
+        if (kMode != kScanState || values) {
+          tmem_ld16(tlane + tVAh + t_lo + g * 16, vt);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) vt[i] = 0.f;
+        }
         tmem_ld_wait();
 #pragma unroll
         for (int i4 = 0; i4 < 16; i4 += 4) {
@@ -379,9 +496,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
 #pragma unroll
         for (int i = 0; i < 16; ++i) vn[i] = (t_lo + g * 16 + i < rows) ? vn[i] : 0.f;
         uint32_t hi[8], lo[8];
-        split16(vn, hi, lo);
-        tmem_st8u(tlane + tZAh + cs * (kFwdTT / 2) + g * 8, hi);
-        tmem_st8u(tlane + tZAl + cs * (kFwdTT / 2) + g * 8, lo);
+        if (kMode != kScanState) {
+          split16(vn, hi, lo);
+          tmem_st8u(tlane + tZAh + cs * (kFwdTT / 2) + g * 8, hi);
+          tmem_st8u(tlane + tZAl + cs * (kFwdTT / 2) + g * 8, lo);
+        }
         if (kSave) {                                 // v_new image: strips t_lo / 8 + g * 2 and the next one
           uint8_t* dst = reinterpret_cast<uint8_t*>(p.vn_img + cidx * 16384) + (vrow >> 6) * 16384 + (cs * (kFwdTT / 8) + g * 2) * 1024 + (vrow & 63) * 16;
           *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -404,26 +523,42 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
     tc_fence_before();
     scan_sync();                                   // sync 3
     tc_fence_after();
-    if (warp_u == 0) dead = scan_fwd_mma3(tbase_u, sb_u, c, bars, p.status, dead, elect_one());
+    if (warp_u == 0) dead = scan_fwd_mma3<kMode>(tbase_u, sb_u, c, bars, p.status, dead, elect_one());
     wait_or_mark(&mma_bar, mphase, dead, p.status);    // the state update has completed (the output product may still run)
     tc_fence_after();
   }
 
-  if (nt > 0) {
+  if (kMode != kScanState && nt > 0) {
     wait_or_mark(&o_bar, ophase, dead, p.status);
     tc_fence_after();
     form_o(nt - 1);
     store_o(nt - 1);
   }
-  if (!dead && p.ht) {
-    float* dst = p.ht + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow;
+  float* dst = p.ht && (!kSplit || pos.s + 1 == pos.ns) ? p.ht + ((int64_t(n) * p.HV + hv) * kK + k_lo) * p.V + vb * 128 + vrow : nullptr;
+  int64_t ld = p.V;
+  if (kMode == kScanState) {
+    dst = values ? p.seg_h + ((int64_t(seg) * p.HV + hv) * (p.V / 128) + vb) * (kK * 128) + k_lo * 128 + vrow : nullptr;
+    ld = 128;
+  }
+  if (!dead && (dst || (kMode == kScanState && !values))) {
 #pragma unroll
     for (int part = 0; part < kFwdKT / 16; ++part) {
       float s16[16];
       tmem_ld16(tlane + tST + k_lo + part * 16, s16);
       tmem_ld_wait();
+      if (kMode == kScanState && !values) {                 // M as an operand image, [64 start dims][value | residual][16 strips of 8 end dims]
+        uint32_t hi[8], lo[8];
+        split16(s16, hi, lo);
+        uint8_t* img = reinterpret_cast<uint8_t*>(p.seg_m + (int64_t(seg) * p.HV + hv) * 32768) + (vrow >> 6) * 32768 + (vrow & 63) * 16 +
+                       (k_lo / 8 + part * 2) * 1024;
+        *reinterpret_cast<uint4*>(img) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(img + 1024) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+        *reinterpret_cast<uint4*>(img + 16384) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint4*>(img + 16384 + 1024) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+      } else {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) dst[int64_t(part * 16 + i) * p.V] = s16[i];
+        for (int i = 0; i < 16; ++i) dst[int64_t(part * 16 + i) * ld] = s16[i];
+      }
     }
   }
   tc_fence_before();

@@ -52,6 +52,13 @@ std::tuple<Tensor, Tensor, GdnSaved> gdn_fwd(const Tensor& q_, const Tensor& k_,
   a.gam = desc(s.gam), a.x_inv = desc(s.x_inv), a.s_img = desc(s.s_img), a.vn_img = desc(s.vn_img), a.p_img = desc(s.p_img);
   a.cu_seqlens = desc(s.geo.cu), a.chunk_offsets = desc(s.geo.co);
   a.scale = float(scale), a.chunk_size = kChunk, a.max_seqlen = int32_t(s.geo.max_len), a.total_chunks = int32_t(s.geo.chunks);
+  if (save) {
+    uint64_t bytes = 0;
+    c10::cuda::CUDAGuard guard(d);
+    ok_or_throw("gdn_chunk_segments_size", lib.gdn_chunk_segments_size(&a, &bytes));
+    if (bytes) s.seg_m = empty({int64_t(bytes / 2)}, at::kBFloat16, d);
+    a.seg_m = desc(s.seg_m);
+  }
   two_phase("gdn_chunk_fwd", lib.gdn_chunk_fwd_workspace_size, lib.gdn_chunk_fwd, a, d, true);
   return {o, ht, s};
 }
@@ -71,7 +78,7 @@ std::vector<Tensor> gdn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, c
          dbeta = empty({B, T, HV}, ty.beta, d), dh0;
   if (want_dh0) dh0 = empty(hs, at::kFloat, d);
   fla_gdn_chunk_bwd_args a{};
-  a.q_rstd = desc(s.q_rstd), a.k_rstd = desc(s.k_rstd);
+  a.q_rstd = desc(s.q_rstd), a.k_rstd = desc(s.k_rstd), a.seg_m = desc(s.seg_m);
   a.q = desc(q), a.k = desc(k), a.v = desc(v), a.beta = desc(beta);
   a.gam = desc(s.gam), a.x_inv = desc(s.x_inv), a.s_img = desc(s.s_img), a.vn_img = desc(s.vn_img), a.p_img = desc(s.p_img);
   a.d_o = desc(d_o), a.dht = desc(dht);
@@ -131,7 +138,7 @@ struct GdnFn : torch::autograd::Function<GdnFn> {
                               out < 0 ? std::nullopt : std::optional<at::ScalarType>(at::ScalarType(out)), l2norm);
     if (in.folded) std::tie(o, ht) = unfold_outputs(o, ht, q.size(0));
     ctx->save_for_backward({l2norm ? s.qn : in.q, l2norm ? s.kn : in.k, in.v, in.beta, s.gam, s.x_inv, s.s_img, s.vn_img, s.p_img, s.q_rstd,
-                            s.k_rstd, s.geo.cu, s.geo.co});
+                            s.k_rstd, s.geo.cu, s.geo.co, s.seg_m});
     auto& m = ctx->saved_data;
     m["geo"] = std::vector<int64_t>{s.geo.N, s.geo.max_len, s.geo.chunks};
     m["types"] = std::vector<int64_t>{int64_t(q.scalar_type()), int64_t(k.scalar_type()), int64_t(v.scalar_type()), int64_t(g.scalar_type()),
@@ -147,7 +154,7 @@ struct GdnFn : torch::autograd::Function<GdnFn> {
     const variable_list sv = ctx->get_saved_variables();
     auto& m = ctx->saved_data;
     const std::vector<int64_t> geo = m["geo"].toIntVector(), ty = m["types"].toIntVector();
-    GdnSaved s{sv[4], sv[5], sv[6], sv[7], sv[8], Tensor(), Tensor(), sv[9], sv[10], Geometry{sv[11], sv[12], geo[0], geo[1], geo[2]}};
+    GdnSaved s{sv[4], sv[5], sv[6], sv[7], sv[8], sv[13], Tensor(), Tensor(), sv[9], sv[10], Geometry{sv[11], sv[12], geo[0], geo[1], geo[2]}};
     const int64_t B = m["fold"].toInt();
     Tensor d_o = grads[0].defined() ? grads[0] : at::zeros(m["o"].toIntVector(), sv[2].options());
     Tensor dht = grads.size() > 1 ? grads[1] : Tensor();

@@ -20,7 +20,7 @@ using at::Tensor;
 #define FLA_HOST_FNS(X)                                                                                                    \
   X(recurrent_gdn_workspace_size) X(recurrent_gdn) X(causal_conv1d_fwd_workspace_size) X(causal_conv1d_fwd)                \
   X(causal_conv1d_bwd_workspace_size) X(causal_conv1d_bwd) X(causal_conv1d_update_workspace_size) X(causal_conv1d_update)  \
-  X(gdn_chunk_fwd_workspace_size) X(gdn_chunk_fwd) X(gdn_chunk_bwd_workspace_size) X(gdn_chunk_bwd)                        \
+  X(gdn_chunk_fwd_workspace_size) X(gdn_chunk_segments_size) X(gdn_chunk_fwd) X(gdn_chunk_bwd_workspace_size) X(gdn_chunk_bwd)                        \
   X(kda_chunk_fwd_workspace_size) X(kda_chunk_fwd) X(kda_chunk_bwd_workspace_size) X(kda_chunk_bwd) X(kda_chunk_saved_size) \
   X(l2norm_fwd) X(l2norm_bwd) X(convert) X(chunk_offsets)
 struct Library {
@@ -152,6 +152,7 @@ Pair recurrent_kda(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
 
 struct GdnSaved {
   Tensor gam, x_inv, s_img, vn_img, p_img;
+  Tensor seg_m;                       // transition matrices of split chains
   Tensor qn, kn, q_rstd, k_rstd;      // normalised rows and their factors, when the operator normalises q and k
   Geometry geo;
 };

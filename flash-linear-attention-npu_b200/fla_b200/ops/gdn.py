@@ -55,10 +55,10 @@ def gdn_chunk_fwd(q, k, v, g, beta, scale, initial_state, output_final_state, cu
                   output_dtype=None):
     """Launch the forward kernels.  Returns (o, final_state, saved) where saved holds gam, X and, when
     `save_for_backward`, the split per-chunk states and v_new that the backward kernels consume."""
-    o, ht, gam, x_inv, s_img, vn_img, p_img, geo = host().gdn_fwd(q, k, v, g, beta, scale, initial_state, output_final_state,
+    o, ht, gam, x_inv, s_img, vn_img, p_img, seg_m, geo = host().gdn_fwd(q, k, v, g, beta, scale, initial_state, output_final_state,
                                                                   cu_seqlens, save_for_backward, output_dtype)
     cu, co, n, max_len, total_chunks = geo
-    return o, ht, dict(gam=gam, x_inv=x_inv, s_img=s_img, vn_img=vn_img, p_img=p_img, cu=cu, co=co, max_len=max_len,
+    return o, ht, dict(gam=gam, x_inv=x_inv, s_img=s_img, vn_img=vn_img, p_img=p_img, seg_m=seg_m, cu=cu, co=co, max_len=max_len,
                        total_chunks=total_chunks, N=n)
 
 
@@ -66,7 +66,7 @@ def gdn_chunk_bwd(q, k, v, beta, saved, do, dht, scale, want_dh0, grad_dtype=Non
     """Launch the backward kernels on the tensors the forward saved.
     Returns (dq, dk, dv, dg, dbeta, dh0 | None); gradients are bf16 unless `grad_dtype` says fp32."""
     s = saved
-    return host().gdn_bwd(q, k, v, beta, s["gam"], s["x_inv"], s["s_img"], s["vn_img"], s["p_img"], s["cu"], s["co"], s["N"],
+    return host().gdn_bwd(q, k, v, beta, s["gam"], s["x_inv"], s["s_img"], s["vn_img"], s["p_img"], s["seg_m"], s["cu"], s["co"], s["N"],
                           s["max_len"], s["total_chunks"], do, dht, scale, want_dh0, *(grad_dtype,) * 5)
 
 

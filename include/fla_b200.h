@@ -225,6 +225,8 @@ FLA_API int fla_b200_causal_conv1d_update(const fla_causal_conv1d_update_args* a
  *   q_norm, k_norm [B, T, HK, 128] bf16 dense and q_rstd, k_rstd [B, T, HK] f32 dense, optional out (all four or none): when given,
  *          the rows of q and k are normalised first, x * rsqrt(sum x^2 + 1e-6) rounded to bf16 (use_qk_l2norm_in_kernel), and left
  *          here with their factors; the backward takes q_norm, k_norm as its q, k
+ *   seg_m [fla_b200_gdn_chunk_segments_size / 2] bf16, optional out (for backward): the transition matrices of the segments into which
+ *          the chains of this shape are split; without it a call that saves for the backward does not split them
  *   cu_seqlens int32 [N+1] device (requires B == 1) with chunk_offsets int32 [N+1] device (prefix sum of
  *   ceil(len/64)), max_seqlen and total_chunks given by the host.  All four are ignored for dense batches.
  * Token tensors need a contiguous last dim, 16-byte aligned rows and batch rows laid out back to back.
@@ -235,12 +237,14 @@ typedef struct fla_gdn_chunk_fwd_args {
   fla_tensor_t o, final_state, gam, x_inv, s_img, vn_img, p_img;
   fla_tensor_t cu_seqlens, chunk_offsets;
   fla_tensor_t q_norm, k_norm, q_rstd, k_rstd;
+  fla_tensor_t seg_m;
   float scale;
   int32_t chunk_size;
   int32_t max_seqlen;
   int32_t total_chunks;
 } fla_gdn_chunk_fwd_args;
 FLA_API int fla_b200_gdn_chunk_fwd_workspace_size(const fla_gdn_chunk_fwd_args* args, uint64_t* bytes);
+FLA_API int fla_b200_gdn_chunk_segments_size(const fla_gdn_chunk_fwd_args* args, uint64_t* bytes);
 FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* args, void* workspace, uint64_t workspace_bytes,
                                    void* stream);
 
@@ -255,6 +259,7 @@ FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* args, void* wor
  *   d_o [B, T, HV, V] bf16;   dht [N, HV, 128, V] f32, optional
  *   dq, dk [B, T, HK, 128], dv [B, T, HV, V], dg, dbeta [B, T, HV]: each bf16 or f32;  dh0 [N, HV, 128, V] f32, optional
  *   dq / dk are summed over the value heads of each GVA group inside the kernel (deterministic).
+ *   seg_m: the forward's, optional
  *   q_rstd, k_rstd [B, T, HK] f32 dense, optional (both or none): q, k are then the normalised rows the forward left, and dq, dk
  *          become the gradients of the rows before the normalisation, rstd (dq - q (q . dq))
  * Workspace (size from the _workspace_size call): status block + state-gradient images + [dO; dZ] images + row sums. */
@@ -263,6 +268,7 @@ typedef struct fla_gdn_chunk_bwd_args {
   fla_tensor_t dq, dk, dv, dg, dbeta, dh0;
   fla_tensor_t cu_seqlens, chunk_offsets;
   fla_tensor_t q_rstd, k_rstd;
+  fla_tensor_t seg_m;
   float scale;
   int32_t chunk_size;
   int32_t max_seqlen;
