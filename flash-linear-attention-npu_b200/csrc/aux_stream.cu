@@ -15,6 +15,12 @@ int sm_count(int dev) {
   return g_sm_count[dev];
 }
 
+int current_sm_count() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  return sm_count(dev);
+}
+
 AuxStream* aux_stream_for(int dev, cudaStream_t user) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(user, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;

@@ -14,6 +14,7 @@ struct AuxStream {
 };
 
 int sm_count(int dev);
+int current_sm_count();      // of the current device
 // nullptr when `user` is being captured, when eight caller streams of the device already have one, or when creation failed
 AuxStream* aux_stream_for(int dev, cudaStream_t user);
 

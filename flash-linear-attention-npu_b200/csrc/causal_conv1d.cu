@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
+#include "aux_stream.h"
 
 namespace fla {
 
@@ -71,9 +72,14 @@ struct ConvFwdParams {
   int64_t y_sh;       // head-first output [B, H, T, D/H]: stride between heads (0 with the [B, T, D] output)
   int y_hd;           // channels per head of the output (D with the [B, T, D] output)
   int B, T, D, nseq, silu;
+  int tile;           // tokens per CTA
+  int f_packed;       // final_state is dense [N, D, W-1] with 16-byte aligned sequences
 };
 
-constexpr int kConvTile = 64;     // tokens per CTA tile
+// Tokens per CTA: 64 (3 rows in 67 are read twice) as long as that gives every SM two CTAs, shorter tiles below: a CTA walks its tokens one
+// group after the other, so a short input in long tiles is a chain of a few memory round trips on a few SMs (100 tokens x 8,192 channels in
+// 64-token tiles: 16 CTAs, 12.8 us).
+constexpr int kConvTile = 64, kConvTileMin = 8;
 constexpr int kConvGroup = 4;     // tokens processed per inner step (independent 16-byte loads in flight); 4 keeps 128 registers = 4 CTAs per SM
 constexpr int kConvThreads = 128;
 
@@ -83,8 +89,8 @@ __global__ void __launch_bounds__(kConvThreads, 4) conv_fwd_kernel(ConvFwdParams
   const int d0 = (blockIdx.x * kConvThreads + threadIdx.x) * 8;
   if (d0 >= p.D) return;
   const int b = blockIdx.z;
-  const int t_begin = blockIdx.y * kConvTile;
-  const int t_end = min(p.T, t_begin + kConvTile);
+  const int t_begin = blockIdx.y * p.tile;
+  const int t_end = min(p.T, t_begin + p.tile);
   if (t_begin >= t_end) return;
 
   float w[W][8], bias[8];
@@ -191,7 +197,16 @@ __global__ void __launch_bounds__(kConvThreads, 4) conv_fwd_kernel(ConvFwdParams
         }
       }
     }
-    if (p.final_state && seg_end == seq_end) {  // the sequence ended in this tile: its last W-1 inputs are the state
+    if (p.final_state && seg_end == seq_end && p.f_packed) {  // the state with taps contiguous: my 8 channels are W - 1 16-byte pieces
+      float flat[8 * (W - 1)];
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int j = 0; j < W - 1; ++j) flat[c * (W - 1) + j] = win[j][c];
+#pragma unroll
+      for (int j = 0; j < W - 1; ++j)
+        *reinterpret_cast<uint4*>(p.final_state + seq * p.f_sn + int64_t(d0) * (W - 1) + j * 8) = pack8f(flat + j * 8);
+    } else if (p.final_state && seg_end == seq_end) {  // the sequence ended in this tile: its last W-1 inputs are the state
 #pragma unroll
       for (int j = 0; j < W - 1; ++j)
 #pragma unroll
@@ -381,13 +396,17 @@ extern "C" FLA_API int fla_b200_causal_conv1d_fwd(const fla_causal_conv1d_fwd_ar
     if (!s.data) continue;
     if (s.ndim != 3 || s.dtype != FLA_BF16 || s.shape[0] != nseq || s.shape[1] != D || s.shape[2] != W - 1)
       return FLA_ERR_SHAPE;
-    if (which) { p.final_state = static_cast<bf16*>(s.data); p.f_sn = s.stride[0]; p.f_sd = s.stride[1]; p.f_sw = s.stride[2]; }
+    if (which) { p.final_state = static_cast<bf16*>(s.data); p.f_sn = s.stride[0]; p.f_sd = s.stride[1]; p.f_sw = s.stride[2];
+      p.f_packed = s.stride[2] == 1 && s.stride[1] == W - 1 && s.stride[0] % 8 == 0 && aligned16(s.data); }
     else { p.init = static_cast<const bf16*>(s.data); p.i_sn = s.stride[0]; p.i_sd = s.stride[1]; p.i_sw = s.stride[2]; }
   }
   p.cu_seqlens = static_cast<const int32_t*>(a->cu_seqlens.data);
   p.B = int(B); p.T = int(T); p.D = int(D); p.nseq = nseq; p.silu = a->activation_silu;
   if (T == 0) return FLA_OK;
-  const dim3 grid(unsigned((D / 8 + kConvThreads - 1) / kConvThreads), unsigned((T + kConvTile - 1) / kConvTile), unsigned(B));
+  const int64_t blocks_d = (D / 8 + kConvThreads - 1) / kConvThreads;
+  p.tile = kConvTile;
+  while (p.tile > kConvTileMin && blocks_d * ((T + p.tile - 1) / p.tile) * B < 2 * current_sm_count()) p.tile /= 2;
+  const dim3 grid(unsigned(blocks_d), unsigned((T + p.tile - 1) / p.tile), unsigned(B));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   KernelTimer kt("causal_conv1d_fwd", st);
 #define FLA_LAUNCH_FWD(WW)                                                                           \

@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
+#include "aux_stream.h"
 
 namespace fla {
 
@@ -39,10 +40,11 @@ struct ConvBwdParams {
   const int32_t* cu_seqlens;
   int64_t x_sb, x_st, dy_sb, dy_st, yp_sb, yp_st, dx_sb, dx_st, w_sd, w_sw;
   int64_t i_sn, i_sd, i_sw, t_sn, t_sd, t_sw, h_sn, h_sd, h_sw;
-  int B, T, D, nseq, dh0_is_f32, tiles_per_row;
+  int B, T, D, nseq, dh0_is_f32, tiles_per_row, tile;
 };
 
-constexpr int kBwdTile = 128;    // tokens per CTA tile
+// Tokens per CTA: 128 as long as that fills two CTAs on every SM, shorter tiles below (8,191 tokens x 2,048 channels: 128 CTAs of 296, 46 us)
+constexpr int kBwdTile = 128, kBwdTileMin = 16;
 constexpr int kBwdThreads = 128;
 
 // derivative of SiLU at pre-activation p: s (1 + p (1 - s)), s = sigmoid(p)
@@ -145,8 +147,8 @@ __global__ void __launch_bounds__(kBwdThreads, 2) conv_bwd_kernel(ConvBwdParams 
   const int d0 = (blockIdx.x * kBwdThreads + threadIdx.x) * 8;
   if (d0 >= p.D) return;
   const int b = blockIdx.z;
-  const int s0 = blockIdx.y * kBwdTile;
-  const int s1 = min(p.T, s0 + kBwdTile);
+  const int s0 = blockIdx.y * p.tile;
+  const int s1 = min(p.T, s0 + p.tile);
   const f2 half2 = mk2(0.5f, 0.5f), one2 = mk2(1.f, 1.f), neg2 = mk2(-1.f, -1.f), zero2 = mk2(0.f, 0.f);
 
   f2 w[W][4], bias[4];
@@ -411,12 +413,22 @@ struct ConvBwdReduceParams {
   int tiles, W, D, dw_f32, db_f32;
 };
 
-__global__ void conv_bwd_reduce_kernel(ConvBwdReduceParams p) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
+// 32 channels x 8 groups of tiles per block: eight loads in flight per channel, added up in a fixed order
+__global__ void __launch_bounds__(256) conv_bwd_reduce_kernel(ConvBwdReduceParams p) {
+  __shared__ float part_s[8][32];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  const int d = blockIdx.x * 32 + lane;
   const int j = blockIdx.y;   // 0 .. W-1: dw tap, W: db
-  if (d >= p.D) return;
   float acc = 0.f;
-  for (int t = 0; t < p.tiles; ++t) acc += p.part[(int64_t(t) * (p.W + 1) + j) * p.D + d];
+  if (d < p.D) {
+#pragma unroll 4
+    for (int t = grp; t < p.tiles; t += 8) acc += p.part[(int64_t(t) * (p.W + 1) + j) * p.D + d];
+  }
+  part_s[grp][lane] = acc;
+  __syncthreads();
+  if (grp || d >= p.D) return;
+#pragma unroll
+  for (int g = 1; g < 8; ++g) acc += part_s[g][lane];
   void* out = j < p.W ? p.dw : p.db;
   const int64_t off = j < p.W ? d * p.dw_sd + j * p.dw_sw : d;
   if (!out) return;
@@ -428,8 +440,15 @@ inline bool vec_ok3(const fla_tensor_t& t) {
   return t.stride[2] == 1 && aligned16(t.data) && t.stride[1] % 8 == 0 && t.stride[0] % 8 == 0;
 }
 
+int bwd_tile(const fla_causal_conv1d_bwd_args* a) {
+  const int64_t B = a->x.shape[0], T = a->x.shape[1], blocks_d = (a->x.shape[2] / 8 + kBwdThreads - 1) / kBwdThreads;
+  int tile = kBwdTile;
+  while (tile > kBwdTileMin && blocks_d * ((T + tile - 1) / tile) * B < 2 * current_sm_count()) tile /= 2;
+  return tile;
+}
 int bwd_tiles(const fla_causal_conv1d_bwd_args* a) {
-  return int((a->x.shape[1] + kBwdTile - 1) / kBwdTile);
+  const int tile = bwd_tile(a);
+  return int((a->x.shape[1] + tile - 1) / tile);
 }
 
 }  // namespace
@@ -496,7 +515,7 @@ extern "C" FLA_API int fla_b200_causal_conv1d_bwd(const fla_causal_conv1d_bwd_ar
   }
   p.cu_seqlens = static_cast<const int32_t*>(a->cu_seqlens.data);
   const int tiles = bwd_tiles(a);
-  p.B = int(B); p.T = int(T); p.D = int(D); p.nseq = nseq; p.tiles_per_row = tiles;
+  p.B = int(B); p.T = int(T); p.D = int(D); p.nseq = nseq; p.tiles_per_row = tiles; p.tile = bwd_tile(a);
   const uint64_t need = uint64_t(B) * tiles * (W + 1) * D * 4;
   if (!workspace || workspace_bytes < need || !aligned16(workspace)) return FLA_ERR_WORKSPACE;
   p.part = static_cast<float*>(workspace);
@@ -514,6 +533,6 @@ extern "C" FLA_API int fla_b200_causal_conv1d_bwd(const fla_causal_conv1d_bwd_ar
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   ConvBwdReduceParams r{p.part, dw.data, db, dw.stride[0], dw.stride[1], int(B) * tiles, int(W), int(D), dw.dtype == FLA_F32, a->db.dtype == FLA_F32};
-  conv_bwd_reduce_kernel<<<dim3(unsigned((D + 255) / 256), unsigned(W + 1)), 256, 0, st>>>(r);
+  conv_bwd_reduce_kernel<<<dim3(unsigned((D + 31) / 32), unsigned(W + 1)), 256, 0, st>>>(r);
   return cuda_status(cudaGetLastError());
 }
