@@ -90,7 +90,7 @@ STAGE_BYTES = {
     "prepare_wy_repr_bwd_group_sum": lambda c: _th(c, "HV", 128, 4) + _th(c, "HK", 128, 2),
 }
 KERNEL_SYMBOL = {"gdn_fwd": "gdn_scan_fwd_kernel", "gdn_bwd_dhu": "gdn_scan_bwd_kernel", "gdn_bwd_par": "gdn_bwd_par_kernel",
-                 "kda_fwd": "kda_fwd_kernel", "kda_prep": "kda_prep_kernel", "kda_bwd_dhu": "kda_bwd_dhu_kernel", "kda_bwd_par": "kda_bwd_par_kernel", "gdn_prep": "gdn_prep_kernel",
+                 "kda_fwd": "kda_scan_fwd_kernel", "kda_prep": "kda_prep_kernel", "kda_bwd_dhu": "kda_scan_bwd_kernel", "kda_bwd_par": "kda_bwd_par_kernel", "gdn_prep": "gdn_prep_kernel",
                  "recurrent_gdn": "recurrent_gdn_kernel", "causal_conv1d_fwd": "conv_fwd_kernel",
                  "causal_conv1d_update": "conv_update1_kernel", "causal_conv1d_bwd": "conv_bwd_kernel",
                  "chunk_local_cumsum": "stage_cumsum_kernel", "chunk_scaled_dot_kkt": "stage_kkt_kernel",
@@ -298,7 +298,7 @@ class Workload:
         c = self.cfg
         if self.name in ("gdn_fwd_bwd", "kda_fwd_bwd") and c["B"] >= 2:
             # the backward launches its two kernels once per half of the batch when its scan has more chains than SMs
-            chains = c["B"] * c["HV"] * (c["V"] // (128 if self.name == "gdn_fwd_bwd" else 64))
+            chains = c["B"] * c["HV"] * (c["V"] // 128)
             if chains > torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count:
                 n += 2
         return n

@@ -493,7 +493,7 @@ static SegPlan bwd_plan(const fla_gdn_chunk_bwd_args* a, int64_t total_chunks, i
   whole.count = N;
   if (!a->seg_m.data) return whole;
   const bool packed = a->cu_seqlens.data != nullptr;
-  return gdn_segments(N, total_chunks, packed ? a->max_seqlen : a->q.shape[1], packed, a->v.shape[2], a->v.shape[3]);
+  return scan_plan(N, total_chunks, packed ? a->max_seqlen : a->q.shape[1], packed, a->v.shape[2], a->v.shape[3]);
 }
 
 extern "C" FLA_API int fla_b200_gdn_chunk_bwd_workspace_size(const fla_gdn_chunk_bwd_args* a, uint64_t* bytes) {

@@ -268,13 +268,6 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
 
 using namespace fla;
 
-// A forward step is 1; a state-only step takes as long (its outputs and score products are off the chain).
-fla::SegPlan fla::gdn_segments(int64_t N, int64_t total_chunks, int64_t max_len, bool packed, int64_t HV, int64_t V) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
-  return plan_segments(N, total_chunks, (max_len + kC - 1) / kC, packed, HV * (V / 128), HV, 1.0, sm_count(dev));
-}
-
 static int geometry(const fla_gdn_chunk_fwd_args* a, int64_t* total_chunks, int* N, int* max_len) {
   const int64_t B = a->q.shape[0], T = a->q.shape[1];
   *N = int(B);
@@ -294,7 +287,7 @@ static SegPlan plan_of(const fla_gdn_chunk_fwd_args* a, int64_t total_chunks, in
   SegPlan whole;
   whole.count = N;
   if (a->s_img.data && !a->seg_m.data) return whole;      // the backward has to find the same segments' M
-  return gdn_segments(N, total_chunks, max_len, a->cu_seqlens.data != nullptr, a->v.shape[2], a->v.shape[3]);
+  return scan_plan(N, total_chunks, max_len, a->cu_seqlens.data != nullptr, a->v.shape[2], a->v.shape[3]);
 }
 
 // Size of the seg_m buffer a training forward keeps for its backward (0: the chains of this shape are not split).
@@ -303,7 +296,7 @@ extern "C" FLA_API int fla_b200_gdn_chunk_segments_size(const fla_gdn_chunk_fwd_
   if (!a->q.data || a->q.ndim != 4 || !a->v.data || a->v.ndim != 4) return FLA_ERR_SHAPE;
   int64_t total_chunks; int N, max_len;
   if (int st = geometry(a, &total_chunks, &N, &max_len)) return st;
-  const SegPlan plan = gdn_segments(N, total_chunks, max_len, a->cu_seqlens.data != nullptr, a->v.shape[2], a->v.shape[3]);
+  const SegPlan plan = scan_plan(N, total_chunks, max_len, a->cu_seqlens.data != nullptr, a->v.shape[2], a->v.shape[3]);
   *bytes = plan.split ? uint64_t(plan.count) * a->v.shape[2] * kSegMBytes : 0;
   return FLA_OK;
 }

@@ -13,10 +13,6 @@ constexpr int kK = 128;    // key head dim
 constexpr int kV = 128;    // value head dim
 constexpr int kBV = 64;    // value columns owned by one CTA of the sequential kernels
 
-struct SegPlan;
-// How both GDN scans split their chains (scan_segments.cuh); the same in the forward and the backward of one call.
-SegPlan gdn_segments(int64_t N, int64_t total_chunks, int64_t max_len, bool packed, int64_t HV, int64_t V);
-
 struct SeqInfo {
   int bos;   // first token (flat index) of the sequence
   int len;   // tokens in the sequence

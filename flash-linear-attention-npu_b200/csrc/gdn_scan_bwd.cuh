@@ -113,21 +113,6 @@ __device__ __forceinline__ bool scan_bwd_walk(uint32_t tbase, uint32_t sb, uint6
   return dead;
 }
 
-// 32 values per lane -> lane l keeps the sum over the warp of value l (recursive halving: 31 shuffles)
-__device__ __forceinline__ float warp_transpose_reduce32(float* x, int lane) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    const bool up = (lane & off) != 0;
-#pragma unroll
-    for (int i = 0; i < off; ++i) {
-      const float send = up ? x[i] : x[i + off];
-      const float keep = up ? x[i + off] : x[i];
-      x[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  return x[0];
-}
-
 template <bool kState, bool kSplit>     // kState: dH of a segment only.  kSplit: chains are split (whole chains have an instance without the walk)
 __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdParams p, const __grid_constant__ CUtensorMap tm_q,
                                                                         const __grid_constant__ CUtensorMap tm_k,

@@ -49,46 +49,6 @@ constexpr uint32_t kScanFwdSmem = 188416;
 __host__ __device__ constexpr uint32_t walk_piece(int i) { return i < 2 ? sQK + 32768 + i * 16384 : i == 2 ? sX + 16384 : sP + 16384; }
 enum { kScanInfer = 0, kScanSave = 1, kScanState = 2 };
 
-// Epilogue warps of the forward scan: TMEM lane quadrant = warp % 4, warp / 4 selects which of the kFwdSplit column
-// ranges of a tile the warp owns (64 / kFwdSplit tokens, 128 / kFwdSplit key dims); the helper warp comes after them.
-// Sixteen warps with a quarter of the columns each against eight with a half: 0.577 -> 0.564 ms (training) and
-// 0.498 -> 0.485 ms (inference); the per-chunk chain is mostly hand-off latency, not epilogue issue.
-constexpr int kFwdSplit = 4;
-constexpr int kFwdEpiWarps = 4 * kFwdSplit, kFwdEpiThreads = 32 * kFwdEpiWarps, kFwdThreads = kFwdEpiThreads + 32;
-constexpr int kFwdTT = 64 / kFwdSplit, kFwdKT = 128 / kFwdSplit;     // tokens / key dims per thread
-__device__ __forceinline__ void fwd_epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kFwdEpiThreads) : "memory"); }
-template <int kRowBytes, int kRows>
-__device__ __forceinline__ void fwd_copy_out_tile(const uint8_t* tile, uint8_t* gbase, int64_t g_row_bytes, int rows, int tid) {
-  constexpr int kPerRow = kRowBytes / 16, kIters = kRows * kPerRow / kFwdEpiThreads;
-#pragma unroll
-  for (int i = 0; i < kIters; ++i) {
-    const int id = tid + i * kFwdEpiThreads, r = id / kPerRow, c16 = id % kPerRow;
-    if (r < rows) *reinterpret_cast<uint4*>(gbase + r * g_row_bytes + c16 * 16) = *reinterpret_cast<const uint4*>(tile + r * kRowBytes + c16 * 16);
-  }
-}
-// Each epilogue thread holds one channel (`vrow`) of kFwdTT tokens (cs * kFwdTT ..) of a [64 tokens][128 channels] result.
-// The tile is transposed through a 16 KB shared-memory buffer: bf16 results in one pass, fp32 results in two (32 tokens each).
-__device__ __forceinline__ void fwd_store_rows_transposed(uint8_t* tile, const float* ov, void* g, int64_t g_row_elems, bool f32, int rows,
-                                                          int cs, int vrow, int tid) {
-  if (f32) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if ((cs * kFwdTT) / 32 == h) {
-#pragma unroll
-        for (int i = 0; i < kFwdTT; ++i) *reinterpret_cast<float*>(tile + ((cs * kFwdTT) % 32 + i) * 512 + vrow * 4) = ov[i];
-      }
-      fwd_epi_sync();
-      fwd_copy_out_tile<512, 32>(tile, reinterpret_cast<uint8_t*>(static_cast<float*>(g) + h * 32 * g_row_elems), g_row_elems * 4, rows - h * 32, tid);
-      fwd_epi_sync();
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kFwdTT; ++i) *reinterpret_cast<bf16*>(tile + (cs * kFwdTT + i) * 256 + vrow * 2) = __float2bfloat16_rn(ov[i]);
-    fwd_epi_sync();
-    fwd_copy_out_tile<256, 64>(tile, static_cast<uint8_t*>(g), g_row_elems * 2, rows, tid);
-  }
-}
-
 struct ScanBars {
   uint64_t *mma_bar, *o_bar, *qk_bar, *x_bar, *p_bar, *v_bar;   // two barriers each (index = chunk parity) but the first two
 };

@@ -7,9 +7,9 @@
 //   gk = chunk cumsum(g), a = gk at the middle token, Qp = Q e^{gk-a}, Kp = K e^{gk-a}, Kn = K e^{a-gk},
 //   P = tril(Qp Kn^T), M = strict_tril(Kp Kn^T), X = (I + beta M)^-1, Sa = diag(e^a) S, D = e^{gk_L-a}:
 //   Vn = X (beta (V - Kp Sa)),  O = scale (Qp Sa + P Vn),  S' = diag(D) (Sa + Kn^T Vn).
-// The entry point recomputes the forward (prep -> inverse -> forward scan, saving Sa and Vn as panel images) and runs
+// The entry point recomputes the forward (prep -> inverse -> forward scan, saving Sa and Vn as strip images) and runs
 //
-//  kda_bwd_dhu_kernel  (reverse-sequential over chunks, one CTA per (sequence, value head, 64-column block of V)):
+//  kda_scan_bwd_kernel  (kda_scan_bwd.cuh; reverse-sequential over chunks, one CTA per (sequence, value head, 128 channels of V)):
 //      dS'a = diag(D) dS'          dVn = scale P^T dO + Kn dS'a          dZ = X^T dVn          dV = beta dZ
 //      dSa  = dS'a + Qp^T (scale dO) + Kp^T (-beta dZ)                   dS = diag(e^a) dSa    dh0 = dS after the first chunk
 //  kda_bwd_par_kernel  (parallel over chunks, one CTA per (chunk, q/k head), looping over the value heads of the group):
@@ -25,6 +25,7 @@
 #include "kernel_timer.h"
 #include "aux_stream.h"
 #include "kda_common.cuh"
+#include "scan_segments.cuh"
 #include "tensor_map.h"
 
 namespace fla {
@@ -37,8 +38,12 @@ struct KdaBwdParams {
   const bf16* qk_img; const bf16* kn_img; const bf16* p_img; const bf16* x_img;
   const float* vec; const float* gk;
   const bf16* s_img; const bf16* vn_img;
-  bf16* ds_img;        // [chunks, HV, V/64, {hi, lo}, 128x64]  dS'a entering each chunk
-  bf16* dz_img;        // [chunks, HV, V/64, {64x64 dO, 64x64 dZ hi, 64x64 dZ lo}]
+  bf16* ds_img;        // [chunks, HV, V/64, {hi, lo}, 16 strips of 8 key dims, 64 channels]  dS'a entering each chunk
+  bf16* dz_img;        // [chunks, HV, V/64, {dO, dZ hi, dZ lo}, 8 strips of 8 tokens, 64 channels]
+  const bf16* seg_m;   // split chains: the forward's transition matrices
+  float* seg_dh;       // split chains: [segments, HV, V/128, 128, 128]
+  int seg_len;         // chunks per segment
+  int clear;           // the scan is the call's first kernel: it clears the status word
   float* bz;           // [V/32, tokens, HV] partial sums of dZ * V over the 32-column slices of V
   const float* dht; float* dh0;
   void* dq; void* dk; void* dv; void* dg; void* dbeta;
@@ -56,300 +61,15 @@ struct KdaBwdParams {
 
 constexpr int64_t kKdaDsImg = 16384, kKdaDzImg = 12288;   // bf16 elements per (chunk, head, 64-column block of V)
 
-// ============================================================================================= dhu
-constexpr uint32_t dOffQKH = 0, dOffQKL = 32768, dOffKNH = 65536, dOffKNL = 81920;
-constexpr uint32_t dOffDSH = 98304, dOffDSL = 114688;     // dS'a hi / lo, later rows 0-63 scale dO, rows 64-127 -beta dZ
-constexpr uint32_t dOffDO = 131072;                        // raw dO rows of this V block
-constexpr uint32_t dOffPH = 139264, dOffPL = 147456;      // P, then dVn, then dZ (hi / lo)
-constexpr uint32_t dOffXH = 155648, dOffXL = 163840;
-constexpr uint32_t kKdaDhuSmem = 172032;
-constexpr uint32_t dColDS = 0, dColW1 = 64, dColDZ = 128, dColU1 = 192;
-
-__global__ void __launch_bounds__(256, 1) kda_bwd_dhu_kernel(KdaBwdParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ float vec_s[2][2][kK];     // [chunk parity][e^a | e^{gk_L - a}][channel]
-  __shared__ float beta_s[2][kC];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(8) uint64_t bar, pbar, qk_bar, kn_bar, x_bar;
-
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int vb = blockIdx.x, hv = blockIdx.y, n = blockIdx.z + p.n0;
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
-  const int quad = warp & 3, half = warp >> 2;   // TMEM lane quadrant; which 32 of the tile's 64 columns
-  const bool kside = quad >= 2;
-  const int row = quad * 32 + lane, tok = row & 63, c0 = half * 32;
-
-  if (warp == 0) {
-    tmem_alloc(&tmem_base_s, 256);
-    tmem_relinquish();
-  }
-  if (tid == 0) {
-    clear_status(p.status, vb + hv + n == 0);
-    mbar_init(&bar, 1);
-    mbar_init(&pbar, 1);
-    mbar_init(&qk_bar, 1);
-    mbar_init(&kn_bar, 1);
-    mbar_init(&x_bar, 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  const uint32_t tbase = tmem_base_s;
-  const uint32_t trow = tmem_addr(tbase, quad * 32, c0);
-  uint32_t phase = 0, pphase = 0, qkphase = 0, knphase = 0, xphase = 0;
-  bool dead = false;
-  const uint32_t sb = smem_u32(smem);
-  auto chunk_head = [&](int c) { return (int64_t(sq.cbase) + c) * p.HV + hv; };
-  auto issue_p_load = [&](int c) {
-    mbar_arrive_expect_tx(&pbar, 16384);
-    bulk_load(sb + dOffPH, p.p_img + chunk_head(c) * kKdaPImg, 16384, &pbar);
-  };
-  auto issue_qk_load = [&](int c) {
-    mbar_arrive_expect_tx(&qk_bar, 65536);
-    bulk_load(sb + dOffQKH, p.qk_img + chunk_head(c) * kKdaQkImg, 65536, &qk_bar);
-  };
-  auto issue_kn_load = [&](int c) {
-    mbar_arrive_expect_tx(&kn_bar, 32768);
-    bulk_load(sb + dOffKNH, p.kn_img + chunk_head(c) * kKdaKnImg, 32768, &kn_bar);
-  };
-  auto issue_x_load = [&](int c) {
-    mbar_arrive_expect_tx(&x_bar, 16384);
-    bulk_load(sb + dOffXH, p.x_img + chunk_head(c) * kKdaXImg, 16384, &x_bar);
-  };
-
-  // per-chunk vectors, beta and my dO / v row travel through registers one chunk ahead
-  float pf_vec = 0.f, pf_beta = 0.f;
-  uint4 pf_row[4], rcur[4];
-  auto prefetch_load = [&](int c) {
-    const int t0 = c * kC;
-    const int rows = min(kC, sq.len - t0);
-    const int64_t tok0 = int64_t(sq.bos) + t0;
-    pf_vec = p.vec[chunk_head(c) * kKdaVecs * kK + tid];      // 256 threads: e^a then e^{gk_L - a}
-    const bf16* rsrc = kside ? p.v + (tok0 + tok) * p.v_st + hv * p.v_sh + vb * kBV + c0
-                             : p.dO + (tok0 + tok) * p.do_st + hv * p.do_sh + vb * kBV + c0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      pf_row[i] = make_uint4(0, 0, 0, 0);
-      if (tok < rows) pf_row[i] = *reinterpret_cast<const uint4*>(rsrc + i * 8);
-    }
-    if (kside) pf_beta = tok < rows ? ld_scalar(p.beta, (tok0 + tok) * p.beta_st + hv, p.beta_is_f32) : 0.f;
-  };
-  auto prefetch_store = [&](int c) {
-    vec_s[c & 1][tid / kK][tid % kK] = pf_vec;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) rcur[i] = pf_row[i];
-    if (kside) {
-      if (half == 0) beta_s[c & 1][tok] = pf_beta;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(smem + dOffDO + panel_chunk_off(tok, half * 4 + i)) = pf_row[i];
-    }
-  };
-
-  const Operand opKnAh{sb + dOffKNH - 8192, 8192, 0}, opKnAl{sb + dOffKNL - 8192, 8192, 0};   // Kn as A, valid rows 64..127
-  const Operand opDSH{sb + dOffDSH, 16384, 1}, opDSL{sb + dOffDSL, 16384, 1};
-  const Operand opPTh{sb + dOffPH - 8192, 8192, 1}, opPTl{sb + dOffPL - 8192, 8192, 1};       // P^T, valid rows 64..127
-  const Operand opDO{sb + dOffDO, 8192, 1};
-  const Operand opXTh{sb + dOffXH - 8192, 8192, 1}, opXTl{sb + dOffXL - 8192, 8192, 1};       // X^T, valid rows 64..127
-  const Operand opDVh{sb + dOffPH, 8192, 1}, opDVl{sb + dOffPL, 8192, 1};
-  const Operand opQKTh{sb + dOffQKH, 16384, 1}, opQKTl{sb + dOffQKL, 16384, 1};               // [Qp^T | Kp^T]
-
-  float srow[32];   // this thread's 32 columns of the fp32 state-gradient row (row = key channel)
-  const int c_last = sq.nt - 1;
-  if (sq.nt > 0) {   // a sequence without tokens requests nothing: dh0 = dht below
-    if (tid == 0) {
-      issue_kn_load(c_last);
-      issue_p_load(c_last);
-      issue_x_load(c_last);
-      issue_qk_load(c_last);
-    }
-    prefetch_load(c_last);
-    prefetch_store(c_last);
-  }
-  if (p.dht) {
-    const float* src = p.dht + ((int64_t(n) * p.HV + hv) * kK + row) * p.V + vb * kBV + c0;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      const float4 t = *reinterpret_cast<const float4*>(src + i);
-      srow[i] = t.x; srow[i + 1] = t.y; srow[i + 2] = t.z; srow[i + 3] = t.w;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) srow[i] = 0.f;
-  }
-  __syncthreads();
-
-  for (int c = c_last; c >= 0; --c) {
-    const int cur = c & 1;
-    const int t0 = c * kC;
-    const int rows = min(kC, sq.len - t0);
-    const int64_t tok0 = int64_t(sq.bos) + t0;
-    const int64_t cidx = chunk_head(c);
-
-    // ---- stage 0: dS'a = diag(e^{gk_L - a}) dS' as split copy (MMA operand and image) and as the fp32 master in TMEM
-    {
-      const float el = vec_s[cur][1][row];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) srow[i] *= el;
-      row32_to_hilo(smem + dOffDSH, smem + dOffDSL, row, half, srow);
-      tmem_st_row32(trow + dColDS, srow);
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-
-    // ---- stage 1: W1 = Kn dS'a  and  U1 = P^T dO  (valid accumulator rows 64..127)
-    if (tid == 0) {
-      bulk_store(p.ds_img + (cidx * p.nvb + vb) * 16384, sb + dOffDSH, 32768);
-      bulk_commit();
-      if (!mbar_wait(&kn_bar, knphase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-      mma_tile(tbase + dColW1, opKnAh, opDSH, 128, 64, 8, false);
-      mma_tile(tbase + dColW1, opKnAh, opDSL, 128, 64, 8, true);
-      mma_tile(tbase + dColW1, opKnAl, opDSH, 128, 64, 8, true);
-      if (!mbar_wait(&pbar, pphase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-      mma_tile(tbase + dColU1, opPTh, opDO, 128, 64, 4, false);
-      mma_tile(tbase + dColU1, opPTl, opDO, 128, 64, 4, true);
-      mma_commit(&bar);
-    }
-    knphase ^= 1;
-    pphase ^= 1;
-    wait_or_mark(&bar, phase, dead, p.status);
-    tc_fence_after();
-    if (tid == 0 && c > 0) issue_kn_load(c - 1);   // the Kn panels are free again
-
-    // ---- stage 2: k-side rows: dVn = scale U1 + W1
-    float acc[32];
-    if (kside) {
-      float w1[32];
-      tmem_ld32(trow + dColW1, w1);
-      tmem_ld32(trow + dColU1, acc);
-      tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 32; ++i) acc[i] = p.scale * acc[i] + w1[i];
-      row32_to_hilo(smem + dOffPH, smem + dOffPL, tok, half, acc);
-    }
-    if (tid == 0) bulk_wait_read();  // the dS'a images have left shared memory (it is reused in stage 4)
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-
-    // ---- stage 3: dZ = X^T dVn  (valid accumulator rows 64..127)
-    if (tid == 0) {
-      if (!mbar_wait(&x_bar, xphase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-      mma_tile(tbase + dColDZ, opXTh, opDVh, 128, 64, 4, false);
-      mma_tile(tbase + dColDZ, opXTh, opDVl, 128, 64, 4, true);
-      mma_tile(tbase + dColDZ, opXTl, opDVh, 128, 64, 4, true);
-      mma_commit(&bar);
-    }
-    xphase ^= 1;
-    wait_or_mark(&bar, phase, dead, p.status);
-    tc_fence_after();
-    if (tid == 0 && c > 0) issue_x_load(c - 1);
-
-    // ---- stage 4: k-side rows: dV, sum_v dZ*V, dZ images, -beta dZ;  q-side rows: scale dO
-    if (kside) {
-      tmem_ld_row32(trow + dColDZ, acc);
-      const float bi = beta_s[cur][tok];
-      float bzsum = 0.f;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float vv[8];
-        unpack_bf16x8(rcur[i], vv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) bzsum += acc[i * 8 + j] * vv[j];
-      }
-      row32_to_hilo(smem + dOffPH, smem + dOffPL, tok, half, acc);
-      if (tok < rows) {
-        p.bz[(int64_t(vb * 2 + half) * p.total_tokens + tok0 + tok) * p.HV + hv] = bzsum;
-        const int64_t off = (tok0 + tok) * p.dv_st + hv * p.dv_sh + vb * kBV + c0;
-        if (p.dv_f32) {
-          float* dst = static_cast<float*>(p.dv) + off;
-#pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(dst + i) = make_float4(bi * acc[i], bi * acc[i + 1], bi * acc[i + 2], bi * acc[i + 3]);
-        } else {
-          bf16* dst = static_cast<bf16*>(p.dv) + off;
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            float t[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) t[j] = bi * acc[ch * 8 + j];
-            *reinterpret_cast<uint4*>(dst + ch * 8) = pack8(t);
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 32; ++i) acc[i] *= -bi;
-      row32_to_hilo(smem + dOffDSH, smem + dOffDSL, 64 + tok, half, acc);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float vv[8];
-        unpack_bf16x8(rcur[i], vv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i * 8 + j] = p.scale * vv[j];
-      }
-      row32_to_hilo(smem + dOffDSH, smem + dOffDSL, tok, half, acc);
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-
-    // ---- stage 5: dSa += [Qp^T | Kp^T] [scale dO ; -beta dZ]
-    if (tid == 0) {
-      bf16* dst = p.dz_img + (cidx * p.nvb + vb) * 12288;
-      bulk_store(dst, sb + dOffDO, 8192);            // dO
-      bulk_store(dst + 4096, sb + dOffPH, 16384);    // dZ hi, dZ lo
-      bulk_commit();
-      if (!mbar_wait(&qk_bar, qkphase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-      mma_tile(tbase + dColDS, opQKTh, opDSH, 128, 64, 8, true);
-      mma_tile(tbase + dColDS, opQKTh, opDSL, 128, 64, 8, true);
-      mma_tile(tbase + dColDS, opQKTl, opDSH, 128, 64, 8, true);
-      mma_commit(&bar);
-    }
-    qkphase ^= 1;
-    if (c > 0) prefetch_load(c - 1);
-    wait_or_mark(&bar, phase, dead, p.status);
-    tc_fence_after();
-    if (tid == 0 && c > 0) issue_qk_load(c - 1);
-
-    // ---- stage 6: dS = diag(e^a) dSa to registers; next chunk's operands
-    tmem_ld_row32(trow + dColDS, srow);
-    {
-      const float ea = vec_s[cur][0][row];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) srow[i] *= ea;
-    }
-    if (tid == 0) {
-      bulk_wait_read();                  // the dO / dZ images have left the panels
-      if (c > 0) issue_p_load(c - 1);    // ... which now receive the next chunk's P
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (c > 0) {
-      prefetch_store(c - 1);
-      __syncthreads();
-    }
-  }
-
-  if (!dead && p.dh0) {
-    float* dst = p.dh0 + ((int64_t(n) * p.HV + hv) * kK + row) * p.V + vb * kBV + c0;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(srow[i], srow[i + 1], srow[i + 2], srow[i + 3]);
-  }
-  if (tid == 0) bulk_wait_all();
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tbase, 256);
-}
+}  // namespace fla
+#include "kda_scan_bwd.cuh"
+namespace fla {
 
 // ============================================================================================= par
 constexpr uint32_t qOffQKH = 0, qOffQKL = 32768, qOffKNH = 65536, qOffKNL = 81920;       // per-head operand images
-constexpr uint32_t qOffAH = 98304;              // [dO ; dZ_hi] rows of one V block (128 rows)
-constexpr uint32_t qOffAL = 114688;             // rows 0-63 zero, rows 64-127 dZ_lo
+// Operands of one 64-channel step are strips (sm100.cuh) whose 64 rows are value channels, the reduction dim of its products.
+constexpr uint32_t qOffAH = 98304;              // [dO^T | dZ_hi^T]: 16 strips of 8 tokens
+constexpr uint32_t qOffAL = 114688;             // 8 KB of zeros, then dZ_lo^T
 constexpr uint32_t qOffVNH = 131072, qOffVNL = 139264;
 constexpr uint32_t qOffSH = 147456, qOffSL = 163840, qOffDSH = 180224, qOffDSL = 196608;
 constexpr uint32_t qOffPAH = qOffAH, qOffPAL = qOffAL;   // [dP ; dM] hi / lo reuse the [dO ; dZ] panels
@@ -411,7 +131,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ float beta_s[kC], anchor_s[kK];
   __shared__ float red[2][2][kC];      // rkG, ma : [half][row]
-  __shared__ float sds_s[2][kK];       // sum_v dS'a * Sa per key channel, by column half
+  __shared__ float sds_s[kK];          // sum_v dS'a * Sa per key channel
   __shared__ float colsum_s[2][kK];    // per 32-row part: column sums of the dgk tiles
   __shared__ float ndot_s[NORM ? 2 : 1][2 * kC];  // q.dq / k.dk of the complete rows, per half of the columns (normalised q, k only)
   __shared__ float t1col_s[2][kK];     // per 32-row quadrant: sum_i Kn_i (Vn dS'a^T)_i of the last-row term
@@ -473,11 +193,11 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
   const Operand opQKnh{sb + qOffQKH, 16384, 1}, opQKnl{sb + qOffQKL, 16384, 1};         // as B, N = 128 key dims, reduction over 128 rows
   const Operand opKNbh{sb + qOffKNH, 8192, 0}, opKNbl{sb + qOffKNL, 8192, 0};           // Kn as B, N = 64 tokens
   const Operand opKNnh{sb + qOffKNH, 8192, 1}, opKNnl{sb + qOffKNL, 8192, 1};           // Kn as B, N = 128 key dims, reduction over tokens
-  const Operand opAH{sb + qOffAH, 16384, 0}, opAL{sb + qOffAL, 16384, 0};
-  const Operand opVNbH{sb + qOffVNH, 8192, 0}, opVNbL{sb + qOffVNL, 8192, 0};           // Vn as B (N = 64 tokens)
-  const Operand opVNaH{sb + qOffVNH - 8192, 8192, 0}, opVNaL{sb + qOffVNL - 8192, 8192, 0};  // Vn as A, valid rows 64..127
-  const Operand opSH{sb + qOffSH, 16384, 0}, opSL{sb + qOffSL, 16384, 0};               // Sa block as B (N = 128 key dims)
-  const Operand opDSH{sb + qOffDSH, 16384, 0}, opDSL{sb + qOffDSL, 16384, 0};
+  const Operand opAH{sb + qOffAH, 1024, 2}, opAL{sb + qOffAL, 1024, 2};                 // [dO; dZ], M = 128 tokens
+  const Operand opVNbH{sb + qOffVNH, 1024, 2}, opVNbL{sb + qOffVNL, 1024, 2};           // Vn as B (N = 64 tokens)
+  const Operand opVNaH{sb + qOffVNH - 8192, 1024, 2}, opVNaL{sb + qOffVNL - 8192, 1024, 2};  // Vn as A, valid rows 64..127
+  const Operand opSH{sb + qOffSH, 1024, 2}, opSL{sb + qOffSL, 1024, 2};                 // Sa block as B (N = 128 key dims)
+  const Operand opDSH{sb + qOffDSH, 1024, 2}, opDSL{sb + qOffDSL, 1024, 2};
   const Operand opPAH{sb + qOffPAH, 16384, 0}, opPAL{sb + qOffPAL, 16384, 0};           // [dP; dM], reduction over j
   const Operand opPATh{sb + qOffPAH - 8192, 8192, 1}, opPATl{sb + qOffPAL - 8192, 8192, 1};  // its transpose, valid rows 64..127
 
@@ -500,7 +220,9 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
       issue_images(hv);
       issue_loads(hv, 0);
     }
-    float sds = 0.f;   // my key channel (tid & 127), my 32 columns (tid >> 7) of sum_v dS'a * Sa
+    float sds[8];      // sum_v dS'a * Sa: the 8 key dims of strip tid / 16, value channels tid % 16 (mod 16) of every step
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sds[j] = 0.f;
     for (int vb = 0; vb < NVB; ++vb) {
       if (vb == 0) {
         ok = mbar_wait(&img_bar, iphase, p.status, FLA_ERR_TIMEOUT);
@@ -530,17 +252,17 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
         mma_tile(tbase + qColTB1, opVNaL, opDSH, 128, 128, 4, true);
         mma_commit(&mma_bar);
       }
-      // sum_v dS'a * Sa per key channel over this V block while the MMAs run (elementwise on the panel images)
-      {
-        const int kr = tid & 127, hf = tid >> 7;
+      // sum_v dS'a * Sa per key channel over this V block while the MMAs run (elementwise on the images)
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          float s[8], d[8];
-          chunk_vals(smem + qOffSH, smem + qOffSL, kr, hf * 4 + ch, s);
-          chunk_vals(smem + qOffDSH, smem + qOffDSL, kr, hf * 4 + ch, d);
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t off = (tid >> 4) * 1024 + ((tid & 15) + r * 16) * 16;
+        float s1[8], s2[8], d1[8], d2[8];
+        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffSH + off), s1);
+        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffSL + off), s2);
+        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffDSH + off), d1);
+        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffDSL + off), d2);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) sds += s[j] * d[j];
-        }
+        for (int j = 0; j < 8; ++j) sds[j] += (s1[j] + s2[j]) * (d1[j] + d2[j]);
       }
       ok = mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT);
       mphase ^= 1;
@@ -557,7 +279,19 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
       }
     }
     if (!ok) break;
-    sds_s[tid >> 7][tid & 127] = sds;
+    {      // over the sixteen threads of a strip by halving: thread 2 j (+ 1) of them ends with key dim j
+#pragma unroll
+      for (int o = 8, w = 4; w >= 1; o >>= 1, w >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int j = 0; j < w; ++j) {
+          const float send = up ? sds[j] : sds[j + w], keep = up ? sds[j + w] : sds[j];
+          sds[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      sds[0] += __shfl_xor_sync(0xffffffffu, sds[0], 1);
+      if (!(lane & 1)) sds_s[(tid >> 4) * 8 + ((lane >> 1) & 7)] = sds[0];
+    }
 
     // ---- epilogue 1: score-tile gradients -> [dP; dM] operand; row scaling of the first TA product in place
     const float beta_i = beta_s[tok];
@@ -723,7 +457,7 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
       for (int i = 0; i < 32; ++i) tot += tile_q[(r0 + i) * kTileStride + kc] + tile_k[(r0 + i) * kTileStride + kc];   // rows past the end hold zeros
       colsum_s[part][kc] = tot;
       __syncthreads();
-      float run = sds_s[0][kc] + sds_s[1][kc] + t1col_s[0][kc] + t1col_s[1][kc] + (part == 0 ? colsum_s[1][kc] : 0.f);
+      float run = sds_s[kc] + t1col_s[0][kc] + t1col_s[1][kc] + (part == 0 ? colsum_s[1][kc] : 0.f);
       const int64_t base = tok0 * p.dg_st + hv * p.dg_sh + kc;
       for (int blk = 3; blk >= 0; --blk) {
         float vals[8];
@@ -803,15 +537,17 @@ __global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, con
 using namespace fla;
 
 // Workspace: status | [forward workspace | gk | s_img | vn_img unless the caller passes the forward's saved buffer] | ds_img | dz_img | bz
-static uint64_t kda_bwd_ws_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, bool have_saved, uint64_t* off_saved,
-                                  uint64_t off[3]) {
+static uint64_t kda_bwd_ws_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, bool have_saved, const SegPlan& plan,
+                                  uint64_t* off_saved, uint64_t off[4]) {
   const uint64_t per = uint64_t(total_chunks) * HV;
-  uint64_t o = 256, so[4];
+  uint64_t o = 256, so[5];
   *off_saved = o;
-  if (!have_saved) o += align_up(kda_saved_layout(total_chunks, HV, nvb, tokens, so), 256);
+  if (!have_saved) o += align_up(kda_saved_layout(total_chunks, HV, nvb, tokens, plan.split ? plan.count : 0, so), 256);
   off[0] = o; o += align_up(per * nvb * kKdaDsImg * 2, 256);
   off[1] = o; o += align_up(per * nvb * kKdaDzImg * 2, 256);
   off[2] = o; o += align_up(uint64_t(2 * nvb) * tokens * HV * 4, 256);
+  off[3] = o;      // H of the recomputed forward, then dH
+  if (plan.split) o += uint64_t(plan.count) * HV * (nvb / 2) * kSegHBytes;
   return o;
 }
 
@@ -831,15 +567,21 @@ static int kda_bwd_geometry(const fla_kda_chunk_bwd_args* a, int64_t* total_chun
   return FLA_OK;
 }
 
+static SegPlan kda_bwd_plan(const fla_kda_chunk_bwd_args* a, int64_t total_chunks, int N) {      // that of the forward
+  const bool packed = a->cu_seqlens.data != nullptr;
+  return scan_plan(N, total_chunks, packed ? a->max_seqlen : a->q.shape[1], packed, a->v.shape[2], a->v.shape[3]);
+}
+
 extern "C" FLA_API int fla_b200_kda_chunk_bwd_workspace_size(const fla_kda_chunk_bwd_args* a, uint64_t* bytes) {
   if (!a || !bytes) return FLA_ERR_NULL;
   int64_t total_chunks; int N;
   const int st = kda_bwd_geometry(a, &total_chunks, &N);
   if (st) return st;
-  uint64_t off[3], off_saved;
+  uint64_t off[4], off_saved;
   const int64_t V = a->v.shape[3];
   if (V != kV && V != 2 * kV) return FLA_ERR_SHAPE;
-  *bytes = kda_bwd_ws_layout(total_chunks, a->v.shape[2], V / kBV, a->q.shape[0] * a->q.shape[1], a->saved.data != nullptr, &off_saved, off);
+  *bytes = kda_bwd_ws_layout(total_chunks, a->v.shape[2], V / kBV, a->q.shape[0] * a->q.shape[1], a->saved.data != nullptr,
+                             kda_bwd_plan(a, total_chunks, N), &off_saved, off);
   return FLA_OK;
 }
 
@@ -891,11 +633,12 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   }
   if ((st = kda_check_rstd(a->q_rstd, a->k_rstd, B, T, HK))) return st;
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
-  uint64_t off[3], off_saved, so[4], fo[5];
+  uint64_t off[4], off_saved, so[5], fo[5];
   const bool have_saved = a->saved.data != nullptr;
-  const uint64_t need = kda_bwd_ws_layout(total_chunks, HV, nvb, B * T, have_saved, &off_saved, off);
+  const SegPlan plan = kda_bwd_plan(a, total_chunks, N);
+  const uint64_t need = kda_bwd_ws_layout(total_chunks, HV, nvb, B * T, have_saved, plan, &off_saved, off);
   if (!workspace || workspace_bytes < need || !aligned16(workspace)) return FLA_ERR_WORKSPACE;
-  const uint64_t sbytes = kda_saved_layout(total_chunks, HV, nvb, B * T, so);
+  const uint64_t sbytes = kda_saved_layout(total_chunks, HV, nvb, B * T, plan.split ? plan.count : 0, so);
   if (have_saved && (a->saved.dtype != FLA_BF16 || a->saved.ndim != 1 || uint64_t(a->saved.shape[0]) * 2 < sbytes ||
                      !aligned16(a->saved.data)))
     return FLA_ERR_SHAPE;
@@ -922,6 +665,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   f.N = N; f.T = int(T); f.HK = int(HK); f.HV = int(HV); f.total_tokens = B * T; f.V = int(V); f.nvb = int(nvb);
   f.g_is_f32 = a->g.dtype == FLA_F32; f.beta_is_f32 = a->beta.dtype == FLA_F32;
   f.gate_mode = 0; f.scale = a->scale;
+  f.seg_len = plan.len; f.seg_m = reinterpret_cast<bf16*>(sv + so[4]); f.seg_h = reinterpret_cast<float*>(ws + off[3]);
   f.q_rstd = static_cast<float*>(a->q_rstd.data); f.k_rstd = static_cast<float*>(a->k_rstd.data);   // (written again by the recomputed forward)
 
   KdaBwdParams p{};
@@ -932,6 +676,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   p.s_img = f.s_img; p.vn_img = f.vn_img;
   p.ds_img = reinterpret_cast<bf16*>(ws + off[0]); p.dz_img = reinterpret_cast<bf16*>(ws + off[1]);
   p.bz = reinterpret_cast<float*>(ws + off[2]);
+  p.seg_len = plan.len; p.seg_m = f.seg_m; p.seg_dh = f.seg_h; p.clear = have_saved;
   p.dht = static_cast<const float*>(a->dht.data); p.dh0 = static_cast<float*>(a->dh0.data);
   p.dq = a->dq.data; p.dk = a->dk.data; p.dv = a->dv.data; p.dg = a->dg.data; p.dbeta = a->dbeta.data;
   p.cu_seqlens = f.cu_seqlens; p.chunk_offsets = f.chunk_offsets;
@@ -947,20 +692,27 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   p.status = f.status;
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  if (!have_saved && (st = kda_launch_forward(f, total_chunks, cs))) return st;
+  if (!have_saved && (st = kda_launch_forward(f, total_chunks, plan.count, cs))) return st;
   static std::atomic<bool> attr_done_dev[64] = {};   // per device ordinal; setting the attributes twice is harmless
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
   if (!attr_done_dev[dev]) {
-    if (cudaFuncSetAttribute(kda_bwd_dhu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaDhuSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
+    for (auto* scan : {kda_scan_bwd_kernel<false, false>, kda_scan_bwd_kernel<false, true>, kda_scan_bwd_kernel<true, true>})
+      if (cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaScanBwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     for (auto* par : {kda_bwd_par_kernel<2, false>, kda_bwd_par_kernel<4, false>, kda_bwd_par_kernel<2, true>, kda_bwd_par_kernel<4, true>})
       if (cudaFuncSetAttribute(par, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaParSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     attr_done_dev[dev] = true;
   }
-  CUtensorMap tm_gk;
+  CUtensorMap tm_gk, tm_v, tm_d;
+  if (make_row_tile_map(&tm_v, p.v, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.v_sh), uint64_t(p.v_st)) ||
+      make_row_tile_map(&tm_d, p.dO, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.do_sh), uint64_t(p.do_st)))
+    return FLA_ERR_CUDA;
   if (make_row_tile_map_f32(&tm_gk, p.gk, kK, uint64_t(HV), uint64_t(B * T), uint64_t(kK), uint64_t(HV) * kK)) return FLA_ERR_CUDA;
-  auto launch_scan = [&](const KdaBwdParams& pp, int nseq, cudaStream_t st_) {
-    kda_bwd_dhu_kernel<<<dim3(unsigned(nvb), unsigned(HV), nseq), 256, kKdaDhuSmem + 1024, st_>>>(pp);
+  auto launch_scan = [&](const KdaBwdParams& pp, int64_t segments, cudaStream_t st_) {
+    const dim3 grid(unsigned(HV * (V / 128)), unsigned(segments));
+    if (plan.split) kda_scan_bwd_kernel<true, true><<<grid, kScanThreads, kKdaScanBwdSmem + 1024, st_>>>(pp, tm_v, tm_d);
+    auto* scan = plan.split ? kda_scan_bwd_kernel<false, true> : kda_scan_bwd_kernel<false, false>;
+    scan<<<grid, kScanThreads, kKdaScanBwdSmem + 1024, st_>>>(pp, tm_v, tm_d);
   };
   auto launch_par = [&](const KdaBwdParams& pp, int64_t chunks, cudaStream_t st_) {
     auto* par = nvb == 2 ? (pp.q_rstd ? kda_bwd_par_kernel<2, true> : kda_bwd_par_kernel<2, false>)
@@ -970,7 +722,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   // more scan chains (one CTA per SM each) than SMs: two halves of the batch on two streams, so that the chunk-parallel
   // kernel of the first half fills the SMs the second half's scan leaves idle (aux_stream.h)
   AuxStream* aux = nullptr;
-  if (N >= 2 && int64_t(nvb) * HV * N > sm_count(dev) && !kernel_timing_enabled()) aux = aux_stream_for(dev, cs);
+  if (N >= 2 && !plan.split && HV * (V / 128) * N > sm_count(dev) && !kernel_timing_enabled()) aux = aux_stream_for(dev, cs);
   if (aux) {
     std::lock_guard<std::mutex> lk(aux->mu);
     const int n1 = N / 2;
@@ -988,7 +740,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   }
   {
     KernelTimer kt("kda_bwd_dhu", cs);
-    launch_scan(p, N, cs);
+    launch_scan(p, plan.count, cs);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {

@@ -11,13 +11,14 @@
 // with w, u folded away.  The decay sits inside the K reduction, so the scaled operands cannot be the exact
 // bf16 inputs: kda_prep_kernel (parallel over chunks) builds them once as bf16 hi + residual operand panels,
 // computes both score tiles on tcgen05 and the inverse on CUDA cores, and stores everything as ready-to-load
-// panel images; kda_fwd_kernel (sequential over chunks, fp32 state in TMEM) only bulk-loads them.
+// panel images; kda_scan_fwd_kernel (kda_scan_fwd.cuh; sequential over chunks, fp32 state in TMEM) only bulk-loads them.
 #include "gdn_common.cuh"
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
 #include "tri_inverse.cuh"
 #include "kda_common.cuh"
 #include "tensor_map.h"
+#include "kda_scan_fwd.cuh"
 
 namespace fla {
 
@@ -142,6 +143,9 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
     p.vec[cidx * kKdaVecs * kK + tid] = __expf(a);
     p.vec[cidx * kKdaVecs * kK + kK + tid] = __expf(last_s[tid] - a);
     p.vec[cidx * kKdaVecs * kK + 2 * kK + tid] = a;
+  } else {
+    const int t = tid - kK;
+    p.vec[cidx * kKdaVecs * kK + 3 * kK + t] = t < rows ? ld_scalar(p.beta, (tok0 + t) * p.beta_st + hv, p.beta_is_f32) : 0.f;
   }
   // 3. scaled operands as split bf16 panels
   {
@@ -269,270 +273,6 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
   if (warp == 0) tmem_dealloc(tbase, 64);
 }
 
-// --------------------------------------------------------------------------------------------- forward
-constexpr uint32_t fOffQKH = 0, fOffQKL = 32768, fOffKNH = 65536, fOffKNL = 81920;
-constexpr uint32_t fOffPH = 98304, fOffPL = 106496, fOffX = 114688, fOffXL = 122880;
-constexpr uint32_t fOffSH = 131072, fOffSL = 147456, fOffZH = 163840, fOffZL = 172032;
-constexpr uint32_t kKdaFwdSmem = 180224;
-constexpr uint32_t fColS = 0, fColRQ = 64, fColPV = 128, fColVN = 192;
-
-__global__ void __launch_bounds__(256, 1) kda_fwd_kernel(KdaParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ float vec_s[2][2][kK];     // [chunk parity][e^a | e^{gk_L - a}][channel]
-  __shared__ float beta_s[2][kC];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(8) uint64_t mma_bar, load1_bar, load2_bar;
-
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int vb = blockIdx.x, hv = blockIdx.y, n = blockIdx.z;
-  const SeqInfo sq = seq_info(p.cu_seqlens, p.chunk_offsets, n, p.T);
-  const int quad = warp & 3, half = warp >> 2;
-  const bool kside = quad >= 2;
-  const int row = quad * 32 + lane, tok = row & 63, c0 = half * 32;
-
-  if (warp == 0) {
-    tmem_alloc(&tmem_base_s, 256);
-    tmem_relinquish();
-  }
-  if (tid == 0) {
-    mbar_init(&mma_bar, 1);
-    mbar_init(&load1_bar, 1);
-    mbar_init(&load2_bar, 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  const uint32_t tbase = tmem_base_s;
-  const uint32_t trow = tmem_addr(tbase, quad * 32, c0);
-  const uint32_t sb = smem_u32(smem);
-  uint32_t mphase = 0, l1phase = 0, l2phase = 0;
-  bool dead = false;
-
-  auto issue_load1 = [&](int c) {   // [Qp; Kp] hi + lo
-    const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-    mbar_arrive_expect_tx(&load1_bar, 65536);
-    bulk_load(sb + fOffQKH, p.qk_img + cidx * kKdaQkImg, 65536, &load1_bar);
-  };
-  auto issue_load2 = [&](int c) {   // Kn hi + lo, P hi + lo, X
-    const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-    mbar_arrive_expect_tx(&load2_bar, 32768 + 16384 + 16384);
-    bulk_load(sb + fOffKNH, p.kn_img + cidx * kKdaKnImg, 32768, &load2_bar);
-    bulk_load(sb + fOffPH, p.p_img + cidx * kKdaPImg, 16384, &load2_bar);
-    bulk_load(sb + fOffX, p.x_img + cidx * kKdaXImg, 16384, &load2_bar);
-  };
-  if (tid == 0 && sq.nt > 0) {   // a sequence without tokens requests nothing: its final state is its initial state
-    issue_load1(0);
-    issue_load2(0);
-  }
-
-  const Operand opQKH{sb + fOffQKH, 16384, 0}, opQKL{sb + fOffQKL, 16384, 0};
-  const Operand opKNTh{sb + fOffKNH, 8192, 1}, opKNTl{sb + fOffKNL, 8192, 1};   // Kn^T: M = 128 key dims
-  const Operand opSH{sb + fOffSH, 16384, 1}, opSL{sb + fOffSL, 16384, 1};
-  const Operand opZH{sb + fOffZH, 8192, 1}, opZL{sb + fOffZL, 8192, 1};
-  const Operand opX{sb + fOffX - 8192, 16384, 0};               // rows 64..127 of this tile are X
-  const Operand opXL{sb + fOffXL - 8192, 16384, 0};             // ... and of this one its bf16 residual
-  const Operand opPH{sb + fOffPH, 16384, 0}, opPL{sb + fOffPL, 16384, 0};       // rows 0..63 are P
-
-  // per-chunk scalars / vectors / value rows are staged through registers one chunk ahead
-  float pf_vec = 0.f, pf_beta = 0.f;
-  uint4 pf_v[4], vcur[4];
-  auto prefetch_load = [&](int c) {
-    const int t0 = c * kC;
-    const int rows = min(kC, sq.len - t0);
-    const int64_t tok0 = int64_t(sq.bos) + t0;
-    const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-    pf_vec = p.vec[cidx * kKdaVecs * kK + tid];                       // 256 threads: e^a then e^{gk_L - a}
-    if (kside) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        pf_v[i] = make_uint4(0, 0, 0, 0);
-        if (tok < rows) pf_v[i] = *reinterpret_cast<const uint4*>(p.v + (tok0 + tok) * p.v_st + hv * p.v_sh + vb * kBV + c0 + i * 8);
-      }
-      pf_beta = tok < rows ? ld_scalar(p.beta, (tok0 + tok) * p.beta_st + hv, p.beta_is_f32) : 0.f;
-    }
-  };
-  auto store_scalars = [&](int c) {   // double-buffered by chunk parity: safe to write while chunk c-1 is in flight
-    vec_s[c & 1][tid / kK][tid % kK] = pf_vec;
-    if (kside && half == 0) beta_s[c & 1][tok] = pf_beta;
-  };
-  auto take_values = [&]() {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) vcur[i] = pf_v[i];
-  };
-
-  float srow[32];
-  if (sq.nt > 0) {
-    prefetch_load(0);
-    store_scalars(0);
-    take_values();
-  }
-  if (p.h0) {
-    const float* src = p.h0 + ((int64_t(n) * p.HV + hv) * kK + row) * p.V + vb * kBV + c0;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      const float4 t = *reinterpret_cast<const float4*>(src + i);
-      srow[i] = t.x; srow[i + 1] = t.y; srow[i + 2] = t.z; srow[i + 3] = t.w;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) srow[i] = 0.f;
-  }
-  __syncthreads();
-
-  for (int c = 0; c < sq.nt; ++c) {
-    const int cur = c & 1;
-    const int t0 = c * kC;
-    const int rows = min(kC, sq.len - t0);
-    const int64_t tok0 = int64_t(sq.bos) + t0;
-
-    // ---- stage 0: Sa = diag(e^a) S as split copy and as the fp32 master in TMEM
-    {
-      const float ea = vec_s[cur][0][row];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) srow[i] *= ea;
-      row32_to_hilo(smem + fOffSH, smem + fOffSL, row, half, srow);
-      tmem_st16(trow + fColS, srow);
-      tmem_st16(trow + fColS + 16, srow + 16);
-      tmem_st_wait();
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-
-    // ---- stage 1: [Qp; Kp] Sa
-    if (!dead && !mbar_wait(&load1_bar, l1phase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-    l1phase ^= 1;
-    if (tid == 0) {
-      if (p.s_img) {
-        const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-        bulk_store(p.s_img + (cidx * p.nvb + vb) * 16384, sb + fOffSH, 32768);
-        bulk_commit();
-      }
-      mma_tile(tbase + fColRQ, opQKH, opSH, 128, 64, 8, false);
-      mma_tile(tbase + fColRQ, opQKH, opSL, 128, 64, 8, true);
-      mma_tile(tbase + fColRQ, opQKL, opSH, 128, 64, 8, true);
-      mma_commit(&mma_bar);
-    }
-    if (c + 1 < sq.nt) {
-      prefetch_load(c + 1);
-      store_scalars(c + 1);
-    }
-    if (!dead && !mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-    mphase ^= 1;
-    tc_fence_after();
-    if (tid == 0 && c + 1 < sq.nt) issue_load1(c + 1);   // the [Qp; Kp] buffers are free again
-
-    // ---- stage 2: k-side rows: Z = beta (V - Kp Sa)
-    float acc[32];
-    if (kside) {
-      tmem_ld32(trow + fColRQ, acc);
-      tmem_ld_wait();
-      const float bi = beta_s[cur][tok];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float vv[8];
-        unpack_bf16x8(vcur[i], vv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i * 8 + j] = bi * (vv[j] - acc[i * 8 + j]);
-      }
-      row32_to_hilo(smem + fOffZH, smem + fOffZL, tok, half, acc);
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-
-    // ---- stage 3: v_new = X Z
-    if (!dead && !mbar_wait(&load2_bar, l2phase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-    l2phase ^= 1;
-    if (tid == 0) {
-      mma_tile(tbase + fColVN, opX, opZH, 128, 64, 4, false);
-      mma_tile(tbase + fColVN, opX, opZL, 128, 64, 4, true);
-      mma_tile(tbase + fColVN, opXL, opZH, 128, 64, 4, true);
-      mma_commit(&mma_bar);
-    }
-    if (!dead && !mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-    mphase ^= 1;
-    tc_fence_after();
-
-    // ---- stage 4: k-side rows publish v_new
-    if (kside) {
-      tmem_ld32(trow + fColVN, acc);
-      tmem_ld_wait();
-      row32_to_hilo(smem + fOffZH, smem + fOffZL, tok, half, acc);
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-
-    // ---- stage 5: Aqk v_new and the state update Sa += Kn^T v_new
-    if (tid == 0) {
-      if (p.vn_img) {
-        const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-        bulk_store(p.vn_img + (cidx * p.nvb + vb) * 8192, sb + fOffZH, 16384);
-        bulk_commit();
-      }
-      mma_tile(tbase + fColPV, opPH, opZH, 128, 64, 4, false);
-      mma_tile(tbase + fColPV, opPH, opZL, 128, 64, 4, true);
-      mma_tile(tbase + fColPV, opPL, opZH, 128, 64, 4, true);
-      mma_tile(tbase + fColS, opKNTh, opZH, 128, 64, 4, true);
-      mma_tile(tbase + fColS, opKNTh, opZL, 128, 64, 4, true);
-      mma_tile(tbase + fColS, opKNTl, opZH, 128, 64, 4, true);
-      mma_commit(&mma_bar);
-    }
-    if (!dead && !mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT)) dead = true;
-    mphase ^= 1;
-    tc_fence_after();
-    if (tid == 0 && c + 1 < sq.nt) issue_load2(c + 1);
-    if (p.s_img || p.vn_img) {   // the saved images must have left the S / v_new panels before they are rewritten
-      if (tid == 0) bulk_wait_read();
-      __syncthreads();
-    }
-
-    // ---- stage 6: output rows; next state S = diag(e^{gk_L - a}) (Sa + Kn^T v_new)
-    if (!kside) {
-      float qs[32];
-      tmem_ld32(trow + fColRQ, qs);
-      tmem_ld32(trow + fColPV, acc);
-      tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 32; ++i) acc[i] = p.scale * (qs[i] + acc[i]);
-      if (tok < rows && p.o) {
-        const int64_t off = (tok0 + tok) * p.o_st + hv * p.o_sh + vb * kBV + c0;
-        if (p.o_is_f32) {
-          float* dst = static_cast<float*>(p.o) + off;
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-        } else {
-          bf16* dst = static_cast<bf16*>(p.o) + off;
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch) *reinterpret_cast<uint4*>(dst + ch * 8) = pack8(acc + ch * 8);
-        }
-      }
-    }
-    tmem_ld32(trow + fColS, srow);
-    tmem_ld_wait();
-    {
-      const float el = vec_s[cur][1][row];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) srow[i] *= el;
-    }
-    if (c + 1 < sq.nt) take_values();
-  }
-
-  if (!dead && p.ht) {
-    float* dst = p.ht + ((int64_t(n) * p.HV + hv) * kK + row) * p.V + vb * kBV + c0;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(srow[i], srow[i + 1], srow[i + 2], srow[i + 3]);
-  }
-  if (tid == 0) bulk_wait_all();
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tbase, 256);
-}
-
 // The two 64 x 64 score blocks of every chunk as plain tensors, for callers of the reference's low-level forward
 // (npu_chunk_kda_fwd returns them): Aqk = scale tril(q k^T 2^{gk_i - gk_j}) from the P image and Akk = the chunk inverse
 // from the X image (value + residual panels summed), rows and columns past a short chunk as zeros.
@@ -594,7 +334,7 @@ uint64_t fla::kda_ws_layout(int64_t total_chunks, int64_t HV, uint64_t off[5]) {
   return o;
 }
 
-uint64_t fla::kda_saved_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, uint64_t off[4]) {
+uint64_t fla::kda_saved_layout(int64_t total_chunks, int64_t HV, int64_t nvb, int64_t tokens, int64_t segments, uint64_t off[5]) {
   uint64_t fo[5];
   const uint64_t per = uint64_t(total_chunks) * HV;
   uint64_t o = 0;
@@ -602,6 +342,7 @@ uint64_t fla::kda_saved_layout(int64_t total_chunks, int64_t HV, int64_t nvb, in
   off[1] = o; o += align_up(uint64_t(tokens) * HV * kK * 4, 256);
   off[2] = o; o += align_up(per * nvb * kKdaSImg * 2, 256);
   off[3] = o; o += align_up(per * nvb * kKdaVnImg * 2, 256);
+  off[4] = o; o += uint64_t(segments) * HV * kSegMBytes;
   return o;
 }
 
@@ -623,13 +364,23 @@ static int kda_geometry(const fla_kda_chunk_fwd_args* a, int64_t* total_chunks, 
   return FLA_OK;
 }
 
+static SegPlan kda_plan(const fla_kda_chunk_fwd_args* a, int64_t total_chunks, int N, int max_len) {
+  return scan_plan(N, total_chunks, max_len, a->cu_seqlens.data != nullptr, a->v.shape[2], a->v.shape[3]);
+}
+// Operand images (unless they go into `saved`), then H and (again unless saved) M of the segments of split chains.
+static uint64_t kda_fwd_workspace(const fla_kda_chunk_fwd_args* a, int64_t total_chunks, const SegPlan& plan) {
+  uint64_t off[5];
+  uint64_t b = a->saved.data ? 256 : kda_ws_layout(total_chunks, a->v.shape[2], off);
+  if (plan.split) b += uint64_t(plan.count) * a->v.shape[2] * (kSegHBytes * (a->v.shape[3] / 128) + (a->saved.data ? 0 : kSegMBytes));
+  return b;
+}
+
 extern "C" FLA_API int fla_b200_kda_chunk_fwd_workspace_size(const fla_kda_chunk_fwd_args* a, uint64_t* bytes) {
   if (!a || !bytes) return FLA_ERR_NULL;
   int64_t total_chunks; int N, max_len;
   const int st = kda_geometry(a, &total_chunks, &N, &max_len);
   if (st) return st;
-  uint64_t off[5];
-  *bytes = a->saved.data ? 256 : kda_ws_layout(total_chunks, a->v.shape[2], off);
+  *bytes = kda_fwd_workspace(a, total_chunks, kda_plan(a, total_chunks, N, max_len));
   return FLA_OK;
 }
 
@@ -638,10 +389,11 @@ extern "C" FLA_API int fla_b200_kda_chunk_saved_size(const fla_kda_chunk_fwd_arg
   int64_t total_chunks; int N, max_len;
   const int st = kda_geometry(a, &total_chunks, &N, &max_len);
   if (st) return st;
-  uint64_t off[4];
+  uint64_t off[5];
   const int64_t V = a->v.shape[3];
   if (V != kV && V != 2 * kV) return FLA_ERR_SHAPE;
-  *bytes = kda_saved_layout(total_chunks, a->v.shape[2], V / kBV, a->q.shape[0] * a->q.shape[1], off);
+  const SegPlan plan = kda_plan(a, total_chunks, N, max_len);
+  *bytes = kda_saved_layout(total_chunks, a->v.shape[2], V / kBV, a->q.shape[0] * a->q.shape[1], plan.split ? plan.count : 0, off);
   return FLA_OK;
 }
 
@@ -711,16 +463,17 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
   if ((st = kda_check_rstd(a->q_rstd, a->k_rstd, B, T, HK))) return st;
   if (a->chunk_size != kC) return FLA_ERR_VALUE;
   uint64_t off[5];
-  uint64_t need = kda_ws_layout(total_chunks, HV, off);
+  kda_ws_layout(total_chunks, HV, off);
+  const SegPlan plan = kda_plan(a, total_chunks, N, max_len);
+  const uint64_t need = kda_fwd_workspace(a, total_chunks, plan);
   uint8_t* images = static_cast<uint8_t*>(workspace);   // where the operand images go
-  uint64_t soff[4] = {0, 0, 0, 0};
+  uint64_t soff[5] = {};
   if (a->saved.data) {
-    const uint64_t sbytes = kda_saved_layout(total_chunks, HV, V / kBV, B * T, soff);
+    const uint64_t sbytes = kda_saved_layout(total_chunks, HV, V / kBV, B * T, plan.split ? plan.count : 0, soff);
     if (a->saved.dtype != FLA_BF16 || a->saved.ndim != 1 || uint64_t(a->saved.shape[0]) * 2 < sbytes || !aligned16(a->saved.data))
       return FLA_ERR_SHAPE;
     if (a->gate_mode != 0 || a->gk.data) return FLA_ERR_VALUE;
     images = static_cast<uint8_t*>(a->saved.data) + soff[0];
-    need = 256;
   }
   if (!workspace || workspace_bytes < need || !aligned16(workspace)) return FLA_ERR_WORKSPACE;
 
@@ -741,6 +494,12 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
   p.qk_img = reinterpret_cast<bf16*>(ws + off[0]); p.kn_img = reinterpret_cast<bf16*>(ws + off[1]);
   p.p_img = reinterpret_cast<bf16*>(ws + off[2]); p.x_img = reinterpret_cast<bf16*>(ws + off[3]);
   p.vec = reinterpret_cast<float*>(ws + off[4]);
+  p.seg_len = plan.len;
+  if (plan.split) {
+    uint8_t* end = static_cast<uint8_t*>(workspace) + need - uint64_t(plan.count) * HV * kSegHBytes * (V / 128);
+    p.seg_h = reinterpret_cast<float*>(end);
+    p.seg_m = reinterpret_cast<bf16*>(a->saved.data ? static_cast<uint8_t*>(a->saved.data) + soff[4] : end - uint64_t(plan.count) * HV * kSegMBytes);
+  }
   p.h0 = static_cast<const float*>(a->initial_state.data); p.ht = static_cast<float*>(a->final_state.data);
   p.o = a->o.data;
   p.cu_seqlens = static_cast<const int32_t*>(a->cu_seqlens.data);
@@ -765,7 +524,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   const int nt_max = (max_len + kC - 1) / kC;
-  st = kda_launch_forward(p, total_chunks, cs);
+  st = kda_launch_forward(p, total_chunks, plan.count, cs);
   if (st || (!ep.out[0] && !ep.out[1])) return st;
   ep.img[0] = p.p_img; ep.img[1] = p.x_img;
   ep.cu_seqlens = p.cu_seqlens; ep.chunk_offsets = p.chunk_offsets; ep.T = p.T; ep.HV = p.HV; ep.scale = p.scale;
@@ -774,17 +533,20 @@ extern "C" FLA_API int fla_b200_kda_chunk_fwd(const fla_kda_chunk_fwd_args* a, v
   return cuda_status(cudaGetLastError());
 }
 
-int fla::kda_launch_forward(const KdaParams& p, int64_t total_chunks, cudaStream_t cs) {
+int fla::kda_launch_forward(const KdaParams& p, int64_t total_chunks, int64_t segments, cudaStream_t cs) {
   static std::atomic<bool> attr_done_dev[64] = {};   // per device ordinal; setting the attributes twice is harmless
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return FLA_ERR_CUDA;
   if (!attr_done_dev[dev]) {
     if (cudaFuncSetAttribute(kda_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaPrepSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
-    if (cudaFuncSetAttribute(kda_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaFwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
+    for (auto* scan : {kda_scan_fwd_kernel<false, false, false>, kda_scan_fwd_kernel<true, false, false>, kda_scan_fwd_kernel<false, false, true>,
+                       kda_scan_fwd_kernel<true, false, true>, kda_scan_fwd_kernel<false, true, true>})
+      if (cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kKdaScanFwdSmem) + 1024) != cudaSuccess) return FLA_ERR_CUDA;
     attr_done_dev[dev] = true;
   }
-  CUtensorMap tm_q, tm_k;
-  if (make_row_tile_map(&tm_q, p.q, kK, uint64_t(p.HK), uint64_t(p.total_tokens), uint64_t(p.q_sh), uint64_t(p.q_st)) ||
+  CUtensorMap tm_q, tm_k, tm_v;
+  if (make_row_tile_map(&tm_v, p.v, uint64_t(p.V), uint64_t(p.HV), uint64_t(p.total_tokens), uint64_t(p.v_sh), uint64_t(p.v_st)) ||
+      make_row_tile_map(&tm_q, p.q, kK, uint64_t(p.HK), uint64_t(p.total_tokens), uint64_t(p.q_sh), uint64_t(p.q_st)) ||
       make_row_tile_map(&tm_k, p.k, kK, uint64_t(p.HK), uint64_t(p.total_tokens), uint64_t(p.k_sh), uint64_t(p.k_st)))
     return FLA_ERR_CUDA;
   {
@@ -794,7 +556,12 @@ int fla::kda_launch_forward(const KdaParams& p, int64_t total_chunks, cudaStream
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
     KernelTimer kt("kda_fwd", cs);
-    kda_fwd_kernel<<<dim3(unsigned(p.nvb), unsigned(p.HV), p.N), 256, kKdaFwdSmem + 1024, cs>>>(p);
+    const bool split = p.seg_len != kWholeSequence;
+    const unsigned heads = unsigned(p.HV * (p.V / 128));
+    if (split) kda_scan_fwd_kernel<false, true, true><<<dim3(heads, unsigned(segments), 2), kFwdThreads, kKdaScanFwdSmem + 1024, cs>>>(p, tm_v);
+    auto* scan = split ? (p.s_img ? kda_scan_fwd_kernel<true, false, true> : kda_scan_fwd_kernel<false, false, true>)
+                       : (p.s_img ? kda_scan_fwd_kernel<true, false, false> : kda_scan_fwd_kernel<false, false, false>);
+    scan<<<dim3(heads, unsigned(segments)), kFwdThreads, kKdaScanFwdSmem + 1024, cs>>>(p, tm_v);
   }
   return cuda_status(cudaGetLastError());
 }

@@ -30,8 +30,8 @@ struct KdaInterParams {
   const float* gk;        // [tokens, HV, K] chunk-local cumulative gate (natural log) of the saved buffer
   const bf16* x_img;      // (I + Akk)^-1 per (chunk, head): value + residual panels
   const float* vec;       // per (chunk, head): e^a, e^{gk_L - a}, a
-  const bf16* s_img;      // Sa = diag(e^a) S per (chunk, head, 64-column block of V): value + residual panels
-  const bf16* vn_img;     // v_new per (chunk, head, block): value + residual panels
+  const bf16* s_img;      // Sa = diag(e^a) S per (chunk, head, 64-column block of V): value + residual strips
+  const bf16* vn_img;     // v_new per (chunk, head, block): value + residual strips
   OutView w, u, qg, kg, vn;
   void* h; int h_dtype, h_vfirst;
   const int32_t* cu_seqlens; const int32_t* chunk_offsets;
@@ -42,6 +42,11 @@ __device__ __forceinline__ void put(void* p, int dtype, int64_t idx, float x) {
   if (dtype == FLA_F32) static_cast<float*>(p)[idx] = x;
   else if (dtype == FLA_F16) static_cast<__half*>(p)[idx] = __float2half_rn(x);
   else static_cast<bf16*>(p)[idx] = __float2bfloat16_rn(x);
+}
+// value + residual of element (row, ch) of an image in strips of 8 rows (64 channels)
+__device__ __forceinline__ float strip_val(const uint8_t* img, int lo_off, int row, int ch) {
+  const int off = (row >> 3) * 1024 + ch * 16 + (row & 7) * 2;
+  return __bfloat162float(*reinterpret_cast<const bf16*>(img + off)) + __bfloat162float(*reinterpret_cast<const bf16*>(img + lo_off + off));
 }
 __device__ __forceinline__ float panel_val(const uint8_t* hi, uint32_t lo_off, int row, int col) {
   const uint32_t o = panel_off(row, col);
@@ -144,14 +149,14 @@ __global__ void __launch_bounds__(256) kda_intermediates_kernel(KdaInterParams p
       const uint8_t* img = reinterpret_cast<const uint8_t*>(p.vn_img + (cidx * p.nvb + vb) * kKdaVnImg);
       for (int idx = tid; idx < kC * 64; idx += 256) {
         const int t = idx >> 6, ch = idx & 63;
-        if (t < rows) put(p.vn.p, p.vn.dtype, b * p.vn.sb + (t0 + t) * p.vn.st + hv * p.vn.sh + vb * 64 + ch, panel_val(img, 8192, t, ch));
+        if (t < rows) put(p.vn.p, p.vn.dtype, b * p.vn.sb + (t0 + t) * p.vn.st + hv * p.vn.sh + vb * 64 + ch, strip_val(img, 8192, t, ch));
       }
     }
     if (p.h) {
       const uint8_t* img = reinterpret_cast<const uint8_t*>(p.s_img + (cidx * p.nvb + vb) * kKdaSImg);
       for (int idx = tid; idx < kK * 64; idx += 256) {
         const int kd = idx >> 6, ch = idx & 63;
-        const float x = panel_val(img, 16384, kd, ch) * ea_s[kd];
+        const float x = strip_val(img, 16384, kd, ch) * ea_s[kd];
         const int64_t o = p.h_vfirst ? (cidx * p.V + vb * 64 + ch) * kK + kd : (cidx * kK + kd) * p.V + vb * 64 + ch;
         put(p.h, p.h_dtype, o, x);
       }
@@ -202,8 +207,8 @@ extern "C" FLA_API int fla_b200_kda_chunk_intermediates(const fla_kda_intermedia
     total_chunks = a->total_chunks;
   }
   const int64_t nvb = V / 64;
-  uint64_t soff[4], woff[6];
-  const uint64_t sbytes = kda_saved_layout(total_chunks, HV, nvb, B * T, soff);
+  uint64_t soff[5], woff[5];
+  const uint64_t sbytes = kda_saved_layout(total_chunks, HV, nvb, B * T, 0, soff);
   kda_ws_layout(total_chunks, HV, woff);
   if (a->saved.dtype != FLA_BF16 || a->saved.ndim != 1 || uint64_t(a->saved.shape[0]) * 2 < sbytes || !aligned16(a->saved.data))
     return FLA_ERR_SHAPE;

@@ -10,6 +10,7 @@
 // The reverse scan's gradient is carried by the transpose of the same M.
 #pragma once
 #include "gdn_common.cuh"
+#include "aux_stream.h"
 
 namespace fla {
 
@@ -97,6 +98,11 @@ inline SegPlan plan_segments(int64_t N, int64_t total_chunks, int64_t max_nt, bo
     }
   }
   return best;
+}
+// How the scans of one call split their chains: the same in its forward and its backward.  A state-only step takes as long as a full one
+// (the outputs and score products it leaves out are off the chain).
+inline SegPlan scan_plan(int64_t N, int64_t total_chunks, int64_t max_len, bool packed, int64_t HV, int64_t V) {
+  return plan_segments(N, total_chunks, (max_len + kC - 1) / kC, packed, HV * (V / 128), HV, 1.0, current_sm_count());
 }
 
 }  // namespace fla

@@ -55,3 +55,21 @@ def test_gdn_split_packed(lens, HV):
     names = ("o", "ht", "dq", "dk", "dv", "dg", "dbeta", "dh0", "inference o", "inference ht")
     for n, a, b in zip(names, run(1), run(-(-160 // HV))):
         _close(n, a, b, 2e-3)
+
+
+@pytest.mark.parametrize("keep", [False, True])
+@pytest.mark.parametrize("T,HV,V", [(1024, 1, 128), (1111, 3, 128), (2300, 2, 256)])
+def test_kda_split_forward_and_backward(T, HV, V, keep):
+    from fla_b200.ops import chunk_kda, chunk_kda_fwd_bwd
+    d = _inputs(T, HV, HV, 1, V)
+    d["g"] = (-torch.rand(1, T, HV, 128, generator=torch.Generator(device="cuda").manual_seed(T), device="cuda") / 16).bfloat16()
+
+    def run(copies):
+        x = {n: t.expand(copies, *t.shape[1:]).contiguous() for n, t in d.items()}
+        o, ht, gr = chunk_kda_fwd_bwd(x["q"], x["k"], x["v"], x["g"], x["beta"], x["do"], initial_state=x["h0"], dht=x["dht"],
+                                      output_dtype=torch.float32, disable_recompute=keep)
+        o2, ht2 = chunk_kda(x["q"], x["k"], x["v"], x["g"], x["beta"], initial_state=x["h0"], output_final_state=True, output_dtype=torch.float32)
+        return [t[:1] for t in (o, ht, *gr, o2, ht2)]
+    names = ("o", "ht", "dq", "dk", "dv", "dg", "dbeta", "dh0", "inference o", "inference ht")
+    for n, a, b in zip(names, run(1), run(-(-160 // HV))):
+        _close(n, a, b, 2e-3)
