@@ -65,11 +65,6 @@ namespace fla {
 // of its own and back cost 16 KB each way per tile.  (With four warps
 // and whole rows per thread the kernel took 0.245 ms at the benchmark shape: it is a chain of latencies, and half the
 // work per thread at twice the warps per SM shortens it.)
-// eight consecutive floats of shared memory, 16-byte aligned
-__device__ __forceinline__ void gather8(const float* p, float* f) {
-  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-}
 constexpr int kPrepThreads = 256;
 constexpr int kPrepSmem = 2 * kTriTile * 4;      // [q; k] panels (32 KB), then the A^T tiles of two heads
 static_assert(kPrepSmem >= 32768, "the panels must fit");
@@ -253,8 +248,8 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
       const int grp = tid >> 7, t = tid & 127;
       if (grp < pair) {
         float* tile = reinterpret_cast<float*>(smem) + grp * kTriTile;
-        tri_invert(tile, t, 1 + grp);
-        tri_store_strips(tile, reinterpret_cast<uint8_t*>(p.X + ((int64_t(sq.cbase) + pos.c) * p.HV + hk * G + h0 + grp) * 8192), rows, t);
+        tri_invert<128>(tile, t, 1 + grp);
+        tri_store_strips<128>(tile, reinterpret_cast<uint8_t*>(p.X + ((int64_t(sq.cbase) + pos.c) * p.HV + hk * G + h0 + grp) * 8192), rows, t);
       }
     }
     if (h0 + 2 < G) __syncthreads();

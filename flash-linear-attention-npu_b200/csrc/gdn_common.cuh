@@ -81,6 +81,12 @@ __device__ __forceinline__ float exp2_fast(float x) {
   return y;
 }
 
+// Eight consecutive floats, 16-byte aligned.
+__device__ __forceinline__ void gather8(const float* p, float* f) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+
 // Load 64 consecutive fp32 accumulator columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld_row64(uint32_t taddr, float* v) {
   tmem_ld32(taddr, v);

@@ -25,6 +25,7 @@ namespace fla {
 // --------------------------------------------------------------------------------------------- prep
 constexpr uint32_t pOffQKH = 0, pOffQKL = 32768, pOffKNH = 65536, pOffKNL = 81920;
 constexpr uint32_t kKdaPrepSmem = 98304;           // operand panels only
+constexpr uint32_t kStageP = 32768, kStageX = 49152;   // once the panels are free: the images of P and of X
 
 __device__ __forceinline__ float kda_gate(float g, int mode, float eig, float bias, float lower_bound) {
   if (mode == 0) return g;
@@ -36,15 +37,18 @@ __device__ __forceinline__ float kda_gate(float g, int mode, float eig, float bi
   return lower_bound / (1.f + __expf(-eig * raw));  // lower_bound * sigmoid(exp(A_log) (g + dt_bias))
 }
 
-// Thread layout of the elementwise phases: 16 channel groups (8 channels each) x 16 token segments (4 tokens each).
-// The raw q and k rows arrive as TMA tiles in the residual panels (where each thread later overwrites exactly the
-// 16-byte pieces it read), so their latency is hidden behind the gate phases.
-__global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __grid_constant__ CUtensorMap tm_q,
-                                                          const __grid_constant__ CUtensorMap tm_k) {
+// Sixteen warps.  Thread layout of the elementwise phases: 16 channel groups (8 channels each) x 32 token pairs.  The raw q and k rows
+// arrive as TMA tiles in the residual panels (where each thread later overwrites exactly the 16-byte pieces it read), so their
+// latency is hidden behind the gate phases.  What bounds it: instructions and their latency at the two CTAs that 96 KB of operand panels
+// leave room for - with eight warps per CTA the SM issued 29 % of the time; sixteen halve each thread's chain of work.  8,192 tokens of
+// 32 heads with gate and normalisation: 318 -> 288 us; 32,768 tokens without: 1060 -> 950 us.
+constexpr int kKdaPrepThreads = 512;
+__global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams p, const __grid_constant__ CUtensorMap tm_q,
+                                                                      const __grid_constant__ CUtensorMap tm_k) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ float tot_s[16][kK];          // gate sum of each token segment, per channel
-  __shared__ float anchor_s[kK], last_s[kK];
+  __shared__ __align__(16) float tot_s[16][kK];      // gate sum of each warp's four tokens, per channel
+  __shared__ __align__(16) float anchor_s[kK], last_s[kK];
   __shared__ uint32_t tmem_base_s;
   __shared__ __align__(8) uint64_t bar, qk_bar;
 
@@ -58,7 +62,7 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
   const int rows = min(kC, sq.len - t0);
   const int64_t tok0 = int64_t(sq.bos) + t0;
   const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-  const int cg = tid & 15, seg = tid >> 4, r0 = cg * 8;
+  const int cg = tid & 15, r0 = cg * 8, tb = (tid >> 4) * 2;      // my channels and my first token
 
   if (warp == 0) {
     tmem_alloc(&tmem_base_s, 64);
@@ -77,61 +81,66 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
     tma_load_tile(sbq + pOffQKL + 8192, &tm_k, 0, hk, row0, &qk_bar);           // k rows -> rows 64-127
     tma_load_tile(sbq + pOffQKL + 16384 + 8192, &tm_k, 64, hk, row0, &qk_bar);
   }
-  // 1. activated gates of my 4 tokens x 8 channels, prefix-summed inside the segment (zero past the sequence end)
-  float gk[4][8];
+  // 1. activated gates of my 2 tokens x 8 channels (zero past the sequence end), summed over the warp's tokens before them
+  float gk[2][8];
   {
-    const float eig = (p.gate_mode && p.a_log) ? __expf(p.a_log[hv]) : 1.f;
-    float bias[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) bias[j] = (p.gate_mode && p.dt_bias) ? p.dt_bias[hv * kK + r0 + j] : 0.f;
+    for (int i = 0; i < 2; ++i) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = seg * 4 + i;
-      float raw[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) raw[j] = 0.f;
-      if (t < rows) {
-        const int64_t off = (tok0 + t) * p.g_st + hv * p.g_sh + r0;
-        if (p.g_is_f32) {
-          const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p.g) + off);
-          const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p.g) + off + 4);
-          raw[0] = a.x; raw[1] = a.y; raw[2] = a.z; raw[3] = a.w; raw[4] = b.x; raw[5] = b.y; raw[6] = b.z; raw[7] = b.w;
-        } else {
-          unpack_bf16x8(*reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.g) + off), raw);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float gv = t < rows ? kda_gate(raw[j], p.gate_mode, eig, bias[j], p.lower_bound) : 0.f;
-        gk[i][j] = gv + (i ? gk[i - 1][j] : 0.f);
+      for (int j = 0; j < 8; ++j) gk[i][j] = 0.f;
+      if (tb + i < rows) {
+        const int64_t off = (tok0 + tb + i) * p.g_st + hv * p.g_sh + r0;
+        if (p.g_is_f32) gather8(static_cast<const float*>(p.g) + off, gk[i]);
+        else unpack_bf16x8(*reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.g) + off), gk[i]);
       }
     }
+    if (p.gate_mode) {
+      const float eig = p.a_log ? __expf(p.a_log[hv]) : 1.f;
+      float bias[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) tot_s[seg][r0 + j] = gk[3][j];
+      for (int j = 0; j < 8; ++j) bias[j] = 0.f;
+      if (p.dt_bias) gather8(p.dt_bias + hv * kK + r0, bias);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gk[i][j] = tb + i < rows ? kda_gate(gk[i][j], p.gate_mode, eig, bias[j], p.lower_bound) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      gk[1][j] += gk[0][j];
+      const float below = __shfl_up_sync(0xffffffffu, gk[1][j], 16);
+      if (lane >= 16) {
+        gk[0][j] += below;
+        gk[1][j] += below;
+      }
+    }
+    if (lane >= 16) {
+      *reinterpret_cast<float4*>(&tot_s[warp][r0]) = make_float4(gk[1][0], gk[1][1], gk[1][2], gk[1][3]);
+      *reinterpret_cast<float4*>(&tot_s[warp][r0 + 4]) = make_float4(gk[1][4], gk[1][5], gk[1][6], gk[1][7]);
+    }
   }
   __syncthreads();
-  // 2. add the totals of the earlier segments; publish the anchor row (middle token) and the last valid row
+  // 2. add the totals of the earlier warps; publish the anchor row (middle token) and the last valid row
   {
     float off[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) off[j] = 0.f;
-    for (int sgm = 0; sgm < seg; ++sgm) {
+    for (int w = 0; w < warp; ++w) {
+      float t[8];
+      gather8(&tot_s[w][r0], t);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) off[j] += tot_s[sgm][r0 + j];
+      for (int j = 0; j < 8; ++j) off[j] += t[j];
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) gk[i][j] += off[j];
     const int ta = min(kC / 2 - 1, rows - 1), tl = rows - 1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = seg * 4 + i;
-      if (t == ta) {
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) gk[i][j] += off[j];
+      if (tb + i == ta) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) anchor_s[r0 + j] = gk[i][j];
       }
-      if (t == tl) {
+      if (tb + i == tl) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) last_s[r0 + j] = gk[i][j];
       }
@@ -143,25 +152,33 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
     p.vec[cidx * kKdaVecs * kK + tid] = __expf(a);
     p.vec[cidx * kKdaVecs * kK + kK + tid] = __expf(last_s[tid] - a);
     p.vec[cidx * kKdaVecs * kK + 2 * kK + tid] = a;
-  } else {
+  } else if (tid < 2 * kK) {
     const int t = tid - kK;
     p.vec[cidx * kKdaVecs * kK + 3 * kK + t] = t < rows ? ld_scalar(p.beta, (tok0 + t) * p.beta_st + hv, p.beta_is_f32) : 0.f;
   }
   // 3. scaled operands as split bf16 panels
   {
-    float an[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) an[j] = anchor_s[r0 + j];
     const uint32_t pan = (cg / 8) * 16384, pan64 = (cg / 8) * 8192;
     const bool landed = mbar_wait(&qk_bar, 0, p.status, FLA_ERR_TIMEOUT);
+    if (p.gk_out) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = seg * 4 + i;
-      float qv[8], kv[8], qp[8], kp[8], kn[8];
+      for (int i = 0; i < 2; ++i) {
+        if (tb + i < rows) {
+          float* dst = p.gk_out + ((tok0 + tb + i) * p.HV + hv) * kK + r0;
+          *reinterpret_cast<float4*>(dst) = make_float4(gk[i][0], gk[i][1], gk[i][2], gk[i][3]);
+          *reinterpret_cast<float4*>(dst + 4) = make_float4(gk[i][4], gk[i][5], gk[i][6], gk[i][7]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = tb + i;
+      const uint32_t o1 = panel_chunk_off(t, cg % 8), o2 = panel_chunk_off(64 + t, cg % 8);
+      float qv[8], kv[8];
       uint4 qraw = make_uint4(0, 0, 0, 0), kraw = qraw;
       if (t < rows && landed) {   // rows past the end of the sequence hold foreign tokens in the tile: use zeros
-        qraw = *reinterpret_cast<const uint4*>(smem + pOffQKL + pan + panel_chunk_off(t, cg % 8));
-        kraw = *reinterpret_cast<const uint4*>(smem + pOffQKL + pan + panel_chunk_off(64 + t, cg % 8));
+        qraw = *reinterpret_cast<const uint4*>(smem + pOffQKL + pan + o1);
+        kraw = *reinterpret_cast<const uint4*>(smem + pOffQKL + pan + o2);
       }
       unpack_bf16x8(qraw, qv);
       unpack_bf16x8(kraw, kv);
@@ -179,31 +196,31 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
         const float rq = rsqrtf(sq_q + 1e-6f), rk = rsqrtf(sq_k + 1e-6f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          qv[j] = __bfloat162float(__float2bfloat16_rn(qv[j] * rq));
-          kv[j] = __bfloat162float(__float2bfloat16_rn(kv[j] * rk));
+          qv[j] *= rq;
+          kv[j] *= rk;
         }
+        unpack_bf16x8(pack8(qv), qv);
+        unpack_bf16x8(pack8(kv), kv);
         if (cg == 0 && t < rows && hv == hk * (p.HV / p.HK)) {
           p.q_rstd[(tok0 + t) * p.HK + hk] = rq;
           p.k_rstd[(tok0 + t) * p.HK + hk] = rk;
         }
       }
+      float an[8], kn[8];
+      gather8(&anchor_s[r0], an);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float d = gk[i][j] - an[j];
-        const float e1 = __expf(d), e2 = __expf(-d);
-        qp[j] = qv[j] * e1; kp[j] = kv[j] * e1; kn[j] = kv[j] * e2;
-      }
-      if (p.gk_out && t < rows) {
-        float* dst = p.gk_out + ((tok0 + t) * p.HV + hv) * kK + r0;
-        *reinterpret_cast<float4*>(dst) = make_float4(gk[i][0], gk[i][1], gk[i][2], gk[i][3]);
-        *reinterpret_cast<float4*>(dst + 4) = make_float4(gk[i][4], gk[i][5], gk[i][6], gk[i][7]);
+        const float d = (gk[i][j] - an[j]) * kLog2e;
+        const float e1 = exp2_fast(d);
+        kn[j] = kv[j] * exp2_fast(-d);
+        qv[j] *= e1;
+        kv[j] *= e1;
       }
       uint4 hi, lo;
-      const uint32_t o1 = panel_chunk_off(t, cg % 8), o2 = panel_chunk_off(64 + t, cg % 8);
-      split8(qp, hi, lo);
+      split8(qv, hi, lo);
       *reinterpret_cast<uint4*>(smem + pOffQKH + pan + o1) = hi;
       *reinterpret_cast<uint4*>(smem + pOffQKL + pan + o1) = lo;
-      split8(kp, hi, lo);
+      split8(kv, hi, lo);
       *reinterpret_cast<uint4*>(smem + pOffQKH + pan + o2) = hi;
       *reinterpret_cast<uint4*>(smem + pOffQKL + pan + o2) = lo;
       split8(kn, hi, lo);
@@ -219,58 +236,71 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaParams p, const __g
   const uint32_t sb = smem_u32(smem);
   // 4. save the operand images; both score tiles in one M = 128 product: rows 0-63 Qp Kn^T, rows 64-127 Kp Kn^T
   if (tid == 0) {
-    bulk_store(p.qk_img + cidx * kKdaQkImg, sb + pOffQKH, 65536);
-    bulk_store(p.kn_img + cidx * kKdaKnImg, sb + pOffKNH, 32768);
-    bulk_commit();
     const Operand aH{sb + pOffQKH, 16384, 0}, aL{sb + pOffQKL, 16384, 0};
     const Operand bH{sb + pOffKNH, 8192, 0}, bL{sb + pOffKNL, 8192, 0};
     mma_tile(tbase, aH, bH, 128, 64, 8, false);
     mma_tile(tbase, aH, bL, 128, 64, 8, true);
     mma_tile(tbase, aL, bH, 128, 64, 8, true);
     mma_commit(&bar);
+    bulk_store(p.qk_img + cidx * kKdaQkImg, sb + pOffQKH, 65536);
+    bulk_store(p.kn_img + cidx * kKdaKnImg, sb + pOffKNH, 32768);
+    bulk_commit();
   }
   // 5. q-side rows: P = tril(Aqk) written straight into its split panel image;
   //    k-side rows: Akk^T = (beta_i Kp Kn^T)^T into shared memory, where the operand panels were, and inverted there
-  const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane, tok = row & 63;
+  const int quad = warp & 3, j0 = (warp >> 2) * 16, row = quad * 32 + lane, tok = row & 63;      // my 16 columns of my row
   // requested before the product is waited for
   const float bi = (quad >= 2 && tok < rows) ? ld_scalar(p.beta, (tok0 + tok) * p.beta_st + hv, p.beta_is_f32) : 0.f;
   const bool ok = mbar_wait(&bar, 0, p.status, FLA_ERR_TIMEOUT);
-  if (tid == 0) bulk_wait_read();     // the images have left the panels
+  if (tid == 0) bulk_wait_read();     // the images have left the panels (the end of the kernel completes the writes)
   tc_fence_after();
   __syncthreads();
   float* at = reinterpret_cast<float*>(smem);
+  uint8_t* p_stage = smem + kStageP;
+  uint8_t* x_stage = smem + kStageX;
   if (ok) {
-    float sc[32];
-    tmem_ld32(tmem_addr(tbase, quad * 32, half * 32), sc);
+    float sc[16];
+    tmem_ld16(tmem_addr(tbase, quad * 32, j0), sc);
     tmem_ld_wait();
     if (quad < 2) {
 #pragma unroll
-      for (int jj = 0; jj < 32; ++jj) sc[jj] = (half * 32 + jj <= tok) ? sc[jj] : 0.f;   // select: masked entries may be inf
-      uint8_t* img = reinterpret_cast<uint8_t*>(p.p_img + cidx * kKdaPImg);
+      for (int jj = 0; jj < 16; ++jj) sc[jj] = (j0 + jj <= tok) ? sc[jj] : 0.f;   // select: masked entries may be inf
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
+      for (int ch = 0; ch < 2; ++ch) {
         uint4 hi, lo;
         split8(sc + ch * 8, hi, lo);
-        const uint32_t off = panel_chunk_off(tok, half * 4 + ch);
-        *reinterpret_cast<uint4*>(img + off) = hi;
-        *reinterpret_cast<uint4*>(img + 8192 + off) = lo;
+        const uint32_t off = panel_chunk_off(tok, j0 / 8 + ch);
+        *reinterpret_cast<uint4*>(p_stage + off) = hi;
+        *reinterpret_cast<uint4*>(p_stage + 8192 + off) = lo;
       }
+      fence_async_smem();
     } else {
 #pragma unroll
-      for (int jj = 0; jj < 32; ++jj) {
-        const int j = half * 32 + jj;
+      for (int jj = 0; jj < 16; ++jj) {
+        const int j = j0 + jj;
         at[j * kTriStride + tok] = j < tok ? bi * sc[jj] : 0.f;      // select: entries above the diagonal may be inf
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (tid < 128) {
-    tri_invert(at, tid, 1);
-    tri_store_panels(at, reinterpret_cast<uint8_t*>(p.x_img + cidx * kKdaXImg), rows, tid);
+  if (tid == 256) {
+    bulk_store(p.p_img + cidx * kKdaPImg, sb + kStageP, 16384);
+    bulk_commit();
+    bulk_wait_read();
   }
-  if (tid == 0) bulk_wait_all();
-  if (warp == 0) tmem_dealloc(tbase, 64);
+  if (warp == 12) tmem_dealloc(tbase, 64);
+  if (tid < 256) {
+    tri_invert<256>(at, tid, 1);
+    tri_store_panels<256>(at, x_stage, rows, tid);
+    fence_async_smem();
+    tri_sync<256>(1);
+    if (tid == 0) {
+      bulk_store(p.x_img + cidx * kKdaXImg, sb + kStageX, 16384);
+      bulk_commit();
+      bulk_wait_read();
+    }
+  }
 }
 
 // The two 64 x 64 score blocks of every chunk as plain tensors, for callers of the reference's low-level forward
@@ -551,7 +581,7 @@ int fla::kda_launch_forward(const KdaParams& p, int64_t total_chunks, int64_t se
     return FLA_ERR_CUDA;
   {
     KernelTimer kt("kda_prep", cs);
-    kda_prep_kernel<<<dim3(unsigned(total_chunks), unsigned(p.HV)), 256, kKdaPrepSmem + 1024, cs>>>(p, tm_q, tm_k);
+    kda_prep_kernel<<<dim3(unsigned(total_chunks), unsigned(p.HV)), kKdaPrepThreads, kKdaPrepSmem + 1024, cs>>>(p, tm_q, tm_k);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
