@@ -12,8 +12,10 @@
 // bf16 inputs: kda_prep_kernel (parallel over chunks) builds them once as bf16 hi + residual operand panels,
 // computes both score tiles on tcgen05 and the inverse on CUDA cores, and stores everything as ready-to-load
 // panel images; kda_scan_fwd_kernel (kda_scan_fwd.cuh; sequential over chunks, fp32 state in TMEM) only bulk-loads them.
+#include <algorithm>
 #include "gdn_common.cuh"
 #include "fla_b200_internal.h"
+#include "aux_stream.h"
 #include "kernel_timer.h"
 #include "tri_inverse.cuh"
 #include "kda_common.cuh"
@@ -24,26 +26,35 @@ namespace fla {
 
 // --------------------------------------------------------------------------------------------- prep
 constexpr uint32_t pOffQKH = 0, pOffQKL = 32768, pOffKNH = 65536, pOffKNL = 81920;
-constexpr uint32_t kKdaPrepSmem = 98304;           // operand panels only
-constexpr uint32_t kStageP = 32768, kStageX = 49152;   // once the panels are free: the images of P and of X
+// Once the panels are free: the image of P where Qp was, A^T (inverted in place) and the image of X where Kn was, and the next tile's rows
+// of q and k where the residuals of Qp and Kp were.
+constexpr uint32_t kStageP = pOffQKH, kStageA = pOffKNH, kStageX = pOffKNH + kTriTile * 4;
+constexpr uint32_t kKdaPrepSmem = kStageX + 16384;
+static_assert(kStageX % 1024 == 0 && kKdaPrepSmem >= pOffKNL + 16384, "panel alignment");
 
 __device__ __forceinline__ float kda_gate(float g, int mode, float eig, float bias, float lower_bound) {
   if (mode == 0) return g;
   const float raw = g + bias;
   if (mode == 1) {  // -exp(A_log) * softplus(g + dt_bias)
-    const float sp = raw > 20.f ? raw : log1pf(__expf(raw));
-    return -eig * sp;
+    // softplus(x) = max(x, 0) + log1p(e), e = exp(-|x|);  log1p(e) = 2 atanh(s), s = e / (2 + e) <= 1/3, by its series (what is
+    // left out is below 2e-8 of it)
+    const float e = __expf(-fabsf(raw)), s = __fdividef(e, 2.f + e), z = s * s;
+    float a = 1.f / 13;
+    a = a * z + 1.f / 11; a = a * z + 1.f / 9; a = a * z + 1.f / 7; a = a * z + 1.f / 5; a = a * z + 1.f / 3; a = a * z + 1.f;
+    return -eig * (fmaxf(raw, 0.f) + 2.f * s * a);
   }
-  return lower_bound / (1.f + __expf(-eig * raw));  // lower_bound * sigmoid(exp(A_log) (g + dt_bias))
+  return __fdividef(lower_bound, 1.f + __expf(-eig * raw));  // lower_bound * sigmoid(exp(A_log) (g + dt_bias))
 }
 
-// Sixteen warps.  Thread layout of the elementwise phases: 16 channel groups (8 channels each) x 32 token pairs.  The raw q and k rows
-// arrive as TMA tiles in the residual panels (where each thread later overwrites exactly the 16-byte pieces it read), so their
-// latency is hidden behind the gate phases.  What bounds it: instructions and their latency at the two CTAs that 96 KB of operand panels
-// leave room for - with eight warps per CTA the SM issued 29 % of the time; sixteen halve each thread's chain of work.  8,192 tokens of
-// 32 heads with gate and normalisation: 318 -> 288 us; 32,768 tokens without: 1060 -> 950 us.
-constexpr int kKdaPrepThreads = 512;
-__global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams p, const __grid_constant__ CUtensorMap tm_q,
+// Two CTAs of sixteen warps per SM (what 97 KB of operand panels leave room for), each working through every 2 x #SM-th tile.  Thread
+// layout of the elementwise phases: 16 channel groups (8 channels each) x 32 token pairs.  The raw q and k rows arrive as TMA tiles in the
+// residual panels, where each thread later overwrites exactly the 16-byte pieces it read; those of the next tile are requested as
+// soon as the images have left, and its gates are brought into L2, so that no tile starts with a round trip to HBM.  After the score product the
+// warps part: eight write P, eight invert.  What bounds it: instruction issue in the elementwise phases (45 % over all) and the barriers
+// between the phases.  8,192 tokens of 32 heads with gate and normalisation: 318 us with eight warps per CTA and one tile
+// per CTA, 288 with sixteen warps, 274 now.
+constexpr int kKdaPrepThreads = 512, kLeaderK = 64;      // kLeaderK: the thread that issues for the k-side warps (0 for the q-side)
+__global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams p, unsigned tiles, const __grid_constant__ CUtensorMap tm_q,
                                                                       const __grid_constant__ CUtensorMap tm_k) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -53,34 +64,43 @@ __global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams 
   __shared__ __align__(8) uint64_t bar, qk_bar;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int hv = blockIdx.y;
-  const int hk = hv / (p.HV / p.HK);
-  const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, 0, blockIdx.x);
-  const SeqInfo& sq = pos.sq;
-  const int c = pos.c;
-  const int t0 = c * kC;
-  const int rows = min(kC, sq.len - t0);
-  const int64_t tok0 = int64_t(sq.bos) + t0;
-  const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
   const int cg = tid & 15, r0 = cg * 8, tb = (tid >> 4) * 2;      // my channels and my first token
+  const int quad = warp & 3, j0 = (warp >> 2) * 16, row = quad * 32 + lane, tok = row & 63;      // my 16 score columns of my row
+  const int gva = p.HV / p.HK;
+  const uint32_t sb = smem_u32(smem);
+
+  // a tile is a (chunk, head); heads fastest, so that the CTAs of one moment read neighbouring pieces of the same token rows
+  struct Tile { int hv, tok0, rows; };
+  auto tile_at = [&](unsigned tile) {
+    const unsigned chunk = tile / unsigned(p.HV);
+    const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, 0, int(chunk));
+    return Tile{int(tile - chunk * unsigned(p.HV)), pos.sq.bos + pos.c * kC, min(kC, pos.sq.len - pos.c * kC)};
+  };
+  auto load_qk = [&](const Tile& t) {      // one thread
+    const int hk = t.hv / gva;
+    mbar_arrive_expect_tx(&qk_bar, 4 * 8192);
+    tma_load_tile(sb + pOffQKL, &tm_q, 0, hk, t.tok0, &qk_bar);                  // q rows -> rows 0-63 of the residual panels
+    tma_load_tile(sb + pOffQKL + 16384, &tm_q, 64, hk, t.tok0, &qk_bar);
+    tma_load_tile(sb + pOffQKL + 8192, &tm_k, 0, hk, t.tok0, &qk_bar);           // k rows -> rows 64-127
+    tma_load_tile(sb + pOffQKL + 16384 + 8192, &tm_k, 64, hk, t.tok0, &qk_bar);
+  };
 
   if (warp == 0) {
     tmem_alloc(&tmem_base_s, 64);
     tmem_relinquish();
   }
+  Tile cur = tile_at(blockIdx.x);
   if (tid == 0) {
-    clear_status(p.status, blockIdx.x + hv == 0);
+    clear_status(p.status, blockIdx.x == 0);
     mbar_init(&bar, 1);
     mbar_init(&qk_bar, 1);
     mbar_init_fence();
-    const uint32_t sbq = smem_u32(smem);
-    const int row0 = int(tok0);
-    mbar_arrive_expect_tx(&qk_bar, 4 * 8192);
-    tma_load_tile(sbq + pOffQKL, &tm_q, 0, hk, row0, &qk_bar);                  // q rows -> rows 0-63 of the lo panels
-    tma_load_tile(sbq + pOffQKL + 16384, &tm_q, 64, hk, row0, &qk_bar);
-    tma_load_tile(sbq + pOffQKL + 8192, &tm_k, 0, hk, row0, &qk_bar);           // k rows -> rows 64-127
-    tma_load_tile(sbq + pOffQKL + 16384 + 8192, &tm_k, 64, hk, row0, &qk_bar);
+    load_qk(cur);
   }
+  uint32_t parity = 0;
+  for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x, parity ^= 1) {
+  const int hv = cur.hv, rows = cur.rows;
+  const int64_t tok0 = cur.tok0, cidx = tile;
   // 1. activated gates of my 2 tokens x 8 channels (zero past the sequence end), summed over the warp's tokens before them
   float gk[2][8];
   {
@@ -119,6 +139,7 @@ __global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams 
       *reinterpret_cast<float4*>(&tot_s[warp][r0 + 4]) = make_float4(gk[1][4], gk[1][5], gk[1][6], gk[1][7]);
     }
   }
+  if (tid == 0 || tid == kLeaderK) bulk_wait_read();     // the previous tile's P and X have left shared memory
   __syncthreads();
   // 2. add the totals of the earlier warps; publish the anchor row (middle token) and the last valid row
   {
@@ -159,7 +180,7 @@ __global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams 
   // 3. scaled operands as split bf16 panels
   {
     const uint32_t pan = (cg / 8) * 16384, pan64 = (cg / 8) * 8192;
-    const bool landed = mbar_wait(&qk_bar, 0, p.status, FLA_ERR_TIMEOUT);
+    const bool landed = mbar_wait(&qk_bar, parity, p.status, FLA_ERR_TIMEOUT);
     if (p.gk_out) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -201,9 +222,9 @@ __global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams 
         }
         unpack_bf16x8(pack8(qv), qv);
         unpack_bf16x8(pack8(kv), kv);
-        if (cg == 0 && t < rows && hv == hk * (p.HV / p.HK)) {
-          p.q_rstd[(tok0 + t) * p.HK + hk] = rq;
-          p.k_rstd[(tok0 + t) * p.HK + hk] = rk;
+        if (cg == 0 && t < rows && hv % gva == 0) {
+          p.q_rstd[(tok0 + t) * p.HK + hv / gva] = rq;
+          p.k_rstd[(tok0 + t) * p.HK + hv / gva] = rk;
         }
       }
       float an[8], kn[8];
@@ -233,74 +254,82 @@ __global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams 
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = tmem_base_s;
-  const uint32_t sb = smem_u32(smem);
   // 4. save the operand images; both score tiles in one M = 128 product: rows 0-63 Qp Kn^T, rows 64-127 Kp Kn^T
-  if (tid == 0) {
+  if (tid == kLeaderK) {
     const Operand aH{sb + pOffQKH, 16384, 0}, aL{sb + pOffQKL, 16384, 0};
     const Operand bH{sb + pOffKNH, 8192, 0}, bL{sb + pOffKNL, 8192, 0};
     mma_tile(tbase, aH, bH, 128, 64, 8, false);
     mma_tile(tbase, aH, bL, 128, 64, 8, true);
     mma_tile(tbase, aL, bH, 128, 64, 8, true);
     mma_commit(&bar);
-    bulk_store(p.qk_img + cidx * kKdaQkImg, sb + pOffQKH, 65536);
     bulk_store(p.kn_img + cidx * kKdaKnImg, sb + pOffKNH, 32768);
     bulk_commit();
+  } else if (tid == 0) {
+    bulk_store(p.qk_img + cidx * kKdaQkImg, sb + pOffQKH, 65536);
+    bulk_commit();
   }
-  // 5. q-side rows: P = tril(Aqk) written straight into its split panel image;
-  //    k-side rows: Akk^T = (beta_i Kp Kn^T)^T into shared memory, where the operand panels were, and inverted there
-  const int quad = warp & 3, j0 = (warp >> 2) * 16, row = quad * 32 + lane, tok = row & 63;      // my 16 columns of my row
   // requested before the product is waited for
   const float bi = (quad >= 2 && tok < rows) ? ld_scalar(p.beta, (tok0 + tok) * p.beta_st + hv, p.beta_is_f32) : 0.f;
-  const bool ok = mbar_wait(&bar, 0, p.status, FLA_ERR_TIMEOUT);
-  if (tid == 0) bulk_wait_read();     // the images have left the panels (the end of the kernel completes the writes)
+  const bool more = tile + gridDim.x < tiles;
+  if (more) cur = tile_at(tile + gridDim.x);
+  const bool ok = mbar_wait(&bar, parity, p.status, FLA_ERR_TIMEOUT);
   tc_fence_after();
-  __syncthreads();
-  float* at = reinterpret_cast<float*>(smem);
-  uint8_t* p_stage = smem + kStageP;
-  uint8_t* x_stage = smem + kStageX;
-  if (ok) {
-    float sc[16];
-    tmem_ld16(tmem_addr(tbase, quad * 32, j0), sc);
-    tmem_ld_wait();
-    if (quad < 2) {
-#pragma unroll
-      for (int jj = 0; jj < 16; ++jj) sc[jj] = (j0 + jj <= tok) ? sc[jj] : 0.f;   // select: masked entries may be inf
-#pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {
-        uint4 hi, lo;
-        split8(sc + ch * 8, hi, lo);
-        const uint32_t off = panel_chunk_off(tok, j0 / 8 + ch);
-        *reinterpret_cast<uint4*>(p_stage + off) = hi;
-        *reinterpret_cast<uint4*>(p_stage + 8192 + off) = lo;
-      }
-      fence_async_smem();
-    } else {
-#pragma unroll
-      for (int jj = 0; jj < 16; ++jj) {
-        const int j = j0 + jj;
-        at[j * kTriStride + tok] = j < tok ? bi * sc[jj] : 0.f;      // select: entries above the diagonal may be inf
-      }
-    }
-  }
+  float sc[16];
+  tmem_ld16(tmem_addr(tbase, quad * 32, j0), sc);
+  tmem_ld_wait();
   tc_fence_before();
-  __syncthreads();
-  if (tid == 256) {
-    bulk_store(p.p_img + cidx * kKdaPImg, sb + kStageP, 16384);
-    bulk_commit();
-    bulk_wait_read();
-  }
-  if (warp == 12) tmem_dealloc(tbase, 64);
-  if (tid < 256) {
-    tri_invert<256>(at, tid, 1);
-    tri_store_panels<256>(at, x_stage, rows, tid);
+  if (quad < 2) {
+    // 5a. q-side rows (eight warps): P = tril(Aqk) as split panels, then the next tile's loads
+    if (tid == 0) bulk_wait_read();
+    tri_sync<256>(2);
+    uint8_t* img = smem + kStageP;
+#pragma unroll
+    for (int jj = 0; jj < 16; ++jj) sc[jj] = (ok && j0 + jj <= tok) ? sc[jj] : 0.f;   // select: masked entries may be inf
+#pragma unroll
+    for (int ch = 0; ch < 2; ++ch) {
+      uint4 hi, lo;
+      split8(sc + ch * 8, hi, lo);
+      const uint32_t off = panel_chunk_off(tok, j0 / 8 + ch);
+      *reinterpret_cast<uint4*>(img + off) = hi;
+      *reinterpret_cast<uint4*>(img + 8192 + off) = lo;
+    }
+    fence_async_smem();
+    tri_sync<256>(2);
+    if (tid == 0) {
+      bulk_store(p.p_img + cidx * kKdaPImg, sb + kStageP, 16384);
+      bulk_commit();
+      if (more) load_qk(cur);
+    }
+    if (more) {      // the gates of the next tile as far as L2: four threads a row, 128 bytes each
+      const int t = (warp >> 2) * 64 + (warp & 1) * 32 + lane, es = p.g_is_f32 ? 4 : 2;
+      if (t / 4 < cur.rows && (t & 3) * 128 < kK * es)
+        prefetch_l2(static_cast<const char*>(p.g) + ((int64_t(cur.tok0) + t / 4) * p.g_st + cur.hv * p.g_sh) * es + (t & 3) * 128);
+    }
+  } else {
+    // 5b. k-side rows (eight warps): Akk^T = (beta_i Kp Kn^T)^T, inverted where Kn was
+    const int t = (warp >> 2) * 64 + (warp & 1) * 32 + lane;
+    float* at = reinterpret_cast<float*>(smem + kStageA);
+    if (tid == kLeaderK) bulk_wait_read();
+    tri_sync<256>(1);
+#pragma unroll
+    for (int jj = 0; jj < 16; ++jj) {
+      const int j = j0 + jj;
+      at[j * kTriStride + tok] = ok && j < tok ? bi * sc[jj] : 0.f;      // select: entries above the diagonal may be inf
+    }
+    tri_sync<256>(1);
+    tri_invert<256>(at, t, 1);
+    tri_store_panels<256>(at, smem + kStageX, rows, t);
     fence_async_smem();
     tri_sync<256>(1);
-    if (tid == 0) {
+    if (tid == kLeaderK) {
       bulk_store(p.x_img + cidx * kKdaXImg, sb + kStageX, 16384);
       bulk_commit();
-      bulk_wait_read();
     }
   }
+  }
+  if (tid == 0 || tid == kLeaderK) bulk_wait_read();     // the end of the kernel completes the writes
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem_base_s, 64);
 }
 
 // The two 64 x 64 score blocks of every chunk as plain tensors, for callers of the reference's low-level forward
@@ -581,7 +610,8 @@ int fla::kda_launch_forward(const KdaParams& p, int64_t total_chunks, int64_t se
     return FLA_ERR_CUDA;
   {
     KernelTimer kt("kda_prep", cs);
-    kda_prep_kernel<<<dim3(unsigned(total_chunks), unsigned(p.HV)), kKdaPrepThreads, kKdaPrepSmem + 1024, cs>>>(p, tm_q, tm_k);
+    const unsigned tiles = unsigned(total_chunks) * unsigned(p.HV);
+    kda_prep_kernel<<<std::min(tiles, 2u * unsigned(current_sm_count())), kKdaPrepThreads, kKdaPrepSmem + 1024, cs>>>(p, tiles, tm_q, tm_k);
   }
   if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
