@@ -20,6 +20,7 @@
 //
 // Every operand that is not an exact bf16 input travels as bf16 hi + bf16 residual (three tcgen05.mma passes);
 // accumulation is fp32 in TMEM.
+#include <algorithm>
 #include "gdn_common.cuh"
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
@@ -43,6 +44,7 @@ struct KdaBwdParams {
   const bf16* seg_m;   // split chains: the forward's transition matrices
   float* seg_dh;       // split chains: [segments, HV, V/128, 128, 128]
   int seg_len;         // chunks per segment
+  int* counter;        // tiles the par kernel has handed out beyond its first wave; the scan in front of it sets it to zero
   int clear;           // the scan is the call's first kernel: it clears the status word
   float* bz;           // [V/32, tokens, HV] partial sums of dZ * V over the 32-column slices of V
   const float* dht; float* dh0;
@@ -68,20 +70,23 @@ namespace fla {
 // ============================================================================================= par
 constexpr uint32_t qOffQKH = 0, qOffQKL = 32768, qOffKNH = 65536, qOffKNL = 81920;       // per-head operand images
 // Operands of one 64-channel step are strips (sm100.cuh) whose 64 rows are value channels, the reduction dim of its products.
-constexpr uint32_t qOffAH = 98304;              // [dO^T | dZ_hi^T]: 16 strips of 8 tokens
-constexpr uint32_t qOffAL = 114688;             // 8 KB of zeros, then dZ_lo^T
+constexpr uint32_t qOffAL = 98304;              // 8 KB of zeros (dO has no residual), then dZ_lo^T
+constexpr uint32_t qOffAH = 114688;             // [dO^T | dZ_hi^T]: 16 strips of 8 tokens
 constexpr uint32_t qOffVNH = 131072, qOffVNL = 139264;
 constexpr uint32_t qOffSH = 147456, qOffSL = 163840, qOffDSH = 180224, qOffDSL = 196608;
-constexpr uint32_t qOffPAH = qOffAH, qOffPAL = qOffAL;   // [dP ; dM] hi / lo reuse the [dO ; dZ] panels
-constexpr uint32_t qOffTile = qOffAH;           // two fp32 [64][132] tiles of the dg assembly reuse the step buffers
 constexpr uint32_t kKdaParSmem = 212992;
-constexpr int kTileStride = 132;   // 16-byte aligned rows; float4 row stores and scalar column reads are both conflict-free
+// What reuses the step buffers (all but the zeros): the [dP; dM] panels and the chunk's gk rows (four 64 x 32 fp32 TMA tiles,
+// swizzled), then, over the panels, two fp32 [64][132] tiles of the dg assembly.
+constexpr uint32_t qOffPAH = qOffAL + 8192, qOffPAL = qOffPAH + 16384;
+constexpr uint32_t qOffTile = qOffPAH;
+constexpr int kTileStride = 132;   // 16-byte aligned rows; float4 row stores and float2 column reads are both conflict-free
 constexpr uint32_t kTileBytes = kC * kTileStride * 4;
-constexpr uint32_t qOffGk = 165888;             // the chunk's gk rows: four 64 x 32 fp32 TMA tiles (swizzled), 32 KB
-static_assert(qOffTile + 2 * kTileBytes <= qOffGk && qOffGk % 1024 == 0 && qOffGk + 32768 <= kKdaParSmem &&
-              qOffGk >= qOffSL, "dg tiles and the gk tile must fit in the phase-1 step buffers behind the [dP; dM] panels");
+constexpr uint32_t qOffGk = qOffTile + 2 * kTileBytes;
+static_assert(qOffGk % 1024 == 0 && qOffGk + 32768 <= kKdaParSmem && qOffGk >= qOffPAL + 16384, "dg tiles, panels and gk rows must fit in the step buffers");
 constexpr uint32_t qColQK = 0, qColDV = 64, qColTA = 128, qColTB1 = 256, qColTB2 = 384;
+constexpr uint32_t qColTA2 = 0;                 // [dP; dM] Kn, where the two score tiles were
 constexpr uint32_t kKdaStepBytes = 16384 + 8192 + 16384 + 32768 + 32768;
+constexpr int kParWorkers = 512, kParThreads = kParWorkers + 32;
 
 // sum over 8 columns of (hi + lo panel values) * x
 __device__ __forceinline__ void chunk_vals(const uint8_t* pan_hi, const uint8_t* pan_lo, int row, int ch, float* f) {
@@ -92,439 +97,460 @@ __device__ __forceinline__ void chunk_vals(const uint8_t* pan_hi, const uint8_t*
   for (int j = 0; j < 8; ++j) f[j] += lo[j];
 }
 
-
-// Sum over the 32 lanes (rows) of each of 32 per-lane values (columns): lane l ends up with the total of column l.
+// Sum over the 32 lanes of each of 8 per-lane values: lanes 4 j .. 4 j + 3 end up with the total of value j.
 // Recursive halving: at every step a lane keeps one half of its values and hands the other half to its partner.
-__device__ __forceinline__ float warp_column_sums32(const float* v, int lane) {
-  float a[16], b[8], c[4], d[2];
+__device__ __forceinline__ float warp_column_sums8(const float (&v)[8], int lane) {
+  float a[4], b[2];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float send = (lane & 16) ? v[i] : v[16 + i], keep = (lane & 16) ? v[16 + i] : v[i];
-    a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
+  for (int i = 0; i < 4; ++i) a[i] = ((lane & 16) ? v[4 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, (lane & 16) ? v[i] : v[4 + i], 16);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float send = (lane & 8) ? a[i] : a[8 + i], keep = (lane & 8) ? a[8 + i] : a[i];
-    b[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float send = (lane & 4) ? b[i] : b[4 + i], keep = (lane & 4) ? b[4 + i] : b[i];
-    c[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const float send = (lane & 2) ? c[i] : c[2 + i], keep = (lane & 2) ? c[2 + i] : c[i];
-    d[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-  }
-  const float send = (lane & 1) ? d[0] : d[1], keep = (lane & 1) ? d[1] : d[0];
-  return keep + __shfl_xor_sync(0xffffffffu, send, 1);
+  for (int i = 0; i < 2; ++i) b[i] = ((lane & 8) ? a[2 + i] : a[i]) + __shfl_xor_sync(0xffffffffu, (lane & 8) ? a[i] : a[2 + i], 8);
+  float r = ((lane & 4) ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, (lane & 4) ? b[0] : b[1], 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  return r + __shfl_xor_sync(0xffffffffu, r, 1);
 }
 
-// The chunk's gk rows arrive as TMA tiles once the phase-1 buffers are free; the last epilogue reads them from
-// shared memory (their global loads used to sit, one round trip each, on the critical path).
+__device__ __forceinline__ void par_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kParWorkers) : "memory"); }
+__device__ __forceinline__ bool par_sync_and(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      " .reg .pred p, q;\n"
+      " setp.ne.u32 q, %1, 0;\n"
+      " bar.red.and.pred p, 1, %2, q;\n"
+      " selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(uint32_t(ok)), "n"(kParWorkers)
+      : "memory");
+  return r != 0;
+}
+
+// One CTA per SM; sixteen worker warps and one thread that issues every load and product.  An item is one value head of one
+// (chunk, q/k head) tile; the workers' phases of an item and what the issuing thread does meanwhile:
+//     sum dS'a Sa            score product, then per 64 channels of V: load, three products
+//     [dP; dM] operand       -
+//     -                      the products with [dP; dM], gk rows
+//     dq, dk, dg tiles       -                                            (images free: the next item's are requested)
+//     dg, dq, dk out         score product of the next item, its first step's loads
+// What bounded the one-tile-per-CTA form with eight warps (40,000 cycles a tile, of which the tensor core needs 10,000 and HBM 17,000): nothing
+// overlapped - the prologue and the first loads (5,400), two V steps (9,000), the products with [dP; dM] behind the issuing thread's own
+// epilogue work (5,000), eight warps' worth of fp32 epilogues (12,000), stores (3,000).
+// 32,768 tokens of 32 heads: 2.36 -> 1.78 ms.
+// Tiles are handed out by a counter: next to the other half of the batch's scan (below) the CTAs do not start together.
 // NVB: 64-column blocks of V per head (2 or 4), a compile-time trip count that keeps the block loop unrolled.  NORM: dq, dk go through
-// the q/k normalisation at the end (a kernel of its own: the epilogue's registers would spill in the other: 2.24 -> 2.5 ms).
+// the q/k normalisation at the end (a kernel of its own: the epilogue's registers would spill in the other).
 template <int NVB, bool NORM>
-__global__ void __launch_bounds__(256, 1) kda_bwd_par_kernel(KdaBwdParams p, const __grid_constant__ CUtensorMap tm_gk) {
+__global__ void __launch_bounds__(kParThreads, 1) kda_bwd_par_kernel(KdaBwdParams p, int chunks, const __grid_constant__ CUtensorMap tm_gk) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ float beta_s[kC], anchor_s[kK];
-  __shared__ float red[2][2][kC];      // rkG, ma : [half][row]
+  __shared__ __align__(16) float anchor_s[kK], beta_s[kK];      // neighbours in the prep kernel's record: one load
+  __shared__ float red[2][4][kC];      // rkG, ma : [32-column group of the row][row]
   __shared__ float sds_s[kK];          // sum_v dS'a * Sa per key channel
-  __shared__ float colsum_s[2][kK];    // per 32-row part: column sums of the dgk tiles
-  __shared__ float ndot_s[NORM ? 2 : 1][2 * kC];  // q.dq / k.dk of the complete rows, per half of the columns (normalised q, k only)
+  __shared__ __align__(8) float colsum_s[8][kK];    // per 8-row part: column sums of the dgk tiles
+  __shared__ float ndot_s[NORM ? 4 : 1][2 * kC];    // q.dq / k.dk of the complete rows, per 32-column group (normalised q, k only)
   __shared__ float t1col_s[2][kK];     // per 32-row quadrant: sum_i Kn_i (Vn dS'a^T)_i of the last-row term
+  __shared__ int item_s, tok0_s;
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(8) uint64_t mma_bar, load_bar, img_bar, gk_bar;
+  __shared__ __align__(8) uint64_t img_bar, load_bar, gk_bar;            // loads
+  __shared__ __align__(8) uint64_t step_bar, p1_bar, mma2_bar;           // products: a V step, the last V step, those with [dP; dM]
+  __shared__ __align__(8) uint64_t sds_bar, epi1_bar, epi2_bar, dg_bar;  // workers: step buffers read, [dP; dM] there, images and accumulators read, tiles read
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int hk = blockIdx.y;
-  const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.n0, blockIdx.x);
-  if (pos.n < p.n0 || pos.n >= p.n1) return;      // half of a packed batch: the other half's chunks
-  const SeqInfo& sq = pos.sq;
-  const int c = pos.c;
-  const int t0 = c * kC;
-  const int rows = min(kC, sq.len - t0);
-  const int64_t tok0 = int64_t(sq.bos) + t0;
   const int G = p.HV / p.HK;
-  const int quad = warp & 3, half = warp >> 2;
-  const int row = quad * 32 + lane;           // accumulator row == TMEM lane
-  const bool kside = quad >= 2;
-  const int tok = row & 63;
+  // chunks of this launch: fixed lengths count from the first chunk of sequence n0, a packed batch's half is cut out here
+  int chunk0 = 0;
+  if (p.cu_seqlens) {
+    chunk0 = p.chunk_offsets[p.n0];
+    chunks = p.chunk_offsets[p.n1] - chunk0;
+  }
+  const int tiles = chunks * p.HK;
+  const int flat0 = p.cu_seqlens ? chunk0 : p.n0 * ((p.T + kC - 1) / kC);      // flat index of the launch's first chunk
 
   if (warp == 0) {
     tmem_alloc(&tmem_base_s, 512);
     tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(&mma_bar, 1);
-    mbar_init(&load_bar, 1);
-    mbar_init(&img_bar, 1);
-    mbar_init(&gk_bar, 1);
+    for (uint64_t* b : {&img_bar, &load_bar, &gk_bar, &step_bar, &p1_bar, &mma2_bar}) mbar_init(b, 1);
+    for (uint64_t* b : {&sds_bar, &epi1_bar, &epi2_bar, &dg_bar}) mbar_init(b, kParWorkers / 32);
     mbar_init_fence();
     tma_prefetch_descriptor(&tm_gk);
   }
+  if (tid < kParWorkers) *reinterpret_cast<uint4*>(smem + qOffAL + tid * 16) = make_uint4(0, 0, 0, 0);
+  fence_async_smem();
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
   const uint32_t tbase = tmem_base_s;
-  const uint32_t trow = tmem_addr(tbase, quad * 32, 0);
   const uint32_t sb = smem_u32(smem);
-  uint32_t mphase = 0, lphase = 0, iphase = 0, gphase = 0;
-  bool ok = true;
 
-  auto issue_images = [&](int hv) {           // one thread: [Qp; Kp] and Kn of one value head
-    const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-    mbar_arrive_expect_tx(&img_bar, 65536 + 32768);
-    bulk_load(sb + qOffQKH, p.qk_img + cidx * kKdaQkImg, 65536, &img_bar);
-    bulk_load(sb + qOffKNH, p.kn_img + cidx * kKdaKnImg, 32768, &img_bar);
-  };
-  auto issue_loads = [&](int hv, int vb) {    // one thread: operands of one (value head, V block) step
-    const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-    mbar_arrive_expect_tx(&load_bar, kKdaStepBytes);
-    const bf16* dz = p.dz_img + (cidx * NVB + vb) * 12288;
-    bulk_load(sb + qOffAH, dz, 16384, &load_bar);
-    bulk_load(sb + qOffAL + 8192, dz + 8192, 8192, &load_bar);
-    bulk_load(sb + qOffVNH, p.vn_img + (cidx * NVB + vb) * 8192, 16384, &load_bar);
-    bulk_load(sb + qOffSH, p.s_img + (cidx * NVB + vb) * 16384, 32768, &load_bar);
-    bulk_load(sb + qOffDSH, p.ds_img + (cidx * NVB + vb) * 16384, 32768, &load_bar);
-  };
+  if (warp == kParWorkers / 32) {
+    if (lane == 0) {
+      auto record = [&](int tile, int h) { return int64_t(flat0 + tile / p.HK) * p.HV + (tile % p.HK) * G + h; };
+      auto issue_images = [&](int64_t cidx) {           // [Qp; Kp], Kn, the anchor and beta of one value head
+        mbar_arrive_expect_tx(&img_bar, 65536 + 32768 + 1024);
+        bulk_load(sb + qOffQKH, p.qk_img + cidx * kKdaQkImg, 65536, &img_bar);
+        bulk_load(sb + qOffKNH, p.kn_img + cidx * kKdaKnImg, 32768, &img_bar);
+        bulk_load(smem_u32(anchor_s), p.vec + cidx * kKdaVecs * kK + 2 * kK, 512, &img_bar);
+        bulk_load(smem_u32(beta_s), p.vec + cidx * kKdaVecs * kK + 3 * kK, 512, &img_bar);
+      };
+      auto issue_loads = [&](int64_t cidx, int vb) {    // operands of one (value head, V block) step
+        mbar_arrive_expect_tx(&load_bar, kKdaStepBytes);
+        const bf16* dz = p.dz_img + (cidx * NVB + vb) * kKdaDzImg;
+        bulk_load(sb + qOffAH, dz, 16384, &load_bar);
+        bulk_load(sb + qOffAL + 8192, dz + 8192, 8192, &load_bar);
+        bulk_load(sb + qOffVNH, p.vn_img + (cidx * NVB + vb) * kKdaVnImg, 16384, &load_bar);
+        bulk_load(sb + qOffSH, p.s_img + (cidx * NVB + vb) * kKdaSImg, 32768, &load_bar);
+        bulk_load(sb + qOffDSH, p.ds_img + (cidx * NVB + vb) * kKdaDsImg, 32768, &load_bar);
+      };
+      const Operand opQKh{sb + qOffQKH, 16384, 0}, opQKl{sb + qOffQKL, 16384, 0};           // [Qp; Kp], reduction over key dims
+      const Operand opQKnh{sb + qOffQKH, 16384, 1}, opQKnl{sb + qOffQKL, 16384, 1};         // as B, N = 128 key dims, reduction over 128 rows
+      const Operand opKNbh{sb + qOffKNH, 8192, 0}, opKNbl{sb + qOffKNL, 8192, 0};           // Kn as B, N = 64 tokens
+      const Operand opKNnh{sb + qOffKNH, 8192, 1}, opKNnl{sb + qOffKNL, 8192, 1};           // Kn as B, N = 128 key dims, reduction over tokens
+      const Operand opAH{sb + qOffAH, 1024, 2}, opAL{sb + qOffAL, 1024, 2};                 // [dO; dZ], M = 128 tokens
+      const Operand opVNbH{sb + qOffVNH, 1024, 2}, opVNbL{sb + qOffVNL, 1024, 2};           // Vn as B (N = 64 tokens)
+      const Operand opVNaH{sb + qOffVNH - 8192, 1024, 2}, opVNaL{sb + qOffVNL - 8192, 1024, 2};  // Vn as A, valid rows 64..127
+      const Operand opSH{sb + qOffSH, 1024, 2}, opSL{sb + qOffSL, 1024, 2};                 // Sa block as B (N = 128 key dims)
+      const Operand opDSH{sb + qOffDSH, 1024, 2}, opDSL{sb + qOffDSL, 1024, 2};
+      const Operand opPAH{sb + qOffPAH, 16384, 0}, opPAL{sb + qOffPAL, 16384, 0};           // [dP; dM], reduction over j
+      const Operand opPATh{sb + qOffPAH - 8192, 8192, 1}, opPATl{sb + qOffPAL - 8192, 8192, 1};  // its transpose, valid rows 64..127
 
-  const Operand opQKh{sb + qOffQKH, 16384, 0}, opQKl{sb + qOffQKL, 16384, 0};           // [Qp; Kp], reduction over key dims
-  const Operand opQKnh{sb + qOffQKH, 16384, 1}, opQKnl{sb + qOffQKL, 16384, 1};         // as B, N = 128 key dims, reduction over 128 rows
-  const Operand opKNbh{sb + qOffKNH, 8192, 0}, opKNbl{sb + qOffKNL, 8192, 0};           // Kn as B, N = 64 tokens
-  const Operand opKNnh{sb + qOffKNH, 8192, 1}, opKNnl{sb + qOffKNL, 8192, 1};           // Kn as B, N = 128 key dims, reduction over tokens
-  const Operand opAH{sb + qOffAH, 1024, 2}, opAL{sb + qOffAL, 1024, 2};                 // [dO; dZ], M = 128 tokens
-  const Operand opVNbH{sb + qOffVNH, 1024, 2}, opVNbL{sb + qOffVNL, 1024, 2};           // Vn as B (N = 64 tokens)
-  const Operand opVNaH{sb + qOffVNH - 8192, 1024, 2}, opVNaL{sb + qOffVNL - 8192, 1024, 2};  // Vn as A, valid rows 64..127
-  const Operand opSH{sb + qOffSH, 1024, 2}, opSL{sb + qOffSL, 1024, 2};                 // Sa block as B (N = 128 key dims)
-  const Operand opDSH{sb + qOffDSH, 1024, 2}, opDSL{sb + qOffDSL, 1024, 2};
-  const Operand opPAH{sb + qOffPAH, 16384, 0}, opPAL{sb + qOffPAL, 16384, 0};           // [dP; dM], reduction over j
-  const Operand opPATh{sb + qOffPAH - 8192, 8192, 1}, opPATl{sb + qOffPAL - 8192, 8192, 1};  // its transpose, valid rows 64..127
-
-  float acc_out[64];  // running dq (q-side rows) or dk (k-side rows), this thread's 64 key-dim columns
-#pragma unroll
-  for (int i = 0; i < 64; ++i) acc_out[i] = 0.f;
-  float* tile_q = reinterpret_cast<float*>(smem + qOffTile);
-  float* tile_k = reinterpret_cast<float*>(smem + qOffTile + kTileBytes);
-
-  for (int h = 0; h < G && ok; ++h) {
-    const int hv = hk * G + h;
-    const int64_t cidx = (int64_t(sq.cbase) + c) * p.HV + hv;
-    // zero rows of the lo operand (dO has no residual), this head's scalars, then the loads
-    for (int idx = tid; idx < 512; idx += 256) *reinterpret_cast<uint4*>(smem + qOffAL + idx * 16) = make_uint4(0, 0, 0, 0);
-    if (tid < kC) beta_s[tid] = tid < rows ? ld_scalar(p.beta, (tok0 + tid) * p.beta_st + hv, p.beta_is_f32) : 0.f;
-    if (tid >= 128) anchor_s[tid - 128] = p.vec[cidx * kKdaVecs * kK + 2 * kK + tid - 128];
-    fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      issue_images(hv);
-      issue_loads(hv, 0);
-    }
-    float sds[8];      // sum_v dS'a * Sa: the 8 key dims of strip tid / 16, value channels tid % 16 (mod 16) of every step
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sds[j] = 0.f;
-    for (int vb = 0; vb < NVB; ++vb) {
-      if (vb == 0) {
-        ok = mbar_wait(&img_bar, iphase, p.status, FLA_ERR_TIMEOUT);
-        iphase ^= 1;
-      }
-      ok = mbar_wait(&load_bar, lphase, p.status, FLA_ERR_TIMEOUT) && ok;
-      lphase ^= 1;
-      if (!__syncthreads_and(ok)) { ok = false; break; }
-      if (tid == 0) {
-        tc_fence_after();
-        if (vb == 0) {
-          mma_tile(tbase + qColQK, opQKh, opKNbh, 128, 64, 8, false);
-          mma_tile(tbase + qColQK, opQKh, opKNbl, 128, 64, 8, true);
-          mma_tile(tbase + qColQK, opQKl, opKNbh, 128, 64, 8, true);
-        }
-        const bool accf = vb > 0;
-        // [dO; dZ] . [Vn_lo | Sa_hi]^T as one N = 192 product: the two images are neighbours in shared memory and their
-        // accumulators neighbours in tensor memory, so the A operand is read once for both
-        static_assert(qOffVNL + 8192 == qOffSH && qColDV + 64 == qColTA, "the N = 192 product needs both pairs adjacent");
-        mma_tile(tbase + qColDV, opAH, opVNbL, 128, 192, 4, accf);
-        mma_tile(tbase + qColDV, opAH, opVNbH, 128, 64, 4, true);
-        mma_tile(tbase + qColDV, opAL, opVNbH, 128, 64, 4, true);
-        mma_tile(tbase + qColTA, opAH, opSL, 128, 128, 4, true);
-        mma_tile(tbase + qColTA, opAL, opSH, 128, 128, 4, true);
-        mma_tile(tbase + qColTB1, opVNaH, opDSH, 128, 128, 4, accf);
-        mma_tile(tbase + qColTB1, opVNaH, opDSL, 128, 128, 4, true);
-        mma_tile(tbase + qColTB1, opVNaL, opDSH, 128, 128, 4, true);
-        mma_commit(&mma_bar);
-      }
-      // sum_v dS'a * Sa per key channel over this V block while the MMAs run (elementwise on the images)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const uint32_t off = (tid >> 4) * 1024 + ((tid & 15) + r * 16) * 16;
-        float s1[8], s2[8], d1[8], d2[8];
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffSH + off), s1);
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffSL + off), s2);
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffDSH + off), d1);
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffDSL + off), d2);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) sds[j] += (s1[j] + s2[j]) * (d1[j] + d2[j]);
-      }
-      ok = mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT);
-      mphase ^= 1;
-      if (!__syncthreads_and(ok)) { ok = false; break; }   // also: every thread is done reading the step's buffers
-      tc_fence_after();
-      if (tid == 0) {
-        if (vb + 1 < NVB) {
-          issue_loads(hv, vb + 1);
-        } else {   // the phase-1 buffers are free: this head's gk rows, channels 32 b .. 32 b + 31 in tile b
-          mbar_arrive_expect_tx(&gk_bar, 4 * 8192);
-#pragma unroll
-          for (int b = 0; b < 4; ++b) tma_load_tile(sb + qOffGk + b * 8192, &tm_gk, 32 * b, hv, int(tok0), &gk_bar);
-        }
-      }
-    }
-    if (!ok) break;
-    {      // over the sixteen threads of a strip by halving: thread 2 j (+ 1) of them ends with key dim j
-#pragma unroll
-      for (int o = 8, w = 4; w >= 1; o >>= 1, w >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int j = 0; j < w; ++j) {
-          const float send = up ? sds[j] : sds[j + w], keep = up ? sds[j + w] : sds[j];
-          sds[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-      }
-      sds[0] += __shfl_xor_sync(0xffffffffu, sds[0], 1);
-      if (!(lane & 1)) sds_s[(tid >> 4) * 8 + ((lane >> 1) & 7)] = sds[0];
-    }
-
-    // ---- epilogue 1: score-tile gradients -> [dP; dM] operand; row scaling of the first TA product in place
-    const float beta_i = beta_s[tok];
-    float ma_part = 0.f, rkG = 0.f;
-    {
-      float sc[32], dvv[32];
-      tmem_ld32(trow + qColQK + half * 32, sc);
-      tmem_ld32(trow + qColDV + half * 32, dvv);
-      tmem_ld_wait();
-      if (!kside) {
-#pragma unroll
-        for (int jj = 0; jj < 32; ++jj) dvv[jj] = (half * 32 + jj <= tok) ? p.scale * dvv[jj] : 0.f;
+      auto wait = [&](uint64_t* bar, uint32_t& phase) {
+        const bool r = mbar_wait(bar, phase, p.status, FLA_ERR_TIMEOUT);
+        phase ^= 1;
+        return r;
+      };
+      uint32_t ph_img = 0, ph_load = 0, ph_step = 0, ph_p1 = 0, ph_sds = 0, ph_epi1 = 0, ph_epi2 = 0, ph_dg = 0;
+      int tile = blockIdx.x, h = 0;
+      bool ok = true;
+      if (tile < tiles) {
+        const int64_t cidx = record(tile, 0);
+        item_s = tile * G;
+        issue_images(cidx);
+        issue_loads(cidx, 0);
       } else {
+        item_s = -1;
+        mbar_arrive_expect_tx(&img_bar, 0);
+        ok = false;
+      }
+      int after = ok ? int(gridDim.x) + atomicAdd(p.counter, 1) : 0;      // the tile that follows
+      while (ok) {
+        const int64_t cidx = record(tile, h);
+        const int hv = (tile % p.HK) * G + h;
+        if (!wait(&img_bar, ph_img)) break;
+        tc_fence_after();
+        mma_tile(tbase + qColQK, opQKh, opKNbh, 128, 64, 8, false);
+        mma_tile(tbase + qColQK, opQKh, opKNbl, 128, 64, 8, true);
+        mma_tile(tbase + qColQK, opQKl, opKNbh, 128, 64, 8, true);
+        for (int vb = 0; vb < NVB && ok; ++vb) {
+          ok = wait(&load_bar, ph_load);
+          if (!ok) break;
+          const bool accf = vb > 0;
+          // [dO; dZ] . [Vn_lo | Sa_hi]^T as one N = 192 product: the two images are neighbours in shared memory and their
+          // accumulators neighbours in tensor memory, so the A operand is read once for both
+          static_assert(qOffVNL + 8192 == qOffSH && qColDV + 64 == qColTA, "the N = 192 product needs both pairs adjacent");
+          mma_tile(tbase + qColDV, opAH, opVNbL, 128, 192, 4, accf);
+          mma_tile(tbase + qColDV, opAH, opVNbH, 128, 64, 4, true);
+          mma_tile(tbase + qColDV, opAL, opVNbH, 128, 64, 4, true);
+          mma_tile(tbase + qColTA, opAH, opSL, 128, 128, 4, true);
+          mma_tile(tbase + qColTA, opAL, opSH, 128, 128, 4, true);
+          mma_tile(tbase + qColTB1, opVNaH, opDSH, 128, 128, 4, accf);
+          mma_tile(tbase + qColTB1, opVNaH, opDSL, 128, 128, 4, true);
+          mma_tile(tbase + qColTB1, opVNaL, opDSH, 128, 128, 4, true);
+          if (vb + 1 < NVB) {
+            mma_commit(&step_bar);
+            ok = wait(&sds_bar, ph_sds) && wait(&step_bar, ph_step);
+            if (ok) issue_loads(cidx, vb + 1);
+          } else {
+            mma_commit(&p1_bar);
+            ok = wait(&sds_bar, ph_sds) && wait(&p1_bar, ph_p1);
+            if (ok) {   // the step buffers are free: this head's gk rows, channels 32 b .. 32 b + 31 in tile b
+              mbar_arrive_expect_tx(&gk_bar, 4 * 8192);
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const bool keep = half * 32 + jj < tok;
-          const float dA = keep ? -dvv[jj] : 0.f;
-          ma_part += keep ? dA * sc[jj] : 0.f;      // select: entries above the diagonal of M may be huge
-          dvv[jj] = dA * beta_i;
+              for (int b = 0; b < 4; ++b) tma_load_tile(sb + qOffGk + b * 8192, &tm_gk, 32 * b, hv, tok0_s, &gk_bar);
+            }
+          }
         }
-      }
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        uint4 hi, lo;
-        split8(dvv + ch * 8, hi, lo);
-        const uint32_t off = panel_chunk_off(row, half * 4 + ch);
-        *reinterpret_cast<uint4*>(smem + qOffPAH + off) = hi;
-        *reinterpret_cast<uint4*>(smem + qOffPAL + off) = lo;
-      }
-    }
-    {
-      float ta[64];
-      tmem_ld_row64(trow + qColTA + half * 64, ta);
-      float f = p.scale;
-      if (kside) {
-        // Kp_i . (dZ Sa^T)_i over my 64 key dims
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          float kp[8];
-          chunk_vals(smem + qOffQKH + half * 16384, smem + qOffQKL + half * 16384, 64 + tok, ch, kp);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) rkG += kp[j] * ta[ch * 8 + j];
+        if (!ok || !wait(&epi1_bar, ph_epi1)) break;
+        // TA2 = [dP; dM] Kn   and   TB2 = [dP^T | dM^T] [Qp; Kp]
+        tc_fence_after();
+        mma_tile(tbase + qColTA2, opPAH, opKNnh, 128, 128, 4, false);
+        mma_tile(tbase + qColTA2, opPAH, opKNnl, 128, 128, 4, true);
+        mma_tile(tbase + qColTA2, opPAL, opKNnh, 128, 128, 4, true);
+        mma_tile(tbase + qColTB2, opPATh, opQKnh, 128, 128, 8, false);
+        mma_tile(tbase + qColTB2, opPATh, opQKnl, 128, 128, 8, true);
+        mma_tile(tbase + qColTB2, opPATl, opQKnh, 128, 128, 8, true);
+        mma_commit(&mma2_bar);
+        if (++h == G) {
+          h = 0;
+          tile = after;
+          if (tile < tiles) after = int(gridDim.x) + atomicAdd(p.counter, 1);
         }
-        f = -beta_i;
+        const bool more = tile < tiles;
+        if (!wait(&epi2_bar, ph_epi2)) break;
+        item_s = more ? tile * G + h : -1;
+        if (!more) {
+          mbar_arrive_expect_tx(&img_bar, 0);
+          break;
+        }
+        issue_images(record(tile, h));
+        if (!wait(&dg_bar, ph_dg)) break;
+        issue_loads(record(tile, h), 0);
       }
+    }
+  } else {
+    const int quad = warp & 3, cg = warp >> 2;  // my 32 accumulator rows, my 32 key-dim columns
+    const int row = quad * 32 + lane;           // accumulator row == TMEM lane
+    const bool kside = quad >= 2;
+    const int tok = row & 63;
+    const uint32_t trow = tmem_addr(tbase, quad * 32, 0);
+    float* tile_q = reinterpret_cast<float*>(smem + qOffTile);
+    float* tile_k = reinterpret_cast<float*>(smem + qOffTile + kTileBytes);
+    const uint8_t* qk_h = smem + qOffQKH + (cg >> 1) * 16384;      // the panels of my columns
+    const uint8_t* qk_l = smem + qOffQKL + (cg >> 1) * 16384;
+    const uint8_t* kn_h = smem + qOffKNH + (cg >> 1) * 8192;
+    const uint8_t* kn_l = smem + qOffKNL + (cg >> 1) * 8192;
+    auto signal = [&](uint64_t* bar) {      // my warp is done with what the barrier stands for
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    uint32_t ph_load = 0, ph = 0;
+    bool ok = true;
+    float acc[32];      // running dq (q-side rows) or dk (k-side rows), my 32 key-dim columns
 #pragma unroll
-      for (int i = 0; i < 64; ++i) ta[i] *= f;
-      tmem_st_row64(trow + qColTA + half * 64, ta);
-    }
-    if (kside) {
-      red[0][half][tok] = rkG;
-      red[1][half][tok] = ma_part;
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
+    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
 
-    // ---- TA += [dP; dM] Kn   and   TB2 = [dP^T | dM^T] [Qp; Kp]
-    if (tid == 0) {
-      tc_fence_after();
-      mma_tile(tbase + qColTA, opPAH, opKNnh, 128, 128, 4, true);
-      mma_tile(tbase + qColTA, opPAH, opKNnl, 128, 128, 4, true);
-      mma_tile(tbase + qColTA, opPAL, opKNnh, 128, 128, 4, true);
-      mma_tile(tbase + qColTB2, opPATh, opQKnh, 128, 128, 8, false);
-      mma_tile(tbase + qColTB2, opPATh, opQKnl, 128, 128, 8, true);
-      mma_tile(tbase + qColTB2, opPATl, opQKnh, 128, 128, 8, true);
-      mma_commit(&mma_bar);
-    }
-    // dbeta while the MMAs run
-    if (tid < rows) {
-      const int i = tid;
-      const int64_t gidx = (tok0 + i) * p.HV + hv;
-      const int64_t bzs = p.total_tokens * p.HV;
+    while (true) {
+      // a wait that runs out makes this thread skip the rest of its waits; all leave together at the next turn
+      ok = ok && mbar_wait(&img_bar, ph, p.status, FLA_ERR_TIMEOUT);
+      const int item = item_s;
+      if (!par_sync_and(ok) || item < 0) break;
+      const int tile = item / G, h = item - tile * G, hk = tile % p.HK, hv = hk * G + h;
+      const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.n0, chunk0 + tile / p.HK);
+      const int t0 = pos.c * kC, rows = min(kC, pos.sq.len - t0);
+      const int64_t tok0 = int64_t(pos.sq.bos) + t0;
+      if (tid == 0) tok0_s = int(tok0);
       float bz = 0.f;
-      for (int s = 0; s < NVB; ++s) bz += p.bz[(2 * s) * bzs + gidx] + p.bz[(2 * s + 1) * bzs + gidx];
-      const float db = bz - (red[0][0][i] + red[0][1][i]) + (red[1][0][i] + red[1][1][i]);
-      if (p.dbeta_f32) static_cast<float*>(p.dbeta)[gidx] = db;
-      else static_cast<bf16*>(p.dbeta)[gidx] = __float2bfloat16_rn(db);
-    }
-    ok = mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT);
-    mphase ^= 1;
-    if (!__syncthreads_and(ok)) { ok = false; break; }
-    tc_fence_after();
-
-    // ---- epilogue 2: dq / dk rows of this head and the three dg tiles (the step buffers are free now)
-    {
-      const int pan = half;   // my 64 key dims are panel `half` of the 128-wide images
-      const bool live = tok < rows;
-      ok = mbar_wait(&gk_bar, gphase, p.status, FLA_ERR_TIMEOUT) && ok;
-      gphase ^= 1;
+      if (tid < rows) {
+        const int64_t gidx = (tok0 + tid) * p.HV + hv, bzs = p.total_tokens * p.HV;
 #pragma unroll
-      for (int sub = 0; sub < 2; ++sub) {
-        float x[32];
-        tmem_ld32(trow + qColTA + half * 64 + sub * 32, x);
+        for (int s = 0; s < 2 * NVB; ++s) bz += p.bz[s * bzs + gidx];
+      }
+      {      // sum_v dS'a * Sa per key channel while the products run: strip `warp` is 8 key dims
+        float sds[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sds[j] = 0.f;
+        for (int vb = 0; vb < NVB; ++vb) {
+          ok = ok && mbar_wait(&load_bar, ph_load, p.status, FLA_ERR_TIMEOUT);
+          ph_load ^= 1;
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const uint32_t off = warp * 1024 + (lane + r * 32) * 16;
+            float s1[8], s2[8], d1[8], d2[8];
+            unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffSH + off), s1);
+            unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffSL + off), s2);
+            unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffDSH + off), d1);
+            unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + qOffDSL + off), d2);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sds[j] += (s1[j] + s2[j]) * (d1[j] + d2[j]);
+          }
+          signal(&sds_bar);
+        }
+        const float t = warp_column_sums8(sds, lane);
+        if (!(lane & 3)) sds_s[warp * 8 + (lane >> 2)] = t;
+      }
+
+      // ---- epilogue 1: score-tile gradients -> [dP; dM] operand
+      ok = ok && mbar_wait(&p1_bar, ph, p.status, FLA_ERR_TIMEOUT);
+      tc_fence_after();
+      const float beta_i = beta_s[tok];
+      float rkG = 0.f;
+      {
+        float sc[16], dvv[16], ma = 0.f;
+        tmem_ld16(trow + qColQK + cg * 16, sc);
+        tmem_ld16(trow + qColDV + cg * 16, dvv);
         tmem_ld_wait();
         if (!kside) {
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            float qp[8];
-            chunk_vals(smem + qOffQKH + pan * 16384, smem + qOffQKL + pan * 16384, tok, sub * 4 + ch, qp);
-            const uint8_t* gt = smem + qOffGk + (half * 2 + sub) * 8192 + tok * 128;
-            const float4 g0 = *reinterpret_cast<const float4*>(gt + (((2 * ch) ^ (tok & 7)) << 4));
-            const float4 g1 = *reinterpret_cast<const float4*>(gt + (((2 * ch + 1) ^ (tok & 7)) << 4));
-            const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-            float tq[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int col = sub * 32 + ch * 8 + j;
-              const float xv = x[ch * 8 + j];
-              const float e1 = __expf(gv[j] - anchor_s[half * 64 + col]);
-              acc_out[col] += live ? xv * e1 : 0.f;
-              tq[j] = live ? qp[j] * xv : 0.f;
-            }
-            float* dq_ = tile_q + tok * kTileStride + half * 64 + sub * 32 + ch * 8;
-            *reinterpret_cast<float4*>(dq_) = make_float4(tq[0], tq[1], tq[2], tq[3]);
-            *reinterpret_cast<float4*>(dq_ + 4) = make_float4(tq[4], tq[5], tq[6], tq[7]);
-          }
+          for (int jj = 0; jj < 16; ++jj) dvv[jj] = (cg * 16 + jj <= tok) ? p.scale * dvv[jj] : 0.f;
         } else {
-          float y1[32], y2[32], t1v[32];
-          tmem_ld32(trow + qColTB1 + half * 64 + sub * 32, y1);
-          tmem_ld32(trow + qColTB2 + half * 64 + sub * 32, y2);
+#pragma unroll
+          for (int jj = 0; jj < 16; ++jj) {
+            const bool keep = cg * 16 + jj < tok;
+            const float dA = keep ? -dvv[jj] : 0.f;
+            ma += keep ? dA * sc[jj] : 0.f;      // select: entries above the diagonal of M may be huge
+            dvv[jj] = dA * beta_i;
+          }
+          red[1][cg][tok] = ma;
+        }
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+          uint4 hi, lo;
+          split8(dvv + ch * 8, hi, lo);
+          const uint32_t off = panel_chunk_off(row, cg * 2 + ch);
+          *reinterpret_cast<uint4*>(smem + qOffPAH + off) = hi;
+          *reinterpret_cast<uint4*>(smem + qOffPAL + off) = lo;
+        }
+      }
+      fence_async_smem();
+      tc_fence_before();
+      signal(&epi1_bar);
+
+      // ---- epilogue 2: dq / dk rows of this head and the two dg tiles (the panels are free then)
+      ok = ok && mbar_wait(&gk_bar, ph, p.status, FLA_ERR_TIMEOUT) && mbar_wait(&mma2_bar, ph, p.status, FLA_ERR_TIMEOUT);
+      tc_fence_after();
+      const bool live = tok < rows;
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) {
+        const int c8 = cg * 32 + ch * 8, pc = (cg & 1) * 4 + ch;      // my 8 columns, their 16-byte piece of the panel row
+        float x[8], x2[8], gv[8];
+        tmem_ld8(trow + qColTA + c8, x);
+        tmem_ld8(trow + qColTA2 + c8, x2);
+        {
+          const uint8_t* gt = smem + qOffGk + cg * 8192 + tok * 128;
+          const float4 g0 = *reinterpret_cast<const float4*>(gt + (((2 * ch) ^ (tok & 7)) << 4));
+          const float4 g1 = *reinterpret_cast<const float4*>(gt + (((2 * ch + 1) ^ (tok & 7)) << 4));
+          float an[8];
+          gather8(anchor_s + c8, an);
+          gv[0] = g0.x; gv[1] = g0.y; gv[2] = g0.z; gv[3] = g0.w; gv[4] = g1.x; gv[5] = g1.y; gv[6] = g1.z; gv[7] = g1.w;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) gv[j] = (gv[j] - an[j]) * kLog2e;
+        }
+        float tv[8];
+        if (!kside) {
+          float qp[8];
+          chunk_vals(qk_h, qk_l, tok, pc, qp);
           tmem_ld_wait();
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            float kp[8], kn[8];
-            chunk_vals(smem + qOffQKH + pan * 16384, smem + qOffQKL + pan * 16384, 64 + tok, sub * 4 + ch, kp);
-            chunk_vals(smem + qOffKNH + pan * 8192, smem + qOffKNL + pan * 8192, tok, sub * 4 + ch, kn);
-            const uint8_t* gt = smem + qOffGk + (half * 2 + sub) * 8192 + tok * 128;
-            const float4 g0 = *reinterpret_cast<const float4*>(gt + (((2 * ch) ^ (tok & 7)) << 4));
-            const float4 g1 = *reinterpret_cast<const float4*>(gt + (((2 * ch + 1) ^ (tok & 7)) << 4));
-            const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-            float tk[8];
+          for (int j = 0; j < 8; ++j) {
+            const float xv = p.scale * x[j] + x2[j];
+            acc[ch * 8 + j] += live ? xv * exp2_fast(gv[j]) : 0.f;
+            tv[j] = live ? qp[j] * xv : 0.f;
+          }
+        } else {
+          float y1[8], y2[8], kp[8], kn[8], t1v[8];
+          tmem_ld8(trow + qColTB1 + c8, y1);
+          tmem_ld8(trow + qColTB2 + c8, y2);
+          chunk_vals(qk_h, qk_l, 64 + tok, pc, kp);
+          chunk_vals(kn_h, kn_l, tok, pc, kn);
+          tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int col = sub * 32 + ch * 8 + j;
-              const float d = gv[j] - anchor_s[half * 64 + col];
-              const float e1 = __expf(d), e2 = __expf(-d);
-              const float dkp = x[ch * 8 + j], t1 = y1[ch * 8 + j], dkn = t1 + y2[ch * 8 + j];
-              acc_out[col] += live ? dkp * e1 + dkn * e2 : 0.f;
-              tk[j] = live ? kp[j] * dkp - kn[j] * dkn : 0.f;
-              t1v[ch * 8 + j] = live ? kn[j] * t1 : 0.f;
-            }
-            float* dk_ = tile_k + tok * kTileStride + half * 64 + sub * 32 + ch * 8;
-            *reinterpret_cast<float4*>(dk_) = make_float4(tk[0], tk[1], tk[2], tk[3]);
-            *reinterpret_cast<float4*>(dk_ + 4) = make_float4(tk[4], tk[5], tk[6], tk[7]);
+          for (int j = 0; j < 8; ++j) {
+            rkG += kp[j] * x[j];      // Kp_i . (dZ Sa^T)_i
+            const float dkp = x2[j] - beta_i * x[j], dkn = y1[j] + y2[j];
+            acc[ch * 8 + j] += live ? dkp * exp2_fast(gv[j]) + dkn * exp2_fast(-gv[j]) : 0.f;
+            tv[j] = live ? kp[j] * dkp - kn[j] * dkn : 0.f;
+            t1v[j] = live ? kn[j] * y1[j] : 0.f;
           }
           // last-row term: column sums of Kn * (Vn dS'a^T) over my warp's 32 rows
-          t1col_s[quad - 2][half * 64 + sub * 32 + lane] = warp_column_sums32(t1v, lane);
+          const float t = warp_column_sums8(t1v, lane);
+          if (!(lane & 3)) t1col_s[quad - 2][c8 + (lane >> 2)] = t;
         }
+        float* dst = (kside ? tile_k : tile_q) + tok * kTileStride + c8;
+        *reinterpret_cast<float4*>(dst) = make_float4(tv[0], tv[1], tv[2], tv[3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(tv[4], tv[5], tv[6], tv[7]);
       }
-    }
-    tc_fence_before();
-    if (!__syncthreads_and(ok)) { ok = false; break; }
-    // dg = reverse chunk-local cumulative sum of dgk; the last row additionally carries
-    // sum_v dS'a Sa + sum_i Kn_i (Vn dS'a^T)_i, which therefore reaches every row.
-    {
-      // Two threads per key channel, 32 rows each: local totals first, then the suffix sums.  Each group of eight rows is
-      // read into registers before any of its results is stored: a global store between two shared-memory loads would keep
-      // the compiler from overlapping them (it cannot tell the generic pointers apart).
-      const int kc = tid & (kK - 1), part = tid >> 7, r0 = part * 32;
-      float tot = 0.f;
-#pragma unroll 8
-      for (int i = 0; i < 32; ++i) tot += tile_q[(r0 + i) * kTileStride + kc] + tile_k[(r0 + i) * kTileStride + kc];   // rows past the end hold zeros
-      colsum_s[part][kc] = tot;
-      __syncthreads();
-      float run = sds_s[kc] + t1col_s[0][kc] + t1col_s[1][kc] + (part == 0 ? colsum_s[1][kc] : 0.f);
-      const int64_t base = tok0 * p.dg_st + hv * p.dg_sh + kc;
-      for (int blk = 3; blk >= 0; --blk) {
-        float vals[8];
+      if (kside) red[0][cg][tok] = rkG;
+      tc_fence_before();
+      signal(&epi2_bar);
+      ok = par_sync_and(ok);
+      // dg = reverse chunk-local cumulative sum of dgk; the last row additionally carries
+      // sum_v dS'a Sa + sum_i Kn_i (Vn dS'a^T)_i, which therefore reaches every row.
+      {
+        // A thread has two key channels and 8 rows: local totals first, then the suffix sums.
+        const int kc = (tid & 63) * 2, part = tid >> 6, r0 = part * 8;
+        float2 v[8];      // rows past the end hold zeros
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int t = r0 + blk * 8 + j;
-          vals[j] = tile_q[t * kTileStride + kc] + tile_k[t * kTileStride + kc];
+        for (int i = 0; i < 8; ++i) {
+          const float2 a = *reinterpret_cast<const float2*>(tile_q + (r0 + i) * kTileStride + kc);
+          const float2 b = *reinterpret_cast<const float2*>(tile_k + (r0 + i) * kTileStride + kc);
+          v[i] = make_float2(a.x + b.x, a.y + b.y);
         }
+        float2 run = make_float2(sds_s[kc] + t1col_s[0][kc] + t1col_s[1][kc], sds_s[kc + 1] + t1col_s[0][kc + 1] + t1col_s[1][kc + 1]);
+        float db = 0.f;
+        if (tid < kC) {
+          db = bz;
 #pragma unroll
-        for (int j = 7; j >= 0; --j) {
-          run += vals[j];
-          vals[j] = run;
+          for (int s = 0; s < 4; ++s) db += red[1][s][tid] - red[0][s][tid];
         }
+        fence_async_smem();
+        signal(&dg_bar);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int t = r0 + blk * 8 + j;
-          if (t < rows) {
-            if (p.dg_f32) static_cast<float*>(p.dg)[base + t * p.dg_st] = vals[j];
-            else static_cast<bf16*>(p.dg)[base + t * p.dg_st] = __float2bfloat16_rn(vals[j]);
+        for (int i = 6; i >= 0; --i) {      // suffix sums of my rows
+          v[i].x += v[i + 1].x;
+          v[i].y += v[i + 1].y;
+        }
+        *reinterpret_cast<float2*>(&colsum_s[part][kc]) = v[0];
+        if (tid < rows) {
+          const int64_t gidx = (tok0 + tid) * p.HV + hv;
+          if (p.dbeta_f32) static_cast<float*>(p.dbeta)[gidx] = db;
+          else static_cast<bf16*>(p.dbeta)[gidx] = __float2bfloat16_rn(db);
+        }
+        par_sync();
+        for (int s = part + 1; s < 8; ++s) {
+          const float2 t = *reinterpret_cast<const float2*>(&colsum_s[s][kc]);
+          run.x += t.x;
+          run.y += t.y;
+        }
+        const int64_t base = tok0 * p.dg_st + hv * p.dg_sh + kc;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int t = r0 + i;
+          if (ok && t < rows) {
+            if (p.dg_f32) *reinterpret_cast<float2*>(static_cast<float*>(p.dg) + base + t * p.dg_st) = make_float2(run.x + v[i].x, run.y + v[i].y);
+            else *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.dg) + base + t * p.dg_st) = pack_bf16(run.x + v[i].x, run.y + v[i].y);
           }
         }
       }
-    }
-    __syncthreads();
-  }
+      ph ^= 1;
+      if (h + 1 < G) continue;
 
-  if constexpr (NORM) {   // the rows are complete: rstd (dx - x (x . dx)) with x the normalised row, made again from the raw one
-    const int64_t r = tok0 + min(tok, rows - 1);
-    const float rs = (kside ? p.k_rstd : p.q_rstd)[r * p.HK + hk];
-    const bf16* src = kside ? p.k + r * p.k_st + hk * p.k_sh : p.q + r * p.q_st + hk * p.q_sh;
-    uint4 raw[8];
+      if constexpr (NORM) {   // the rows are complete: rstd (dx - x (x . dx)) with x the normalised row, made again from the raw one
+        const int64_t r = tok0 + min(tok, rows - 1);
+        const float rs = (kside ? p.k_rstd : p.q_rstd)[r * p.HK + hk];
+        const bf16* src = (kside ? p.k + r * p.k_st + hk * p.k_sh : p.q + r * p.q_st + hk * p.q_sh) + cg * 32;
+        uint4 raw[4];
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) raw[ch] = *reinterpret_cast<const uint4*>(src + half * 64 + ch * 8);
-    float t = 0.f;
+        for (int ch = 0; ch < 4; ++ch) raw[ch] = *reinterpret_cast<const uint4*>(src + ch * 8);
+        float t = 0.f;
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      float f[8];
-      unpack_bf16x8(raw[ch], f);
+        for (int ch = 0; ch < 4; ++ch) {
+          float f[8];
+          unpack_bf16x8(raw[ch], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = f[j] * rs;
-      raw[ch] = pack8(f);
-      unpack_bf16x8(raw[ch], f);
+          for (int j = 0; j < 8; ++j) f[j] = f[j] * rs;
+          raw[ch] = pack8(f);
+          unpack_bf16x8(raw[ch], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) t += f[j] * acc_out[ch * 8 + j];
-    }
-    ndot_s[half][row] = t;
-    __syncthreads();
-    t = ndot_s[0][row] + ndot_s[1][row];
+          for (int j = 0; j < 8; ++j) t += f[j] * acc[ch * 8 + j];
+        }
+        ndot_s[cg][row] = t;
+        par_sync();
+        t = (ndot_s[0][row] + ndot_s[1][row]) + (ndot_s[2][row] + ndot_s[3][row]);
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      float f[8];
-      unpack_bf16x8(raw[ch], f);
+        for (int ch = 0; ch < 4; ++ch) {
+          float f[8];
+          unpack_bf16x8(raw[ch], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc_out[ch * 8 + j] = (acc_out[ch * 8 + j] - t * f[j]) * rs;
-    }
-  }
-  if (ok && tok < rows) {
-    void* base = kside ? p.dk : p.dq;
-    const int64_t off = kside ? (tok0 + tok) * p.dk_st + hk * p.dk_sh + half * 64 : (tok0 + tok) * p.dq_st + hk * p.dq_sh + half * 64;
-    if (kside ? p.dk_f32 : p.dq_f32) {
-      float* dst = static_cast<float*>(base) + off;
+          for (int j = 0; j < 8; ++j) acc[ch * 8 + j] = (acc[ch * 8 + j] - t * f[j]) * rs;
+        }
+      }
+      if (ok && live) {
+        void* base = kside ? p.dk : p.dq;
+        const int64_t off = (kside ? (tok0 + tok) * p.dk_st + hk * p.dk_sh : (tok0 + tok) * p.dq_st + hk * p.dq_sh) + cg * 32;
+        if (kside ? p.dk_f32 : p.dq_f32) {
+          float* dst = static_cast<float*>(base) + off;
 #pragma unroll
-      for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(acc_out[i], acc_out[i + 1], acc_out[i + 2], acc_out[i + 3]);
-    } else {
-      bf16* dst = static_cast<bf16*>(base) + off;
+          for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+        } else {
+          bf16* dst = static_cast<bf16*>(base) + off;
 #pragma unroll
-      for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<uint4*>(dst + ch * 8) = pack8(acc_out + ch * 8);
+          for (int ch = 0; ch < 4; ++ch) *reinterpret_cast<uint4*>(dst + ch * 8) = pack8(acc + ch * 8);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) acc[i] = 0.f;
     }
   }
   tc_fence_before();
@@ -690,6 +716,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   p.dg_f32 = a->dg.dtype == FLA_F32; p.dbeta_f32 = a->dbeta.dtype == FLA_F32;
   p.scale = a->scale;
   p.status = f.status;
+  p.counter = f.status + 16;      // both inside the workspace's 256-byte head
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   if (!have_saved && (st = kda_launch_forward(f, total_chunks, plan.count, cs))) return st;
@@ -717,7 +744,7 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   auto launch_par = [&](const KdaBwdParams& pp, int64_t chunks, cudaStream_t st_) {
     auto* par = nvb == 2 ? (pp.q_rstd ? kda_bwd_par_kernel<2, true> : kda_bwd_par_kernel<2, false>)
                          : (pp.q_rstd ? kda_bwd_par_kernel<4, true> : kda_bwd_par_kernel<4, false>);
-    par<<<dim3(unsigned(chunks), unsigned(HK)), 256, kKdaParSmem + 1024, st_>>>(pp, tm_gk);
+    par<<<unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads, kKdaParSmem + 1024, st_>>>(pp, int(chunks), tm_gk);
   };
   // more scan chains (one CTA per SM each) than SMs: two halves of the batch on two streams, so that the chunk-parallel
   // kernel of the first half fills the SMs the second half's scan leaves idle (aux_stream.h)
@@ -728,10 +755,11 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
     const int n1 = N / 2;
     KdaBwdParams p2 = p;
     p.n1 = p2.n0 = n1;
+    p2.counter = p.counter + 16;
     if (cudaEventRecord(aux->fork, cs) != cudaSuccess || cudaStreamWaitEvent(aux->s, aux->fork, 0) != cudaSuccess) return FLA_ERR_CUDA;
     launch_scan(p, n1, cs);
     launch_scan(p2, N - n1, aux->s);
-    // a packed batch's halves hold chunk counts the host does not have: both launches cover all chunks and skip the other half's
+    // a packed batch's halves hold chunk counts the host does not have: the kernel looks up its own
     const int64_t nt = (T + kC - 1) / kC;
     launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs);
     launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s);
