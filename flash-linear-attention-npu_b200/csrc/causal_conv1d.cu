@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
+#include "common/pdl.cuh"
 #include "aux_stream.h"
 
 namespace fla {
@@ -229,65 +230,83 @@ struct ConvUpdParams {
 
 // Fast path: one token per sequence, state holds exactly W-1 inputs.
 // STATE_DMAJOR: state is [slots, W-1, D] (channels contiguous); otherwise [slots, D, W-1] (taps contiguous).
-template <int W, bool STATE_DMAJOR>
+// A thread takes NS sequences of its 8 channels: the taps (64 bytes per thread, a full pass over L1 for every warp) are read once
+// for all of them and NS times W 16-byte loads are in flight.
+template <int W, bool STATE_DMAJOR, int NS>
 __global__ void __launch_bounds__(kConvThreads) conv_update1_kernel(ConvUpdParams p) {
   constexpr int S = W - 1;
+  pdl_trigger();
+  pdl_wait();
   const int d0 = (blockIdx.x * kConvThreads + threadIdx.x) * 8;
   if (d0 >= p.D) return;
-  const int n = blockIdx.y;
-  int slot = n;
-  if (p.cache_indices) slot = p.cache_indices[n];
-  if (slot == p.pad_slot_id || slot < 0 || slot >= p.nslots) return;
-
-  float w[W][8], acc[8], xv[8], h[S][8];
-  load_weights<W>(p.weight, p.w_sd, p.w_sw, d0, w);
-  if (p.bias) unpack8(*reinterpret_cast<const uint4*>(p.bias + d0), acc);
-  else {
+  uint4 xr[NS], hr[NS][S];
+  int64_t so[NS];         // offset of the sequence's state; negative: nothing to do
 #pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c] = 0.f;
-  }
-  unpack8(*reinterpret_cast<const uint4*>(p.x + n * p.x_sn + d0), xv);
-  bf16* st = p.state + slot * p.s_sn;
-  if constexpr (STATE_DMAJOR) {
-#pragma unroll
-    for (int s = 0; s < S; ++s) unpack8(*reinterpret_cast<const uint4*>(st + s * p.s_ss + d0), h[s]);
-  } else {
-    // 8 channels x S taps are 8*S contiguous elements = S 16-byte vectors
-    float flat[S * 8];
-#pragma unroll
-    for (int s = 0; s < S; ++s) unpack8(*reinterpret_cast<const uint4*>(st + int64_t(d0) * S + s * 8), flat + s * 8);
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-#pragma unroll
-      for (int s = 0; s < S; ++s) h[s][c] = flat[c * S + s];
-  }
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float a = acc[c] + w[W - 1][c] * xv[c];
-#pragma unroll
-    for (int s = 0; s < S; ++s) a += w[s][c] * h[s][c];
-    acc[c] = p.silu ? silu(a) : a;
-  }
-  if (p.residual) {
-    float rv[8];
-    unpack8(*reinterpret_cast<const uint4*>(p.residual + n * p.r_sn + d0), rv);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c] += rv[c];
-  }
-  *reinterpret_cast<uint4*>(p.y + n * p.y_sn + d0) = pack8f(acc);
-  // new state = (h[1], ..., h[S-1], x)
-  if constexpr (STATE_DMAJOR) {
+  for (int i = 0; i < NS; ++i) {
+    const int n = blockIdx.y * NS + i;
+    int slot = n;
+    if (p.cache_indices && n < p.N) slot = p.cache_indices[n];
+    so[i] = (n >= p.N || slot == p.pad_slot_id || slot < 0 || slot >= p.nslots) ? -1 : slot * p.s_sn;
+    if (so[i] < 0) continue;
+    xr[i] = *reinterpret_cast<const uint4*>(p.x + n * p.x_sn + d0);
+    // taps contiguous: 8 channels x S taps are 8*S contiguous elements = S 16-byte vectors
 #pragma unroll
     for (int s = 0; s < S; ++s)
-      *reinterpret_cast<uint4*>(st + s * p.s_ss + d0) = (s + 1 < S) ? pack8f(h[s + 1]) : pack8f(xv);
-  } else {
-    float flat[S * 8];
+      hr[i][s] = *reinterpret_cast<const uint4*>(p.state + so[i] + (STATE_DMAJOR ? s * p.s_ss + d0 : int64_t(d0) * S + s * 8));
+  }
+  float w[W][8], bias[8];
+  load_weights<W>(p.weight, p.w_sd, p.w_sw, d0, w);
+  if (p.bias) unpack8(*reinterpret_cast<const uint4*>(p.bias + d0), bias);
+  else {
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
+    for (int c = 0; c < 8; ++c) bias[c] = 0.f;
+  }
 #pragma unroll
-      for (int s = 0; s < S; ++s) flat[c * S + s] = (s + 1 < S) ? h[s + 1][c] : xv[c];
+  for (int i = 0; i < NS; ++i) {
+    if (so[i] < 0) continue;
+    const int n = blockIdx.y * NS + i;
+    float acc[8], xv[8], h[S][8];
+    unpack8(xr[i], xv);
+    if constexpr (STATE_DMAJOR) {
 #pragma unroll
-    for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(st + int64_t(d0) * S + s * 8) = pack8f(flat + s * 8);
+      for (int s = 0; s < S; ++s) unpack8(hr[i][s], h[s]);
+    } else {
+      float flat[S * 8];
+#pragma unroll
+      for (int s = 0; s < S; ++s) unpack8(hr[i][s], flat + s * 8);
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int s = 0; s < S; ++s) h[s][c] = flat[c * S + s];
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      float a = bias[c] + w[W - 1][c] * xv[c];
+#pragma unroll
+      for (int s = 0; s < S; ++s) a += w[s][c] * h[s][c];
+      acc[c] = p.silu ? silu(a) : a;
+    }
+    if (p.residual) {
+      float rv[8];
+      unpack8(*reinterpret_cast<const uint4*>(p.residual + n * p.r_sn + d0), rv);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[c] += rv[c];
+    }
+    *reinterpret_cast<uint4*>(p.y + n * p.y_sn + d0) = pack8f(acc);
+    // new state = (h[1], ..., h[S-1], x)
+    bf16* st = p.state + so[i];
+    if constexpr (STATE_DMAJOR) {
+#pragma unroll
+      for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(st + s * p.s_ss + d0) = (s + 1 < S) ? hr[i][s + 1] : xr[i];
+    } else {
+      float flat[S * 8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int s = 0; s < S; ++s) flat[c * S + s] = (s + 1 < S) ? h[s + 1][c] : xv[c];
+#pragma unroll
+      for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(st + int64_t(d0) * S + s * 8) = pack8f(flat + s * 8);
+    }
   }
 }
 
@@ -479,15 +498,19 @@ extern "C" FLA_API int fla_b200_causal_conv1d_update(const fla_causal_conv1d_upd
   const bool dmajor = s.stride[1] == 1 && s.stride[2] % 8 == 0 && s.stride[0] % 8 == 0 && aligned16(s.data);
   const bool smajor = s.stride[2] == 1 && s.stride[1] == S && s.stride[0] % 8 == 0 && aligned16(s.data);
   if (vec && w_ok && T == 1 && S == W - 1 && !spec && (dmajor || smajor)) {
-    const dim3 grid(unsigned((D / 8 + kConvThreads - 1) / kConvThreads), unsigned(N));
-#define FLA_LAUNCH_UPD(WW)                                                               \
-  if (dmajor) conv_update1_kernel<WW, true><<<grid, kConvThreads, 0, st>>>(p);          \
-  else conv_update1_kernel<WW, false><<<grid, kConvThreads, 0, st>>>(p);
+    const unsigned gx = unsigned((D / 8 + kConvThreads - 1) / kConvThreads);
+    // two sequences per thread once that leaves every SM three CTAs
+    const bool many = gx * ((N + 1) / 2) >= 3 * 148;
+    const dim3 grid(gx, unsigned(many ? (N + 1) / 2 : N));
+    void (*kernel)(ConvUpdParams) = nullptr;
+#define FLA_LAUNCH_UPD(WW)                                                                              \
+  kernel = dmajor ? (many ? conv_update1_kernel<WW, true, 2> : conv_update1_kernel<WW, true, 1>)        \
+                  : (many ? conv_update1_kernel<WW, false, 2> : conv_update1_kernel<WW, false, 1>);
     if (W == 4) { FLA_LAUNCH_UPD(4) } else if (W == 3) { FLA_LAUNCH_UPD(3) } else { FLA_LAUNCH_UPD(2) }
 #undef FLA_LAUNCH_UPD
-  } else {
-    const dim3 grid(unsigned((D + 127) / 128), unsigned(N));
-    conv_update_generic_kernel<<<grid, 128, 0, st>>>(p);
+    return cuda_status(launch_pdl(kernel, grid, dim3(kConvThreads), 0, st, p));
   }
+  const dim3 grid(unsigned((D + 127) / 128), unsigned(N));
+  conv_update_generic_kernel<<<grid, 128, 0, st>>>(p);
   return cuda_status(cudaGetLastError());
 }

@@ -1,6 +1,6 @@
 // Fused-recurrent gated delta rule (decode / short-sequence step) over a pool of per-sequence states.
 //
-// One CTA owns one (sequence, value-head) state matrix (128 of its value channels when V = 256), streams it from HBM once with 16-byte
+// One CTA owns 32 value channels of one (sequence, value-head) state matrix, streams them from HBM once with 16-byte
 // loads, applies up to a few tokens of
 //     S <- exp(g) S  (scalar g per head and / or a per-key-channel gate gk: S <- diag(exp(gk)) S) ;
 //     d = beta (v - S^T k) ;  S <- S + k d^T ;  o = S^T (scale q)
@@ -14,6 +14,7 @@
 #include <cuda_fp16.h>
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
+#include "common/pdl.cuh"
 
 namespace fla {
 
@@ -167,273 +168,288 @@ __device__ __forceinline__ void store_out(const RecurrentParams& p, int64_t off,
   else static_cast<__nv_bfloat16*>(p.out)[off] = __float2bfloat16_rn(o);
 }
 
-constexpr int kRecThreads = 256;
+// A CTA takes 32 value channels of one head: 128 threads with 32 state values each.  Whole heads (256 threads, three CTAs per SM) left
+// 45 sequences x 32 heads at 3.24 waves of CTAs that all load, compute and store in step, and a single sequence on 32 SMs.  A token costs
+// three barriers: everything it reads is requested one token ahead and published by the first, each dot product takes one more.
+// HBM-bound from a few dozen sequences on: 256 sequences x 32 heads (1.07 GB) 170 -> 163 us, with the conv update in front 191 -> 176
+// (94 % of the measured copy rate); one sequence 5.3 -> 3.5 us.
+constexpr int kRecThreads = 128, kRecTile = 32;
 
-// K-first states ([K][V] in memory).  The columns of V are independent recurrences, so a CTA owns VT of the V value channels:
-// a thread keeps 4 channels of every RG-th key row.
-template <int K, int V, int VT, typename ST>
-__global__ void __launch_bounds__(kRecThreads, 3) recurrent_gdn_kernel(RecurrentParams p) {
-  constexpr int ROWS = K, COLS = VT, LD = V;
-  constexpr int NVB = V / VT;
-  constexpr int TPR = COLS / 4;              // threads per row
+// K-first states ([K][V] in memory).  The columns of V are independent recurrences; a thread keeps 4 channels of every 16th key row.
+template <int K, int V, typename ST>
+__global__ void __launch_bounds__(kRecThreads, 8) recurrent_gdn_kernel(RecurrentParams p) {
+  constexpr int NVB = V / kRecTile;
+  constexpr int TPR = kRecTile / 4;          // threads per row
   constexpr int RG = kRecThreads / TPR;      // row groups handled per pass
-  constexpr int R = ROWS / RG;               // rows per thread
-  static_assert(ROWS % RG == 0 && TPR <= 32, "unsupported head dims");
+  constexpr int R = K / RG;                  // rows per thread
+  constexpr int NW = kRecThreads / 32;
+  static_assert(K % RG == 0 && V % kRecTile == 0 && K <= kRecThreads, "unsupported head dims");
 
-  __shared__ float k_s[K], q_s[K], dk_s[K];
-  __shared__ __align__(16) float red[RG][COLS];
-  __shared__ float norm_s[2];
+  __shared__ float k_s[2][K], q_s[2][K], dk_s[2][K];          // double-buffered: one barrier publishes a token
+  __shared__ float norm_s[2][2][NW];
+  __shared__ __align__(16) float red_k[NW][kRecTile], red_q[NW][kRecTile];
 
   const int vb = blockIdx.x % NVB;
   const int seq = (blockIdx.x / NVB) / p.HV, hv = (blockIdx.x / NVB) % p.HV;
-  const int v0 = vb * VT;                                   // first value channel of this CTA
-  const int64_t tile_off = v0;                              // offset of the tile inside the stored K x V matrix
+  const int v0 = vb * kRecTile;                             // first value channel of this CTA
   const int hk = hv / (p.HV / p.HK);
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int rg = tid / TPR, c0 = (tid % TPR) * 4;
 
+  pdl_trigger();
+  // the state of a plain batch can be on its way while the kernel in front (the conv update of the same step) finishes
+  if (!p.cu_seqlens && !p.state_indices && tid < K)
+    prefetch_l2(static_cast<const ST*>(p.state_in) + seq * p.state_in_stride_b + hv * p.state_in_stride_h + v0 + int64_t(tid) * V);
+  pdl_wait();
   int t0, t1, blk;
   if (!sequence_of(p, seq, tid, t0, t1, blk)) return;
 
   float4 s[R];
   {
-    const ST* src = static_cast<const ST*>(p.state_in) + blk * p.state_in_stride_b + hv * p.state_in_stride_h;
+    const ST* src = static_cast<const ST*>(p.state_in) + blk * p.state_in_stride_b + hv * p.state_in_stride_h + v0 + c0;
 #pragma unroll
-    for (int i = 0; i < R; ++i) s[i] = load4<ST>(src + tile_off + int64_t(rg + i * RG) * LD + c0);
+    for (int i = 0; i < R; ++i) s[i] = load4<ST>(src + (rg + i * RG) * V);
   }
-
-  for (int t = t0; t < t1; ++t) {
-    __syncthreads();  // previous token's readers of k_s/q_s/red are done
+  // the next token's elements, requested one token ahead
+  float pk = 0.f, pq = 0.f, pg = 0.f, pdecay = 0.f, pbeta = 1.f;
+  float4 pv;
+  int pblk = -1;
+  auto request = [&](int t) {
     if (tid < K) {
-      k_s[tid] = load_act(p.k, t * p.k_stride_t + hk * p.k_stride_h + tid, p.act_f16);
-    } else if (tid < 2 * K) {
-      q_s[tid - K] = load_act(p.q, t * p.q_stride_t + hk * p.q_stride_h + (tid - K), p.act_f16);
+      pk = load_act(p.k, t * p.k_stride_t + hk * p.k_stride_h + tid, p.act_f16);
+      pq = load_act(p.q, t * p.q_stride_t + hk * p.q_stride_h + tid, p.act_f16);
+      if (p.gk) pg = load_scalar(p.gk, t * p.gk_stride_t + hv * p.gk_stride_h + tid, p.gk_is_f32);
     }
-    if (p.gk && tid < K) {   // per-channel decay of this token: exp(gate(gk))
-      dk_s[tid] = __expf(channel_gate<K>(p, load_scalar(p.gk, t * p.gk_stride_t + hv * p.gk_stride_h + tid, p.gk_is_f32), hv, tid));
+    if (p.g) pdecay = load_scalar(p.g, t * p.g_stride_t + hv, p.g_is_f32);
+    if (p.beta) pbeta = load_scalar(p.beta, t * p.beta_stride_t + hv, p.beta_is_f32);
+    const int64_t voff = t * p.v_stride_t + hv * p.v_stride_h + v0 + c0;
+    pv = p.act_f16 ? load4<__half>(static_cast<const __half*>(p.v) + voff) : load4<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.v) + voff);
+    pblk = p.state_indices ? p.state_indices[t] : (t == t1 - 1 ? seq : -1);
+  };
+  request(t0);
+  for (int t = t0; t < t1; ++t) {
+    const int b = (t - t0) & 1;
+    if (tid < K) {
+      k_s[b][tid] = pk;
+      q_s[b][tid] = pq;
+      if (p.gk) dk_s[b][tid] = __expf(channel_gate<K>(p, pg, hv, tid));     // per-channel decay of this token: exp(gate(gk))
     }
-    const float decay = p.g ? expf(load_scalar(p.g, t * p.g_stride_t + hv, p.g_is_f32)) : 1.f;
-    float beta = p.beta ? load_scalar(p.beta, t * p.beta_stride_t + hv, p.beta_is_f32) : 1.f;
-    if (p.beta_mode) beta = float(p.beta_mode) / (1.f + __expf(-beta));
+    if (p.l2norm) {
+      float nk = pk * pk, nq = pq * pq;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        nk += __shfl_xor_sync(0xffffffffu, nk, o);
+        nq += __shfl_xor_sync(0xffffffffu, nq, o);
+      }
+      if (lane == 0) {
+        norm_s[b][0][warp] = nk;
+        norm_s[b][1][warp] = nq;
+      }
+    }
+    const float decay = p.g ? expf(pdecay) : 1.f;
+    const float beta = p.beta_mode ? float(p.beta_mode) / (1.f + __expf(-pbeta)) : pbeta;
+    const float4 vv = pv;
+    const int wblk = pblk;
+    if (t + 1 < t1) request(t + 1);
     __syncthreads();
     float kscale = 1.f, qscale = p.scale;
     if (p.l2norm) {
-      if (tid < 64) {  // warp 0: |k|^2, warp 1: |q|^2
-        const float* src = tid < 32 ? k_s : q_s;
-        float acc = 0.f;
-        for (int i = tid % 32; i < K; i += 32) acc += src[i] * src[i];
+      float nk = 0.f, nq = 0.f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (tid % 32 == 0) norm_s[tid / 32] = rsqrtf(acc + 1e-6f);
+      for (int w = 0; w < K / 32; ++w) {
+        nk += norm_s[b][0][w];
+        nq += norm_s[b][1][w];
       }
-      __syncthreads();
-      kscale = norm_s[0];
-      qscale = p.scale * norm_s[1];
+      kscale = rsqrtf(nk + 1e-6f);
+      qscale = p.scale * rsqrtf(nq + 1e-6f);
     }
-
     if (p.gk) {   // S <- diag(exp(gate)) S
 #pragma unroll
       for (int i = 0; i < R; ++i) {
-        const float d = dk_s[rg + i * RG];
+        const float d = dk_s[b][rg + i * RG];
         s[i].x *= d; s[i].y *= d; s[i].z *= d; s[i].w *= d;
       }
     }
+    // sums over the key rows: over mine, over the row groups of the warp, over the warps
+    auto total = [&](float4 x, float (*red)[kRecTile], bool all) {
+#pragma unroll
+      for (int o = TPR; o < 32; o <<= 1) {
+        x.x += __shfl_xor_sync(0xffffffffu, x.x, o); x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
+        x.z += __shfl_xor_sync(0xffffffffu, x.z, o); x.w += __shfl_xor_sync(0xffffffffu, x.w, o);
+      }
+      if (lane < TPR) *reinterpret_cast<float4*>(&red[warp][c0]) = x;
+      __syncthreads();
+      float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (all || rg == 0) {
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+          const float4 y = *reinterpret_cast<const float4*>(&red[w][c0]);
+          r.x += y.x; r.y += y.y; r.z += y.z; r.w += y.w;
+        }
+      }
+      return r;
+    };
     // rows are k, my 4 columns are v.  dot[v] = sum_k S[k][v] k[k]
     float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const float kk = k_s[rg + i * RG] * kscale;
+      const float kk = k_s[b][rg + i * RG] * kscale;
       part.x += s[i].x * kk; part.y += s[i].y * kk; part.z += s[i].z * kk; part.w += s[i].w * kk;
     }
-    *reinterpret_cast<float4*>(&red[rg][c0]) = part;
-    __syncthreads();
-    float4 dot = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int r = 0; r < RG; ++r) {
-      const float4 x = *reinterpret_cast<const float4*>(&red[r][c0]);
-      dot.x += x.x; dot.y += x.y; dot.z += x.z; dot.w += x.w;
-    }
-    const int64_t voff = t * p.v_stride_t + hv * p.v_stride_h + v0 + c0;
-    const float4 vv = p.act_f16 ? load4<__half>(static_cast<const __half*>(p.v) + voff)
-                                : load4<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.v) + voff);
+    const float4 dot = total(part, red_k, true);
     float4 d;
     d.x = beta * (vv.x - decay * dot.x); d.y = beta * (vv.y - decay * dot.y);
     d.z = beta * (vv.z - decay * dot.z); d.w = beta * (vv.w - decay * dot.w);
     float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const float kk = k_s[rg + i * RG] * kscale, qq = q_s[rg + i * RG] * qscale;
+      const float kk = k_s[b][rg + i * RG] * kscale, qq = q_s[b][rg + i * RG] * qscale;
       s[i].x = decay * s[i].x + kk * d.x; s[i].y = decay * s[i].y + kk * d.y;
       s[i].z = decay * s[i].z + kk * d.z; s[i].w = decay * s[i].w + kk * d.w;
       po.x += s[i].x * qq; po.y += s[i].y * qq; po.z += s[i].z * qq; po.w += s[i].w * qq;
     }
-    __syncthreads();  // everyone has consumed red[] for the dot
-    *reinterpret_cast<float4*>(&red[rg][c0]) = po;
-    __syncthreads();
-    if (rg == 0) {
-      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (wblk >= 0 && wblk < p.nblocks_out) {
+      ST* dst = static_cast<ST*>(p.state_out) + wblk * p.state_out_stride_b + hv * p.state_out_stride_h + v0 + c0;
 #pragma unroll
-      for (int r = 0; r < RG; ++r) {
-        const float4 x = *reinterpret_cast<const float4*>(&red[r][c0]);
-        o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
-      }
+      for (int i = 0; i < R; ++i) store4<ST>(dst + (rg + i * RG) * V, s[i]);
+    }
+    const float4 o = total(po, red_q, false);
+    if (rg == 0) {
       const int64_t off = t * p.out_stride_t + hv * p.out_stride_h + v0 + c0;
       if (p.out_is_f32) store4<float>(static_cast<float*>(p.out) + off, o);
       else if (p.out_is_f16) store4<__half>(static_cast<__half*>(p.out) + off, o);
       else store4<__nv_bfloat16>(static_cast<__nv_bfloat16*>(p.out) + off, o);
-    }
-
-    const bool last = (t == t1 - 1);
-    int wblk = -1;
-    if (p.state_indices) wblk = p.state_indices[t];
-    else if (last) wblk = seq;
-    if (wblk >= 0 && wblk < p.nblocks_out) {
-      ST* dst = static_cast<ST*>(p.state_out) + wblk * p.state_out_stride_b + hv * p.state_out_stride_h;
-#pragma unroll
-      for (int i = 0; i < R; ++i) store4<ST>(dst + tile_off + int64_t(rg + i * RG) * LD + c0, s[i]);
     }
   }
 }
 
 // V-first states ([V][K] in memory; the state-pool operators).  Four lanes share a value row (K / 4 key channels each, in 16-byte
 // pieces dealt out in turn so that the four lanes read 64 contiguous bytes), so the two dot products of a token take two
-// shuffles each, for VT / 64 rows per thread.  A whole warp per row, which the 4-channel layout of the K-first kernel would
+// shuffles each.  A whole warp per row, which the 4-channel layout of the K-first kernel would
 // give, spent ten shuffles and a dependent global load of v on each of sixteen rows: 36.7 us for 24 sequences x 16 heads with one
 // to four draft tokens (bf16 pool) against the 7 us its bytes take.  The next token's q, k, v are requested before the current one is worked on
 // (q, k, v are double-buffered: one barrier per token, two with the normalisation).
-template <int K, int V, int VT, typename ST>
-__global__ void __launch_bounds__(kRecThreads, 2) recurrent_gdn_vfirst_kernel(RecurrentParams p) {
-  constexpr int NVB = V / VT;
+template <int K, int V, typename ST>
+__global__ void __launch_bounds__(kRecThreads, 5) recurrent_gdn_vfirst_kernel(RecurrentParams p) {
+  constexpr int VT = kRecTile, NVB = V / VT;
   constexpr int E = 16 / sizeof(ST);               // channels per 16-byte piece
   constexpr int P = K / (4 * E);                   // pieces per lane
-  constexpr int R = VT / 64;                       // rows per thread
-  static_assert(VT % 64 == 0 && K % (4 * E) == 0 && 2 * K <= kRecThreads && VT <= kRecThreads, "unsupported head dims");
+  static_assert(V % VT == 0 && 4 * VT == kRecThreads && K % (4 * E) == 0 && K <= kRecThreads, "unsupported head dims");
   __shared__ __align__(16) float k_s[2][K], q_s[2][K], dk_s[2][K];
-  __shared__ float v_s[2][VT], norm_s[2][2];
+  __shared__ float norm_s[2][2][kRecThreads / 32];
 
   const int tid = threadIdx.x, lane4 = tid & 3, row = tid >> 2;
   const int vb = blockIdx.x % NVB, seq = (blockIdx.x / NVB) / p.HV, hv = (blockIdx.x / NVB) % p.HV;
   const int v0 = vb * VT, hk = hv / (p.HV / p.HK);
+  pdl_trigger();
+  pdl_wait();
   int t0, t1, blk;
   if (!sequence_of(p, seq, tid, t0, t1, blk)) return;
 
-  float s[R][P * E];
+  float s[P * E];
   {
-    const ST* src = static_cast<const ST*>(p.state_in) + blk * p.state_in_stride_b + hv * p.state_in_stride_h + int64_t(v0) * K;
+    const ST* src = static_cast<const ST*>(p.state_in) + blk * p.state_in_stride_b + hv * p.state_in_stride_h + int64_t(v0 + row) * K;
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int j = 0; j < P; ++j) load16<ST>(src + (row + r * 64) * K + (j * 4 + lane4) * E, &s[r][j * E]);
+    for (int j = 0; j < P; ++j) load16<ST>(src + (j * 4 + lane4) * E, &s[j * E]);
   }
-  float pqk = 0.f, pv = 0.f, pg = 0.f, pdecay = 0.f, pbeta = 1.f;     // the next token's elements
+  float pk = 0.f, pq = 0.f, pv = 0.f, pg = 0.f, pdecay = 0.f, pbeta = 1.f;     // the next token's elements
+  int pblk = -1;
   auto request = [&](int t) {
-    if (tid < K) pqk = load_act(p.k, t * p.k_stride_t + hk * p.k_stride_h + tid, p.act_f16);
-    else if (tid < 2 * K) pqk = load_act(p.q, t * p.q_stride_t + hk * p.q_stride_h + (tid - K), p.act_f16);
-    if (tid < VT) pv = load_act(p.v, t * p.v_stride_t + hv * p.v_stride_h + v0 + tid, p.act_f16);
-    if (p.gk && tid < K) pg = load_scalar(p.gk, t * p.gk_stride_t + hv * p.gk_stride_h + tid, p.gk_is_f32);
+    if (tid < K) {
+      pk = load_act(p.k, t * p.k_stride_t + hk * p.k_stride_h + tid, p.act_f16);
+      pq = load_act(p.q, t * p.q_stride_t + hk * p.q_stride_h + tid, p.act_f16);
+      if (p.gk) pg = load_scalar(p.gk, t * p.gk_stride_t + hv * p.gk_stride_h + tid, p.gk_is_f32);
+    }
+    pv = load_act(p.v, t * p.v_stride_t + hv * p.v_stride_h + v0 + row, p.act_f16);
     if (p.g) pdecay = load_scalar(p.g, t * p.g_stride_t + hv, p.g_is_f32);
     if (p.beta) pbeta = load_scalar(p.beta, t * p.beta_stride_t + hv, p.beta_is_f32);
+    pblk = p.state_indices ? p.state_indices[t] : (t == t1 - 1 ? seq : -1);
   };
   request(t0);
   for (int t = t0; t < t1; ++t) {
     const int b = (t - t0) & 1;
-    if (tid < K) k_s[b][tid] = pqk;
-    else if (tid < 2 * K) q_s[b][tid - K] = pqk;
-    if (tid < VT) v_s[b][tid] = pv;
-    if (p.gk && tid < K) dk_s[b][tid] = __expf(channel_gate<K>(p, pg, hv, tid));
+    if (tid < K) {
+      k_s[b][tid] = pk;
+      q_s[b][tid] = pq;
+      if (p.gk) dk_s[b][tid] = __expf(channel_gate<K>(p, pg, hv, tid));
+    }
+    if (p.l2norm) {
+      float nk = pk * pk, nq = pq * pq;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        nk += __shfl_xor_sync(0xffffffffu, nk, o);
+        nq += __shfl_xor_sync(0xffffffffu, nq, o);
+      }
+      if (tid % 32 == 0) {
+        norm_s[b][0][tid / 32] = nk;
+        norm_s[b][1][tid / 32] = nq;
+      }
+    }
     const float decay = p.g ? expf(pdecay) : 1.f;
     const float beta = p.beta_mode ? float(p.beta_mode) / (1.f + __expf(-pbeta)) : pbeta;
+    const float vv = pv;
+    const int wblk = pblk;
     if (t + 1 < t1) request(t + 1);
     __syncthreads();
     float kscale = 1.f, qscale = p.scale;
     if (p.l2norm) {
-      if (tid < 64) {  // warp 0: |k|^2, warp 1: |q|^2
-        const float* src = tid < 32 ? k_s[b] : q_s[b];
-        float acc = 0.f;
-        for (int i = tid % 32; i < K; i += 32) acc += src[i] * src[i];
+      float nk = 0.f, nq = 0.f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (tid % 32 == 0) norm_s[b][tid / 32] = rsqrtf(acc + 1e-6f);
+      for (int w = 0; w < K / 32; ++w) {
+        nk += norm_s[b][0][w];
+        nq += norm_s[b][1][w];
       }
-      __syncthreads();
-      kscale = norm_s[b][0];
-      qscale = p.scale * norm_s[b][1];
+      kscale = rsqrtf(nk + 1e-6f);
+      qscale = p.scale * rsqrtf(nq + 1e-6f);
     }
-    float dot[R], o[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) dot[r] = o[r] = 0.f;
+    float dot = 0.f, o = 0.f;
 #pragma unroll
     for (int j = 0; j < P; ++j) {
 #pragma unroll
       for (int e4 = 0; e4 < E; e4 += 4) {
         const int c = (j * 4 + lane4) * E + e4;
+        float* x = &s[j * E + e4];
         const float4 kk = *reinterpret_cast<const float4*>(&k_s[b][c]);
         if (p.gk) {      // S <- diag(exp(gate)) S
           const float4 d = *reinterpret_cast<const float4*>(&dk_s[b][c]);
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            float* x = &s[r][j * E + e4];
-            x[0] *= d.x; x[1] *= d.y; x[2] *= d.z; x[3] *= d.w;
-          }
+          x[0] *= d.x; x[1] *= d.y; x[2] *= d.z; x[3] *= d.w;
         }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const float* x = &s[r][j * E + e4];
-          dot[r] += x[0] * kk.x + x[1] * kk.y + x[2] * kk.z + x[3] * kk.w;
-        }
+        dot += x[0] * kk.x + x[1] * kk.y + x[2] * kk.z + x[3] * kk.w;
       }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 1);
-      dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 2);
-      dot[r] = beta * (v_s[b][row + r * 64] - decay * dot[r] * kscale) * kscale;     // d, times the factor of k
-    }
+    dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+    dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+    dot = beta * (vv - decay * dot * kscale) * kscale;     // d, times the factor of k
 #pragma unroll
     for (int j = 0; j < P; ++j) {
 #pragma unroll
       for (int e4 = 0; e4 < E; e4 += 4) {
         const int c = (j * 4 + lane4) * E + e4;
+        float* x = &s[j * E + e4];
         const float4 kk = *reinterpret_cast<const float4*>(&k_s[b][c]), qq = *reinterpret_cast<const float4*>(&q_s[b][c]);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          float* x = &s[r][j * E + e4];
-          x[0] = decay * x[0] + dot[r] * kk.x; x[1] = decay * x[1] + dot[r] * kk.y;
-          x[2] = decay * x[2] + dot[r] * kk.z; x[3] = decay * x[3] + dot[r] * kk.w;
-          o[r] += x[0] * qq.x + x[1] * qq.y + x[2] * qq.z + x[3] * qq.w;
-        }
+        x[0] = decay * x[0] + dot * kk.x; x[1] = decay * x[1] + dot * kk.y;
+        x[2] = decay * x[2] + dot * kk.z; x[3] = decay * x[3] + dot * kk.w;
+        o += x[0] * qq.x + x[1] * qq.y + x[2] * qq.z + x[3] * qq.w;
       }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      o[r] += __shfl_xor_sync(0xffffffffu, o[r], 1);
-      o[r] += __shfl_xor_sync(0xffffffffu, o[r], 2);
-      if (lane4 == 0) store_out(p, t * p.out_stride_t + hv * p.out_stride_h + v0 + row + r * 64, o[r] * qscale);
-    }
-    const int wblk = p.state_indices ? p.state_indices[t] : (t == t1 - 1 ? seq : -1);
+    o += __shfl_xor_sync(0xffffffffu, o, 1);
+    o += __shfl_xor_sync(0xffffffffu, o, 2);
+    if (lane4 == 0) store_out(p, t * p.out_stride_t + hv * p.out_stride_h + v0 + row, o * qscale);
     if (wblk >= 0 && wblk < p.nblocks_out) {
-      ST* dst = static_cast<ST*>(p.state_out) + wblk * p.state_out_stride_b + hv * p.state_out_stride_h + int64_t(v0) * K;
+      ST* dst = static_cast<ST*>(p.state_out) + wblk * p.state_out_stride_b + hv * p.state_out_stride_h + int64_t(v0 + row) * K;
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int j = 0; j < P; ++j) store16<ST>(dst + (row + r * 64) * K + (j * 4 + lane4) * E, &s[r][j * E]);
+      for (int j = 0; j < P; ++j) store16<ST>(dst + (j * 4 + lane4) * E, &s[j * E]);
     }
   }
 }
 
 template <int K, int V>
 int launch_recurrent(const RecurrentParams& p, int nseq, bool state_f32, bool vfirst, cudaStream_t st) {
-  constexpr int VT = V > 128 ? 128 : V;
-  const dim3 grid(nseq * p.HV * (V / VT)), block(kRecThreads);
+  const dim3 grid(nseq * p.HV * (V / kRecTile)), block(kRecThreads);
   KernelTimer kt("recurrent_gdn", st);
-  if (state_f32) {
-    if (vfirst) recurrent_gdn_vfirst_kernel<K, V, VT, float><<<grid, block, 0, st>>>(p);
-    else recurrent_gdn_kernel<K, V, VT, float><<<grid, block, 0, st>>>(p);
-  } else {
-    if (vfirst) recurrent_gdn_vfirst_kernel<K, V, VT, __nv_bfloat16><<<grid, block, 0, st>>>(p);
-    else recurrent_gdn_kernel<K, V, VT, __nv_bfloat16><<<grid, block, 0, st>>>(p);
-  }
-  return cuda_status(cudaGetLastError());
+  void (*kernel)(RecurrentParams) = state_f32 ? (vfirst ? recurrent_gdn_vfirst_kernel<K, V, float> : recurrent_gdn_kernel<K, V, float>)
+                                              : (vfirst ? recurrent_gdn_vfirst_kernel<K, V, __nv_bfloat16> : recurrent_gdn_kernel<K, V, __nv_bfloat16>);
+  return cuda_status(launch_pdl(kernel, grid, block, 0, st, p));
 }
 
 }  // namespace fla

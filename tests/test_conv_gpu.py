@@ -108,6 +108,26 @@ def test_update_cache_indices_and_pad_slot():
     assert torch.equal(pool[untouched], before[untouched])
 
 
+@pytest.mark.parametrize("layout,W,N", [("taps_contiguous", 4, 887), ("channels_contiguous", 3, 888), ("taps_contiguous", 2, 889)])
+def test_update_two_sequences_per_thread(layout, W, N):
+    """Batches large enough for the kernel that gives a thread two sequences, odd ones and a padded slot among them."""
+    from fla_b200.ops import causal_conv1d_update
+    D = 1024
+    inp = oracle.make_conv_inputs(N, 1, D, W, seed=14, with_state=True)
+    x, idx = inp["x"][:, 0], torch.arange(N - 1, -1, -1, dtype=torch.int32)
+    idx[5] = -1
+    st_ref = inp["state"][idx.clamp(min=0).long()].double().clone()
+    ref = oracle.causal_conv1d_update_ref(x.double(), st_ref, inp["weight"].double(), None, "silu")
+    pool = inp["state"].cuda().contiguous()
+    if layout == "channels_contiguous":
+        pool = pool.transpose(1, 2).contiguous().transpose(1, 2)
+    y = causal_conv1d_update(x.cuda(), pool, weight=inp["weight"].cuda(), activation="silu", cache_indices=idx.cuda(), pad_slot_id=-1)
+    live = idx >= 0
+    assert_close("y", y[live.cuda()], ref[live], TOL, stored_bf16=True)
+    assert torch.equal(pool.cpu()[idx[live].long()].float(), st_ref[live].float())
+    assert torch.equal(pool.cpu()[N - 6].float(), inp["state"][N - 6].float())
+
+
 def test_update_multi_token_and_speculative_window():
     from fla_b200.ops import causal_conv1d_update
     N, D, W, T = 3, 64, 4, 3
