@@ -23,6 +23,7 @@
 //
 // Operands the gradients are sensitive to travel as bf16 hi + bf16 residual and are multiplied in two or three
 // tcgen05.mma passes; q, k, dO enter as the exact bf16 inputs; accumulation is fp32 in TMEM.
+#include <algorithm>
 #include "gdn_common.cuh"
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
@@ -37,13 +38,14 @@ struct GdnBwdParams {
   const float* q_rstd; const float* k_rstd;   // [tokens, HK] or null: q, k are normalised rows, dq / dk go through the normalisation
   const float* gam; const bf16* X;
   const bf16* s_img; const bf16* vn_img; const bf16* p_img;
-  bf16* ds_img;        // [chunks, HV, V/64, 2, 128x64]  state gradient entering each chunk (hi, lo)
-  bf16* dz_img;        // [chunks, HV, V/64, 192x64: rows 0-63 dO, rows 64-127 dZ rounded to bf16, rows 128-191 the residual of dZ]
+  bf16* ds_img;        // [chunks, HV, V/32, 2, 128x32]  state gradient entering each chunk (hi, lo)
+  bf16* dz_img;        // [chunks, HV, V/32, 192x32: rows 0-63 dO, rows 64-127 dZ rounded to bf16, rows 128-191 the residual of dZ]
   float* bz;           // [V/32, tokens, HV] partial sums of dZ * V over the 32-column slices of V
   const float* dht; float* dh0;
   const bf16* seg_m;   // [segments, HV, 128x128 (value, residual)]  the forward's transition matrices (split chains only)
   float* seg_dh;       // [segments, HV, V/128, 128, 128]
   int seg_len;         // chunks per segment
+  int* counter;        // tiles the par kernel has handed out beyond its first wave; the scan in front of it sets it to zero
   void* dq; void* dk; void* dv; void* dg; void* dbeta;
   const int32_t* cu_seqlens; const int32_t* chunk_offsets;
   int64_t q_st, q_sh, k_st, k_sh, v_st, v_sh, do_st, do_sh, beta_st;
@@ -67,391 +69,539 @@ constexpr int64_t kDzImg = kDzHalf;   // per (chunk, head, block): 64x64 dO, 64x
 
 // ============================================================================================= par
 constexpr uint32_t rOffQK = 0, rQKPanel = 16384;
-constexpr uint32_t rOffAH = 49152;             // [dO^T | dZ^T] strips of one 64-channel step (16 KB)
-constexpr uint32_t rOffAL = 32768;             // [0 | residual of dZ^T]: 8 KB of zeros written once, then the step's 8 KB of strips
-// v_new^T and S strips, value / residual, interleaved so that [Vn_lo | S_hi] and [Vn_hi | S_lo] are each one contiguous B operand
-// of 24 strips.  As an A operand with valid rows 64..127 the view of v_new^T starts 8 KB earlier, inside the dZ^T strips or the
-// S strips (any finite contents do).
-constexpr uint32_t rOffVNL = 65536, rOffSH = 73728, rOffVNH = 90112, rOffSL = 98304, rOffDSH = 114688, rOffDSL = 131072;
-constexpr uint32_t rOffPAH = 147456, rOffPAL = 163840;   // [dP ; dAt] hi / lo (128 rows x 64)
-constexpr uint32_t kParSmem = 180224;
-constexpr uint32_t rColQK = 0, rColDV = 64, rColTA = 128, rColTB = 256;
-constexpr uint32_t rColAcc = 384;   // running dq (q-side rows) / dk (k-side rows) over the value heads of the group: 128 columns
-constexpr uint32_t kStepBytes = 16384 + 8192 + 16384 + 32768 + 32768;
+// Two stages, each the operands of 32 value channels (un-swizzled strips of 512 bytes, sm100.cuh, whose 32 rows are value channels: the
+// reduction dim of these products).  [0 | residual of dZ^T]: the zeros are written once.  v_new^T and S strips, value / residual, are interleaved so
+// that [Vn_lo | S_hi] and [Vn_hi | S_lo] are each one contiguous B operand of 24 strips.  As an A operand with valid rows 64..127 the view of
+// v_new^T starts 4 KB earlier, inside the dZ^T strips or the S strips (any finite contents do).
+constexpr uint32_t rOffStage = 32768, kStageStride = 57344;
+constexpr uint32_t sOffAL = 0, sOffAH = 8192, sOffVNL = 16384, sOffSH = 20480, sOffVNH = 28672, sOffSL = 32768, sOffDSH = 40960, sOffDSL = 49152;
+constexpr uint32_t kStageBytes = 12288 + 8192 + 16384 + 16384;      // loaded per stage
+// [dP ; dAt] value / residual (128 rows x 64), behind 16 KB of zeros: read along the reduction over i, the zeros are the rows 0..63 of
+// [0 ; dP^T | dAt^T], whose product then adds to the k-side rows alone and shares the accumulator of [dP; dAt] K.
+constexpr uint32_t rOffZero = rOffStage + 2 * kStageStride, rOffPAH = rOffZero + 16384, rOffPAL = rOffPAH + 16384;
+constexpr uint32_t kParSmem = rOffPAL + 16384;
+constexpr uint32_t rColQK = 0, rColDV = 64, rColTA = 128, rColTB = 256, rColT2 = 384;
+constexpr int kParWorkers = 512, kParThreads = kParWorkers + 128;      // + products, loader, two tail warps
 
-__device__ __forceinline__ void row_dot64(const uint8_t* pan0, uint32_t panel_stride, int row, int col0, const float* x,
-                                          float& acc) {
-  // acc += sum_c bf16_panel[row][col0 + c] * x[c], c in [0, 64); col0 is 0 or 64 (one panel)
-  const uint8_t* pan = pan0 + (col0 / 64) * panel_stride;
-#pragma unroll
-  for (int ch = 0; ch < 8; ++ch) {
-    float f[8];
-    unpack_bf16x8(*reinterpret_cast<const uint4*>(pan + panel_chunk_off(row, ch)), f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc += f[j] * x[ch * 8 + j];
-  }
+// barrier `id` over `threads` threads that tells all of them whether all are fine
+template <int kId, int kThreads>
+__device__ __forceinline__ bool par_sync_and(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      " .reg .pred p, q;\n"
+      " setp.ne.u32 q, %1, 0;\n"
+      " bar.red.and.pred p, %2, %3, q;\n"
+      " selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(uint32_t(ok)), "n"(kId), "n"(kThreads)
+      : "memory");
+  return r != 0;
 }
 
+// Four neighbouring lanes hold four 16-byte pieces each: afterwards lane l has piece l % 4 of each of the four lanes.
+__device__ __forceinline__ void transpose4x4(uint4 (&v)[4], int lane) {
+  auto trade = [&](uint4& keep0, uint4& keep1, int bit) {      // the lane with the bit set keeps its second piece, the other its first
+    const bool up = (lane & bit) != 0;
+    const uint4 out = up ? keep0 : keep1;
+    uint4 in;
+    in.x = __shfl_xor_sync(0xffffffffu, out.x, bit); in.y = __shfl_xor_sync(0xffffffffu, out.y, bit);
+    in.z = __shfl_xor_sync(0xffffffffu, out.z, bit); in.w = __shfl_xor_sync(0xffffffffu, out.w, bit);
+    if (up) keep0 = in;
+    else keep1 = in;
+  };
+  trade(v[0], v[1], 1);
+  trade(v[2], v[3], 1);
+  trade(v[0], v[2], 2);
+  trade(v[1], v[3], 2);
+}
 
-template <int NVB>   // 64-column blocks of V per head (2 or 4): a compile-time trip count keeps the block loop unrolled
-__global__ void __launch_bounds__(256, 1) gdn_bwd_par_kernel(GdnBwdParams p, const __grid_constant__ CUtensorMap tm_q,
-                                                                const __grid_constant__ CUtensorMap tm_k) {
+struct ParItem {      // one value head of one (chunk, q/k head) tile
+  int tile, h;        // h < 0: no more items
+  int tok0, rows;
+};
+
+// One CTA per SM walks over (chunk, q/k head) tiles, handed out by a counter (next to the other half of the batch's scan, below, the CTAs do
+// not start together); an item is one value head of a tile.
+//     loader     operands of 32 value channels at a time into two stages; q, k of the next tile once the last item's readers are through
+//     products   per stage [dO; dZ] . [Vn | S]^T and Vn . dS'^T; then, once [dP; dAt] is there, T2 = [dP; dAt] K + [0; dP^T | dAt^T] [Q; K]
+//     workers    (sixteen warps) <S, dS'> of each stage; epilogue 1: score gradients -> [dP; dAt], first parts of dq / dk from the accumulators,
+//                which the next item's products may overwrite from there on; epilogue 2: T2, row dots; after the last head dq, dk
+//     tail       (two warps) gates and beta of the next item, dg and dbeta of the item before
+// Loads, the products of the next item and the epilogues of this one overlap.  What bounded the one-tile-per-CTA form with eight warps (41,000
+// cycles for a tile of two heads, of which shared memory needs 16,000 and HBM 19,000) was that they did not: load, products, load,
+// products, epilogue, products, epilogue ran one after the other, each waited for by everything else.  Now about 20,000 - 25,000:
+// 32,768 tokens, 16 / 32 heads 1.26 -> 0.86 ms, 8,191 packed tokens with 4 / 8 heads 112 -> 87 us.
+// The products are issued from a one-thread branch: by the whole converged warp they go out faster than the tensor core takes them and the
+// loads and epilogues that run beside them slow everything down (95 us for the packed batch).
+// NVB: 64-column blocks of V per head (2 or 4), a compile-time trip count that keeps the stage loop unrolled.
+template <int NVB>
+__global__ void __launch_bounds__(kParThreads, 1) gdn_bwd_par_kernel(GdnBwdParams p, int chunks, const __grid_constant__ CUtensorMap tm_q,
+                                                                     const __grid_constant__ CUtensorMap tm_k) {
+  constexpr int NS = 2 * NVB;      // stages per item
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // per-head row scalars and row reductions, double-buffered by head parity: the dg / dbeta rows of a head are
-  // finished while the tensor cores work on the next head
-  __shared__ float gam_s2[2][kC], beta_s2[2][kC];
-  __shared__ float red2[2][5][2][kC];  // qdq, kdk, rkG, rkB, ma : [half][row]
-  __shared__ float sds_s2[2][8];
-  __shared__ float ndot_s[2][2 * kC];  // q.dq / k.dk of the complete rows, per half of the columns (normalised q, k only)
-  __shared__ float fin_s[2][2];
+  // double-buffered by item parity
+  __shared__ __align__(16) float gam_s2[2][kC], beta_s2[2][kC];
+  __shared__ float red2[2][5][4][kC];      // q.dq, k.dk, rkG, rkB, ma : [32-column group of the row][row]
+  __shared__ float sds_s2[2][kParWorkers / 32], ndot_s[4][2 * kC], fin_s[2][2];
+  __shared__ ParItem item_s[2];
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(8) uint64_t mma_bar, load_bar, qk_bar;
+  __shared__ __align__(8) uint64_t item_bar[2], qk_bar, full_bar[2];     // from the loader
+  __shared__ __align__(8) uint64_t empty_bar[2];                         // stage read by the products and by every worker warp
+  __shared__ __align__(8) uint64_t scal_bar[2], red_bar[2];              // tail: gam_s, beta_s there; worker warps: red2 there
+  __shared__ __align__(8) uint64_t p1_bar, t2_bar;                       // products: all stages of an item, T2
+  __shared__ __align__(8) uint64_t pa_bar, acc_bar, free_bar;            // worker warps: [dP; dAt] there, accumulators read, q and k read
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int hk = blockIdx.y;
-  const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.n0, blockIdx.x);
-  if (pos.n < p.n0 || pos.n >= p.n1) return;      // half of a packed batch: the other half's chunks
-  const SeqInfo& sq = pos.sq;
-  const int c = pos.c;
-  const int t0 = c * kC;
-  const int rows = min(kC, sq.len - t0);
-  const int64_t tok0 = int64_t(sq.bos) + t0;
   const int G = p.HV / p.HK;
-  const int quad = warp & 3, half = warp >> 2;
-  const int row = quad * 32 + lane;           // accumulator row == TMEM lane
-  const bool kside = quad >= 2;
-  const int tok = row & 63;
+  // chunks of this launch: fixed lengths count from the first chunk of sequence n0, a packed batch's half is cut out here
+  int chunk0 = 0;
+  if (p.cu_seqlens) {
+    chunk0 = p.chunk_offsets[p.n0];
+    chunks = p.chunk_offsets[p.n1] - chunk0;
+  }
+  const int tiles = chunks * p.HK;
+  const int flat0 = p.cu_seqlens ? chunk0 : p.n0 * ((p.T + kC - 1) / kC);      // flat index of the launch's first chunk
 
   if (warp == 0) {
     tmem_alloc(&tmem_base_s, 512);
     tmem_relinquish();
   }
-  const uint32_t sb = smem_u32(smem);
-  // One thread: operands of one (value head, 64-channel half of a block of V) step.  The scans store every saved operand
-  // per half, so a step is four contiguous pieces.
-  auto issue_loads = [&](int hv, int vb) {
-    const int64_t blk = ((int64_t(sq.cbase) + c) * p.HV + hv) * (NVB / 2) + (vb >> 1);
-    const int64_t hf = vb & 1;
-    mbar_arrive_expect_tx(&load_bar, kStepBytes);
-    bulk_load(sb + rOffAH, p.dz_img + blk * (2 * kDzHalf) + hf * kDzHalf, 16384, &load_bar);      // [dO^T | dZ^T] strips
-    bulk_load(sb + rOffAL + 8192, p.dz_img + blk * (2 * kDzHalf) + hf * kDzHalf + 8192, 8192, &load_bar);   // residual of dZ^T
-    bulk_load(sb + rOffVNH, p.vn_img + blk * 16384 + hf * 8192, 8192, &load_bar);           // value
-    bulk_load(sb + rOffVNL, p.vn_img + blk * 16384 + hf * 8192 + 4096, 8192, &load_bar);    // residual
-    bulk_load(sb + rOffSH, p.s_img + blk * 32768 + hf * 16384, 16384, &load_bar);           // value, 16 strips
-    bulk_load(sb + rOffSL, p.s_img + blk * 32768 + hf * 16384 + 8192, 16384, &load_bar);    // residual
-    bulk_load(sb + rOffDSH, p.ds_img + blk * 32768 + hf * 16384, 32768, &load_bar);
-  };
-  // the same four pieces asked into L2 one step ahead: the buffer they will land in is still being read, so the load itself
-  // cannot be issued yet, but the DRAM part of its latency can be spent meanwhile
-  auto prefetch_loads = [&](int hv, int vb) {
-    const int64_t blk = ((int64_t(sq.cbase) + c) * p.HV + hv) * (NVB / 2) + (vb >> 1);
-    const int64_t hf = vb & 1;
-    bulk_prefetch_l2(p.dz_img + blk * (2 * kDzHalf) + hf * kDzHalf, 24576);
-    bulk_prefetch_l2(p.vn_img + blk * 16384 + hf * 8192, 16384);
-    bulk_prefetch_l2(p.s_img + blk * 32768 + hf * 16384, 32768);
-    bulk_prefetch_l2(p.ds_img + blk * 32768 + hf * 16384, 32768);
-  };
   if (tid == 0) {
-    mbar_init(&mma_bar, 1);
-    mbar_init(&load_bar, 1);
-    mbar_init(&qk_bar, 1);
+    for (uint64_t* b : {&item_bar[0], &item_bar[1], &qk_bar, &full_bar[0], &full_bar[1], &p1_bar, &t2_bar}) mbar_init(b, 1);
+    for (uint64_t* b : {&pa_bar, &acc_bar, &free_bar, &red_bar[0], &red_bar[1]}) mbar_init(b, kParWorkers / 32);
+    for (uint64_t* b : {&scal_bar[0], &scal_bar[1]}) mbar_init(b, 2);
+    for (uint64_t* b : {&empty_bar[0], &empty_bar[1]}) mbar_init(b, kParWorkers / 32 + 1);
     mbar_init_fence();
-    // q, k rows of the chunk (shared by the value heads of the group): four 64 x 64 tiles into the [q; k] panels.
-    // Rows past the end of the sequence hold whatever follows in memory; every product with them meets a zero
-    // row or column of dO, dZ, v_new or the masked score gradients, and those rows are never stored.
-    mbar_arrive_expect_tx(&qk_bar, 32768);
-    tma_load_tile(sb + rOffQK, &tm_q, 0, hk, int(tok0), &qk_bar);
-    tma_load_tile(sb + rOffQK + 8192, &tm_k, 0, hk, int(tok0), &qk_bar);
-    tma_load_tile(sb + rOffQK + rQKPanel, &tm_q, 64, hk, int(tok0), &qk_bar);
-    tma_load_tile(sb + rOffQK + rQKPanel + 8192, &tm_k, 64, hk, int(tok0), &qk_bar);
-    issue_loads(hk * G, 0);
   }
-  // per-row scalars of the first value head (later heads: fetched one head ahead)
-  float pf_gam = 0.f, pf_beta = 0.f;
-  auto prefetch_scalars = [&](int hv) {
-    if (tid < kC) {
-      pf_gam = p.gam[(tok0 + min(tid, rows - 1)) * p.HV + hv];
-      pf_beta = tid < rows ? ld_scalar(p.beta, (tok0 + tid) * p.beta_st + hv, p.beta_is_f32) : 0.f;
-    }
-  };
-  prefetch_scalars(hk * G);
-  reinterpret_cast<uint4*>(smem + rOffAL)[tid] = make_uint4(0, 0, 0, 0);          // the zero rows of [0 | residual of dZ^T]
-  reinterpret_cast<uint4*>(smem + rOffAL)[tid + 256] = make_uint4(0, 0, 0, 0);
+  if (tid < kParWorkers) {
+    const uint4 z = make_uint4(0, 0, 0, 0);
+    if (tid < 256) *reinterpret_cast<uint4*>(smem + rOffStage + sOffAL + tid * 16) = z;
+    else *reinterpret_cast<uint4*>(smem + rOffStage + kStageStride + sOffAL + (tid - 256) * 16) = z;
+    *reinterpret_cast<uint4*>(smem + rOffZero + tid * 16) = z;
+    *reinterpret_cast<uint4*>(smem + rOffZero + 8192 + tid * 16) = z;
+  }
   fence_async_smem();
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
   const uint32_t tbase = tmem_base_s;
-  const uint32_t trow = tmem_addr(tbase, quad * 32, 0);
-  uint32_t mphase = 0, lphase = 0;
-  bool ok = true;
+  const uint32_t sb = smem_u32(smem);
+  auto wait = [&](uint64_t* bar, uint32_t& phase) {
+    const bool r = mbar_wait(bar, phase, p.status, FLA_ERR_TIMEOUT);
+    phase ^= 1;
+    return r;
+  };
+  // barriers that exist twice serve alternate items: their users may be an item apart
+  auto wait_item = [&](uint64_t* bars, int n) { return mbar_wait(bars + (n & 1), (n >> 1) & 1, p.status, FLA_ERR_TIMEOUT); };
+  auto signal = [&](uint64_t* bar) {      // my warp is done with what the barrier stands for
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+  };
 
-  const Operand opQK{sb + rOffQK, rQKPanel, 0};                      // [q; k], reduction over key dims
-  const Operand opKb{sb + rOffQK + 8192, rQKPanel, 0};               // k as B, N = 64 tokens
-  const Operand opKn{sb + rOffQK + 8192, rQKPanel, 1};               // k as B, N = 128 key dims, reduction over tokens
-  const Operand opQKn{sb + rOffQK, rQKPanel, 1};                     // [q; k] as B, N = 128 key dims, reduction over 128 rows
-  // operands of a step: un-swizzled strips (sm100.cuh) whose 64 rows are value channels, the reduction dim of these products
-  const Operand opAH{sb + rOffAH, 1024, 2};                                               // [dO; dZ]: M = 128 tokens = 16 strips
-  const Operand opAL{sb + rOffAL, 1024, 2};                                               // [0; residual of dZ]: enters dA = -tril(dZ Vn^T) only
-  const Operand opVNbH{sb + rOffVNH, 1024, 2}, opVNbL{sb + rOffVNL, 1024, 2};            // Vn as B (N = 64 tokens = 8 strips)
-  const Operand opVNaH{sb + rOffVNH - 8192, 1024, 2}, opVNaL{sb + rOffVNL - 8192, 1024, 2};  // Vn as A: accumulator rows 64..127 are valid
-  // (the S block, N = 128 key dims = 16 strips, follows each Vn image: the B operands of the N = 192 products start at Vn)
-  const Operand opDSH{sb + rOffDSH, 1024, 2}, opDSL{sb + rOffDSL, 1024, 2};
-  const Operand opPAH{sb + rOffPAH, 16384, 0}, opPAL{sb + rOffPAL, 16384, 0};            // [dP; dAt], reduction over j
-  const Operand opPATh{sb + rOffPAH - 8192, 8192, 1}, opPATl{sb + rOffPAL - 8192, 8192, 1};  // its transpose, valid rows 64..127
+  if (warp == kParWorkers / 32 + 1) {      // ---------------------------------------------------------------- loader
+    auto first_stage = [&](int tile, int h) { return (int64_t(flat0 + tile / p.HK) * p.HV + (tile % p.HK) * G + h) * NS; };
+    // A stage is seven copies, and the stage after next is asked into L2 in four pieces: its buffer is still being read, but the DRAM part of
+    // its latency can be spent meanwhile.  One lane each: a single thread took 1,000 cycles to issue them.
+    //               dO dZ   dZ_lo  Vn_hi  Vn_lo  S_hi   S_lo   dS       into L2: dZ, Vn, S, dS
+    const int img = lane < 2 ? 0 : lane < 4 ? 1 : lane < 6 ? 2 : lane == 6 ? 3 : min(lane - 7, 3);
+    const int64_t stride = img == 0 ? 6144 : img == 1 ? 4096 : 8192;      // bf16 elements per stage
+    const uint32_t dst = lane == 0 ? sOffAH : lane == 1 ? sOffAL + 4096 : lane == 2 ? sOffVNH : lane == 3 ? sOffVNL : lane == 4 ? sOffSH : lane == 5 ? sOffSL : sOffDSH;
+    const uint32_t bytes = lane == 0 ? 8192 : lane < 4 ? 4096 : lane < 6 ? 8192 : lane == 6 ? 16384 : uint32_t(stride) * 2;
+    const bf16* src = (img == 0 ? p.dz_img : img == 1 ? p.vn_img : img == 2 ? p.s_img : p.ds_img) + (lane == 1 ? 4096 : lane == 3 ? 2048 : lane == 5 ? 4096 : 0);
+    auto position = [&](int tile) { return chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.n0, chunk0 + tile / p.HK); };
 
-  // The running dq (q-side rows) / dk (k-side rows) of the group lives in the last 128 tensor-memory columns, this thread's
-  // 64 key-dim columns at rColAcc + half * 64: in registers it would leave none for the issuing code of warp 0.
-
-  // dg / dbeta rows of one value head from its row reductions (threads 0..63 = the two warps that own the 64 rows).
-  // dg = reverse chunk-local cumulative sum of dgam; the last row additionally carries
-  // e^{gam_L} <S, dS'> + sum_i e^{gam_L - gam_i} k_i.(Vn dS'^T)_i, which therefore reaches every row.
-  auto finish_head = [&](int hvf, int fb, float bz) {
-    const int i = tid;
-    const float (*rd)[2][kC] = red2[fb];
-    const float qdq = rd[0][0][i] + rd[0][1][i], kdk = rd[1][0][i] + rd[1][1][i];
-    const float g_ = rd[2][0][i] + rd[2][1][i], b_ = rd[3][0][i] + rd[3][1][i], ma = rd[4][0][i] + rd[4][1][i];
-    const float gi = gam_s2[fb][i], bi = beta_s2[fb][i], egi = __expf(gi), gl = gam_s2[fb][rows - 1], el = __expf(gl - gi);
-    const bool live = i < rows;
-    float suf = live ? qdq - kdk + 2.f * bi * ma - 2.f * bi * egi * g_ : 0.f;
-    float tot3 = live ? el * b_ : 0.f;
-    const int64_t gidx = (tok0 + i) * p.HV + hvf;
-    if (live) {
-      const float db = bz - egi * g_ + ma;
-      if (p.dbeta_f32) static_cast<float*>(p.dbeta)[gidx] = db;
-      else static_cast<bf16*>(p.dbeta)[gidx] = __float2bfloat16_rn(db);
+    uint32_t ph_empty[2] = {0, 0}, ph_free = 0;
+    int tile = blockIdx.x, h = 0;
+    int tok0 = 0, rows = 0;
+    int64_t b0 = 0;
+    if (tile < tiles) {
+      const ChunkPos pos = position(tile);
+      tok0 = pos.sq.bos + pos.c * kC;
+      rows = min(kC, pos.sq.len - pos.c * kC);
+      b0 = first_stage(tile, 0);
     }
+    bool ok = true;
+    for (int n = 0; ok; ++n) {
+      if (lane == 0) {
+        item_s[n & 1] = ParItem{tile, tile < tiles ? h : -1, tok0, rows};
+        mbar_arrive(&item_bar[n & 1]);
+      }
+      if (tile >= tiles) break;
+      int next = tile, hn = h + 1, tok0n = tok0, rowsn = rows;      // the item that follows
+      int64_t bn = b0 + NS;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float dn = __shfl_down_sync(0xffffffffu, suf, o);
-      if (lane + o < 32) suf += dn;
+      for (int st = 0; st < NS; ++st) {
+        const int s = st & 1;
+        if (n > 0 || st >= 2) ok = ok && wait(&empty_bar[s], ph_empty[s]);
+        ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
+        if (!ok) break;
+        if (lane == 0) mbar_arrive_expect_tx(&full_bar[s], kStageBytes);
+        __syncwarp();
+        if (lane < 7) bulk_load(sb + rOffStage + s * kStageStride + dst, src + (b0 + st) * stride, bytes, &full_bar[s]);
+        if (st == 1 && hn == G) {      // (while the stages are being read)
+          hn = 0;
+          if (lane == 0) next = int(gridDim.x) + atomicAdd(p.counter, 1);
+          next = __shfl_sync(0xffffffffu, next, 0);
+          if (next < tiles) {
+            const ChunkPos pos = position(next);
+            tok0n = pos.sq.bos + pos.c * kC;
+            rowsn = min(kC, pos.sq.len - pos.c * kC);
+            bn = first_stage(next, 0);
+          }
+        }
+        if (lane >= 7 && lane < 11 && (st + 2 < NS || next < tiles)) bulk_prefetch_l2(src + (st + 2 < NS ? b0 + st + 2 : bn + (st + 2 - NS)) * stride, bytes);
+      }
+      if (!ok) break;
+      // q, k rows of the chunk (shared by the value heads of the group): four 64 x 64 tiles, for the score product at the end of the stages.  Rows
+      // past the end of the sequence hold whatever follows in memory; every product with them meets a zero row or column of dO, dZ, v_new or
+      // the masked score gradients, and those rows are never stored.
+      if (h == 0) {
+        if (n > 0) ok = wait(&free_bar, ph_free);
+        if (lane == 0 && ok) {
+          const int hk = tile % p.HK;
+          mbar_arrive_expect_tx(&qk_bar, 32768);
+          tma_load_tile(sb + rOffQK, &tm_q, 0, hk, tok0, &qk_bar);
+          tma_load_tile(sb + rOffQK + 8192, &tm_k, 0, hk, tok0, &qk_bar);
+          tma_load_tile(sb + rOffQK + rQKPanel, &tm_q, 64, hk, tok0, &qk_bar);
+          tma_load_tile(sb + rOffQK + rQKPanel + 8192, &tm_k, 64, hk, tok0, &qk_bar);
+        }
+        __syncwarp();
+      }
+      tile = next, h = hn, tok0 = tok0n, rows = rowsn, b0 = bn;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot3 += __shfl_xor_sync(0xffffffffu, tot3, o);
+  } else if (warp == kParWorkers / 32) {      // ------------------------------------------------------------ products
     if (lane == 0) {
-      fin_s[0][warp] = suf;      // total of this warp's 32 rows (suffix sum at its first row)
-      fin_s[1][warp] = tot3;
-    }
-    asm volatile("bar.sync 2, 64;" ::: "memory");
-    if (warp == 0) suf += fin_s[0][1];
-    float tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) tot += sds_s2[fb][w];
-    const float dgv = suf + __expf(gl) * tot + fin_s[1][0] + fin_s[1][1];
-    if (live) {
-      if (p.dg_f32) static_cast<float*>(p.dg)[gidx] = dgv;
-      else static_cast<bf16*>(p.dg)[gidx] = __float2bfloat16_rn(dgv);
-    }
-    asm volatile("bar.sync 2, 64;" ::: "memory");   // fin_s is free again
-  };
-  auto load_bz = [&](int hvf) -> float {   // sum of the reverse scan's partial row sums of dZ . V (one per 32 columns of V)
-    if (tid >= rows) return 0.f;
-    const int64_t gidx = (tok0 + tid) * p.HV + hvf;
-    const int64_t bzs = p.total_tokens * p.HV;
-    float acc = 0.f;
-    for (int i = 0; i < NVB; ++i) acc += p.bz[(2 * i) * bzs + gidx] + p.bz[(2 * i + 1) * bzs + gidx];
-    return acc;
-  };
-
-  float bz_prev = 0.f;
-  for (int h = 0; h < G && ok; ++h) {
-    const int hv = hk * G + h;
-    const int hb = h & 1;
-    float* gam_s = gam_s2[hb];
-    float* beta_s = beta_s2[hb];
-    float (*red)[2][kC] = red2[hb];
-    if (tid < kC) {
-      gam_s[tid] = pf_gam;
-      beta_s[tid] = pf_beta;
-    }
-    if (h + 1 < G) prefetch_scalars(hv + 1);
-    const float bz_cur = load_bz(hv);     // lands while the step's operands are awaited
-    float sds = 0.f;
-    for (int vb = 0; vb < NVB; ++vb) {
-      ok = mbar_wait(&load_bar, lphase, p.status, FLA_ERR_TIMEOUT);
-      lphase ^= 1;
-      if (h == 0 && vb == 0) ok = mbar_wait(&qk_bar, 0, p.status, FLA_ERR_TIMEOUT) && ok;
-      if (!__syncthreads_and(ok)) { ok = false; break; }
-      if (tid == 0) {
+      const Operand opQK{sb + rOffQK, rQKPanel, 0};                      // [q; k], reduction over key dims
+      const Operand opKb{sb + rOffQK + 8192, rQKPanel, 0};               // k as B, N = 64 tokens
+      const Operand opKn{sb + rOffQK + 8192, rQKPanel, 1};               // k as B, N = 128 key dims, reduction over tokens
+      const Operand opQKn{sb + rOffQK, rQKPanel, 1};                     // [q; k] as B, N = 128 key dims, reduction over 128 rows
+      const Operand opPAH{sb + rOffPAH, 16384, 0}, opPAL{sb + rOffPAL, 16384, 0};                                            // [dP; dAt], reduction over j
+      const Operand opPATh{sb + rOffZero, rOffPAH - rOffZero, 1}, opPATl{sb + rOffZero, rOffPAL - rOffZero, 1};              // [0; its transpose]
+      uint32_t ph_full[2] = {0, 0}, ph_qk = 0, ph_pa = 0, ph_acc = 0;
+      for (int n = 0;; ++n) {
+        if (!wait_item(item_bar, n)) break;
+        const int h = item_s[n & 1].h;
+        if (h < 0) break;
+        if (n > 0 && !wait(&acc_bar, ph_acc)) break;
         tc_fence_after();
-        if (h == 0 && vb == 0) mma_tile(tbase + rColQK, opQK, opKb, 128, 64, 8, false);
-        const bool accf = vb > 0;
-        // [dO; dZ] . [Vn_lo | S_hi]^T and [dO; dZ] . [Vn_hi | S_lo]^T as N = 192 products (the images are neighbours in shared memory, their
-        // accumulators neighbours in tensor memory): the A operand is read once for both
-        static_assert(rOffVNL + 8192 == rOffSH && rOffVNH + 8192 == rOffSL && rColDV + 64 == rColTA, "the N = 192 products need these adjacent");
-        mma_tile(tbase + rColDV, opAH, opVNbL, 128, 192, 4, accf);
-        mma_tile(tbase + rColDV, opAH, opVNbH, 128, 192, 4, true);     // [Vn_hi | S_lo]
-        mma_tile(tbase + rColDV, opAL, opVNbH, 128, 64, 4, true);
-        mma_tile(tbase + rColTB, opVNaH, opDSH, 128, 128, 4, accf);
-        mma_tile(tbase + rColTB, opVNaH, opDSL, 128, 128, 4, true);
-        mma_tile(tbase + rColTB, opVNaL, opDSH, 128, 128, 4, true);
-        mma_commit(&mma_bar);
-        if (vb + 1 < NVB) prefetch_loads(hv, vb + 1);
-        else if (h + 1 < G) prefetch_loads(hv + 1, 0);
-      }
-      if (h > 0 && vb == 0 && tid < kC) finish_head(hv - 1, hb ^ 1, bz_prev);   // while the MMAs run
-      // <S, dS'> over this V block while the MMAs run (elementwise on the raw images).  Values and residuals: the terms
-      // have either sign, so the sum is no larger than its rounding noise would be with the values alone (ragged chunks,
-      // where this term dominates dg, then miss the bar by 10x).
+        bool ok = true;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t off = (tid + i * 256) * 16;
-        float s1[8], s2[8], d1[8], d2[8];
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + rOffSH + off), s1);
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + rOffSL + off), s2);
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + rOffDSH + off), d1);
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(smem + rOffDSL + off), d2);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) sds += (s1[j] + s2[j]) * (d1[j] + d2[j]);
-      }
-      ok = mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT);
-      mphase ^= 1;
-      if (!__syncthreads_and(ok)) { ok = false; break; }   // also: every thread is done reading the step's buffers
-      tc_fence_after();
-      if (tid == 0) {
-        if (vb + 1 < NVB) issue_loads(hv, vb + 1);
-        else if (h + 1 < G) issue_loads(hv + 1, 0);
+        for (int st = 0; st < NS; ++st) {
+          const int s = st & 1;
+          ok = ok && wait(&full_bar[s], ph_full[s]);
+          if (!ok) break;
+          const uint32_t base = sb + rOffStage + s * kStageStride;
+          const Operand opAH{base + sOffAH, 512, 2};                                       // [dO; dZ]: M = 128 tokens = 16 strips
+          const Operand opAL{base + sOffAL, 512, 2};                                       // [0; residual of dZ]: enters dA = -tril(dZ Vn^T) only
+          const Operand opVNbL{base + sOffVNL, 512, 2}, opVNbH{base + sOffVNH, 512, 2};    // Vn as B (N = 64 tokens), S (N = 128 key dims) behind it
+          const Operand opVNaH{base + sOffVNH - 4096, 512, 2}, opVNaL{base + sOffVNL - 4096, 512, 2};   // Vn as A: rows 64..127 are valid
+          const Operand opDSH{base + sOffDSH, 512, 2}, opDSL{base + sOffDSL, 512, 2};
+          const bool acc = st > 0;
+          // [dO; dZ] . [Vn_lo | S_hi]^T and [dO; dZ] . [Vn_hi | S_lo]^T as N = 192 products: the A operand is read once for both
+          static_assert(sOffVNL + 4096 == sOffSH && sOffVNH + 4096 == sOffSL && rColDV + 64 == rColTA, "the N = 192 products need these adjacent");
+          mma_tile(tbase + rColDV, opAH, opVNbL, 128, 192, 2, acc);
+          mma_tile(tbase + rColDV, opAH, opVNbH, 128, 192, 2, true);
+          mma_tile(tbase + rColDV, opAL, opVNbH, 128, 64, 2, true);
+          mma_tile(tbase + rColTB, opVNaH, opDSH, 128, 128, 2, acc);
+          mma_tile(tbase + rColTB, opVNaH, opDSL, 128, 128, 2, true);
+          mma_tile(tbase + rColTB, opVNaL, opDSH, 128, 128, 2, true);
+          mma_commit(&empty_bar[s]);
+        }
+        if (ok && h == 0) {      // the score tiles of the chunk, kept for all heads of the group
+          ok = wait(&qk_bar, ph_qk);
+          if (ok) mma_tile(tbase + rColQK, opQK, opKb, 128, 64, 8, false);
+        }
+        if (!ok) break;
+        mma_commit(&p1_bar);
+        if (!wait(&pa_bar, ph_pa)) break;
+        tc_fence_after();
+        mma_tile(tbase + rColT2, opPAH, opKn, 128, 128, 4, false);
+        mma_tile(tbase + rColT2, opPAL, opKn, 128, 128, 4, true);
+        mma_tile(tbase + rColT2, opPATh, opQKn, 128, 128, 8, true);
+        mma_tile(tbase + rColT2, opPATl, opQKn, 128, 128, 8, true);
+        mma_commit(&t2_bar);
       }
     }
-    if (!ok) break;
+  } else if (warp > kParWorkers / 32) {      // ------------------------------------------------------------------ tail
+    const int i = tid - (kParThreads - 64), w = i >> 5;      // my token
+    bool ok = true;
+    int rows0 = 0;          // of the item before: row count (0: none), where its dg / dbeta element goes, its scalars
+    int64_t gidx0 = 0;
+    float gv0 = 0.f, bv0 = 0.f, bz0 = 0.f;
+    for (int n = 0;; ++n) {
+      ok = ok && wait_item(item_bar, n);
+      const ParItem it = ok ? item_s[n & 1] : ParItem{0, 0, 0, 1};
+      const bool more = it.h >= 0;
+      const int hv = (it.tile % p.HK) * G + it.h;
+      const int64_t gidx = (int64_t(it.tok0) + min(i, it.rows - 1)) * p.HV + hv;
+      float gv = 0.f, bv = 0.f, bz = 0.f;
+      if (more) {
+        gv = p.gam[gidx] * kLog2e;
+        if (i < it.rows) bv = ld_scalar(p.beta, (int64_t(it.tok0) + i) * p.beta_st + hv, p.beta_is_f32);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sds += __shfl_xor_sync(0xffffffffu, sds, o);
-    if (lane == 0) sds_s2[hb][warp] = sds;
+        for (int s = 0; s < 2 * NVB; ++s) bz += p.bz[s * p.total_tokens * p.HV + gidx];
+        gam_s2[n & 1][i] = gv;
+        beta_s2[n & 1][i] = bv;
+        signal(&scal_bar[n & 1]);
+      }
+      // dg / dbeta rows of the item before.  dg = reverse chunk-local cumulative sum of dgam; the last row additionally carries
+      // e^{gam_L} <S, dS'> + sum_i e^{gam_L - gam_i} k_i.(Vn dS'^T)_i, which therefore reaches every row.
+      if (n > 0) ok = ok && wait_item(red_bar, n - 1);
+      float suf = 0.f, tot3 = 0.f, tot = 0.f, gl = 0.f;
+      const bool live = i < rows0;
+      if (rows0) {
+        float (*red)[4][kC] = red2[(n - 1) & 1];
+        auto sum4 = [&](int r) { return (red[r][0][i] + red[r][1][i]) + (red[r][2][i] + red[r][3][i]); };
+        const float qdq = sum4(0), kdk = sum4(1), g_ = sum4(2), b_ = sum4(3), ma = sum4(4), egi = exp2_fast(gv0);
+        gl = gam_s2[(n - 1) & 1][rows0 - 1];
+#pragma unroll
+        for (int j = 0; j < kParWorkers / 32; ++j) tot += sds_s2[(n - 1) & 1][j];
+        if (live) {
+          suf = qdq - kdk + 2.f * bv0 * ma - 2.f * bv0 * egi * g_;
+          tot3 = exp2_fast(gl - gv0) * b_;
+          const float db = bz0 - egi * g_ + ma;
+          if (p.dbeta_f32) static_cast<float*>(p.dbeta)[gidx0] = db;
+          else static_cast<bf16*>(p.dbeta)[gidx0] = __float2bfloat16_rn(db);
+        }
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float dn = __shfl_down_sync(0xffffffffu, suf, o);
+        if (lane + o < 32) suf += dn;
+        tot3 += __shfl_xor_sync(0xffffffffu, tot3, o);
+      }
+      if (lane == 0) {
+        fin_s[0][w] = suf;      // total of this warp's 32 rows (suffix sum at its first row)
+        fin_s[1][w] = tot3;
+      }
+      ok = par_sync_and<2, 64>(ok);
+      if (live && ok) {
+        if (w == 0) suf += fin_s[0][1];
+        const float dgv = suf + exp2_fast(gl) * tot + fin_s[1][0] + fin_s[1][1];
+        if (p.dg_f32) static_cast<float*>(p.dg)[gidx0] = dgv;
+        else static_cast<bf16*>(p.dg)[gidx0] = __float2bfloat16_rn(dgv);
+      }
+      if (!ok || !more) break;
+      par_sync_and<2, 64>(true);      // fin_s is free again
+      rows0 = it.rows, gidx0 = gidx, gv0 = gv, bv0 = bv, bz0 = bz;
+    }
+  } else {      // ------------------------------------------------------------------------------------------ workers
+    const int quad = warp & 3, cg = warp >> 2;  // my 32 accumulator rows, my 32 key-dim columns
+    const int row = quad * 32 + lane;           // accumulator row == TMEM lane
+    const bool kside = quad >= 2;
+    const int tok = row & 63;
+    const uint32_t trow = tmem_addr(tbase, quad * 32, 0);
+    const uint8_t* qk = smem + rOffQK + (cg >> 1) * rQKPanel;      // the panel of my columns
+    auto qk8 = [&](int ch, float* f) {      // eight elements of my row of [q; k]
+      unpack_bf16x8(*reinterpret_cast<const uint4*>(qk + panel_chunk_off(row, (cg & 1) * 4 + ch)), f);
+    };
+    uint32_t ph_full[2] = {0, 0}, ph_qk = 0, ph = 0;
+    bool ok = true;
+    float acc[32];      // running dq (q-side rows) or dk (k-side rows), my 32 key-dim columns
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+    float xsum = 0.f;   // their dot product with q or k
+    // My part of <S, dS'> of a stage, elementwise on the raw images.  Values and residuals: the terms have either sign, so the sum is no
+    // larger than its rounding noise would be with the values alone (ragged chunks, where this term dominates dg, then miss by 10x).
+    float sds = 0.f;
+    auto stage_dot = [&](int s) {
+      ok = ok && wait(&full_bar[s], ph_full[s]);
+      const uint8_t* base = smem + rOffStage + s * kStageStride + tid * 16;
+      const uint4 r1 = *reinterpret_cast<const uint4*>(base + sOffSH), r2 = *reinterpret_cast<const uint4*>(base + sOffSL);
+      const uint4 r3 = *reinterpret_cast<const uint4*>(base + sOffDSH), r4 = *reinterpret_cast<const uint4*>(base + sOffDSL);
+      float s1[8], s2[8], d1[8], d2[8];
+      unpack_bf16x8(r1, s1);
+      unpack_bf16x8(r2, s2);
+      unpack_bf16x8(r3, d1);
+      unpack_bf16x8(r4, d2);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sds += (s1[j] + s2[j]) * (d1[j] + d2[j]);
+      signal(&empty_bar[s]);
+    };
+    ParItem it, next;
+    // An item's first two stages are read while the products of the one before are waited for.  A wait that runs out makes this thread
+    // skip the rest of its waits; all leave together at the barrier behind the stages.
+    auto take = [&](int n) {
+      ok = ok && wait_item(item_bar, n);
+      next = ok ? item_s[n & 1] : ParItem{0, 0, 0, 1};
+      sds = 0.f;
+      if (next.h >= 0) {
+        stage_dot(0);
+        stage_dot(1);
+      }
+    };
+    take(0);
+    for (int n = 0;; ++n) {
+      it = next;
+      if (it.h < 0) {
+        par_sync_and<1, kParWorkers>(true);
+        break;
+      }
+#pragma unroll
+      for (int st = 2; st < NS; ++st) stage_dot(st & 1);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sds += __shfl_xor_sync(0xffffffffu, sds, o);
+      const int hk = it.tile % p.HK, rows = it.rows;
+      const int64_t tok0 = it.tok0;
+      const float *gam_s = gam_s2[n & 1], *beta_s = beta_s2[n & 1];
+      float (*red)[4][kC] = red2[n & 1];
+      ok = ok && wait_item(scal_bar, n);
+      if (lane == 0) sds_s2[n & 1][warp] = sds;
+      if (it.h == 0) ok = ok && wait(&qk_bar, ph_qk);
+      ok = par_sync_and<1, kParWorkers>(ok);
+      if (!ok) break;
 
-    // ---- epilogue 1: score-tile gradients -> [dP; dAt] operand, first parts of this head's dq / dk rows
-    const float gam_i = gam_s[tok], beta_i = beta_s[tok], gam_last = gam_s[rows - 1];
-    const float eg = __expf(gam_i);
-    float ma_part = 0.f;
-    {
-      float sc[32], dvv[32];
-      tmem_ld32(trow + rColQK + half * 32, sc);
-      tmem_ld32(trow + rColDV + half * 32, dvv);
-      tmem_ld_wait();
+      // ---- epilogue 1: score-tile gradients -> [dP; dAt] operand, first parts of this head's dq / dk rows
+      ok = mbar_wait(&p1_bar, ph, p.status, FLA_ERR_TIMEOUT);
+      tc_fence_after();
+      const float gam_i = gam_s[tok], beta_i = beta_s[tok], eg = exp2_fast(gam_i);
+      {
+        float sc[16], dvv[16];
+        tmem_ld16(trow + rColQK + cg * 16, sc);
+        tmem_ld16(trow + rColDV + cg * 16, dvv);
+        float ma = 0.f;
+        tmem_ld_wait();
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+          float t[8];
+          gather8(gam_s + cg * 16 + ch * 8, t);
+          if (!kside) {
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) {
+              const float e = p.scale * exp2_fast(fminf(gam_i - t[jj], 0.f));
+              dvv[ch * 8 + jj] *= (cg * 16 + ch * 8 + jj <= tok) ? e : 0.f;
+            }
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) {
+              const float e = exp2_fast(fminf(gam_i - t[jj], 0.f));
+              const float dA = (cg * 16 + ch * 8 + jj < tok) ? -dvv[ch * 8 + jj] * e : 0.f;
+              ma += dA * sc[ch * 8 + jj];
+              dvv[ch * 8 + jj] = dA * beta_i;
+            }
+          }
+          uint4 hi, lo;
+          split8(dvv + ch * 8, hi, lo);
+          const uint32_t off = panel_chunk_off(row, cg * 2 + ch);
+          *reinterpret_cast<uint4*>(smem + rOffPAH + off) = hi;
+          *reinterpret_cast<uint4*>(smem + rOffPAL + off) = lo;
+        }
+        if (kside) red[4][cg][tok] = ma;
+      }
+      fence_async_smem();
+      tc_fence_before();
+      signal(&pa_bar);
+      float xdx = 0.f;      // q.dq (q-side) or k.dk (k-side) over my columns, this head's part
       if (!kside) {
+        const float f = p.scale * eg;
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const int j = half * 32 + jj;
-          const float e = p.scale * __expf(fminf(gam_i - gam_s[j], 0.f));
-          dvv[jj] *= (j <= tok) ? e : 0.f;
+        for (int c2 = 0; c2 < 2; ++c2) {
+          float x[16];
+          tmem_ld16(trow + rColTA + cg * 32 + c2 * 16, x);
+          float qv[16];
+          qk8(c2 * 2, qv);
+          qk8(c2 * 2 + 1, qv + 8);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            x[i] *= f;
+            xdx += qv[i] * x[i];
+            acc[c2 * 16 + i] += x[i];
+          }
         }
       } else {
+        const float f1 = -beta_i * eg, f2 = exp2_fast(gam_s[rows - 1] - gam_i);
+        float rkG = 0.f, rkB = 0.f;
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const int j = half * 32 + jj;
-          const float e = __expf(fminf(gam_i - gam_s[j], 0.f));
-          const float dec = (j < tok) ? e : 0.f;
-          const float dA = -dvv[jj] * dec;
-          ma_part += dA * sc[jj];
-          dvv[jj] = dA * beta_i;
+        for (int ch = 0; ch < 4; ++ch) {
+          float x[8], y[8], kv[8];
+          tmem_ld8(trow + rColTA + cg * 32 + ch * 8, x);
+          tmem_ld8(trow + rColTB + cg * 32 + ch * 8, y);
+          qk8(ch, kv);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            rkG += kv[i] * x[i];
+            rkB += kv[i] * y[i];
+            acc[ch * 8 + i] += f1 * x[i] + f2 * y[i];
+          }
         }
+        red[2][cg][tok] = rkG;
+        red[3][cg][tok] = rkB;
+        xdx = f1 * rkG + f2 * rkB;
       }
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        uint4 hi, lo;
-        split8(dvv + ch * 8, hi, lo);
-        const uint32_t off = panel_chunk_off(row, half * 4 + ch);
-        *reinterpret_cast<uint4*>(smem + rOffPAH + off) = hi;
-        *reinterpret_cast<uint4*>(smem + rOffPAL + off) = lo;
-      }
-    }
-    float part[64];   // this head's contribution to my dq / dk row (64 key-dim columns)
-    float rkG = 0.f, rkB = 0.f;
-    tmem_ld_row64(trow + rColTA + half * 64, part);
-    if (!kside) {
-      const float f = p.scale * eg;
-#pragma unroll
-      for (int i = 0; i < 64; ++i) part[i] *= f;
-    } else {
-      row_dot64(smem + rOffQK, rQKPanel, 64 + tok, half * 64, part, rkG);
-      float bk[64];
-      tmem_ld_row64(trow + rColTB + half * 64, bk);
-      row_dot64(smem + rOffQK, rQKPanel, 64 + tok, half * 64, bk, rkB);
-      const float f1 = -beta_i * eg, f2 = __expf(gam_last - gam_i);
-#pragma unroll
-      for (int i = 0; i < 64; ++i) part[i] = f1 * part[i] + f2 * bk[i];
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
+      tc_fence_before();
+      signal(&acc_bar);
+      take(n + 1);
 
-    // ---- [dP; dAt] K  and  [dP^T | dAt^T] [Q; K]
-    if (tid == 0) {
+      // ---- epilogue 2: finish the rows, row dots for dg / dbeta
+      const bool last = it.h + 1 == G;
+      float rs = 0.f;
+      if (last && p.q_rstd) rs = (kside ? p.k_rstd : p.q_rstd)[(tok0 + min(tok, rows - 1)) * p.HK + hk];
+      ok = ok && mbar_wait(&t2_bar, ph, p.status, FLA_ERR_TIMEOUT);
       tc_fence_after();
-      mma_tile(tbase + rColTA, opPAH, opKn, 128, 128, 4, false);
-      mma_tile(tbase + rColTA, opPAL, opKn, 128, 128, 4, true);
-      mma_tile(tbase + rColTB, opPATh, opQKn, 128, 128, 8, false);
-      mma_tile(tbase + rColTB, opPATl, opQKn, 128, 128, 8, true);
-      mma_commit(&mma_bar);
-    }
-    ok = mbar_wait(&mma_bar, mphase, p.status, FLA_ERR_TIMEOUT);
-    mphase ^= 1;
-    if (!__syncthreads_and(ok)) { ok = false; break; }
-    tc_fence_after();
+#pragma unroll
+      for (int c2 = 0; c2 < 2; ++c2) {
+        float x[16], v[16];
+        tmem_ld16(trow + rColT2 + cg * 32 + c2 * 16, x);
+        qk8(c2 * 2, v);
+        qk8(c2 * 2 + 1, v + 8);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          xdx += v[i] * x[i];
+          acc[c2 * 16 + i] += x[i];
+        }
+      }
+      red[kside ? 1 : 0][cg][tok] = xdx;
+      tc_fence_before();
+      xsum += xdx;
+      if (last && p.q_rstd) ndot_s[cg][row] = xsum;
+      signal(&red_bar[n & 1]);
+      ph ^= 1;
+      if (!last) continue;
 
-    // ---- epilogue 2: finish the rows, row dots for dg / dbeta
-    {
-      float t[64];
-      tmem_ld_row64(trow + rColTA + half * 64, t);
+      if (p.q_rstd) {   // the rows are complete: through the normalisation, rstd (dx - x (x . dx))
+        ok = par_sync_and<1, kParWorkers>(ok);
+        const float t = (ndot_s[0][row] + ndot_s[1][row]) + (ndot_s[2][row] + ndot_s[3][row]);
 #pragma unroll
-      for (int i = 0; i < 64; ++i) part[i] += t[i];
-      if (kside) {
-        tmem_ld_row64(trow + rColTB + half * 64, t);
+        for (int ch = 0; ch < 4; ++ch) {
+          float f[8];
+          qk8(ch, f);
 #pragma unroll
-        for (int i = 0; i < 64; ++i) part[i] += t[i];
+          for (int j = 0; j < 8; ++j) acc[ch * 8 + j] = (acc[ch * 8 + j] - t * f[j]) * rs;
+        }
       }
-    }
-    float xdx = 0.f;  // q.dq (q-side) or k.dk (k-side) over my columns
-    row_dot64(smem + rOffQK, rQKPanel, row, half * 64, part, xdx);
-    if (h > 0) {
-      float t[64];
-      tmem_ld_row64(trow + rColAcc + half * 64, t);
+      signal(&free_bar);
+      {
+        void* base = kside ? p.dk : p.dq;
+        const int64_t st_ = kside ? p.dk_st : p.dq_st;
+        const int64_t off = tok0 * st_ + hk * (kside ? p.dk_sh : p.dq_sh) + cg * 32;
+        if (kside ? p.dk_f32 : p.dq_f32) {
+          float* dst = static_cast<float*>(base) + off + tok * st_;
+          if (tok < rows) {
 #pragma unroll
-      for (int i = 0; i < 64; ++i) part[i] += t[i];
-    }
-    if (h + 1 < G) {
-      tmem_st_row64(trow + rColAcc + half * 64, part);
-    } else if (p.q_rstd) {   // the rows are complete: through the normalisation, rstd (dx - x (x . dx)), while they are in registers
-      float t = 0.f;
-      row_dot64(smem + rOffQK, rQKPanel, row, half * 64, part, t);
-      ndot_s[half][row] = t;
-      __syncthreads();
-      t = ndot_s[0][row] + ndot_s[1][row];
-      const float rs = (kside ? p.k_rstd : p.q_rstd)[(tok0 + min(tok, rows - 1)) * p.HK + hk];
-      const uint8_t* pan = smem + rOffQK + half * rQKPanel;
+            for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+          }
+        } else {      // four lanes trade pieces so that they store 64 contiguous bytes of one row after the other
+          uint4 v[4];
 #pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        float f[8];
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(pan + panel_chunk_off(row, ch)), f);
+          for (int ch = 0; ch < 4; ++ch) v[ch] = pack8(acc + ch * 8);
+          transpose4x4(v, lane);
+          bf16* dst = static_cast<bf16*>(base) + off + (tok & ~3) * st_ + (lane & 3) * 8;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) part[ch * 8 + j] = (part[ch * 8 + j] - t * f[j]) * rs;
+          for (int j = 0; j < 4; ++j)
+            if ((tok & ~3) + j < rows) *reinterpret_cast<uint4*>(dst + j * st_) = v[j];
+        }
       }
-    }
-    if (h + 1 == G && tok < rows) {   // the last head
-      void* base = kside ? p.dk : p.dq;
-      const int64_t off = kside ? (tok0 + tok) * p.dk_st + hk * p.dk_sh + half * 64 : (tok0 + tok) * p.dq_st + hk * p.dq_sh + half * 64;
-      if (kside ? p.dk_f32 : p.dq_f32) {
-        float* dst = static_cast<float*>(base) + off;
+      xsum = 0.f;
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(part[i], part[i + 1], part[i + 2], part[i + 3]);
-      } else {
-        bf16* dst = static_cast<bf16*>(base) + off;
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<uint4*>(dst + ch * 8) = pack8(part + ch * 8);
-      }
+      for (int i = 0; i < 32; ++i) acc[i] = 0.f;
     }
-    if (!kside) {
-      red[0][half][tok] = xdx;
-    } else {
-      red[1][half][tok] = xdx;
-      red[2][half][tok] = rkG;
-      red[3][half][tok] = rkB;
-      red[4][half][tok] = ma_part;
-    }
-    tc_fence_before();
-    __syncthreads();
-    bz_prev = bz_cur;
   }
-  if (__syncthreads_and(ok) && tid < kC) finish_head(hk * G + G - 1, (G - 1) & 1, bz_prev);
-
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tbase, 512);
@@ -592,6 +742,7 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   p.p_img = static_cast<const bf16*>(a->p_img.data);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   p.status = reinterpret_cast<int*>(ws);
+  p.counter = p.status + 16;      // both inside the workspace's 256-byte head
   p.ds_img = reinterpret_cast<bf16*>(ws + off_ds);
   p.dz_img = reinterpret_cast<bf16*>(ws + off_dz);
   p.bz = reinterpret_cast<float*>(ws + off_bz);
@@ -638,8 +789,8 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
     scan<<<grid, kScanThreads, kScanBwdSmem + 1024, st>>>(pp, tm_q, tm_k, tm_v, tm_d);
   };
   auto launch_par = [&](const GdnBwdParams& pp, int64_t chunks, cudaStream_t st) {
-    if (nvb == 2) gdn_bwd_par_kernel<2><<<dim3(unsigned(chunks), unsigned(HK)), 256, kParSmem + 1024, st>>>(pp, tm_q, tm_k);
-    else gdn_bwd_par_kernel<4><<<dim3(unsigned(chunks), unsigned(HK)), 256, kParSmem + 1024, st>>>(pp, tm_q, tm_k);
+    auto* par = nvb == 2 ? gdn_bwd_par_kernel<2> : gdn_bwd_par_kernel<4>;
+    par<<<unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads, kParSmem + 1024, st>>>(pp, int(chunks), tm_q, tm_k);
   };
   // The reverse scan launches one CTA per (sequence, value head, 128 channels) and each needs a whole SM: when there are
   // more chains than SMs the last round leaves SMs idle for the length of a chain.  The batch is then launched as two
@@ -653,11 +804,12 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
     const int n1 = N / 2;
     GdnBwdParams p2 = p;
     p.n1 = p2.n0 = n1;
+    p2.counter = p.counter + 16;
     bool okc = cudaEventRecord(aux->fork, cs) == cudaSuccess && cudaStreamWaitEvent(aux->s, aux->fork, 0) == cudaSuccess;
     if (!okc) return FLA_ERR_CUDA;
     launch_scan(p, n1, cs);
     launch_scan(p2, N - n1, aux->s);
-    // a packed batch's halves hold chunk counts the host does not have: both launches cover all chunks and skip the other half's
+    // a packed batch's halves hold chunk counts the host does not have: the kernel looks up its own
     const int64_t nt = (T + kC - 1) / kC;
     launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs);
     launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s);

@@ -13,8 +13,8 @@
 // dO^T and V^T reach tensor memory through identity products.  For the chunk-parallel kernel the scan saves, per
 // (chunk, head, block), operands in the un-swizzled strip layout (sm100.cuh) whose rows are value channels, stored by
 // the thread that owns the channel (coalesced):
-//     ds_img  dS' as [64-channel half][value | residual][16 strips of 8 key dims][64 rows x 16 bytes]   = 64 KB
-//     dz_img  [64-channel half][dO^T | dZ^T | residual of dZ^T][8 strips of 8 tokens][64 rows x 16 bytes] = 48 KB
+//     ds_img  dS' as [32-channel quarter][value | residual][16 strips of 8 key dims][32 rows x 16 bytes]   = 64 KB
+//     dz_img  [32-channel quarter][dO^T | dZ^T | residual of dZ^T][8 strips of 8 tokens][32 rows x 16 bytes] = 48 KB
 //
 // Split chains (scan_segments.cuh): a state-only pass gives each segment's dH (the gradient that leaves it on the left when none enters on
 // the right; the last segment starts from dht), the walk to a segment's own start goes through the transposes of the forward's M.
@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
   const int seg = blockIdx.y + p.n0, hv = blockIdx.x / (p.V / 128), vb = blockIdx.x % (p.V / 128);   // neighbours share q, k: heads first
   const int hk = hv / (p.HV / p.HK);
   if (tid == 0) clear_status(p.status, seg + blockIdx.x == 0 && (kState || !kSplit));   // the backward's first kernel
+  if (tid == 0 && blockIdx.y + blockIdx.x == 0) *p.counter = 0;      // of the par kernel that follows
   SegPos pos;
   if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos)) return;
   if (kState && pos.s == 0) return;
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
     // ---- A: publish dS' (the gradient entering this chunk): bf16 value + residual as A operand, decayed copy as accumulator
     {
       const float dl = f.dl;
-      uint8_t* s_row = reinterpret_cast<uint8_t*>(p.ds_img + cidx * 32768) + (vrow >> 6) * 32768 + (vrow & 63) * 16;
+      uint8_t* s_row = reinterpret_cast<uint8_t*>(p.ds_img + cidx * 32768) + quad * 16384 + lane * 16;
 #pragma unroll 1
       for (int g4 = 0; g4 < 4; ++g4) {
         float s16[16];
@@ -345,11 +346,11 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
         tmem_st8u(tlane + uAh + half * 32 + g4 * 8, hi);
         tmem_st8u(tlane + uAl + half * 32 + g4 * 8, lo);
         if (!kState) {   // the dS' image for the chunk-parallel kernel: strips half * 8 + g4 * 2 and the next one of my channel's row
-          uint8_t* dst = s_row + (half * 8 + g4 * 2) * 1024;
+          uint8_t* dst = s_row + (half * 8 + g4 * 2) * 512;
           *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(dst + 1024) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
-          *reinterpret_cast<uint4*>(dst + 16384) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          *reinterpret_cast<uint4*>(dst + 16384 + 1024) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+          *reinterpret_cast<uint4*>(dst + 512) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+          *reinterpret_cast<uint4*>(dst + 8192) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          *reinterpret_cast<uint4*>(dst + 8192 + 512) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) s16[i] *= dl;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
     // ---- C: dZ^T -> dV rows, partial sums of dZ V, the [dO^T | dZ^T] image, the operand [scale e^gam dO^T | -beta e^gam dZ^T]
     {
       // the [dO^T | dZ^T] image: my channel's row of strips half * 4 + g * 2 and the next one
-      uint8_t* img = reinterpret_cast<uint8_t*>(p.dz_img + cidx * (2 * kDzHalf)) + (vrow >> 6) * (2 * kDzHalf) + (vrow & 63) * 16;
+      uint8_t* img = reinterpret_cast<uint8_t*>(p.dz_img + cidx * (2 * kDzHalf)) + quad * kDzHalf + lane * 16;     // kDzHalf bytes per 32 channels
       float pr[32];
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
@@ -415,10 +416,10 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
           for (int i = 0; i < 16; ++i) pr[g * 16 + i] = dz[i] * t16[i];
           uint32_t zl[8];
           split16(dz, w8, zl);     // dZ as value + residual: dA = -tril(dZ Vn^T) feeds dk, dg, dbeta through cancelling sums
-          *reinterpret_cast<uint4*>(img + 8192 + (half * 4 + g * 2) * 1024) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
-          *reinterpret_cast<uint4*>(img + 8192 + (half * 4 + g * 2 + 1) * 1024) = make_uint4(w8[4], w8[5], w8[6], w8[7]);
-          *reinterpret_cast<uint4*>(img + 16384 + (half * 4 + g * 2) * 1024) = make_uint4(zl[0], zl[1], zl[2], zl[3]);
-          *reinterpret_cast<uint4*>(img + 16384 + (half * 4 + g * 2 + 1) * 1024) = make_uint4(zl[4], zl[5], zl[6], zl[7]);
+          *reinterpret_cast<uint4*>(img + 4096 + (half * 4 + g * 2) * 512) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
+          *reinterpret_cast<uint4*>(img + 4096 + (half * 4 + g * 2 + 1) * 512) = make_uint4(w8[4], w8[5], w8[6], w8[7]);
+          *reinterpret_cast<uint4*>(img + 8192 + (half * 4 + g * 2) * 512) = make_uint4(zl[0], zl[1], zl[2], zl[3]);
+          *reinterpret_cast<uint4*>(img + 8192 + (half * 4 + g * 2 + 1) * 512) = make_uint4(zl[4], zl[5], zl[6], zl[7]);
         }
 #pragma unroll
         for (int i4 = 0; i4 < 16; i4 += 4) {
@@ -437,8 +438,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_bwd_kernel(GdnBwdPar
         tmem_ld_wait();
         if (!kState) {
           pack16(t16, w8);                                // exact: these are the bf16 inputs
-          *reinterpret_cast<uint4*>(img + (half * 4 + g * 2) * 1024) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
-          *reinterpret_cast<uint4*>(img + (half * 4 + g * 2 + 1) * 1024) = make_uint4(w8[4], w8[5], w8[6], w8[7]);
+          *reinterpret_cast<uint4*>(img + (half * 4 + g * 2) * 512) = make_uint4(w8[0], w8[1], w8[2], w8[3]);
+          *reinterpret_cast<uint4*>(img + (half * 4 + g * 2 + 1) * 512) = make_uint4(w8[4], w8[5], w8[6], w8[7]);
         }
 #pragma unroll
         for (int i4 = 0; i4 < 16; i4 += 4) {

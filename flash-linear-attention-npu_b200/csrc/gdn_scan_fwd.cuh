@@ -15,8 +15,8 @@
 // un-swizzled strip layout (sm100.cuh), rows = value channels: a thread owns one channel, so the 16 bytes it stores for a
 // strip lie next to its neighbours' (512 contiguous bytes per warp store).  Swizzled panels, whose rows are 128 bytes
 // apart, had to be staged in shared memory and written by bulk copies: 0.83 ms per launch against 0.7x ms.
-//     s_img   [64-channel half][value | residual][16 strips of 8 key dims][64 rows x 16 bytes]   = 64 KB
-//     vn_img  [64-channel half][value | residual][8 strips of 8 tokens][64 rows x 16 bytes]      = 32 KB
+//     s_img   [32-channel quarter][value | residual][16 strips of 8 key dims][32 rows x 16 bytes]   = 64 KB
+//     vn_img  [32-channel quarter][value | residual][8 strips of 8 tokens][32 rows x 16 bytes]      = 32 KB
 //
 // Long chains may be split into segments (scan_segments.cuh): the kernel then also runs as the state-only pass that gives each
 // segment's M and H.
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
     //         fp32 copy as accumulator
     {
       const float dl = f.dl;
-      uint8_t* s_row = kSave ? reinterpret_cast<uint8_t*>(p.s_img + cidx * 32768) + (vrow >> 6) * 32768 + (vrow & 63) * 16 : nullptr;
+      uint8_t* s_row = kSave ? reinterpret_cast<uint8_t*>(p.s_img + cidx * 32768) + quad * 16384 + lane * 16 : nullptr;
 #pragma unroll 1
       for (int g4 = 0; g4 < kFwdKT / 16; ++g4) {         // 16 key dims at a time: 8 packed columns per operand store
         float s16[16];
@@ -382,11 +382,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
         tmem_st8u(tlane + tSAh + cs * (kFwdKT / 2) + g4 * 8, hi);
         tmem_st8u(tlane + tSAl + cs * (kFwdKT / 2) + g4 * 8, lo);
         if (kSave) {   // strips k_lo / 8 + g4 * 2 and the next one of my channel's row
-          uint8_t* dst = s_row + (cs * (kFwdKT / 8) + g4 * 2) * 1024;
+          uint8_t* dst = s_row + (cs * (kFwdKT / 8) + g4 * 2) * 512;
           *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(dst + 1024) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
-          *reinterpret_cast<uint4*>(dst + 16384) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          *reinterpret_cast<uint4*>(dst + 16384 + 1024) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+          *reinterpret_cast<uint4*>(dst + 512) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+          *reinterpret_cast<uint4*>(dst + 8192) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          *reinterpret_cast<uint4*>(dst + 8192 + 512) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) s16[i] *= dl;
@@ -462,11 +462,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
           tmem_st8u(tlane + tZAl + cs * (kFwdTT / 2) + g * 8, lo);
         }
         if (kSave) {                                 // v_new image: strips t_lo / 8 + g * 2 and the next one
-          uint8_t* dst = reinterpret_cast<uint8_t*>(p.vn_img + cidx * 16384) + (vrow >> 6) * 16384 + (cs * (kFwdTT / 8) + g * 2) * 1024 + (vrow & 63) * 16;
+          uint8_t* dst = reinterpret_cast<uint8_t*>(p.vn_img + cidx * 16384) + quad * 8192 + (cs * (kFwdTT / 8) + g * 2) * 512 + lane * 16;
           *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(dst + 1024) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
-          *reinterpret_cast<uint4*>(dst + 8192) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          *reinterpret_cast<uint4*>(dst + 8192 + 1024) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+          *reinterpret_cast<uint4*>(dst + 512) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+          *reinterpret_cast<uint4*>(dst + 4096) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          *reinterpret_cast<uint4*>(dst + 4096 + 512) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
         }
 #pragma unroll
         for (int i4 = 0; i4 < 16; i4 += 4) {

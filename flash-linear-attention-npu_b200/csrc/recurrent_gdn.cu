@@ -15,6 +15,7 @@
 #include "fla_b200_internal.h"
 #include "kernel_timer.h"
 #include "common/pdl.cuh"
+#include "common/sm100.cuh"
 
 namespace fla {
 

@@ -57,6 +57,29 @@ def test_value_dim_256(B, T, HK, HV, cu):
         assert_close(name, got, ref[name], TOL)
 
 
+@pytest.mark.parametrize("B,T,HK,HV,norm", [(9, 1090, 1, 1, False), (9, 1090, 1, 3, True), (4, 129, 37, 37, True)])
+def test_more_tiles_than_sms(B, T, HK, HV, norm):
+    """The chunk-parallel kernel's CTAs take several (chunk, q/k head) tiles each, of one or three value heads, ragged ones among them."""
+    from fla_b200.ops import chunk_gated_delta_rule
+    ref, d = _ref_and_inputs(B, T, HK, HV, seed=2500 + HV)
+    if norm:      # rows of another length: the operator's own normalisation, whose gradient is orthogonal to the row
+        d["q"], d["k"] = 2 * d["q"], 2 * d["k"]
+    wrt = [d[n].requires_grad_() for n in ("q", "k", "v", "g", "beta", "h0")]
+    o, ht = chunk_gated_delta_rule(*wrt[:5], initial_state=wrt[5], output_final_state=True, use_qk_l2norm_in_kernel=norm,
+                                   output_dtype=torch.float32)
+    grads = dict(zip(NAMES + ("dh0",), torch.autograd.grad([o, ht], wrt, [d["do"].float(), d["dht"]])))
+    if norm:
+        for n, x in (("dq", d["q"]), ("dk", d["k"])):
+            x = torch.nn.functional.normalize(x.detach().double().cpu(), dim=-1)
+            ref[n] = (ref[n] - x * (x * ref[n]).sum(-1, keepdim=True)) / 2
+    for name in ("dv", "dg", "dbeta", "dh0") + (() if norm else ("dq", "dk")):
+        assert_close(name, grads[name], ref[name], TOL, stored_bf16=grads[name].dtype == torch.bfloat16)
+    if norm:      # the projection leaves bf16 rows of a norm near one: compare as vectors
+        for name in ("dq", "dk"):
+            g, r = grads[name].double().cpu(), ref[name]
+            assert ((g - r).norm() / r.norm()).item() < 2e-2, name
+
+
 @pytest.mark.parametrize("T", [1, 17, 63, 65, 130])
 def test_backward_ragged_lengths(T):
     from fla_b200.ops import chunk_gated_delta_rule_fwd_bwd
