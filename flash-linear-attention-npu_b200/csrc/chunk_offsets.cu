@@ -5,8 +5,15 @@
 namespace fla {
 
 // One warp walks the sequences 32 at a time: N is a batch of sequences (tens to a few thousand), so this is latency, not work.
-__global__ void chunk_offsets_kernel(const int32_t* cu, int32_t* co, int n) {
+// host (optional): pinned host memory that receives the boundaries in [1, n + 1] and then, in [0], `tag`.
+__global__ void chunk_offsets_kernel(const int32_t* cu, int32_t* co, int n, int32_t* host, int32_t tag) {
   const int lane = threadIdx.x;
+  if (host) {
+    for (int i = lane; i <= n; i += 32) host[1 + i] = cu[i];
+    __threadfence_system();
+    __syncwarp();
+    if (lane == 0) *const_cast<volatile int32_t*>(host) = tag;
+  }
   int base = 0;
   if (lane == 0) co[0] = 0;
   for (int i0 = 0; i0 < n; i0 += 32) {
@@ -25,6 +32,10 @@ __global__ void chunk_offsets_kernel(const int32_t* cu, int32_t* co, int n) {
 }  // namespace fla
 
 extern "C" FLA_API int fla_b200_chunk_offsets(const fla_tensor_t* cu, const fla_tensor_t* co, void* stream) {
+  return fla_b200_chunk_bounds(cu, co, nullptr, 0, stream);
+}
+
+extern "C" FLA_API int fla_b200_chunk_bounds(const fla_tensor_t* cu, const fla_tensor_t* co, int32_t* host, int32_t tag, void* stream) {
   if (!cu || !co || !cu->data || !co->data) return FLA_ERR_NULL;
   for (const fla_tensor_t* t : {cu, co}) {
     if (t->dtype != FLA_I32) return FLA_ERR_DTYPE;
@@ -32,6 +43,6 @@ extern "C" FLA_API int fla_b200_chunk_offsets(const fla_tensor_t* cu, const fla_
     if (t->stride[0] != 1) return FLA_ERR_LAYOUT;
   }
   fla::chunk_offsets_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const int32_t*>(cu->data),
-                                                                             static_cast<int32_t*>(co->data), int(cu->shape[0] - 1));
+                                                                             static_cast<int32_t*>(co->data), int(cu->shape[0] - 1), host, tag);
   return fla::cuda_status(cudaGetLastError());
 }

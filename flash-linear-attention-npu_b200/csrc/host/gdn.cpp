@@ -9,9 +9,44 @@ using torch::autograd::variable_list;
 
 static Tensor state_f32(const Tensor& t) { return t.defined() ? t.to(at::kFloat).contiguous() : t; }
 
+struct GdnShape {
+  int64_t B, T, HK, HV, K, V, tiles, seg_bytes;
+};
+static at::ScalarType piece_type(int i) { return i == GdnSaved::kGam || i >= GdnSaved::kQr ? at::kFloat : at::kBFloat16; }
+static fla_tensor_t gdn_desc(const GdnShape& s, int i, void* data) {
+  const at::ScalarType t = piece_type(i);
+  switch (i) {
+    case GdnSaved::kGam: return desc_at(data, t, {s.B, s.T, s.HV});
+    case GdnSaved::kX: return desc_at(data, t, {s.tiles * 8192});                          // (I + A)^-1 per chunk: value + residual strips
+    case GdnSaved::kS: return desc_at(data, t, {s.tiles * (s.V / 64) * 16384});
+    case GdnSaved::kVn: return desc_at(data, t, {s.tiles * (s.V / 64) * 8192});
+    case GdnSaved::kP: return desc_at(data, t, {s.tiles * 8768});                          // P tile (16 KB) + the chunk's factor record
+    case GdnSaved::kSegM: return desc_at(data, t, {s.seg_bytes / 2});
+    case GdnSaved::kQn: case GdnSaved::kKn: return desc_at(data, t, {s.B, s.T, s.HK, s.K});
+    default: return desc_at(data, t, {s.B, s.T, s.HK});
+  }
+}
+// Bytes of the pieces this call has, 0: absent.
+static std::array<int64_t, GdnSaved::kPieces> piece_bytes(const GdnShape& s, bool save, bool l2norm) {
+  std::array<int64_t, GdnSaved::kPieces> r{};
+  for (int i = 0; i < GdnSaved::kPieces; ++i) {
+    if ((i == GdnSaved::kS || i == GdnSaved::kVn || i == GdnSaved::kP) && !save) continue;
+    if (i >= GdnSaved::kQn && !l2norm) continue;
+    const fla_tensor_t d = gdn_desc(s, i, nullptr);
+    int64_t n = d.dtype == FLA_F32 ? 4 : 2;
+    for (int j = 0; j < d.ndim; ++j) n *= d.shape[j];
+    r[i] = n;
+  }
+  return r;
+}
+static fla_tensor_t& piece_desc(fla_gdn_chunk_fwd_args& a, int i) {
+  fla_tensor_t* const p[] = {&a.gam, &a.x_inv, &a.s_img, &a.vn_img, &a.p_img, &a.seg_m, &a.q_norm, &a.k_norm, &a.q_rstd, &a.k_rstd};
+  return *p[i];
+}
+
 std::tuple<Tensor, Tensor, GdnSaved> gdn_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, double scale,
                                              const Tensor& h0_, bool want_final, const Tensor& cu, bool save, std::optional<at::ScalarType> out,
-                                             bool l2norm) {
+                                             bool l2norm, bool one) {
   const char* op = "chunk_gated_delta_rule";
   for (auto& [name, t] : {std::pair<const char*, const Tensor&>{"q", q_}, {"k", k_}, {"v", v_}})
     TORCH_CHECK_TYPE(t.scalar_type() == at::kBFloat16, op, ": ", name, " must be bfloat16 (fp32 inputs are rejected like in the reference), got ", t.scalar_type());
@@ -34,53 +69,70 @@ std::tuple<Tensor, Tensor, GdnSaved> gdn_fwd(const Tensor& q_, const Tensor& k_,
   const Tensor h0 = state_f32(h0_);
   Tensor o = empty({B, T, HV, V}, out.value_or(q.scalar_type()), d), ht;
   if (want_final) ht = empty({N, HV, K, V}, at::kFloat, d);
-  s.gam = empty({B, T, HV}, at::kFloat, d);
-  s.x_inv = empty({tiles * 8192}, at::kBFloat16, d);      // (I + A)^-1 per chunk: value + residual strips
-  if (save) {
-    s.s_img = empty({tiles * (V / 64) * 16384}, at::kBFloat16, d);
-    s.vn_img = empty({tiles * (V / 64) * 8192}, at::kBFloat16, d);
-    s.p_img = empty({tiles * 8768}, at::kBFloat16, d);    // P tile (16 KB) + the chunk's factor record
-  }
-  if (l2norm) {
-    s.qn = empty({B, T, HK, K}, at::kBFloat16, d), s.kn = empty({B, T, HK, K}, at::kBFloat16, d);
-    s.q_rstd = empty({B, T, HK}, at::kFloat, d), s.k_rstd = empty({B, T, HK}, at::kFloat, d);
-  }
   fla_gdn_chunk_fwd_args a{};
-  a.q_norm = desc(s.qn), a.k_norm = desc(s.kn), a.q_rstd = desc(s.q_rstd), a.k_rstd = desc(s.k_rstd);
   a.q = desc(q), a.k = desc(k), a.v = desc(v), a.g = desc(g), a.beta = desc(beta);
   a.initial_state = desc(h0), a.o = desc(o), a.final_state = desc(ht);
-  a.gam = desc(s.gam), a.x_inv = desc(s.x_inv), a.s_img = desc(s.s_img), a.vn_img = desc(s.vn_img), a.p_img = desc(s.p_img);
   a.cu_seqlens = desc(s.geo.cu), a.chunk_offsets = desc(s.geo.co);
   a.scale = float(scale), a.chunk_size = kChunk, a.max_seqlen = int32_t(s.geo.max_len), a.total_chunks = int32_t(s.geo.chunks);
-  if (save) {
-    uint64_t bytes = 0;
-    c10::cuda::CUDAGuard guard(d);
-    ok_or_throw("gdn_chunk_segments_size", lib.gdn_chunk_segments_size(&a, &bytes));
-    if (bytes) s.seg_m = empty({int64_t(bytes / 2)}, at::kBFloat16, d);
-    a.seg_m = desc(s.seg_m);
+  c10::cuda::CUDAGuard guard(d);
+  uint64_t seg_bytes = 0;
+  if (save) ok_or_throw("gdn_chunk_segments_size", lib.gdn_chunk_segments_size(&a, &seg_bytes));
+  GdnShape shape{B, T, HK, HV, K, V, tiles, int64_t(seg_bytes)};
+  const auto bytes = piece_bytes(shape, save, l2norm);
+  int64_t total = 0;
+  for (int i = 0; i < GdnSaved::kPieces; ++i) {
+    s.at[i] = bytes[i] ? total : -1;
+    total += (bytes[i] + 255) / 256 * 256;
+    if (bytes[i] && !one) {
+      const fla_tensor_t t = gdn_desc(shape, i, nullptr);
+      s.piece[i] = empty(at::IntArrayRef(t.shape, t.ndim), piece_type(i), d);
+    }
   }
-  two_phase("gdn_chunk_fwd", lib.gdn_chunk_fwd_workspace_size, lib.gdn_chunk_fwd, a, d, true);
+  // inference keeps nothing: the workspace goes into the same allocation
+  uint64_t ws_bytes = 0;
+  const bool ws_inside = one && !save;
+  if (one) {
+    for (int i = 0; i < GdnSaved::kPieces; ++i)
+      if (bytes[i]) piece_desc(a, i) = gdn_desc(shape, i, reinterpret_cast<void*>(uintptr_t(256)));      // (for the query: what is there)
+    if (ws_inside) ok_or_throw("gdn_chunk_fwd workspace query", lib.gdn_chunk_fwd_workspace_size(&a, &ws_bytes));
+    s.slab = empty({total + int64_t(ws_bytes)}, at::kByte, d);
+  }
+  for (int i = 0; i < GdnSaved::kPieces; ++i)
+    if (bytes[i]) piece_desc(a, i) = one ? gdn_desc(shape, i, static_cast<char*>(s.slab.data_ptr()) + s.at[i]) : desc(s.piece[i]);
+  if (ws_inside) {
+    ok_or_throw("gdn_chunk_fwd", lib.gdn_chunk_fwd(&a, static_cast<char*>(s.slab.data_ptr()) + total, ws_bytes, current_stream(d)));
+    if (check_status) raise_device_status("gdn_chunk_fwd", s.slab.narrow(0, total, int64_t(ws_bytes)));
+  } else {
+    two_phase("gdn_chunk_fwd", lib.gdn_chunk_fwd_workspace_size, lib.gdn_chunk_fwd, a, d, true);
+  }
   return {o, ht, s};
 }
 
 std::vector<Tensor> gdn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const GdnSaved& s, const Tensor& do_in,
                             const Tensor& dht_in, double scale, bool want_dh0, GradTypes ty) {
   const char* op = "chunk_gated_delta_rule_bwd";
-  const int64_t B = q.size(0), T = q.size(1), HK = q.size(2), K = q.size(3), HV = v.size(2), V = v.size(3);
+  const int64_t B = v.size(0), T = v.size(1), HK = q.defined() ? q.size(2) : s.hk, K = 128, HV = v.size(2), V = v.size(3);
   const at::Device d = Device("gdn_chunk_bwd")(q)(k)(v)(beta)(do_in)(dht_in).get();
   const Tensor d_o = as_rows(do_in.scalar_type() == at::kBFloat16 ? do_in : convert(do_in, at::kBFloat16, op));
   const std::array<int64_t, 4> os{B, T, HV, V}, hs{s.geo.N, HV, K, V};
   TORCH_CHECK(d_o.sizes() == at::IntArrayRef(os), op, ": do must be ", at::IntArrayRef(os), ", got ", d_o.sizes());
-  TORCH_CHECK(s.s_img.defined(), op, ": the forward was not run with save_for_backward=True");
+  TORCH_CHECK(s.slab.defined() || s.piece[GdnSaved::kS].defined(), op, ": the forward was not run with save_for_backward=True");
   if (dht_in.defined()) TORCH_CHECK(dht_in.sizes() == at::IntArrayRef(hs), op, ": dht must be ", at::IntArrayRef(hs), ", got ", dht_in.sizes());
   const Tensor dht = state_f32(dht_in);
   Tensor dq = empty({B, T, HK, K}, ty.q, d), dk = empty({B, T, HK, K}, ty.k, d), dv = empty(os, ty.v, d), dg = empty({B, T, HV}, ty.g, d),
          dbeta = empty({B, T, HV}, ty.beta, d), dh0;
   if (want_dh0) dh0 = empty(hs, at::kFloat, d);
   fla_gdn_chunk_bwd_args a{};
-  a.q_rstd = desc(s.q_rstd), a.k_rstd = desc(s.k_rstd), a.seg_m = desc(s.seg_m);
-  a.q = desc(q), a.k = desc(k), a.v = desc(v), a.beta = desc(beta);
-  a.gam = desc(s.gam), a.x_inv = desc(s.x_inv), a.s_img = desc(s.s_img), a.vn_img = desc(s.vn_img), a.p_img = desc(s.p_img);
+  const int64_t seg_end = s.at[GdnSaved::kQn] >= 0 ? s.at[GdnSaved::kQn] : s.slab.defined() ? s.slab.numel() : 0;
+  const GdnShape shape{B, T, HK, HV, K, V, s.geo.chunks * HV, s.slab.defined() && s.at[GdnSaved::kSegM] >= 0 ? seg_end - s.at[GdnSaved::kSegM] : 0};
+  auto piece = [&](GdnSaved::Piece i) {
+    if (!s.slab.defined()) return desc(s.piece[i]);
+    return s.at[i] < 0 ? fla_tensor_t{} : gdn_desc(shape, i, static_cast<char*>(s.slab.data_ptr()) + s.at[i]);
+  };
+  a.q_rstd = piece(GdnSaved::kQr), a.k_rstd = piece(GdnSaved::kKr), a.seg_m = piece(GdnSaved::kSegM);
+  const bool normed = s.slab.defined() && s.at[GdnSaved::kQn] >= 0;      // the kernels go on with the normalised rows
+  a.q = normed ? piece(GdnSaved::kQn) : desc(q), a.k = normed ? piece(GdnSaved::kKn) : desc(k), a.v = desc(v), a.beta = desc(beta);
+  a.gam = piece(GdnSaved::kGam), a.x_inv = piece(GdnSaved::kX), a.s_img = piece(GdnSaved::kS), a.vn_img = piece(GdnSaved::kVn), a.p_img = piece(GdnSaved::kP);
   a.d_o = desc(d_o), a.dht = desc(dht);
   a.dq = desc(dq), a.dk = desc(dk), a.dv = desc(dv), a.dg = desc(dg), a.dbeta = desc(dbeta), a.dh0 = desc(dh0);
   a.cu_seqlens = desc(s.geo.cu), a.chunk_offsets = desc(s.geo.co);
@@ -135,12 +187,14 @@ struct GdnFn : torch::autograd::Function<GdnFn> {
     const Tensor h0 = value(h0_), cu = value(cu_);
     const GdnInputs in = gdn_inputs(q, k, v, g, beta, h0, cu);
     auto [o, ht, s] = gdn_fwd(in.q, in.k, in.v, in.g, in.beta, scale, in.h0, want_final, cu, true,
-                              out < 0 ? std::nullopt : std::optional<at::ScalarType>(at::ScalarType(out)), l2norm);
+                              out < 0 ? std::nullopt : std::optional<at::ScalarType>(at::ScalarType(out)), l2norm, true);
     if (in.folded) std::tie(o, ht) = unfold_outputs(o, ht, q.size(0));
-    ctx->save_for_backward({l2norm ? s.qn : in.q, l2norm ? s.kn : in.k, in.v, in.beta, s.gam, s.x_inv, s.s_img, s.vn_img, s.p_img, s.q_rstd,
-                            s.k_rstd, s.geo.cu, s.geo.co, s.seg_m});
+    // with the normalisation in the operator the slab has the rows the backward works on
+    ctx->save_for_backward({l2norm ? Tensor() : in.q, l2norm ? Tensor() : in.k, in.v, in.beta, s.slab, s.geo.cu, s.geo.co});
     auto& m = ctx->saved_data;
-    m["geo"] = std::vector<int64_t>{s.geo.N, s.geo.max_len, s.geo.chunks};
+    std::vector<int64_t> geo{s.geo.N, s.geo.max_len, s.geo.chunks, in.q.size(2)};
+    geo.insert(geo.end(), s.at.begin(), s.at.end());
+    m["geo"] = std::move(geo);
     m["types"] = std::vector<int64_t>{int64_t(q.scalar_type()), int64_t(k.scalar_type()), int64_t(v.scalar_type()), int64_t(g.scalar_type()),
                                       int64_t(beta.scalar_type())};
     m["fold"] = in.folded ? q.size(0) : int64_t(0);
@@ -154,7 +208,11 @@ struct GdnFn : torch::autograd::Function<GdnFn> {
     const variable_list sv = ctx->get_saved_variables();
     auto& m = ctx->saved_data;
     const std::vector<int64_t> geo = m["geo"].toIntVector(), ty = m["types"].toIntVector();
-    GdnSaved s{sv[4], sv[5], sv[6], sv[7], sv[8], sv[13], Tensor(), Tensor(), sv[9], sv[10], Geometry{sv[11], sv[12], geo[0], geo[1], geo[2]}};
+    GdnSaved s;
+    s.slab = sv[4];
+    s.geo = Geometry{sv[5], sv[6], geo[0], geo[1], geo[2]};
+    s.hk = geo[3];
+    std::copy(geo.begin() + 4, geo.end(), s.at.begin());
     const int64_t B = m["fold"].toInt();
     Tensor d_o = grads[0].defined() ? grads[0] : at::zeros(m["o"].toIntVector(), sv[2].options());
     Tensor dht = grads.size() > 1 ? grads[1] : Tensor();
@@ -201,7 +259,7 @@ Pair gdn(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_,
   } else {
     Device(op)(q)(k)(v).get();
     const GdnInputs in = gdn_inputs(q, k, v, g, beta, h0, cu);
-    auto [o, ht, s] = gdn_fwd(in.q, in.k, in.v, in.g, in.beta, scale, in.h0, want_final, cu, false, inner, l2norm);
+    auto [o, ht, s] = gdn_fwd(in.q, in.k, in.v, in.g, in.beta, scale, in.h0, want_final, cu, false, inner, l2norm, true);
     r = in.folded ? unfold_outputs(o, ht, q.size(0)) : Pair{o, ht};
   }
   if (half) r.first = to_dtype(r.first, out.value_or(at::kHalf), op);

@@ -204,13 +204,16 @@ FLA_PY(py_gdn_fwd, 11) {
   const bool fin = a.flag();
   const Tensor cu = a.boundaries();
   const bool save = a.flag();
-  auto [o, ht, s] = gdn_fwd(q, k, v, g, beta, scale, h0, fin, cu, save, a.dtype());
-  return pack({wrap(o), wrap(ht), wrap(s.gam), wrap(s.x_inv), wrap(s.s_img), wrap(s.vn_img), wrap(s.p_img), wrap(s.seg_m), geometry_items(s.geo)});
+  auto [o, ht, s] = gdn_fwd(q, k, v, g, beta, scale, h0, fin, cu, save, a.dtype(), false, false);
+  const Tensor* t = s.piece;
+  return pack({wrap(o), wrap(ht), wrap(t[GdnSaved::kGam]), wrap(t[GdnSaved::kX]), wrap(t[GdnSaved::kS]), wrap(t[GdnSaved::kVn]), wrap(t[GdnSaved::kP]),
+               wrap(t[GdnSaved::kSegM]), geometry_items(s.geo)});
 }
 FLA_PY(py_gdn_bwd, 24) {
   const Tensor q = a.tensor(), k = a.tensor(), v = a.tensor(), beta = a.tensor();
   GdnSaved s;
-  s.gam = a.tensor(), s.x_inv = a.tensor(), s.s_img = a.tensor(), s.vn_img = a.tensor(), s.p_img = a.tensor(), s.seg_m = a.tensor();
+  for (int i = GdnSaved::kGam; i <= GdnSaved::kSegM; ++i) s.piece[i] = a.tensor();
+  s.at.fill(-1);
   s.geo = geometry_of(a);
   const Tensor d_o = a.tensor(), dht = a.tensor();
   const double scale = a.number();

@@ -1,6 +1,8 @@
 #include "runtime.h"
 #include <ATen/cuda/CUDAContext.h>
 #include <Python.h>
+#include <c10/cuda/CUDAException.h>
+#include <vector>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -93,9 +95,46 @@ Tensor to_dtype(const Tensor& t, at::ScalarType dtype, const char* op) {
   return ConvertFn::apply(t, int64_t(dtype), op);
 }
 
+// Boundaries that are on the device, read back by the kernel that makes the chunk offsets: it writes them into pinned memory, where this
+// thread polls for the tag of the call.  A copy into pageable memory and the offsets' launch behind it took 12 us more per packed call, all of
+// it with an idle device.  False where the plain copy has to do (a captured stream, whose copy reports the error; very many sequences).
+static bool read_bounds(const char* op, const Tensor& cu, const Tensor& co, at::Device d, std::vector<int32_t>& out) {
+  struct Pinned {
+    int32_t* p = nullptr;
+    int32_t tag = 0;
+  };
+  constexpr int64_t kMost = 4095;
+  thread_local Pinned pin;      // (lives as long as the process: CUDA may be gone when a thread ends)
+  const int64_t n = cu.numel();
+  if (n < 2 || n > kMost) return false;
+  c10::cuda::CUDAGuard guard(d);
+  const cudaStream_t stream = static_cast<cudaStream_t>(current_stream(d));
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+  if (!pin.p) {
+    if (cudaHostAlloc(reinterpret_cast<void**>(&pin.p), (kMost + 1) * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      pin.p = nullptr;
+      return false;
+    }
+    pin.p[0] = 0;
+  }
+  pin.tag = pin.tag == 0x7fffffff ? 1 : pin.tag + 1;
+  const fla_tensor_t a = desc(cu), b = desc(co);
+  ok_or_throw(op, lib.chunk_bounds(&a, &b, pin.p, pin.tag, stream));
+  for (uint32_t spin = 0; __atomic_load_n(pin.p, __ATOMIC_ACQUIRE) != pin.tag; ++spin) {
+    if ((spin & 0xfff) != 0xfff) continue;
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) continue;
+    C10_CUDA_CHECK(e);
+    TORCH_CHECK(__atomic_load_n(pin.p, __ATOMIC_ACQUIRE) == pin.tag, op, ": the sequence boundaries did not arrive");
+  }
+  out.assign(pin.p + 1, pin.p + 1 + n);
+  return true;
+}
+
 // Packed batches: the kernels' grids and the sizes of the saved tensors follow from the lengths, so the boundaries have to be
-// known on the host.  A device tensor is read back once (its stream is waited for); the chunk offsets are then made on the
-// device from the boundaries that are already there, instead of two copies from pageable host memory.
+// known on the host.  A device tensor is read back once (its stream is waited for); the chunk offsets are made on the
+// device from the boundaries that are already there.
 Geometry geometry(const char* op, int64_t B, int64_t T, const Tensor& cu_seqlens, at::Device d) {
   Geometry geo;
   if (!cu_seqlens.defined()) {
@@ -106,18 +145,23 @@ Geometry geometry(const char* op, int64_t B, int64_t T, const Tensor& cu_seqlens
   }
   TORCH_CHECK(B == 1, op, ": cu_seqlens requires batch size 1 (packed sequences)");
   Tensor host;
+  std::vector<int32_t> bounds;
+  if (cu_seqlens.device() == d && cu_seqlens.dim() == 1) {
+    geo.cu = cu_seqlens.to(at::kInt).contiguous();
+    geo.co = empty({cu_seqlens.numel()}, at::kInt, d);
+  }
   {
     PyThreadState* ts = PyGILState_Check() ? PyEval_SaveThread() : nullptr;
     try {
-      host = cu_seqlens.to(at::kCPU, at::kInt).contiguous();
+      if (!geo.co.defined() || !read_bounds(op, geo.cu, geo.co, d, bounds)) host = cu_seqlens.to(at::kCPU, at::kInt).contiguous();
     } catch (...) {
       if (ts) PyEval_RestoreThread(ts);
       throw;
     }
     if (ts) PyEval_RestoreThread(ts);
   }
-  const int32_t* cu = host.data_ptr<int32_t>();
-  const int64_t n = host.numel();
+  const int32_t* cu = host.defined() ? host.data_ptr<int32_t>() : bounds.data();
+  const int64_t n = host.defined() ? host.numel() : int64_t(bounds.size());
   bool fine = n >= 2 && cu[0] == 0;
   for (int64_t i = 0; fine && i + 1 < n; ++i) fine = cu[i + 1] >= cu[i];
   TORCH_CHECK(fine, "cu_seqlens must start at 0 and be non-decreasing, got ", std::vector<int64_t>(cu, cu + n));
@@ -128,8 +172,11 @@ Geometry geometry(const char* op, int64_t B, int64_t T, const Tensor& cu_seqlens
     geo.chunks += (len + kChunk - 1) / kChunk;
   }
   TORCH_CHECK(cu[n - 1] == T, op, ": cu_seqlens[-1]=", cu[n - 1], " must equal T=", T);
-  geo.cu = cu_seqlens.device() == d ? cu_seqlens.to(at::kInt).contiguous() : host.to(d);
-  geo.co = empty({n}, at::kInt, d);
+  if (!host.defined()) return geo;
+  if (!geo.co.defined()) {
+    geo.cu = host.to(d);
+    geo.co = empty({n}, at::kInt, d);
+  }
   const fla_tensor_t a = desc(geo.cu), b = desc(geo.co);
   one_phase(op, d, lib.chunk_offsets, &a, &b);
   return geo;

@@ -22,7 +22,7 @@ using at::Tensor;
   X(causal_conv1d_bwd_workspace_size) X(causal_conv1d_bwd) X(causal_conv1d_update_workspace_size) X(causal_conv1d_update)  \
   X(gdn_chunk_fwd_workspace_size) X(gdn_chunk_segments_size) X(gdn_chunk_fwd) X(gdn_chunk_bwd_workspace_size) X(gdn_chunk_bwd)                        \
   X(kda_chunk_fwd_workspace_size) X(kda_chunk_fwd) X(kda_chunk_bwd_workspace_size) X(kda_chunk_bwd) X(kda_chunk_saved_size) \
-  X(l2norm_fwd) X(l2norm_bwd) X(convert) X(chunk_offsets)
+  X(l2norm_fwd) X(l2norm_bwd) X(convert) X(chunk_offsets) X(chunk_bounds)
 struct Library {
 #define FLA_DECL(n) decltype(&fla_b200_##n) n = nullptr;
   FLA_HOST_FNS(FLA_DECL)
@@ -49,6 +49,21 @@ inline fla_tensor_t desc(const Tensor& t, const char* name = "tensor") {
   for (int i = 0; i < d.ndim; ++i) {
     d.shape[i] = t.size(i);
     d.stride[i] = t.stride(i);
+  }
+  return d;
+}
+
+// A dense tensor that is part of a larger allocation.
+inline fla_tensor_t desc_at(void* data, at::ScalarType t, std::initializer_list<int64_t> sizes) {
+  fla_tensor_t d{};
+  d.data = data;
+  d.dtype = dtype_code(t, "tensor");
+  d.ndim = int32_t(sizes.size());
+  int64_t stride = 1;
+  for (int i = d.ndim - 1; i >= 0; --i) {
+    d.shape[i] = sizes.begin()[i];
+    d.stride[i] = stride;
+    stride *= d.shape[i];
   }
   return d;
 }
@@ -150,14 +165,18 @@ Pair recurrent_kda(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
                    const Tensor& indices, const Tensor& a_log, const Tensor& dt_bias, const Tensor& accepted, double scale, bool inplace,
                    bool l2norm, int64_t gate_mode, int64_t beta_mode, double lower_bound, bool v_first, int64_t seq_num);
 
+// What the GDN forward leaves for its backward.  The operators keep all of it in one allocation (`slab`): a dozen small tensors cost the
+// host more than the launches of a short prompt.  Callers that want the tensors themselves get them one by one.
 struct GdnSaved {
-  Tensor gam, x_inv, s_img, vn_img, p_img;
-  Tensor seg_m;                       // transition matrices of split chains
-  Tensor qn, kn, q_rstd, k_rstd;      // normalised rows and their factors, when the operator normalises q and k
+  enum Piece { kGam, kX, kS, kVn, kP, kSegM, kQn, kKn, kQr, kKr, kPieces };      // kSegM: transition matrices of split chains
+  Tensor slab, piece[kPieces];
+  std::array<int64_t, kPieces> at{};      // byte offsets in the slab, -1: absent
+  int64_t hk = 0;                         // q/k heads
   Geometry geo;
 };
 std::tuple<Tensor, Tensor, GdnSaved> gdn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, double scale,
-                                             const Tensor& h0, bool want_final, const Tensor& cu, bool save, std::optional<at::ScalarType> out, bool l2norm = false);
+                                             const Tensor& h0, bool want_final, const Tensor& cu, bool save, std::optional<at::ScalarType> out, bool l2norm,
+                                             bool slab);
 struct GradTypes {
   at::ScalarType q, k, v, g, beta;
 };

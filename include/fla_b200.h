@@ -482,6 +482,9 @@ FLA_API int fla_b200_convert(const fla_tensor_t* src, const fla_tensor_t* dst, v
 /* Chunk bookkeeping of a packed batch on the device: chunk_offsets[n] = sum over i < n of ceil(length_i / 64), from the
  * sequence boundaries cu_seqlens (both int32 [N+1], dense).  Single-phase (no workspace). */
 FLA_API int fla_b200_chunk_offsets(const fla_tensor_t* cu_seqlens, const fla_tensor_t* chunk_offsets, void* stream);
+/* The same, and the boundaries themselves into pinned host memory: host[1 .. N+1] = cu_seqlens, then host[0] = tag.  A caller that polls
+ * host[0] has them a few microseconds after the work in front of the call is done, without a copy and a stream synchronisation. */
+FLA_API int fla_b200_chunk_bounds(const fla_tensor_t* cu_seqlens, const fla_tensor_t* chunk_offsets, int32_t* host, int32_t tag, void* stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Stand-alone stages of the chunked gated-delta-rule forward: one entry point per low-level reference operator,

@@ -101,6 +101,38 @@ def test_backward_varlen_packed_no_initial_state():
     assert grads[5] is None
 
 
+@pytest.mark.parametrize("N", [2, 33, 64, 65])
+def test_packed_batch_of_many_lengths(N):
+    """Whole chains start longest first (up to 64 sequences, two per lane): ties, empty sequences, and one sequence more."""
+    from fla_b200.ops import chunk_gated_delta_rule_fwd_bwd
+    gen = torch.Generator().manual_seed(N)
+    lens = torch.randint(0, 6, (N,), generator=gen) * 13
+    lens[N // 2] = 140
+    cu = [0] + lens.cumsum(0).tolist()
+    ref, d = _ref_and_inputs(1, cu[-1], 1, 2, seed=2600 + N, cu=cu)
+    o, ht, grads = chunk_gated_delta_rule_fwd_bwd(d["q"], d["k"], d["v"], d["g"], d["beta"], d["do"], initial_state=d["h0"], dht=d["dht"],
+                                                  output_dtype=torch.float32, grad_dtype=torch.float32,
+                                                  cu_seqlens=torch.tensor(cu, dtype=torch.int32, device="cuda"))
+    assert_close("o", o, ref["o"], TOL)
+    assert_close("ht", ht, ref["ht"], TOL)
+    for name, got in zip(NAMES + ("dh0",), grads):
+        assert_close(name, got, ref[name], TOL)
+
+
+@pytest.mark.parametrize("N", [4094, 4095])
+def test_boundaries_of_very_many_sequences(N):
+    """The boundaries of up to 4,094 sequences are read back by the kernel, of more by a copy."""
+    from fla_b200.ops import chunk_gated_delta_rule
+    inp = oracle.make_gdn_inputs(1, N, 1, 1, seed=27, with_grad=False)
+    d = {n: inp[n].cuda() for n in ("q", "k", "v", "g", "beta")}
+    cu = torch.arange(N + 1, device="cuda", dtype=torch.int64)
+    o, _ = chunk_gated_delta_rule(*d.values(), output_dtype=torch.float32, cu_seqlens=cu)
+    q, k, v, beta = (d[n].double() for n in ("q", "k", "v", "beta"))
+    assert_close("o", o, (128 ** -0.5 * (q * k).sum(-1, keepdim=True) * beta[..., None] * v).cpu(), TOL)
+    with pytest.raises(RuntimeError):
+        chunk_gated_delta_rule(*d.values(), cu_seqlens=cu.flip(0))
+
+
 def test_autograd_function_bf16_grads_and_determinism():
     from fla_b200.ops import chunk_gated_delta_rule
     ref, d = _ref_and_inputs(2, 192, 2, 4, seed=5)
