@@ -87,6 +87,8 @@ constexpr int kConvThreads = 128;
 template <int W, bool HAS_RES, bool SILU>
 __global__ void __launch_bounds__(kConvThreads, 4) conv_fwd_kernel(ConvFwdParams p) {
   constexpr int G = kConvGroup;
+  pdl_trigger();
+  pdl_wait();
   const int d0 = (blockIdx.x * kConvThreads + threadIdx.x) * 8;
   if (d0 >= p.D) return;
   const int b = blockIdx.z;
@@ -428,17 +430,13 @@ extern "C" FLA_API int fla_b200_causal_conv1d_fwd(const fla_causal_conv1d_fwd_ar
   const dim3 grid(unsigned(blocks_d), unsigned((T + p.tile - 1) / p.tile), unsigned(B));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   KernelTimer kt("causal_conv1d_fwd", st);
-#define FLA_LAUNCH_FWD(WW)                                                                           \
-  if (p.residual) {                                                                                  \
-    if (p.silu) conv_fwd_kernel<WW, true, true><<<grid, kConvThreads, 0, st>>>(p);                   \
-    else conv_fwd_kernel<WW, true, false><<<grid, kConvThreads, 0, st>>>(p);                         \
-  } else {                                                                                           \
-    if (p.silu) conv_fwd_kernel<WW, false, true><<<grid, kConvThreads, 0, st>>>(p);                  \
-    else conv_fwd_kernel<WW, false, false><<<grid, kConvThreads, 0, st>>>(p);                        \
-  }
+  void (*kernel)(ConvFwdParams) = nullptr;
+#define FLA_LAUNCH_FWD(WW)                                                                                  \
+  kernel = p.residual ? (p.silu ? conv_fwd_kernel<WW, true, true> : conv_fwd_kernel<WW, true, false>)       \
+                      : (p.silu ? conv_fwd_kernel<WW, false, true> : conv_fwd_kernel<WW, false, false>);
   if (W == 4) { FLA_LAUNCH_FWD(4) } else if (W == 3) { FLA_LAUNCH_FWD(3) } else { FLA_LAUNCH_FWD(2) }
 #undef FLA_LAUNCH_FWD
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_pdl(kernel, grid, dim3(kConvThreads), 0, st, p));
 }
 
 extern "C" FLA_API int fla_b200_causal_conv1d_update_workspace_size(const fla_causal_conv1d_update_args* a,

@@ -155,6 +155,8 @@ __global__ void __launch_bounds__(kParThreads, 1) gdn_bwd_par_kernel(GdnBwdParam
   __shared__ __align__(8) uint64_t pa_bar, acc_bar, free_bar;            // worker warps: [dP; dAt] there, accumulators read, q and k read
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  pdl_trigger();
+  pdl_wait();
   const int G = p.HV / p.HK;
   // chunks of this launch: fixed lengths count from the first chunk of sequence n0, a packed batch's half is cut out here
   int chunk0 = 0;
@@ -784,13 +786,16 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
     return FLA_ERR_CUDA;
   auto launch_scan = [&](const GdnBwdParams& pp, int64_t segments, cudaStream_t st) {
     const dim3 grid(unsigned(HV * (V / 128)), unsigned(segments));
-    if (plan.split) gdn_scan_bwd_kernel<true, true><<<grid, kScanThreads, kScanBwdSmem + 1024, st>>>(pp, tm_q, tm_k, tm_v, tm_d);
-    auto* scan = plan.split ? gdn_scan_bwd_kernel<false, true> : gdn_scan_bwd_kernel<false, false>;
-    scan<<<grid, kScanThreads, kScanBwdSmem + 1024, st>>>(pp, tm_q, tm_k, tm_v, tm_d);
+    if (plan.split) {
+      const cudaError_t e = launch_pdl(gdn_scan_bwd_kernel<true, true>, grid, kScanThreads, kScanBwdSmem + 1024, st, pp, tm_q, tm_k, tm_v, tm_d);
+      if (e != cudaSuccess) return e;
+    }
+    return launch_pdl(plan.split ? gdn_scan_bwd_kernel<false, true> : gdn_scan_bwd_kernel<false, false>, grid, kScanThreads, kScanBwdSmem + 1024, st, pp, tm_q,
+                      tm_k, tm_v, tm_d);
   };
   auto launch_par = [&](const GdnBwdParams& pp, int64_t chunks, cudaStream_t st) {
-    auto* par = nvb == 2 ? gdn_bwd_par_kernel<2> : gdn_bwd_par_kernel<4>;
-    par<<<unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads, kParSmem + 1024, st>>>(pp, int(chunks), tm_q, tm_k);
+    return launch_pdl(nvb == 2 ? gdn_bwd_par_kernel<2> : gdn_bwd_par_kernel<4>, unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads,
+                      kParSmem + 1024, st, pp, int(chunks), tm_q, tm_k);
   };
   // The reverse scan launches one CTA per (sequence, value head, 128 channels) and each needs a whole SM: when there are
   // more chains than SMs the last round leaves SMs idle for the length of a chain.  The batch is then launched as two
@@ -807,26 +812,23 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
     p2.counter = p.counter + 16;
     bool okc = cudaEventRecord(aux->fork, cs) == cudaSuccess && cudaStreamWaitEvent(aux->s, aux->fork, 0) == cudaSuccess;
     if (!okc) return FLA_ERR_CUDA;
-    launch_scan(p, n1, cs);
-    launch_scan(p2, N - n1, aux->s);
+    bool launched = launch_scan(p, n1, cs) == cudaSuccess && launch_scan(p2, N - n1, aux->s) == cudaSuccess;
     // a packed batch's halves hold chunk counts the host does not have: the kernel looks up its own
     const int64_t nt = (T + kC - 1) / kC;
-    launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs);
-    launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s);
+    launched = launched && launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs) == cudaSuccess &&
+               launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s) == cudaSuccess;
     okc = cudaEventRecord(aux->join, aux->s) == cudaSuccess && cudaStreamWaitEvent(cs, aux->join, 0) == cudaSuccess;
     if (!okc) return FLA_ERR_CUDA;
-    return cuda_status(cudaGetLastError());
+    return launched ? FLA_OK : FLA_ERR_CUDA;
   }
   {
     KernelTimer kt("gdn_bwd_dhu", cs);
-    launch_scan(p, plan.count, cs);
+    if (launch_scan(p, plan.count, cs) != cudaSuccess) return FLA_ERR_CUDA;
   }
-  if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
     KernelTimer kt("gdn_bwd_par", cs);
-    launch_par(p, total_chunks, cs);
+    return cuda_status(launch_par(p, total_chunks, cs));
   }
-  return cuda_status(cudaGetLastError());
 }
 
 extern "C" FLA_API int fla_b200_gdn_chunk_bwd(const fla_gdn_chunk_bwd_args* a, void* workspace, uint64_t workspace_bytes,

@@ -78,6 +78,8 @@ __global__ void __launch_bounds__(kPrepThreads, 4) gdn_prep_kernel(GdnFwdParams 
   __shared__ __align__(8) uint64_t bar;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  pdl_trigger();
+  pdl_wait();
   const int hk = blockIdx.y;
   const ChunkPos pos = chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, 0, blockIdx.x);
   const SeqInfo& sq = pos.sq;
@@ -448,9 +450,8 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   }
   {
     KernelTimer kt("gdn_prep", cs);
-    gdn_prep_kernel<<<dim3(unsigned(total_chunks), unsigned(HK)), kPrepThreads, prep_smem, cs>>>(p);
+    if (launch_pdl(gdn_prep_kernel, dim3(unsigned(total_chunks), unsigned(HK)), kPrepThreads, prep_smem, cs, p) != cudaSuccess) return FLA_ERR_CUDA;
   }
-  if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   CUtensorMap tm_q, tm_k;
   const uint64_t nst = uint64_t(HK) * kK;   // the normalised rows are dense
   if (p.qn ? (make_row_tile_map(&tm_q, p.qn, kK, uint64_t(HK), uint64_t(B * T), kK, nst) ||
@@ -463,13 +464,13 @@ extern "C" FLA_API int fla_b200_gdn_chunk_fwd(const fla_gdn_chunk_fwd_args* a, v
   {
     KernelTimer kt("gdn_fwd", cs);
     const unsigned heads = unsigned(HV * (V / 128));
-    if (plan.split)
-      gdn_scan_fwd_kernel<kScanState, true><<<dim3(heads, unsigned(plan.count), 2), kFwdThreads, kScanFwdSmem + 1024, cs>>>(p, tm_q, tm_k, tm_v);
+    if (plan.split && launch_pdl(gdn_scan_fwd_kernel<kScanState, true>, dim3(heads, unsigned(plan.count), 2), kFwdThreads, kScanFwdSmem + 1024, cs, p, tm_q,
+                                 tm_k, tm_v) != cudaSuccess)
+      return FLA_ERR_CUDA;
     auto* scan = plan.split ? (p.s_img ? gdn_scan_fwd_kernel<kScanSave, true> : gdn_scan_fwd_kernel<kScanInfer, true>)
                             : (p.s_img ? gdn_scan_fwd_kernel<kScanSave, false> : gdn_scan_fwd_kernel<kScanInfer, false>);
-    scan<<<dim3(heads, unsigned(plan.count)), kFwdThreads, kScanFwdSmem + 1024, cs>>>(p, tm_q, tm_k, tm_v);
+    return cuda_status(launch_pdl(scan, dim3(heads, unsigned(plan.count)), kFwdThreads, kScanFwdSmem + 1024, cs, p, tm_q, tm_k, tm_v));
   }
-  return cuda_status(cudaGetLastError());
 }
 
 

@@ -1,6 +1,7 @@
 // Shared pieces of the chunked GDN kernels: parameter block, sequence/chunk geometry and small
 // row-wise helpers for moving fp32 accumulator rows between TMEM, registers and operand panels.
 #pragma once
+#include "common/pdl.cuh"
 #include <cuda_fp16.h>
 #include "common/sm100.cuh"
 

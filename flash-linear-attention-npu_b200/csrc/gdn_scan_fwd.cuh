@@ -140,10 +140,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gdn_scan_fwd_kernel(GdnFwdPara
   constexpr bool kSave = kMode == kScanSave;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  pdl_trigger();
+  pdl_wait();
   const int seg = blockIdx.y, hv = blockIdx.x / (p.V / 128), vb = blockIdx.x % (p.V / 128);   // neighbours share q, k: heads first
   const int hk = hv / (p.HV / p.HK);
   SegPos pos;
-  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos)) return;
+  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos, 0, p.N)) return;
   const bool values = blockIdx.z == 0;                     // (state-only) H, from the values; else M, from the identity
   if (kMode == kScanState) {                               // H of every segment but the last, M of those between the first and the last
     if (pos.s + 1 == pos.ns || (!values && (pos.s == 0 || vb > 0))) return;

@@ -157,6 +157,8 @@ __global__ void __launch_bounds__(kParThreads, 1) kda_bwd_par_kernel(KdaBwdParam
   __shared__ __align__(8) uint64_t sds_bar, epi1_bar, epi2_bar, dg_bar;  // workers: step buffers read, [dP; dM] there, images and accumulators read, tiles read
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  pdl_trigger();
+  pdl_wait();
   const int G = p.HV / p.HK;
   // chunks of this launch: fixed lengths count from the first chunk of sequence n0, a packed batch's half is cut out here
   int chunk0 = 0;
@@ -737,14 +739,17 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
   if (make_row_tile_map_f32(&tm_gk, p.gk, kK, uint64_t(HV), uint64_t(B * T), uint64_t(kK), uint64_t(HV) * kK)) return FLA_ERR_CUDA;
   auto launch_scan = [&](const KdaBwdParams& pp, int64_t segments, cudaStream_t st_) {
     const dim3 grid(unsigned(HV * (V / 128)), unsigned(segments));
-    if (plan.split) kda_scan_bwd_kernel<true, true><<<grid, kScanThreads, kKdaScanBwdSmem + 1024, st_>>>(pp, tm_v, tm_d);
-    auto* scan = plan.split ? kda_scan_bwd_kernel<false, true> : kda_scan_bwd_kernel<false, false>;
-    scan<<<grid, kScanThreads, kKdaScanBwdSmem + 1024, st_>>>(pp, tm_v, tm_d);
+    if (plan.split) {
+      const cudaError_t e = launch_pdl(kda_scan_bwd_kernel<true, true>, grid, kScanThreads, kKdaScanBwdSmem + 1024, st_, pp, tm_v, tm_d);
+      if (e != cudaSuccess) return e;
+    }
+    return launch_pdl(plan.split ? kda_scan_bwd_kernel<false, true> : kda_scan_bwd_kernel<false, false>, grid, kScanThreads, kKdaScanBwdSmem + 1024, st_, pp,
+                      tm_v, tm_d);
   };
   auto launch_par = [&](const KdaBwdParams& pp, int64_t chunks, cudaStream_t st_) {
     auto* par = nvb == 2 ? (pp.q_rstd ? kda_bwd_par_kernel<2, true> : kda_bwd_par_kernel<2, false>)
                          : (pp.q_rstd ? kda_bwd_par_kernel<4, true> : kda_bwd_par_kernel<4, false>);
-    par<<<unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads, kKdaParSmem + 1024, st_>>>(pp, int(chunks), tm_gk);
+    return launch_pdl(par, unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads, kKdaParSmem + 1024, st_, pp, int(chunks), tm_gk);
   };
   // more scan chains (one CTA per SM each) than SMs: two halves of the batch on two streams, so that the chunk-parallel
   // kernel of the first half fills the SMs the second half's scan leaves idle (aux_stream.h)
@@ -757,24 +762,21 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
     p.n1 = p2.n0 = n1;
     p2.counter = p.counter + 16;
     if (cudaEventRecord(aux->fork, cs) != cudaSuccess || cudaStreamWaitEvent(aux->s, aux->fork, 0) != cudaSuccess) return FLA_ERR_CUDA;
-    launch_scan(p, n1, cs);
-    launch_scan(p2, N - n1, aux->s);
+    bool launched = launch_scan(p, n1, cs) == cudaSuccess && launch_scan(p2, N - n1, aux->s) == cudaSuccess;
     // a packed batch's halves hold chunk counts the host does not have: the kernel looks up its own
     const int64_t nt = (T + kC - 1) / kC;
-    launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs);
-    launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s);
+    launched = launched && launch_par(p, p.cu_seqlens ? total_chunks : n1 * nt, cs) == cudaSuccess &&
+               launch_par(p2, p.cu_seqlens ? total_chunks : (N - n1) * nt, aux->s) == cudaSuccess;
     if (cudaEventRecord(aux->join, aux->s) != cudaSuccess || cudaStreamWaitEvent(cs, aux->join, 0) != cudaSuccess) return FLA_ERR_CUDA;
-    return cuda_status(cudaGetLastError());
+    return launched ? FLA_OK : FLA_ERR_CUDA;
   }
   {
     KernelTimer kt("kda_bwd_dhu", cs);
-    launch_scan(p, plan.count, cs);
+    if (launch_scan(p, plan.count, cs) != cudaSuccess) return FLA_ERR_CUDA;
   }
-  if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
     KernelTimer kt("kda_bwd_par", cs);
-    launch_par(p, total_chunks, cs);
+    return cuda_status(launch_par(p, total_chunks, cs));
   }
-  return cuda_status(cudaGetLastError());
 }
 

@@ -64,6 +64,8 @@ __global__ void __launch_bounds__(kKdaPrepThreads, 2) kda_prep_kernel(KdaParams 
   __shared__ __align__(8) uint64_t bar, qk_bar;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  pdl_trigger();
+  pdl_wait();
   const int cg = tid & 15, r0 = cg * 8, tb = (tid >> 4) * 2;      // my channels and my first token
   const int quad = warp & 3, j0 = (warp >> 2) * 16, row = quad * 32 + lane, tok = row & 63;      // my 16 score columns of my row
   const int gva = p.HV / p.HK;
@@ -611,17 +613,17 @@ int fla::kda_launch_forward(const KdaParams& p, int64_t total_chunks, int64_t se
   {
     KernelTimer kt("kda_prep", cs);
     const unsigned tiles = unsigned(total_chunks) * unsigned(p.HV);
-    kda_prep_kernel<<<std::min(tiles, 2u * unsigned(current_sm_count())), kKdaPrepThreads, kKdaPrepSmem + 1024, cs>>>(p, tiles, tm_q, tm_k);
+    if (launch_pdl(kda_prep_kernel, std::min(tiles, 2u * unsigned(current_sm_count())), kKdaPrepThreads, kKdaPrepSmem + 1024, cs, p, tiles, tm_q, tm_k) != cudaSuccess)
+      return FLA_ERR_CUDA;
   }
-  if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
   {
     KernelTimer kt("kda_fwd", cs);
     const bool split = p.seg_len != kWholeSequence;
     const unsigned heads = unsigned(p.HV * (p.V / 128));
-    if (split) kda_scan_fwd_kernel<false, true, true><<<dim3(heads, unsigned(segments), 2), kFwdThreads, kKdaScanFwdSmem + 1024, cs>>>(p, tm_v);
+    if (split && launch_pdl(kda_scan_fwd_kernel<false, true, true>, dim3(heads, unsigned(segments), 2), kFwdThreads, kKdaScanFwdSmem + 1024, cs, p, tm_v) != cudaSuccess)
+      return FLA_ERR_CUDA;
     auto* scan = split ? (p.s_img ? kda_scan_fwd_kernel<true, false, true> : kda_scan_fwd_kernel<false, false, true>)
                        : (p.s_img ? kda_scan_fwd_kernel<true, false, false> : kda_scan_fwd_kernel<false, false, false>);
-    scan<<<dim3(heads, unsigned(segments)), kFwdThreads, kKdaScanFwdSmem + 1024, cs>>>(p, tm_v);
+    return cuda_status(launch_pdl(scan, dim3(heads, unsigned(segments)), kFwdThreads, kKdaScanFwdSmem + 1024, cs, p, tm_v));
   }
-  return cuda_status(cudaGetLastError());
 }

@@ -110,11 +110,13 @@ __global__ void __launch_bounds__(kScanThreads, 1) kda_scan_bwd_kernel(KdaBwdPar
   __shared__ __align__(8) uint64_t mma_bar, m_bar, qk_bar, kn_bar, x_bar, p_bar, v_bar, d_bar[2], f_bar[3];
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  pdl_trigger();
+  pdl_wait();
   const int seg = blockIdx.y + p.n0, hv = blockIdx.x / (p.V / 128), vb = blockIdx.x % (p.V / 128);
   if (tid == 0) clear_status(p.status, p.clear && seg + blockIdx.x == 0 && (kState || !kSplit));   // the backward's first kernel
   if (tid == 0 && blockIdx.y + blockIdx.x == 0) *p.counter = 0;      // of the par kernel that follows
   SegPos pos;
-  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos)) return;
+  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos, p.n0, p.n1)) return;
   if (kState && pos.s == 0) return;
   const SeqInfo& sq = pos.sq;
   const int n = pos.n, nt = pos.nt;

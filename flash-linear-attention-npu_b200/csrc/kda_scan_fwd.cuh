@@ -114,9 +114,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) kda_scan_fwd_kernel(KdaParams 
   __shared__ __align__(8) uint64_t mma_bar, o_bar, m_bar, qk_bar, kn_bar, x_bar[2], p_bar[2], v_bar[2], f_bar[3];
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  pdl_trigger();
+  pdl_wait();
   const int seg = blockIdx.y, hv = blockIdx.x / (p.V / 128), vb = blockIdx.x % (p.V / 128);
   SegPos pos;
-  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos)) return;
+  if (!segment_pos<kSplit>(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.seg_len, seg, pos, 0, p.N)) return;
   const bool values = blockIdx.z == 0;
   if (kState) {                                            // H of every segment but the last, M of those between the first and the last
     if (pos.s + 1 == pos.ns || (!values && (pos.s == 0 || vb > 0))) return;

@@ -20,11 +20,31 @@ struct SegPos {
   int n, s, ns;     // sequence, segment inside it, segments of the sequence
   int nt;           // chunks of the segment
 };
-// Called by whole warps: segment `flat` of the batch; false past the last one (packed batches launch an upper bound).
+// Called by whole warps: the sequence of [first, first + count) with the `place`-th most chunks.  Whole chains start in this order: hardware hands
+// out CTAs in order, and a long chain that starts last is what all other SMs wait for (22 prompts x 32 heads, 11,003 tokens: 282 -> 240 us).
+__device__ __forceinline__ int by_length(const int32_t* chunk_offsets, int first, int count, int place) {
+  const int lane = threadIdx.x & 31;
+  int nt[2], rank[2] = {0, 0};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int n = lane + i * 32;
+    nt[i] = n < count ? chunk_offsets[first + n + 1] - chunk_offsets[first + n] : -1;
+  }
+  for (int j = 0; j < count; ++j) {
+    const int other = __shfl_sync(0xffffffffu, j < 32 ? nt[0] : nt[1], j & 31);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) rank[i] += other > nt[i] || (other == nt[i] && j < lane + i * 32);
+  }
+  const unsigned lo = __ballot_sync(0xffffffffu, nt[0] >= 0 && rank[0] == place), hi = __ballot_sync(0xffffffffu, nt[1] >= 0 && rank[1] == place);
+  return first + (lo ? __ffs(lo) - 1 : hi ? 31 + __ffs(hi) : place);
+}
+constexpr int kMostByLength = 64;      // sequences that are put in order
+// Called by whole warps: segment `flat` of the batch; false past the last one (packed batches launch an upper bound).  [n0, n1): the sequences of
+// this launch.
 template <bool kSplit>
-__device__ __forceinline__ bool segment_pos(const int32_t* cu_seqlens, const int32_t* chunk_offsets, int N, int T, int seg_len, int flat, SegPos& r) {
+__device__ __forceinline__ bool segment_pos(const int32_t* cu_seqlens, const int32_t* chunk_offsets, int N, int T, int seg_len, int flat, SegPos& r, int n0, int n1) {
   if (!kSplit) {
-    r.n = flat;
+    r.n = cu_seqlens && n1 - n0 <= kMostByLength ? by_length(chunk_offsets, n0, n1 - n0, flat - n0) : flat;
     r.s = 0;
     r.ns = 1;
   } else if (!cu_seqlens) {
