@@ -15,8 +15,10 @@ namespace fla {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// overlap = false: an ordinary launch of such a kernel, for streams that share the SMs with another one - CTAs that only wait for their
+// predecessor would keep the other stream's work from SMs that are free.
 template <class... P, class... A>
-cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -26,8 +28,12 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  return launch_after(true, kernel, grid, block, smem, stream, std::forward<A>(args)...);
 }
 
 }  // namespace fla

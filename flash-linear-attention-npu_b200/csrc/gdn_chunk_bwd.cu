@@ -784,19 +784,6 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
       make_row_tile_map(&tm_v, p.v, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.v_sh), uint64_t(p.v_st)) ||
       make_row_tile_map(&tm_d, p.dO, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.do_sh), uint64_t(p.do_st)))
     return FLA_ERR_CUDA;
-  auto launch_scan = [&](const GdnBwdParams& pp, int64_t segments, cudaStream_t st) {
-    const dim3 grid(unsigned(HV * (V / 128)), unsigned(segments));
-    if (plan.split) {
-      const cudaError_t e = launch_pdl(gdn_scan_bwd_kernel<true, true>, grid, kScanThreads, kScanBwdSmem + 1024, st, pp, tm_q, tm_k, tm_v, tm_d);
-      if (e != cudaSuccess) return e;
-    }
-    return launch_pdl(plan.split ? gdn_scan_bwd_kernel<false, true> : gdn_scan_bwd_kernel<false, false>, grid, kScanThreads, kScanBwdSmem + 1024, st, pp, tm_q,
-                      tm_k, tm_v, tm_d);
-  };
-  auto launch_par = [&](const GdnBwdParams& pp, int64_t chunks, cudaStream_t st) {
-    return launch_pdl(nvb == 2 ? gdn_bwd_par_kernel<2> : gdn_bwd_par_kernel<4>, unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads,
-                      kParSmem + 1024, st, pp, int(chunks), tm_q, tm_k);
-  };
   // The reverse scan launches one CTA per (sequence, value head, 128 channels) and each needs a whole SM: when there are
   // more chains than SMs the last round leaves SMs idle for the length of a chain.  The batch is then launched as two
   // halves on two streams, so that the chunk-parallel kernel of the first half fills the SMs the second half's scan
@@ -804,6 +791,19 @@ static int gdn_chunk_bwd_impl(const fla_gdn_chunk_bwd_args* a, void* workspace, 
   // for the allocation-free entry (creating the second stream may allocate).
   AuxStream* aux = nullptr;
   if (allow_split && N >= 2 && !plan.split && int64_t(V / 128) * HV * N > sm_count(dev) && !kernel_timing_enabled()) aux = aux_stream_for(dev, cs);
+  auto launch_scan = [&](const GdnBwdParams& pp, int64_t segments, cudaStream_t st) {
+    const dim3 grid(unsigned(HV * (V / 128)), unsigned(segments));
+    if (plan.split) {
+      const cudaError_t e = launch_after(!aux, gdn_scan_bwd_kernel<true, true>, grid, kScanThreads, kScanBwdSmem + 1024, st, pp, tm_q, tm_k, tm_v, tm_d);
+      if (e != cudaSuccess) return e;
+    }
+    return launch_after(!aux, plan.split ? gdn_scan_bwd_kernel<false, true> : gdn_scan_bwd_kernel<false, false>, grid, kScanThreads, kScanBwdSmem + 1024, st, pp, tm_q,
+                      tm_k, tm_v, tm_d);
+  };
+  auto launch_par = [&](const GdnBwdParams& pp, int64_t chunks, cudaStream_t st) {
+    return launch_after(!aux, nvb == 2 ? gdn_bwd_par_kernel<2> : gdn_bwd_par_kernel<4>, unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads,
+                      kParSmem + 1024, st, pp, int(chunks), tm_q, tm_k);
+  };
   if (aux) {
     std::lock_guard<std::mutex> lk(aux->mu);   // the fork / join events are shared by the callers of this stream
     const int n1 = N / 2;

@@ -737,24 +737,24 @@ extern "C" FLA_API int fla_b200_kda_chunk_bwd(const fla_kda_chunk_bwd_args* a, v
       make_row_tile_map(&tm_d, p.dO, uint64_t(V), uint64_t(HV), uint64_t(B * T), uint64_t(p.do_sh), uint64_t(p.do_st)))
     return FLA_ERR_CUDA;
   if (make_row_tile_map_f32(&tm_gk, p.gk, kK, uint64_t(HV), uint64_t(B * T), uint64_t(kK), uint64_t(HV) * kK)) return FLA_ERR_CUDA;
+  // more scan chains (one CTA per SM each) than SMs: two halves of the batch on two streams, so that the chunk-parallel
+  // kernel of the first half fills the SMs the second half's scan leaves idle (aux_stream.h)
+  AuxStream* aux = nullptr;
+  if (N >= 2 && !plan.split && HV * (V / 128) * N > sm_count(dev) && !kernel_timing_enabled()) aux = aux_stream_for(dev, cs);
   auto launch_scan = [&](const KdaBwdParams& pp, int64_t segments, cudaStream_t st_) {
     const dim3 grid(unsigned(HV * (V / 128)), unsigned(segments));
     if (plan.split) {
-      const cudaError_t e = launch_pdl(kda_scan_bwd_kernel<true, true>, grid, kScanThreads, kKdaScanBwdSmem + 1024, st_, pp, tm_v, tm_d);
+      const cudaError_t e = launch_after(!aux, kda_scan_bwd_kernel<true, true>, grid, kScanThreads, kKdaScanBwdSmem + 1024, st_, pp, tm_v, tm_d);
       if (e != cudaSuccess) return e;
     }
-    return launch_pdl(plan.split ? kda_scan_bwd_kernel<false, true> : kda_scan_bwd_kernel<false, false>, grid, kScanThreads, kKdaScanBwdSmem + 1024, st_, pp,
+    return launch_after(!aux, plan.split ? kda_scan_bwd_kernel<false, true> : kda_scan_bwd_kernel<false, false>, grid, kScanThreads, kKdaScanBwdSmem + 1024, st_, pp,
                       tm_v, tm_d);
   };
   auto launch_par = [&](const KdaBwdParams& pp, int64_t chunks, cudaStream_t st_) {
     auto* par = nvb == 2 ? (pp.q_rstd ? kda_bwd_par_kernel<2, true> : kda_bwd_par_kernel<2, false>)
                          : (pp.q_rstd ? kda_bwd_par_kernel<4, true> : kda_bwd_par_kernel<4, false>);
-    return launch_pdl(par, unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads, kKdaParSmem + 1024, st_, pp, int(chunks), tm_gk);
+    return launch_after(!aux, par, unsigned(std::min<int64_t>(chunks * HK, sm_count(dev))), kParThreads, kKdaParSmem + 1024, st_, pp, int(chunks), tm_gk);
   };
-  // more scan chains (one CTA per SM each) than SMs: two halves of the batch on two streams, so that the chunk-parallel
-  // kernel of the first half fills the SMs the second half's scan leaves idle (aux_stream.h)
-  AuxStream* aux = nullptr;
-  if (N >= 2 && !plan.split && HV * (V / 128) * N > sm_count(dev) && !kernel_timing_enabled()) aux = aux_stream_for(dev, cs);
   if (aux) {
     std::lock_guard<std::mutex> lk(aux->mu);
     const int n1 = N / 2;

