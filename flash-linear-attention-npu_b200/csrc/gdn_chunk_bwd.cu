@@ -205,13 +205,13 @@ __global__ void __launch_bounds__(kParThreads, 1) gdn_bwd_par_kernel(GdnBwdParam
 
   if (warp == kParWorkers / 32 + 1) {      // ---------------------------------------------------------------- loader
     auto first_stage = [&](int tile, int h) { return (int64_t(flat0 + tile / p.HK) * p.HV + (tile % p.HK) * G + h) * NS; };
-    // A stage is seven copies, and the stage after next is asked into L2 in four pieces: its buffer is still being read, but the DRAM part of
-    // its latency can be spent meanwhile.  One lane each: a single thread took 1,000 cycles to issue them.
-    //               dO dZ   dZ_lo  Vn_hi  Vn_lo  S_hi   S_lo   dS       into L2: dZ, Vn, S, dS
-    const int img = lane < 2 ? 0 : lane < 4 ? 1 : lane < 6 ? 2 : lane == 6 ? 3 : min(lane - 7, 3);
+    // A stage is seven copies, one lane each: a single thread took 1,000 cycles to issue them.  (Asking the stages after next into L2 as
+    // well changed nothing at 4,096 to 32,768 tokens.)
+    //               dO dZ   dZ_lo  Vn_hi  Vn_lo  S_hi   S_lo   dS
+    const int img = lane < 2 ? 0 : lane < 4 ? 1 : lane < 6 ? 2 : 3;
     const int64_t stride = img == 0 ? 6144 : img == 1 ? 4096 : 8192;      // bf16 elements per stage
     const uint32_t dst = lane == 0 ? sOffAH : lane == 1 ? sOffAL + 4096 : lane == 2 ? sOffVNH : lane == 3 ? sOffVNL : lane == 4 ? sOffSH : lane == 5 ? sOffSL : sOffDSH;
-    const uint32_t bytes = lane == 0 ? 8192 : lane < 4 ? 4096 : lane < 6 ? 8192 : lane == 6 ? 16384 : uint32_t(stride) * 2;
+    const uint32_t bytes = lane == 0 ? 8192 : lane < 4 ? 4096 : lane < 6 ? 8192 : 16384;
     const bf16* src = (img == 0 ? p.dz_img : img == 1 ? p.vn_img : img == 2 ? p.s_img : p.ds_img) + (lane == 1 ? 4096 : lane == 3 ? 2048 : lane == 5 ? 4096 : 0);
     auto position = [&](int tile) { return chunk_pos(p.cu_seqlens, p.chunk_offsets, p.N, p.T, p.n0, chunk0 + tile / p.HK); };
 
@@ -254,7 +254,6 @@ __global__ void __launch_bounds__(kParThreads, 1) gdn_bwd_par_kernel(GdnBwdParam
             bn = first_stage(next, 0);
           }
         }
-        if (lane >= 7 && lane < 11 && (st + 2 < NS || next < tiles)) bulk_prefetch_l2(src + (st + 2 < NS ? b0 + st + 2 : bn + (st + 2 - NS)) * stride, bytes);
       }
       if (!ok) break;
       // q, k rows of the chunk (shared by the value heads of the group): four 64 x 64 tiles, for the score product at the end of the stages.  Rows
